@@ -336,6 +336,148 @@ neg2(float2 a)
   return make_float2(-a.x, -a.y);
 }
 
+// ---------------------------------------------------------------------------
+// FP64 arithmetic of the FMA build.  The FP64 kernels are bound by GB300's
+// FP64 pipe (ncu: 78-84 % busy with 8 % of the issue slots used), which takes
+// one warp instruction per 16 cycles and SM and serves not only additions and
+// products but also comparisons, minima, maxima, negations and conversions
+// (probe, independent chains: FMA 617 Gop/s, fmax 490, 1/x 115, c/x 70, sqrt
+// 70, rsqrt 108).  The helpers below keep what need not be there on the
+// integer and special-function pipes.
+// ---------------------------------------------------------------------------
+template <class R>
+constexpr bool kFast64 = sizeof(R) == 8 && kShareRecip;
+
+__device__ __forceinline__ int
+hi32(double x)
+{
+  return __double2hiint(x);
+}
+__device__ __forceinline__ double
+with_hi(int hi, double x)
+{
+  return __hiloint2double(hi, __double2loint(x));
+}
+// zero, infinity or NaN (the seed instructions below return no subnormals)
+__device__ __forceinline__ bool
+seed_special(double y)
+{
+  return ((hi32(y) + 0x00100000) & 0x7fe00000) == 0;
+}
+// 1/x: the hardware's 20-bit seed y (rcp.approx.ftz.f64), then the geometric
+// series of 1/(1 - e), e = 1 - x y, to second order: e^3 is below 2^-58, so
+// the error is that of the last rounding.  Measured over 2^-40..2^40: 1.003 x
+// 2^-53 at most, 1.000 for the division; 182 Gop/s, 115 for the division.
+// Subnormal x give infinity, |x| above 2^1022 zero.
+__device__ __forceinline__ double
+rcp64(double x)
+{
+  double y;
+  asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(x));
+  const double e = fma(-x, y, 1.0);
+  const double r = fma(y, fma(e, e, e), y);
+  return seed_special(y) ? y : r;
+}
+// 1/sqrt(x): the hardware's seed (rsqrt.approx.ftz.f64) and the binomial
+// series of (1 - r)^(-1/2), r = 1 - x y^2, to second order.  Error 1.012 x
+// 2^-53 at most, as CUDA's rsqrt.
+__device__ __forceinline__ double
+rsqrt64(double x)
+{
+  double y;
+  asm("rsqrt.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(x));
+  const double r = fma(-x, y * y, 1.0);
+  const double q = fma(y * r, fma(r, 0.375, 0.5), y);
+  return seed_special(y) ? y : q;
+}
+// sqrt(x) from the same series; error 1.5 x 2^-53 at most (84 Gop/s, 70 for
+// the correctly rounded root).  Zero, infinity and subnormals return x.
+__device__ __forceinline__ double
+sqrt64(double x)
+{
+  double y;
+  asm("rsqrt.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(x));
+  const double g = x * y;
+  const double r = fma(-g, y, 1.0);
+  const double q = fma(g * r, fma(r, 0.375, 0.5), g);
+  return seed_special(y) ? ((hi32(y) & 0x000fffff) != 0 ? y : x) : q;
+}
+// sqrt(n / d) for n >= 0, d > 0; 0 for n = 0
+__device__ __forceinline__ double
+sqrt_ratio64(double n, double d)
+{
+  const double c = n * rsqrt64(n * d);
+  return hi32(n) == 0 ? 0.0 : c;
+}
+__device__ __forceinline__ bool
+positive64(double x) // x > 0 (true for a positive NaN)
+{
+  return __double_as_longlong(x) > 0;
+}
+__device__ __forceinline__ bool
+negative64(double x) // the sign bit
+{
+  return hi32(x) < 0;
+}
+// the larger of x (any sign) and f >= 0; the smaller of two non-negative
+// values: the integer order of the bit patterns is the numbers' order
+__device__ __forceinline__ double
+max_floor64(double x, double f)
+{
+  return __longlong_as_double(max(__double_as_longlong(x), __double_as_longlong(f)));
+}
+__device__ __forceinline__ double
+min_pos64(double a, double b)
+{
+  return __longlong_as_double(min(__double_as_longlong(a), __double_as_longlong(b)));
+}
+// x with the sign flipped when f
+__device__ __forceinline__ double
+flip64(double x, bool f)
+{
+  return with_hi(hi32(x) ^ (f ? (int)0x80000000 : 0), x);
+}
+// x / 2^K by the exponent (exact); the product where the result or x is not normal
+template <int K>
+__device__ __forceinline__ double
+scale_down64(double x)
+{
+  const int hi = hi32(x);
+  if ((unsigned)(hi & 0x7fffffff) - (unsigned)((K + 1) << 20) < (unsigned)((0x7ff - K - 1) << 20))
+    return with_hi(hi - (K << 20), x);
+  return x * (1.0 / (1 << K));
+}
+// max(p, d floor) for d > 0: the product only where the high words say that
+// p / d may be below 2 floor
+__device__ __forceinline__ double
+floor_ratio64(double p, double d, double floor)
+{
+  // a negative p counts as zero (the difference must not wrap)
+  if (max(hi32(p), 0) - hi32(d) < hi32(floor) - 0x3ff00000 + 0x00100000)
+    p = max_floor64(p, d * floor);
+  return p;
+}
+// running maximum of CFL candidates: NaN is ignored, as fmax does
+__device__ __forceinline__ double
+max_cand64(double m, double v)
+{
+  const long long b = __double_as_longlong(v);
+  return b <= 0x7ff0000000000000ll ? __longlong_as_double(max(__double_as_longlong(m), b)) : m;
+}
+__device__ __forceinline__ float
+max_cand(float m, float v)
+{
+  return fmaxf(m, v);
+}
+__device__ __forceinline__ double
+max_cand(double m, double v)
+{
+  if constexpr (kShareRecip)
+    return max_cand64(m, v);
+  else
+    return fmax(m, v);
+}
+
 // FP64 value in the working precision R
 template <class R>
 __device__ __forceinline__ R

@@ -38,24 +38,6 @@ slope1(R q, R qp, R qm, R st)
       m = fminf(m, fabsf(0.5f * (qp - qm)));
     return (dl * dr > 0.f) ? copysignf(m, dl) : 0.f;
   }
-  if constexpr (kShareRecip)
-  {
-    // FP64 FMA build: the minima of non-negative values as integer minima of
-    // their bit patterns (same order; a NaN pattern is the larger, as fmin
-    // drops NaN) and the sign by copysign, on the integer pipes instead of
-    // GB300's 1/64-rate FP64 pipe.  As in the FP32 form, the scaling by st
-    // (0, 1 or 2) is applied once to the minimum, and the centred difference
-    // only where it can bind (st = 2); a non-zero slope has dl's sign (dl, dr
-    // and dcen share it).  Only the sign of a zero slope can differ.
-    auto minpos = [](double a, double b) {
-      return __longlong_as_double(min(__double_as_longlong(a), __double_as_longlong(b)));
-    };
-    const R dl = q - qm, dr = qp - q;
-    R       m = minpos(fabs(dl), fabs(dr));
-    if (st != R(1))
-      m = minpos(st * m, fabs(R(0.5) * (qp - qm)));
-    return copysign((dl * dr <= R(0)) ? R(0) : m, dl);
-  }
   const R dlft = st * (q - qm);
   const R drgt = st * (qp - q);
   const R dcen = R(0.5) * (qp - qm);
@@ -67,6 +49,39 @@ slope1(R q, R qp, R qm, R st)
   return dsgn * fmin(dlim, fabs(dcen));
 }
 
+// Half of slope1's slope, for the FP64 FMA build: every use of a slope takes
+// its half.  Two differences on the FP64 pipe (three for MC); the minima, the
+// scaling by powers of two and the signs on the integer pipes.  A slope is
+// zero where dl and dr differ in sign or either is zero; with st = 1 (minmod)
+// the centred difference never binds (see the FP32 form above).
+__device__ __forceinline__ double
+half_slope64(double q, double qp, double qm, double st)
+{
+  const double dl = q - qm, dr = qp - q;
+  const double m = min_pos64(fabs(dl), fabs(dr));
+  double       h;
+  if (st == 1.0)
+    h = scale_down64<1>(m);
+  else if (st == 2.0)
+    h = min_pos64(m, scale_down64<2>(fabs(qp - qm)));
+  else
+    h = 0.0;
+  // the sign of dl, or zero
+  const int sl = hi32(dl), differ = (sl ^ hi32(dr)) >> 31; // all ones where the signs differ
+  const int hi = hi32(h) & ~differ, lo = __double2loint(h) & ~differ;
+  return __hiloint2double(hi | (sl & (int)0x80000000), lo);
+}
+// the slope, or its half in the FP64 FMA build (kFast64)
+template <class R>
+__device__ __forceinline__ R
+slope_h(R q, R qp, R qm, R st)
+{
+  if constexpr (kFast64<R>)
+    return half_slope64(q, qp, qm, st);
+  else
+    return slope1<R>(q, qp, qm, st);
+}
+
 // computePrimitives (HydroBaseFunctor2D.h:78-102, HydroBaseFunctor3D.h:80-106).
 // In the mixed form (R = float) the internal energy is recomputed in FP64
 // when E/rho and the kinetic energy cancel to fewer than ~7 significant bits.
@@ -74,16 +89,30 @@ template <class R, int NV>
 __device__ __forceinline__ void
 hydro_prims(const R (&u)[NV], R (&q)[NV], const HydroConst<R> & C)
 {
+  if constexpr (kFast64<R>)
+  {
+    // FP64 FMA build: p = (gamma - 1) (E - rho v^2 / 2), 12 FP64-pipe operations in 3D
+    const R d = max_floor64(u[ID], C.smallr), id = rcp64(d);
+    q[ID] = d;
+    q[IU] = u[IU] * id;
+    q[IV] = u[IV] * id;
+    R k = q[IU] * q[IU] + q[IV] * q[IV];
+    if constexpr (NV == 5)
+    {
+      q[IW] = u[IW] * id;
+      k += q[IW] * q[IW];
+    }
+    q[IP] = floor_ratio64((C.gamma0 - R(1)) * fma(R(-0.5) * d, k, u[IP]), d, C.smallp);
+    return;
+  }
   const R d = fmax(u[ID], C.smallr);
   // one reciprocal of the density for the four quotients (FP32: approximate;
   // FP64 exact build: four divisions)
   R id = R(0);
   if constexpr (sizeof(R) == 4)
     id = rcp_a(d);
-  else if constexpr (kShareRecip)
-    id = R(1) / d;
   auto over_d = [&](R x) {
-    if constexpr (sizeof(R) == 4 || kShareRecip)
+    if constexpr (sizeof(R) == 4)
       return x * id;
     else
       return x / d;
@@ -132,6 +161,8 @@ hydro_sound(R d, R p, const HydroConst<R> & C)
 {
   if constexpr (sizeof(R) == 4)
     return sqrt_a(C.gamma0 * p * rcp_a(d));
+  else if constexpr (kFast64<R>)
+    return sqrt_ratio64(C.gamma0 * p, d);
   else
     return sqrt(C.gamma0 * (p) / d);
 }
@@ -145,13 +176,32 @@ hydro_sources(const R (&q)[NV], const R (&dx)[NV], const R (&dy)[NV], const R (&
               const HydroConst<R> & C)
 {
   const R r = q[ID], p = q[IP], u = q[IU], v = q[IV];
+  if constexpr (kFast64<R>)
+  {
+    // FP64 FMA build, from half slopes (so half the sources): one FMA chain each
+    const R ir = rcp64(r), gp = C.gamma0 * p;
+    R       div = dx[IU] + dy[IV];
+    if constexpr (NV == 5)
+      div += dz[IW];
+    auto adv = [&](int f, R x) { // x - v . grad f
+      x = fma(-v, dy[f], fma(-u, dx[f], x));
+      if constexpr (NV == 5)
+        x = fma(-q[IW], dz[f], x);
+      return x;
+    };
+    s[ID] = adv(ID, -div * r);
+    s[IP] = adv(IP, -div * gp);
+    s[IU] = adv(IU, -dx[IP] * ir);
+    s[IV] = adv(IV, -dy[IP] * ir);
+    if constexpr (NV == 5)
+      s[IW] = adv(IW, -dz[IP] * ir);
+    return;
+  }
   R       ir = R(0);
   if constexpr (sizeof(R) == 4)
     ir = rcp_a(r);
-  else if constexpr (kShareRecip)
-    ir = R(1) / r;
   auto over_r = [&](R x) {
-    if constexpr (sizeof(R) == 4 || kShareRecip)
+    if constexpr (sizeof(R) == 4)
       return x * ir;
     else
       return x / r;
@@ -181,9 +231,9 @@ __device__ __forceinline__ void
 hydro_face(const R (&q)[NV], const R (&d)[NV], const R (&s)[NV], R dtd, bool plus, R (&f)[NV],
            R smallr)
 {
-  if constexpr (sizeof(R) == 4 || kShareRecip)
+  if constexpr (sizeof(R) == 4)
   {
-    // mixed form and FP64 FMA build: two fused multiply-adds per variable
+    // mixed form: two fused multiply-adds per variable
     const R hdtd = R(0.5) * dtd, hd = plus ? R(0.5) : R(-0.5);
 #pragma unroll
     for (int v = 0; v < NV; ++v)
@@ -203,12 +253,139 @@ hydro_face(const R (&q)[NV], const R (&d)[NV], const R (&s)[NV], R dtd, bool plu
   f[ID] = fmax(smallr, f[ID]);
 }
 
+// The face states of one cell.  In the FP64 FMA build slopes and sources are
+// halves and the time-advanced state q + s dt/dx is computed once for all
+// directions whose dt/dx is the same.
+template <class R, int NV>
+struct FaceStates
+{
+  const R (&q)[NV], (&s)[NV];
+  R dtd, smallr;
+  R b[kFast64<R> ? NV : 1];
+  __device__ __forceinline__
+  FaceStates(const R (&q_)[NV], const R (&s_)[NV], R dtd_, R smallr_)
+    : q(q_), s(s_), smallr(smallr_)
+  {
+    set(dtd_);
+  }
+  __device__ __forceinline__ void
+  set(R dtd_)
+  {
+    dtd = dtd_;
+    if constexpr (kFast64<R>)
+    {
+#pragma unroll
+      for (int v = 0; v < NV; ++v)
+        b[v] = fma(s[v], dtd, q[v]);
+    }
+  }
+  // the next direction; same: its dt/dx is the present one
+  __device__ __forceinline__ void
+  turn(R dtd_, bool same)
+  {
+    if (!kFast64<R> || !same)
+      set(dtd_);
+  }
+  __device__ __forceinline__ void
+  get(const R (&d)[NV], bool plus, R (&f)[NV]) const
+  {
+    if constexpr (kFast64<R>)
+    {
+#pragma unroll
+      for (int v = 0; v < NV; ++v)
+        f[v] = plus ? b[v] + d[v] : b[v] - d[v];
+      f[ID] = max_floor64(f[ID], smallr);
+    }
+    else
+      hydro_face<R, NV>(q, d, s, dtd, plus, f, smallr);
+  }
+};
+
+// Face fluxes are kept scaled by dt/dx, as the reference stores them; the FP64
+// FMA build keeps them unscaled and scales in the update's FMAs.
+template <class R>
+__device__ __forceinline__ R
+flux_scaled(R f, R dtd)
+{
+  return kFast64<R> ? f : f * dtd;
+}
+template <class R>
+__device__ __forceinline__ R
+add_flux(R x, R f, R dtd)
+{
+  return kFast64<R> ? fma(f, dtd, x) : x + f;
+}
+template <class R>
+__device__ __forceinline__ R
+sub_flux(R x, R f, R dtd)
+{
+  return kFast64<R> ? fma(-f, dtd, x) : x - f;
+}
+
+// riemann_hllc (RiemannSolvers.h:445-568) in the FP64 FMA build: the same star
+// state with about 51 FP64-pipe operations per 3D face.  The larger sound speed is one reciprocal square
+// root (densities are positive: p_l / rho_l >= p_r / rho_r where p_l rho_r >=
+// p_r rho_l).  With w = (p_l - p_r - rc_r (u_l - u_r)) / (rc_l + rc_r), u* = u_l
+// + w and p* = p_l - rc_l w; rc = rho |S - u| is also the star density's
+// numerator.  The four-way choice is by sign bits and selects (integer pipes).
+// With the half slopes and the FMA updates: FP64 2D step 74.3 -> 52.1 us at
+// 256^2, two-shock 3D step 2224 -> 1287 us at 33 x 31 x 99.
+template <int NV>
+__device__ __forceinline__ void
+hllc64(const double (&ql)[NV], const double (&qr)[NV], double (&flux)[NV], const HydroConst<double> & C)
+{
+  const double rl = max_floor64(ql[ID], C.smallr), rr = max_floor64(qr[ID], C.smallr);
+  const double pl = floor_ratio64(ql[IP], rl, C.smallp), pr = floor_ratio64(qr[IP], rr, C.smallp);
+  const double ul = ql[IU], ur = qr[IU];
+  double       kl = ul * ul + ql[IV] * ql[IV], kr = ur * ur + qr[IV] * qr[IV];
+  if constexpr (NV == 5)
+  {
+    kl += ql[IW] * ql[IW];
+    kr += qr[IW] * qr[IW];
+  }
+  const double el = fma(pl, C.entho, scale_down64<1>(rl) * kl), er = fma(pr, C.entho, scale_down64<1>(rr) * kr);
+
+  const bool   lbig = __double_as_longlong(pl * rr) >= __double_as_longlong(pr * rl);
+  const double cmax = max_floor64(sqrt_ratio64(C.gamma0 * (lbig ? pl : pr), lbig ? rl : rr), C.smallc);
+
+  const double du = ul - ur;
+  const bool   lslow = negative64(du); // ul < ur
+  const double SL = (lslow ? ul : ur) - cmax, SR = (lslow ? ur : ul) + cmax;
+  const double al = ul - SL, ar = SR - ur;
+  const double rcl = rl * al, rcr = rr * ar;
+  const double w = fma(-rcr, du, pl - pr) * rcp64(rcr + rcl);
+  const double us = ul + w, ps = fma(-rcl, w, pl);
+
+  // the star state on the side of the contact (left when u* > 0)
+  const bool   left = positive64(us);
+  const double Sk = left ? SL : SR, uk = left ? ul : ur, ek = left ? el : er, pk = left ? pl : pr;
+  const double is = rcp64(Sk - us);
+  const double rs = (left ? flip64(rcl, true) : rcr) * is;
+  const double es = fma(ps, us, fma(-pk, uk, (left ? flip64(al, true) : ar) * ek)) * is;
+  const bool   out = left ? positive64(SL) : !positive64(SR); // supersonic: the side's own state
+  const double ro = out ? (left ? rl : rr) : rs, uo = out ? uk : us, po = out ? pk : ps, eo = out ? ek : es;
+
+  const double m = ro * uo;
+  const bool   ml = positive64(m);
+  flux[ID] = m;
+  flux[IU] = fma(m, uo, po);
+  flux[IP] = (eo + po) * uo;
+  flux[IV] = m * (ml ? ql[IV] : qr[IV]);
+  if constexpr (NV == 5)
+    flux[IW] = m * (ml ? ql[IW] : qr[IW]);
+}
+
 // riemann_hllc (RiemannSolvers.h:445-568).  States are in the face frame
 // (normal velocity in IU); NV = 4 (2D) or 5 (3D).
 template <class R, int NV>
 __device__ __forceinline__ void
 hllc(const R (&ql)[NV], const R (&qr)[NV], R (&flux)[NV], const HydroConst<R> & C)
 {
+  if constexpr (kFast64<R>)
+  {
+    hllc64<NV>(ql, qr, flux, C);
+    return;
+  }
   const R entho = C.entho;
   R       rl, pl, ul, etotl, rr, pr, ur, etotr, cmax; // cmax: the larger sound speed
   if constexpr (sizeof(R) == 4)
@@ -248,18 +425,8 @@ hllc(const R (&ql)[NV], const R (&qr)[NV], R (&flux)[NV], const HydroConst<R> & 
       ecinr += R(0.5) * rr * qr[IW] * qr[IW];
     etotr = pr * entho + ecinr;
 
-    if constexpr (kShareRecip)
-    {
-      // FP64 FMA build: the larger sound speed squared with one division (the
-      // densities are positive, so p_l / rho_l >= p_r / rho_r where p_l rho_r
-      // >= p_r rho_l, up to rounding ties), then one square root (a correctly
-      // rounded square root is monotonic)
-      const bool lbig = pl * rr >= pr * rl;
-      cmax = sqrt(fmax(C.gamma0 * (lbig ? pl : pr) / (lbig ? rl : rr), C.smallc * C.smallc));
-    }
-    else
-      cmax = fmax(sqrt(fmax(C.gamma0 * pl / rl, C.smallc * C.smallc)),
-                  sqrt(fmax(C.gamma0 * pr / rr, C.smallc * C.smallc)));
+    cmax = fmax(sqrt(fmax(C.gamma0 * pl / rl, C.smallc * C.smallc)),
+                sqrt(fmax(C.gamma0 * pr / rr, C.smallc * C.smallc)));
   }
   const R ptotl = pl, ptotr = pr;
 
@@ -273,12 +440,6 @@ hllc(const R (&ql)[NV], const R (&qr)[NV], R (&flux)[NV], const HydroConst<R> & 
   if constexpr (sizeof(R) == 4)
   {
     const float irc = rcp_a(rcr + rcl);
-    ustar = (rcr * ur + rcl * ul + (ptotl - ptotr)) * irc;
-    ptotstar = (rcr * ptotl + rcl * ptotr + rcl * rcr * (ul - ur)) * irc;
-  }
-  else if constexpr (kShareRecip)
-  {
-    const R irc = R(1) / (rcr + rcl);
     ustar = (rcr * ur + rcl * ul + (ptotl - ptotr)) * irc;
     ptotstar = (rcr * ptotl + rcl * ptotr + rcl * rcr * (ul - ur)) * irc;
   }
@@ -317,33 +478,15 @@ hllc(const R (&ql)[NV], const R (&qr)[NV], R (&flux)[NV], const HydroConst<R> & 
   {
     uo = ustar;
     ptoto = ptotstar;
-    if constexpr (kShareRecip)
-    {
-      const R is = R(1) / (SL - ustar);
-      ro = rl * (SL - ul) * is;
-      etoto = ((SL - ul) * etotl - ptotl * ul + ptotstar * ustar) * is;
-    }
-    else
-    {
-      ro = rl * (SL - ul) / (SL - ustar);
-      etoto = ((SL - ul) * etotl - ptotl * ul + ptotstar * ustar) / (SL - ustar);
-    }
+    ro = rl * (SL - ul) / (SL - ustar);
+    etoto = ((SL - ul) * etotl - ptotl * ul + ptotstar * ustar) / (SL - ustar);
   }
   else if (SR > R(0))
   {
     uo = ustar;
     ptoto = ptotstar;
-    if constexpr (kShareRecip)
-    {
-      const R is = R(1) / (SR - ustar);
-      ro = rr * (SR - ur) * is;
-      etoto = ((SR - ur) * etotr - ptotr * ur + ptotstar * ustar) * is;
-    }
-    else
-    {
-      ro = rr * (SR - ur) / (SR - ustar);
-      etoto = ((SR - ur) * etotr - ptotr * ur + ptotstar * ustar) / (SR - ustar);
-    }
+    ro = rr * (SR - ur) / (SR - ustar);
+    etoto = ((SR - ur) * etotr - ptotr * ur + ptotstar * ustar) / (SR - ustar);
   }
   else
   {
@@ -378,12 +521,91 @@ cmpflx(const R (&qg)[NV], R (&flux)[NV], const HydroConst<R> & C)
   flux[IP] = qg[IU] * (etot + qg[IP]);
 }
 
+// riemann_approx (RiemannSolvers.h:60-200) in the FP64 FMA build: a Newton
+// iteration takes four reciprocals and reciprocal square roots (about 45
+// FP64-pipe operations) instead of eight divisions and two square roots: with
+// x = c (1 + gamma6 (p - p_k) / p_k), w = x rsqrt(x) and the shock velocity's
+// quotient by w is a product with rsqrt(x).
+template <int NV>
+__device__ __forceinline__ void
+riemann_approx64(const double (&ql)[NV], const double (&qr)[NV], double (&flux)[NV], const HydroConst<double> & C)
+{
+  const double rl = max_floor64(ql[ID], C.smallr), ul = ql[IU], pl = floor_ratio64(ql[IP], rl, C.smallp);
+  const double rr = max_floor64(qr[ID], C.smallr), ur = qr[IU], pr = floor_ratio64(qr[IP], rr, C.smallp);
+  const double cl = C.gamma0 * pl * rl, cr = C.gamma0 * pr * rr;
+  // c gamma6 / p = gamma0 gamma6 rho
+  const double kl = C.gamma0 * C.gamma6 * rl, kr = C.gamma0 * C.gamma6 * rr;
+  const double du = ul - ur;
+  double       wl = sqrt64(cl), wr = sqrt64(cr);
+  double       p = max_floor64(fma(wl * wr, du, fma(wr, pl, wl * pr)) * rcp64(wl + wr), 0.0);
+  double       yl, yr;
+  for (int iter = 0;; ++iter)
+  {
+    const double dl = p - pl, dr = p - pr;
+    const double xl = fma(kl, dl, cl), xr = fma(kr, dr, cr);
+    yl = rsqrt64(xl);
+    yr = rsqrt64(xr);
+    wl = xl * yl;
+    wr = xr * yr;
+    if (iter == 10)
+      break;
+    // q = 2 w^3 / (w^2 + c)
+    const double gl = xl * wl * rcp64(xl + cl), gr = xr * wr * rcp64(xr + cr);
+    const double dv = fma(-dr, yr, fma(-dl, yl, du)); // u_l* - u_r*
+    double       delp = (gr + gr) * gl * rcp64(gr + gl) * dv;
+    delp = negative64(delp + p) ? -p : delp;
+    p += delp;
+    // |delp / (p + smallpp)| > 1e-6
+    if (__double_as_longlong(fabs(delp)) <= __double_as_longlong(fabs((p + C.smallpp) * 1e-6)))
+    {
+      const double x2l = fma(kl, p - pl, cl), x2r = fma(kr, p - pr, cr);
+      yl = rsqrt64(x2l);
+      yr = rsqrt64(x2r);
+      wl = x2l * yl;
+      wr = x2r * yr;
+      break;
+    }
+  }
+  const double us = 0.5 * (ul + ur + fma(pl - p, yl, -((pr - p) * yr)));
+  const bool   left = !negative64(us);
+  const double ro = left ? rl : rr, po = left ? pl : pr, wo = left ? wl : wr, yo = left ? yl : yr;
+  const double uo = flip64(left ? ul : ur, !left), ss = flip64(us, !left); // sgnm u
+  const double co = max_floor64(sqrt_ratio64(fabs(C.gamma0 * po), ro), C.smallc);
+  // rho / (1 + rho (p_o - p*) / w^2)
+  const double rs = max_floor64(ro * rcp64(fma(ro * (po - p), yo * yo, 1.0)), C.smallr);
+  const double cs = max_floor64(sqrt_ratio64(fabs(C.gamma0 * p), rs), C.smallc);
+  double       spout = co - uo, spin = cs - ss;
+  if (p >= po)
+    spin = spout = fma(wo, rcp64(ro), -uo); // shock
+  const double sum = spout + spin;
+  const double scr = fmax(spout - spin, C.smallc + fabs(sum));
+  double       frac = fma(0.5 * sum, rcp64(scr), 0.5);
+  frac = frac != frac ? 0.0 : (frac >= 1.0 ? 1.0 : (frac <= 0.0 ? 0.0 : frac));
+  double qg[NV];
+  qg[ID] = fma(frac, rs - ro, ro);
+  qg[IU] = fma(frac, us - (left ? ul : ur), left ? ul : ur);
+  qg[IP] = fma(frac, p - po, po);
+  if (negative64(spout))
+    qg[ID] = ro, qg[IU] = left ? ul : ur, qg[IP] = po;
+  if (positive64(spin))
+    qg[ID] = rs, qg[IU] = us, qg[IP] = p;
+  qg[IV] = left ? ql[IV] : qr[IV];
+  if constexpr (NV == 5)
+    qg[IW] = left ? ql[IW] : qr[IW];
+  cmpflx<double, NV>(qg, flux, C);
+}
+
 // riemann_approx (RiemannSolvers.h:60-200): two-shock iterative solver,
 // at most 10 Newton iterations on p*
 template <class R, int NV>
 __device__ __forceinline__ void
 riemann_approx(const R (&ql)[NV], const R (&qr)[NV], R (&flux)[NV], const HydroConst<R> & C)
 {
+  if constexpr (kFast64<R>)
+  {
+    riemann_approx64<NV>(ql, qr, flux, C);
+    return;
+  }
   const R gamma0 = C.gamma0, gamma6 = C.gamma6, smallr = C.smallr, smallc = C.smallc, smallp = C.smallp;
   const R rl = fmax(ql[ID], smallr), ul = ql[IU], pl = fmax(ql[IP], rl * smallp);
   const R rr = fmax(qr[ID], smallr), ur = qr[IU], pr = fmax(qr[IP], rr * smallp);
@@ -478,8 +700,8 @@ riemann_llf(const R (&ql)[NV], const R (&qr)[NV], R (&flux)[NV], const HydroCons
   const R entho = C.entho;
   const R rl = fmax(ql[ID], C.smallr), ul = ql[IU], pl = fmax(ql[IP], rl * C.smallp);
   const R rr = fmax(qr[ID], C.smallr), ur = qr[IU], pr = fmax(qr[IP], rr * C.smallp);
-  const R cl = sqrt(C.gamma0 * pl / rl);
-  const R cr = sqrt(C.gamma0 * pr / rr);
+  const R cl = kFast64<R> ? sqrt_ratio64(C.gamma0 * pl, rl) : sqrt(C.gamma0 * pl / rl);
+  const R cr = kFast64<R> ? sqrt_ratio64(C.gamma0 * pr, rr) : sqrt(C.gamma0 * pr / rr);
   const R cmax = fmax(fabs(ul) + cl, fabs(ur) + cr);
   R       uleft[NV], uright[NV], fleft[NV], fright[NV];
   hydro_uf<R, NV>(ql, uleft, fleft, entho);
@@ -498,8 +720,8 @@ riemann_hll(const R (&ql)[NV], const R (&qr)[NV], R (&flux)[NV], const HydroCons
   const R entho = C.entho;
   const R rl = fmax(ql[ID], C.smallr), ul = ql[IU], pl = fmax(ql[IP], rl * C.smallp);
   const R rr = fmax(qr[ID], C.smallr), ur = qr[IU], pr = fmax(qr[IP], rr * C.smallp);
-  const R cl = sqrt(C.gamma0 * pl / rl);
-  const R cr = sqrt(C.gamma0 * pr / rr);
+  const R cl = kFast64<R> ? sqrt_ratio64(C.gamma0 * pl, rl) : sqrt(C.gamma0 * pl / rl);
+  const R cr = kFast64<R> ? sqrt_ratio64(C.gamma0 * pr, rr) : sqrt(C.gamma0 * pr / rr);
   const R SL = fmin(fmin(ul, ur) - fmax(cl, cr), R(0));
   const R SR = fmax(fmax(ul, ur) + fmax(cl, cr), R(0));
   R       uleft[NV], uright[NV], fleft[NV], fright[NV];
@@ -540,7 +762,7 @@ hydro_invdt(const R (&u)[NV], const HydroConst<R> & C, const KParams & P)
   const R c = hydro_sound<R>(q[ID], q[IP], C);
   const R vx = c + fabs(q[IU]);
   const R vy = c + fabs(q[IV]);
-  if constexpr (sizeof(R) == 8 && !kShareRecip)
+  if constexpr (sizeof(R) == 8 && !kFast64<R>)
   {
     if constexpr (NV == 4)
       return vx / P.dx + vy / P.dy;

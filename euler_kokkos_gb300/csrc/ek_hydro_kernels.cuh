@@ -112,7 +112,7 @@ hydro3d_slot_elems()
   return (int)(((5 * (TX + 4) * (TY + 4) * sizeof(R) + 127) / 128 * 128) / sizeof(R));
 }
 
-// slopes of the cell at tile coordinates (hx, hy) of the planes qm/q0/qp
+// slopes (slope_h) of the cell at tile coordinates (hx, hy) of the planes qm/q0/qp
 template <class R, int NV, int HX, int HY>
 __device__ __forceinline__ void
 cell_slopes(const R * q0, const R * qm, const R * qp, int hx, int hy, R st, R (&c)[NV], R (&dX)[NV],
@@ -124,10 +124,10 @@ cell_slopes(const R * q0, const R * qm, const R * qp, int hx, int hy, R st, R (&
     const R * p = q0 + v * HY * HX;
     const R   x = p[hy * HX + hx];
     c[v] = x;
-    dX[v] = slope1<R>(x, p[hy * HX + hx + 1], p[hy * HX + hx - 1], st);
-    dY[v] = slope1<R>(x, p[(hy + 1) * HX + hx], p[(hy - 1) * HX + hx], st);
+    dX[v] = slope_h<R>(x, p[hy * HX + hx + 1], p[hy * HX + hx - 1], st);
+    dY[v] = slope_h<R>(x, p[(hy + 1) * HX + hx], p[(hy - 1) * HX + hx], st);
     if (three_d)
-      dZ[v] = slope1<R>(x, qp[(v * HY + hy) * HX + hx], qm[(v * HY + hy) * HX + hx], st);
+      dZ[v] = slope_h<R>(x, qp[(v * HY + hy) * HX + hx], qm[(v * HY + hy) * HX + hx], st);
     else
       dZ[v] = R(0);
   }
@@ -175,6 +175,7 @@ hydro2d_tile(const S * __restrict__ Uin, S * __restrict__ Uout, const KParams & 
   }
   const double        t = ss.t, dt = ss.dt;
   const R             dtdx = ss.dtdx, dtdy = ss.dtdy;
+  const bool          same_xy = dtdx == dtdy; // square cells: one time-advanced state for all faces
   const HydroConst<R> C = hydro_const<R>(P);
   const R             hdt = (R)(0.5 * dt);
   const bool          kick = GRAV && P.grav_hancock; // gravity predictor of the face states
@@ -203,25 +204,27 @@ hydro2d_tile(const S * __restrict__ Uin, S * __restrict__ Uout, const KParams & 
     R hg[3];
     if (kick)
       half_g(tx, ty, hg);
-    hydro_face<R, NV>(c, dX, s, dtdx, false, f, C.smallr);
+    FaceStates<R, NV> F(c, s, dtdx, C.smallr);
+    F.get(dX, false, f);
     if (kick)
       grav_kick<R, NV>(f, hg);
 #pragma unroll
     for (int v = 0; v < NV; ++v)
       sXm[(v * TY + ty) * FX + tx + 1] = f[v];
-    hydro_face<R, NV>(c, dX, s, dtdx, true, f, C.smallr);
+    F.get(dX, true, f);
     if (kick)
       grav_kick<R, NV>(f, hg);
 #pragma unroll
     for (int v = 0; v < NV; ++v)
       sXp[(v * TY + ty) * FX + tx + 1] = f[v];
-    hydro_face<R, NV>(c, dY, s, dtdy, false, f, C.smallr);
+    F.turn(dtdy, same_xy);
+    F.get(dY, false, f);
     if (kick)
       grav_kick<R, NV>(f, hg);
 #pragma unroll
     for (int v = 0; v < NV; ++v)
       sYm[(v * (TY + 2) + ty + 1) * TX + tx] = f[v];
-    hydro_face<R, NV>(c, dY, s, dtdy, true, f, C.smallr);
+    F.get(dY, true, f);
     if (kick)
       grav_kick<R, NV>(f, hg);
 #pragma unroll
@@ -256,7 +259,7 @@ hydro2d_tile(const S * __restrict__ Uin, S * __restrict__ Uout, const KParams & 
       half_g(cx, cy, hg);
     if (kind < 2)
     {
-      hydro_face<R, NV>(c, dX, s, dtdx, kind == 0, f, C.smallr);
+      FaceStates<R, NV>(c, s, dtdx, C.smallr).get(dX, kind == 0, f);
       if (kick)
         grav_kick<R, NV>(f, hg);
       R * dst = kind == 0 ? sXp : sXm;
@@ -266,7 +269,7 @@ hydro2d_tile(const S * __restrict__ Uin, S * __restrict__ Uout, const KParams & 
     }
     else
     {
-      hydro_face<R, NV>(c, dY, s, dtdy, kind == 2, f, C.smallr);
+      FaceStates<R, NV>(c, s, dtdy, C.smallr).get(dY, kind == 2, f);
       if (kick)
         grav_kick<R, NV>(f, hg);
       R * dst = kind == 2 ? sYp : sYm;
@@ -278,7 +281,7 @@ hydro2d_tile(const S * __restrict__ Uin, S * __restrict__ Uout, const KParams & 
   __syncthreads();
 
   // fluxes: x-face i (left face of cell i) from XMAX(i-1), XMIN(i); stored
-  // scaled by dt/dx into the XMIN slot of cell i (HydroRunFunctors2D.h:653-661)
+  // scaled by dt/dx (flux_scaled) into the XMIN slot of cell i (HydroRunFunctors2D.h:653-661)
   for (int fidx = threadIdx.x; fidx < (TX + 1) * TY; fidx += NT)
   {
     const int i = fidx % (TX + 1), j = fidx / (TX + 1);
@@ -292,7 +295,7 @@ hydro2d_tile(const S * __restrict__ Uin, S * __restrict__ Uout, const KParams & 
     hydro_riemann<RS, R, NV>(ql, qr, fl, C);
 #pragma unroll
     for (int v = 0; v < NV; ++v)
-      sXm[(v * TY + j) * FX + i + 1] = fl[v] * dtdx;
+      sXm[(v * TY + j) * FX + i + 1] = flux_scaled(fl[v], dtdx);
   }
   // y-faces: swap IU/IV around the solver (HydroRunFunctors2D.h:741-758)
   for (int fidx = threadIdx.x; fidx < TX * (TY + 1); fidx += NT)
@@ -317,7 +320,7 @@ hydro2d_tile(const S * __restrict__ Uin, S * __restrict__ Uout, const KParams & 
     fl[IV] = tmp;
 #pragma unroll
     for (int v = 0; v < NV; ++v)
-      sYm[(v * (TY + 2) + j + 1) * TX + i] = fl[v] * dtdy;
+      sYm[(v * (TY + 2) + j + 1) * TX + i] = flux_scaled(fl[v], dtdy);
   }
   __syncthreads();
 
@@ -334,10 +337,10 @@ hydro2d_tile(const S * __restrict__ Uin, S * __restrict__ Uout, const KParams & 
       R x = (R)ldg(Uin + v * P.vstride + off);
       if (v == ID)
         rho_old = x;
-      x += sXm[(v * TY + ty) * FX + tx + 1];
-      x -= sXm[(v * TY + ty) * FX + tx + 2];
-      x += sYm[(v * (TY + 2) + ty + 1) * TX + tx];
-      x -= sYm[(v * (TY + 2) + ty + 2) * TX + tx];
+      x = add_flux(x, sXm[(v * TY + ty) * FX + tx + 1], dtdx);
+      x = sub_flux(x, sXm[(v * TY + ty) * FX + tx + 2], dtdx);
+      x = add_flux(x, sYm[(v * (TY + 2) + ty + 1) * TX + tx], dtdy);
+      x = sub_flux(x, sYm[(v * (TY + 2) + ty + 2) * TX + tx], dtdy);
       u[v] = x;
     }
     R g[3];
@@ -356,9 +359,9 @@ hydro2d_tile(const S * __restrict__ Uin, S * __restrict__ Uout, const KParams & 
       us[v] = (R)(S)u[v];
     }
     if constexpr (GRAV)
-      tmax = fmax(tmax, hydro_invdt_grav<R, NV>(us, g, C, P));
+      tmax = max_cand(tmax, hydro_invdt_grav<R, NV>(us, g, C, P));
     else
-      tmax = fmax(tmax, hydro_invdt<R, NV>(us, C, P));
+      tmax = max_cand(tmax, hydro_invdt<R, NV>(us, C, P));
   }
   block_max_commit<NT>(cand_key((double)tmax), &clk->key[(step + 1) % 3]);
   if (bx == 0 && by == 0 && threadIdx.x == 0)
@@ -540,6 +543,7 @@ hydro3d_step(const S * __restrict__ Uin, S * __restrict__ Uout, KParams P, DevCl
     return;
   const double        t = sc.t, dt = sc.dt;
   const R             dtdx = to_r<R>(sc.dtdx), dtdy = to_r<R>(sc.dtdy), dtdz = to_r<R>(sc.dtdz);
+  const bool          same_xy = dtdx == dtdy, same_all = same_xy && dtdx == dtdz; // cubic cells
   const HydroConst<R> C = hydro_const<R>(P);
   const R             hdt = (R)(0.5 * dt);
   const bool          kick = GRAV && P.grav_hancock; // gravity predictor of the face states
@@ -643,39 +647,42 @@ hydro3d_step(const S * __restrict__ Uin, S * __restrict__ Uout, KParams P, DevCl
       R hg[3];
       if (kick)
         half_g(gi, gj, kc + gw, hg);
+      FaceStates<R, NV> F(c, s, dtdx, C.smallr);
       if (full)
       {
-        hydro_face<R, NV>(c, dX, s, dtdx, false, f, C.smallr);
+        F.get(dX, false, f);
         if (kick)
           grav_kick<R, NV>(f, hg);
 #pragma unroll
         for (int v = 0; v < NV; ++v)
           sXm[(v * TY + ty) * FX + tx + 1] = f[v];
-        hydro_face<R, NV>(c, dX, s, dtdx, true, f, C.smallr);
+        F.get(dX, true, f);
         if (kick)
           grav_kick<R, NV>(f, hg);
 #pragma unroll
         for (int v = 0; v < NV; ++v)
           sXp[(v * TY + ty) * FX + tx + 1] = f[v];
-        hydro_face<R, NV>(c, dY, s, dtdy, false, f, C.smallr);
+        F.turn(dtdy, same_xy);
+        F.get(dY, false, f);
         if (kick)
           grav_kick<R, NV>(f, hg);
 #pragma unroll
         for (int v = 0; v < NV; ++v)
           sYm[(v * (TY + 2) + ty + 1) * TX + tx] = f[v];
-        hydro_face<R, NV>(c, dY, s, dtdy, true, f, C.smallr);
+        F.get(dY, true, f);
         if (kick)
           grav_kick<R, NV>(f, hg);
 #pragma unroll
         for (int v = 0; v < NV; ++v)
           sYp[(v * (TY + 2) + ty + 1) * TX + tx] = f[v];
       }
+      F.turn(dtdz, same_all);
       if (kc >= k0)
       {
         // z-face between kc-1 and kc: ZMAX(kc-1), ZMIN(kc); swap IU/IW
         // (HydroRunFunctors3D.h:672-707)
         R qr[NV];
-        hydro_face<R, NV>(c, dZ, s, dtdz, false, qr, C.smallr);
+        F.get(dZ, false, qr);
         if (kick)
           grav_kick<R, NV>(qr, hg);
         R ql[NV];
@@ -694,11 +701,11 @@ hydro3d_step(const S * __restrict__ Uin, S * __restrict__ Uout, KParams P, DevCl
         fz[IW] = tmp;
 #pragma unroll
         for (int v = 0; v < NV; ++v)
-          fz[v] = fz[v] * dtdz;
+          fz[v] = flux_scaled(fz[v], dtdz);
       }
       if (kc < k1)
       {
-        hydro_face<R, NV>(c, dZ, s, dtdz, true, zmax_prev, C.smallr);
+        F.get(dZ, true, zmax_prev);
         if (kick)
           grav_kick<R, NV>(zmax_prev, hg);
       }
@@ -732,7 +739,7 @@ hydro3d_step(const S * __restrict__ Uin, S * __restrict__ Uout, KParams P, DevCl
           half_g(gi0 + cx, gj0 + cy, kc + gw, hg);
         if (kind < 2)
         {
-          hydro_face<R, NV>(c, dX, s, dtdx, kind == 0, f, C.smallr);
+          FaceStates<R, NV>(c, s, dtdx, C.smallr).get(dX, kind == 0, f);
           if (kick)
             grav_kick<R, NV>(f, hg);
           R * dst = kind == 0 ? sXp : sXm;
@@ -742,7 +749,7 @@ hydro3d_step(const S * __restrict__ Uin, S * __restrict__ Uout, KParams P, DevCl
         }
         else
         {
-          hydro_face<R, NV>(c, dY, s, dtdy, kind == 2, f, C.smallr);
+          FaceStates<R, NV>(c, s, dtdy, C.smallr).get(dY, kind == 2, f);
           if (kick)
             grav_kick<R, NV>(f, hg);
           R * dst = kind == 2 ? sYp : sYm;
@@ -800,7 +807,7 @@ hydro3d_step(const S * __restrict__ Uin, S * __restrict__ Uout, KParams P, DevCl
         const R dtd = ydir ? dtdy : dtdx;
 #pragma unroll
         for (int v = 0; v < NV; ++v)
-          rsrc[v * vs] = fl[v] * dtd;
+          rsrc[v * vs] = flux_scaled(fl[v], dtd);
       }
       __syncthreads();
     }
@@ -813,7 +820,7 @@ hydro3d_step(const S * __restrict__ Uin, S * __restrict__ Uout, KParams P, DevCl
       const long long off = own_off + (long long)(kc - 1 + gw) * P.plane;
 #pragma unroll
       for (int v = 0; v < NV; ++v)
-        u[v] = acc[v] - fz[v];
+        u[v] = sub_flux(acc[v], fz[v], dtdz);
       R g[3];
       if constexpr (GRAV)
       {
@@ -828,9 +835,9 @@ hydro3d_step(const S * __restrict__ Uin, S * __restrict__ Uout, KParams P, DevCl
         us[v] = (R)(S)u[v];
       }
       if constexpr (GRAV)
-        tmax = fmax(tmax, hydro_invdt_grav<R, NV>(us, g, C, P));
+        tmax = max_cand(tmax, hydro_invdt_grav<R, NV>(us, g, C, P));
       else
-        tmax = fmax(tmax, hydro_invdt<R, NV>(us, C, P));
+        tmax = max_cand(tmax, hydro_invdt<R, NV>(us, C, P));
     }
     if (full && own)
     {
@@ -841,11 +848,11 @@ hydro3d_step(const S * __restrict__ Uin, S * __restrict__ Uout, KParams P, DevCl
         R x = (R)ldg(Uin + v * P.vstride + off);
         if (v == ID)
           rho_prev = x;
-        x += sXm[(v * TY + ty) * FX + tx + 1];
-        x -= sXm[(v * TY + ty) * FX + tx + 2];
-        x += sYm[(v * (TY + 2) + ty + 1) * TX + tx];
-        x -= sYm[(v * (TY + 2) + ty + 2) * TX + tx];
-        x += fz[v];
+        x = add_flux(x, sXm[(v * TY + ty) * FX + tx + 1], dtdx);
+        x = sub_flux(x, sXm[(v * TY + ty) * FX + tx + 2], dtdx);
+        x = add_flux(x, sYm[(v * (TY + 2) + ty + 1) * TX + tx], dtdy);
+        x = sub_flux(x, sYm[(v * (TY + 2) + ty + 2) * TX + tx], dtdy);
+        x = add_flux(x, fz[v], dtdz);
         acc[v] = x;
       }
     }
@@ -877,10 +884,10 @@ hydro_dt_kernel(const S * __restrict__ U, KParams P, unsigned long long * key, D
     {
       R g[3];
       grav_at<S, R, NV>(P, i, j, k, g);
-      tmax = fmax(tmax, hydro_invdt_grav<R, NV>(u, g, C, P));
+      tmax = max_cand(tmax, hydro_invdt_grav<R, NV>(u, g, C, P));
     }
     else
-      tmax = fmax(tmax, hydro_invdt<R, NV>(u, C, P));
+      tmax = max_cand(tmax, hydro_invdt<R, NV>(u, C, P));
   });
   block_max_commit<256>(cand_key((double)tmax), key);
   if (fin)
