@@ -60,6 +60,7 @@ struct KParams
   float     idx, idy, idz; // 1/dx, 1/dy, 1/dz
   double    idxd, idyd, idzd; // 1/dx, 1/dy, 1/dz in FP64 (FP64 FMA build's CFL)
   int       mhd_stage;     // MHD update: stage the trace planes in shared memory
+  double    entho;           // 1 / (gamma0 - 1)
   double    gamma6, smallpp; // riemann_approx constants (HydroParams.cpp:353-356)
   float     gamma6f, smallppf;
   // static gravity (hydro; GravityParams.h:22-37): the field is gfield
@@ -402,17 +403,17 @@ sqrt64(double x)
   const double q = fma(g * r, fma(r, 0.375, 0.5), g);
   return seed_special(y) ? ((hi32(y) & 0x000fffff) != 0 ? y : x) : q;
 }
-// sqrt(n / d) for n >= 0, d > 0; 0 for n = 0
+// sqrt(n / d) for n >= 0, d > 0; 0 where n d is below 2^-1021
 __device__ __forceinline__ double
 sqrt_ratio64(double n, double d)
 {
-  const double c = n * rsqrt64(n * d);
-  return hi32(n) == 0 ? 0.0 : c;
+  const double x = n * d, c = n * rsqrt64(x);
+  return (unsigned)hi32(x) < 0x00200000u ? 0.0 : c;
 }
 __device__ __forceinline__ bool
-positive64(double x) // x > 0 (true for a positive NaN)
+positive64(double x) // x > 0
 {
-  return __double_as_longlong(x) > 0;
+  return (unsigned long long)(__double_as_longlong(x) - 1) < 0x7ff0000000000000ull;
 }
 __device__ __forceinline__ bool
 negative64(double x) // the sign bit
@@ -436,6 +437,18 @@ __device__ __forceinline__ double
 flip64(double x, bool f)
 {
   return with_hi(hi32(x) ^ (f ? (int)0x80000000 : 0), x);
+}
+// integers in the order of the numbers, and back
+__device__ __forceinline__ long long
+order64(double x)
+{
+  const long long b = __double_as_longlong(x);
+  return b ^ ((b >> 63) & 0x7fffffffffffffffll);
+}
+__device__ __forceinline__ double
+from_order64(long long b)
+{
+  return __longlong_as_double(b ^ ((b >> 63) & 0x7fffffffffffffffll));
 }
 // x / 2^K by the exponent (exact); the product where the result or x is not normal
 template <int K>
@@ -749,7 +762,8 @@ block_max_commit(unsigned long long local, unsigned long long * dst)
 __device__ __forceinline__ unsigned long long
 cand_key(double v)
 {
-  return (v != v) ? 0ull : dkey(v);
+  // NaN by its bits (a comparison is an FP64-pipe instruction)
+  return (__double_as_longlong(v) & 0x7fffffffffffffffll) > 0x7ff0000000000000ll ? 0ull : dkey(v);
 }
 
 

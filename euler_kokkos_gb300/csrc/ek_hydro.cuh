@@ -52,8 +52,9 @@ slope1(R q, R qp, R qm, R st)
 // Half of slope1's slope, for the FP64 FMA build: every use of a slope takes
 // its half.  Two differences on the FP64 pipe (three for MC); the minima, the
 // scaling by powers of two and the signs on the integer pipes.  A slope is
-// zero where dl and dr differ in sign or either is zero; with st = 1 (minmod)
-// the centred difference never binds (see the FP32 form above).
+// zero where dl and dr differ in sign or either is zero, and, as the
+// reference's test dl dr <= 0 has it, where their product underflows; with st =
+// 1 (minmod) the centred difference never binds (see the FP32 form above).
 __device__ __forceinline__ double
 half_slope64(double q, double qp, double qm, double st)
 {
@@ -67,9 +68,10 @@ half_slope64(double q, double qp, double qm, double st)
   else
     h = 0.0;
   // the sign of dl, or zero
-  const int sl = hi32(dl), differ = (sl ^ hi32(dr)) >> 31; // all ones where the signs differ
-  const int hi = hi32(h) & ~differ, lo = __double2loint(h) & ~differ;
-  return __hiloint2double(hi | (sl & (int)0x80000000), lo);
+  const int      sl = hi32(dl), sr = hi32(dr);
+  const unsigned e2 = (unsigned)(sl & 0x7fffffff) + (unsigned)(sr & 0x7fffffff); // log2 |dl dr| + 2046, x 2^20
+  const bool     zero = (sl ^ sr) < 0 || e2 < (970u << 20);
+  return __hiloint2double((zero ? 0 : hi32(h)) | (sl & (int)0x80000000), zero ? 0 : __double2loint(h));
 }
 // the slope, or its half in the FP64 FMA build (kFast64)
 template <class R>

@@ -28,7 +28,7 @@ hydro_const(const KParams & P)
     C.slope_type = P.slope_type;
     C.gamma6 = P.gamma6;
     C.smallpp = P.smallpp;
-    C.entho = 1.0 / (P.gamma0 - 1.0);
+    C.entho = P.entho;
   }
   else
   {

@@ -14,7 +14,20 @@ template <class R>
 struct MhdConst
 {
   R gamma0, smallr, smallp, smallc, slope_type;
+  R entho; // 1 / (gamma0 - 1), the value every Riemann solver of the reference computes
 };
+
+// rho c_fast^2 from gamma p, B^2 and Bn^2 in the FP64 FMA build: with all terms
+// multiplied by rho no reciprocal of the density is needed before the outer
+// root, which is one sqrt_ratio64 for the largest of several speeds.  The
+// discriminant, (B^2 - gamma p)^2 / 4 + gamma p Bt^2 by its parts, is not
+// negative.
+__device__ __forceinline__ double
+fast_num64(double gp, double b2, double bn2)
+{
+  const double s = scale_down64<1>(b2 + gp);
+  return s + sqrt64(max_floor64(fma(s, s, -(gp * bn2)), 0.0));
+}
 
 // find_speed_fast<dir> (mhd_utils.h:89-117)
 template <class R, int DIR>
@@ -24,7 +37,9 @@ mhd_speed_fast(const R (&q)[8], R gamma0)
   const R d = q[ID], p = q[IP], a = q[IA], b = q[IB], c = q[IC];
   const R b2 = a * a + b * b + c * c;
   const R bn = DIR == 0 ? a : (DIR == 1 ? b : c);
-  if constexpr (kShareRecip)
+  if constexpr (kFast64<R>)
+    return sqrt_ratio64(fast_num64(gamma0 * p, b2, bn * bn), d);
+  else if constexpr (kShareRecip)
   {
     const R id = R(1) / d;
     const R c2 = gamma0 * p * id;
@@ -34,23 +49,6 @@ mhd_speed_fast(const R (&q)[8], R gamma0)
   const R c2 = gamma0 * p / d;
   const R d2 = R(0.5) * (b2 / d + c2);
   return sqrt(d2 + sqrt(d2 * d2 - c2 * bn * bn / d));
-}
-
-// the square of find_speed_fast<dir> before its outer square root (FP64 FMA
-// build).  A correctly rounded square root is monotonic, so the largest of
-// several speeds is the square root of the largest of these, bit for bit,
-// one square root instead of one per state.
-template <class R, int DIR>
-__device__ __forceinline__ R
-mhd_speed_fast_sq(const R (&q)[8], R gamma0)
-{
-  const R d = q[ID], p = q[IP], a = q[IA], b = q[IB], c = q[IC];
-  const R b2 = a * a + b * b + c * c;
-  const R bn = DIR == 0 ? a : (DIR == 1 ? b : c);
-  const R id = R(1) / d;
-  const R c2 = gamma0 * p * id;
-  const R d2 = R(0.5) * (b2 * id + c2);
-  return d2 + sqrt(d2 * d2 - c2 * bn * bn * id);
 }
 
 // find_speed_info<THREE_D> summed as ComputeDtFunctor3D_MHD does
@@ -75,16 +73,13 @@ mhd_invdt(const R (&q)[8], R gamma0, double dx, double dy, double dz, float idx,
     const float cfz = sqrt_a(d2 + sqrt_a(dd - cr * c * c));
     return (cfx + fabsf(q[IU])) * idx + (cfy + fabsf(q[IV])) * idy + (cfz + fabsf(q[IW])) * idz;
   }
-  if constexpr (kShareRecip)
+  if constexpr (kFast64<R>)
   {
-    // FP64 FMA build: one reciprocal of the density, host-prepared 1/dx
-    const R id = R(1) / d;
-    const R c2 = gamma0 * p * id;
-    const R d2 = R(0.5) * (b2 * id + c2);
-    const R dd = d2 * d2, cr = c2 * id;
-    const R cfx = sqrt(d2 + sqrt(dd - cr * a * a));
-    const R cfy = sqrt(d2 + sqrt(dd - cr * b * b));
-    const R cfz = sqrt(d2 + sqrt(dd - cr * c * c));
+    // FP64 FMA build: host-prepared 1/dx
+    const R gp = gamma0 * p;
+    const R cfx = sqrt_ratio64(fast_num64(gp, b2, a * a), d);
+    const R cfy = sqrt_ratio64(fast_num64(gp, b2, b * b), d);
+    const R cfz = sqrt_ratio64(fast_num64(gp, b2, c * c), d);
     return (cfx + fabs(q[IU])) * idxd + (cfy + fabs(q[IV])) * idyd + (cfz + fabs(q[IW])) * idzd;
   }
   const R c2 = gamma0 * p / d;
@@ -108,18 +103,27 @@ __device__ __forceinline__ void
 mhd_constoprim(const R (&u)[5], const R (&bl)[3], const R (&br)[3], R (&q)[8], const MhdConst<R> & C,
                FB && fp64_faces)
 {
+  if constexpr (kFast64<R>)
+  {
+    // FP64 FMA build: p = (gamma - 1) (E - B^2 / 2 - rho v^2 / 2)
+    const R d = max_floor64(u[ID], C.smallr), id = rcp64(d);
+    q[ID] = d;
+    q[IU] = u[IU] * id;
+    q[IV] = u[IV] * id;
+    q[IW] = u[IW] * id;
+    q[IA] = scale_down64<1>(bl[0] + br[0]);
+    q[IB] = scale_down64<1>(bl[1] + br[1]);
+    q[IC] = scale_down64<1>(bl[2] + br[2]);
+    const R k2 = q[IU] * q[IU] + q[IV] * q[IV] + q[IW] * q[IW];
+    const R b2 = q[IA] * q[IA] + q[IB] * q[IB] + q[IC] * q[IC];
+    q[IP] = floor_ratio64((C.gamma0 - R(1)) * fma(R(-0.5) * d, k2, fma(R(-0.5), b2, u[IP])), d, C.smallp);
+    return;
+  }
   q[ID] = fmax(u[ID], C.smallr);
   R id = R(0);
   if constexpr (sizeof(R) == 4)
   {
     id = rcp_a(q[ID]);
-    q[IU] = u[IU] * id;
-    q[IV] = u[IV] * id;
-    q[IW] = u[IW] * id;
-  }
-  else if constexpr (kShareRecip)
-  {
-    id = R(1) / q[ID];
     q[IU] = u[IU] * id;
     q[IV] = u[IV] * id;
     q[IW] = u[IW] * id;
@@ -136,7 +140,7 @@ mhd_constoprim(const R (&u)[5], const R (&bl)[3], const R (&br)[3], R (&q)[8], c
   const R eken = R(0.5) * (q[IU] * q[IU] + q[IV] * q[IV] + q[IW] * q[IW]);
   const R emag = R(0.5) * (q[IA] * q[IA] + q[IB] * q[IB] + q[IC] * q[IC]);
   R       eint;
-  if constexpr (sizeof(R) == 4 || kShareRecip)
+  if constexpr (sizeof(R) == 4)
     eint = (u[IP] - emag) * id - eken;
   else
     eint = (u[IP] - emag) / q[ID] - eken;
@@ -302,6 +306,109 @@ mhd_hlld_f32(const float (&ql)[8], const float (&qr)[8], float (&flux)[NF], floa
   return true;
 }
 
+// riemann_hlld (RiemannSolvers_MHD.h:130-364) in the FP64 FMA build: the same
+// states with about 180 FP64-pipe operations per face.  Both fast speeds share
+// one outer root (fast_num64); u* and p* follow from one quotient w; the
+// degenerate-state test |estar / Bn^2 - 1| <= 1e-8 is taken without the
+// division; roots and quotients by rsqrt64 / rcp64; regions, minima and signs on
+// the integer pipes.  With the emf and trace below: FP64 2D step 189 -> 122 us at
+// 200 x 136, 3D step 4170 -> 2830 us at 32^3.
+template <int NF>
+__device__ __forceinline__ void
+mhd_hlld64(const double (&ql)[8], const double (&qr)[8], double (&flux)[NF], double gamma0, double entho)
+{
+  const double a = scale_down64<1>(ql[IA] + qr[IA]), a2 = a * a;
+  struct Side
+  {
+    double pt, et, vb, n; // total pressure and energy, v.B, rho c_fast^2
+  };
+  auto side = [&](const double (&q)[8]) {
+    Side         s;
+    const double b2 = fma(q[IC], q[IC], fma(q[IB], q[IB], a2)), em = scale_down64<1>(b2);
+    const double k2 = fma(q[IW], q[IW], fma(q[IV], q[IV], q[IU] * q[IU]));
+    s.pt = q[IP] + em;
+    s.et = fma(q[IP], entho, fma(scale_down64<1>(q[ID]), k2, em));
+    s.vb = fma(q[IW], q[IC], fma(q[IV], q[IB], q[IU] * a));
+    s.n = fast_num64(gamma0 * q[IP], b2, a2);
+    return s;
+  };
+  const Side   L = side(ql), R = side(qr);
+  const double ul = ql[IU], ur = qr[IU];
+  const bool   lbig = __double_as_longlong(L.n * qr[ID]) >= __double_as_longlong(R.n * ql[ID]);
+  const double cmax = sqrt_ratio64(lbig ? L.n : R.n, lbig ? ql[ID] : qr[ID]);
+  const double du = ul - ur;
+  const bool   lslow = negative64(du);
+  const double sl = (lslow ? ul : ur) - cmax, sr = (lslow ? ur : ul) + cmax;
+  const double al = ul - sl, ar = sr - ur;
+  const double rcl = ql[ID] * al, rcr = qr[ID] * ar;
+  const double w = fma(-rcr, du, L.pt - R.pt) * rcp64(rcr + rcl);
+  const double us = ul + w, ps = fma(-rcl, w, L.pt);
+  const double usa = us * a, psus = ps * us;
+
+  struct Star
+  {
+    double r, v, w, b, c, vb, et, sq, al; // sq = sqrt(rho*), al = |Bn| / sqrt(rho*)
+  };
+  // dS = S - u, rd = rho dS, du = u* - u
+  auto star = [&](const double (&q)[8], const Side & s, double S, double dS, double rd, double du) {
+    Star         t;
+    const double sus = S - us, is = rcp64(sus);
+    t.r = rd * is;
+    const double es = fma(rd, sus, -a2), e = fma(rd, dS, -a2), ie = rcp64(es);
+    const bool   deg = positive64(a2) &&
+                     __double_as_longlong(fabs(es - a2)) <= __double_as_longlong(1e-8 * a2);
+    const double h = deg ? 0.0 : a * du * ie, f = deg ? 1.0 : e * ie;
+    t.v = fma(-q[IB], h, q[IV]);
+    t.w = fma(-q[IC], h, q[IW]);
+    t.b = q[IB] * f;
+    t.c = q[IC] * f;
+    t.vb = fma(t.w, t.c, fma(t.v, t.b, usa));
+    t.et = fma(a, s.vb - t.vb, fma(-s.pt, q[IU], fma(dS, s.et, psus))) * is;
+    const double y = rsqrt64(t.r);
+    t.sq = t.r * y;
+    t.al = fabs(a) * y;
+    return t;
+  };
+  const Star   Ls = star(ql, L, sl, flip64(al, true), flip64(rcl, true), w), Rs = star(qr, R, sr, ar, rcr, us - ur);
+  const double sal = us - Ls.al, sar = us + Rs.al;
+  const bool   left = positive64(sl), lstar = !left && positive64(sal);
+  const bool   rside = !left && !lstar && !positive64(us) && !positive64(sar);
+  double       ro, uo, vo, wo, bo, co, po, eo, vbo;
+  if (left || (rside && !positive64(sr)))
+  {
+    ro = left ? ql[ID] : qr[ID], uo = left ? ul : ur, vo = left ? ql[IV] : qr[IV], wo = left ? ql[IW] : qr[IW];
+    bo = left ? ql[IB] : qr[IB], co = left ? ql[IC] : qr[IC];
+    po = left ? L.pt : R.pt, eo = left ? L.et : R.et, vbo = left ? L.vb : R.vb;
+  }
+  else if (lstar || rside)
+  {
+    ro = lstar ? Ls.r : Rs.r, uo = us, vo = lstar ? Ls.v : Rs.v, wo = lstar ? Ls.w : Rs.w;
+    bo = lstar ? Ls.b : Rs.b, co = lstar ? Ls.c : Rs.c;
+    po = ps, eo = lstar ? Ls.et : Rs.et, vbo = lstar ? Ls.vb : Rs.vb;
+  }
+  else
+  {
+    const bool   neg = negative64(a), cl = positive64(us); // sgn(Bn) < 0; left of the contact
+    const double is = rcp64(Ls.sq + Rs.sq), sq2 = Ls.sq * Rs.sq;
+    vo = (fma(Ls.sq, Ls.v, Rs.sq * Rs.v) + flip64(Rs.b - Ls.b, neg)) * is;
+    wo = (fma(Ls.sq, Ls.w, Rs.sq * Rs.w) + flip64(Rs.c - Ls.c, neg)) * is;
+    bo = fma(sq2, flip64(Rs.v - Ls.v, neg), fma(Ls.sq, Rs.b, Rs.sq * Ls.b)) * is;
+    co = fma(sq2, flip64(Rs.w - Ls.w, neg), fma(Ls.sq, Rs.c, Rs.sq * Ls.c)) * is;
+    vbo = fma(wo, co, fma(vo, bo, usa));
+    uo = us, po = ps;
+    ro = cl ? Ls.r : Rs.r;
+    eo = fma(flip64(cl ? Ls.sq : Rs.sq, neg == cl), vbo - (cl ? Ls.vb : Rs.vb), cl ? Ls.et : Rs.et);
+  }
+  const double m = ro * uo;
+  flux[ID] = m;
+  flux[IP] = fma(eo + po, uo, -(a * vbo));
+  flux[IU] = fma(m, uo, po - a2);
+  flux[IV] = fma(m, vo, -(a * bo));
+  flux[IW] = fma(m, wo, -(a * co));
+  if constexpr (NF > 5)
+    flux[5] = fma(co, uo, -(a * wo));
+}
+
 // riemann_hlld (RiemannSolvers_MHD.h:130-364), states in the face frame.
 // The 3D update uses the five hydro components of the flux (NF = 5); the 2D
 // update also uses the Bz component, returned in flux[5] when NF = 6.
@@ -310,13 +417,17 @@ mhd_hlld_f32(const float (&ql)[8], const float (&qr)[8], float (&flux)[NF], floa
 // with mhd_hlld<double> from the same states.
 template <class R, int NF = 5>
 __device__ __forceinline__ bool
-mhd_hlld(R (&ql)[8], R (&qr)[8], R (&flux)[NF], R gamma0)
+mhd_hlld(R (&ql)[8], R (&qr)[8], R (&flux)[NF], R gamma0, R entho)
 {
   if constexpr (sizeof(R) == 4)
     return mhd_hlld_f32<NF>(ql, qr, flux, gamma0);
+  else if constexpr (kFast64<R>)
+  {
+    mhd_hlld64<NF>(ql, qr, flux, gamma0, entho);
+    return true;
+  }
   else
   {
-  const R entho = R(1.0) / (gamma0 - R(1.0));
   const R a = R(0.5) * (ql[IA] + qr[IA]);
   const R sgnm = (a >= R(0)) ? R(1) : R(-1);
   ql[IA] = a;
@@ -334,32 +445,17 @@ mhd_hlld(R (&ql)[8], R (&qr)[8], R (&flux)[NF], R gamma0)
   const R ptotr = pr + emagr;
   const R vdotbr = ur * a + vr * br + wr * cr;
 
-  // the larger fast speed (FP64 FMA build: one outer square root, the same bits)
-  R cmax;
-  if constexpr (kShareRecip)
-    cmax = sqrt(fmax(mhd_speed_fast_sq<R, 0>(ql, gamma0), mhd_speed_fast_sq<R, 0>(qr, gamma0)));
-  else
-    cmax = fmax(mhd_speed_fast<R, 0>(ql, gamma0), mhd_speed_fast<R, 0>(qr, gamma0));
+  const R cmax = fmax(mhd_speed_fast<R, 0>(ql, gamma0), mhd_speed_fast<R, 0>(qr, gamma0));
   const R sl = fmin(ul, ur) - cmax;
   const R sr = fmax(ul, ur) + cmax;
   const R rcl = rl * (ul - sl);
   const R rcr = rr * (sr - ur);
-  // FP64 FMA build: one reciprocal per shared denominator (kShareRecip)
-  const R irc = kShareRecip ? R(1) / (rcr + rcl) : R(0);
-  const R ustar = kShareRecip ? (rcr * ur + rcl * ul + (ptotl - ptotr)) * irc
-                              : (rcr * ur + rcl * ul + (ptotl - ptotr)) / (rcr + rcl);
-  const R ptotstar = kShareRecip ? (rcr * ptotl + rcl * ptotr + rcl * rcr * (ul - ur)) * irc
-                                 : (rcr * ptotl + rcl * ptotr + rcl * rcr * (ul - ur)) / (rcr + rcl);
+  const R ustar = (rcr * ur + rcl * ul + (ptotl - ptotr)) / (rcr + rcl);
+  const R ptotstar = (rcr * ptotl + rcl * ptotr + rcl * rcr * (ul - ur)) / (rcr + rcl);
 
   R estar;
-  // the degenerate-state test divides both sides' estar by a^2: one
-  // reciprocal in the FP64 FMA build
-  const R ia2 = kShareRecip ? R(1) / (a * a) : R(0);
-  auto    degenerate = [&](R e) {
-    return a * a > R(0) && fabs((kShareRecip ? e * ia2 : e / (a * a)) - R(1)) <= R(1e-8);
-  };
-  const R isl = kShareRecip ? R(1) / (sl - ustar) : R(0);
-  const R rstarl = kShareRecip ? rl * (sl - ul) * isl : rl * (sl - ul) / (sl - ustar);
+  auto degenerate = [&](R e) { return a * a > R(0) && fabs(e / (a * a) - R(1)) <= R(1e-8); };
+  const R rstarl = rl * (sl - ul) / (sl - ustar);
   estar = rl * (sl - ul) * (sl - ustar) - a * a;
   const R el = rl * (sl - ul) * (sl - ul) - a * a;
   R       vstarl, wstarl, bstarl, cstarl;
@@ -370,14 +466,6 @@ mhd_hlld(R (&ql)[8], R (&qr)[8], R (&flux)[NF], R gamma0)
     wstarl = wl;
     cstarl = cl;
   }
-  else if constexpr (kShareRecip)
-  {
-    const R ie = R(1) / estar;
-    vstarl = vl - a * bl * (ustar - ul) * ie;
-    bstarl = bl * el * ie;
-    wstarl = wl - a * cl * (ustar - ul) * ie;
-    cstarl = cl * el * ie;
-  }
   else
   {
     vstarl = vl - a * bl * (ustar - ul) / estar;
@@ -387,17 +475,12 @@ mhd_hlld(R (&ql)[8], R (&qr)[8], R (&flux)[NF], R gamma0)
   }
   const R vdotbstarl = ustar * a + vstarl * bstarl + wstarl * cstarl;
   const R etotstarl =
-    kShareRecip ? ((sl - ul) * etotl - ptotl * ul + ptotstar * ustar + a * (vdotbl - vdotbstarl)) * isl
-                : ((sl - ul) * etotl - ptotl * ul + ptotstar * ustar + a * (vdotbl - vdotbstarl)) / (sl - ustar);
-  // sqrt(rho*) and |a| / sqrt(rho*): one reciprocal square root in the FP64
-  // FMA build
-  const R rsl = kShareRecip ? rsqrt(rstarl) : R(0);
-  const R sqrrstarl = kShareRecip ? rstarl * rsl : sqrt(rstarl);
-  const R calfvenl = kShareRecip ? fabs(a) * rsl : fabs(a) / sqrrstarl;
+    ((sl - ul) * etotl - ptotl * ul + ptotstar * ustar + a * (vdotbl - vdotbstarl)) / (sl - ustar);
+  const R sqrrstarl = sqrt(rstarl);
+  const R calfvenl = fabs(a) / sqrrstarl;
   const R sal = ustar - calfvenl;
 
-  const R isr = kShareRecip ? R(1) / (sr - ustar) : R(0);
-  const R rstarr = kShareRecip ? rr * (sr - ur) * isr : rr * (sr - ur) / (sr - ustar);
+  const R rstarr = rr * (sr - ur) / (sr - ustar);
   estar = rr * (sr - ur) * (sr - ustar) - a * a;
   const R er = rr * (sr - ur) * (sr - ur) - a * a;
   R       vstarr, wstarr, bstarr, cstarr;
@@ -408,14 +491,6 @@ mhd_hlld(R (&ql)[8], R (&qr)[8], R (&flux)[NF], R gamma0)
     wstarr = wr;
     cstarr = cr;
   }
-  else if constexpr (kShareRecip)
-  {
-    const R ie = R(1) / estar;
-    vstarr = vr - a * br * (ustar - ur) * ie;
-    bstarr = br * er * ie;
-    wstarr = wr - a * cr * (ustar - ur) * ie;
-    cstarr = cr * er * ie;
-  }
   else
   {
     vstarr = vr - a * br * (ustar - ur) / estar;
@@ -425,11 +500,9 @@ mhd_hlld(R (&ql)[8], R (&qr)[8], R (&flux)[NF], R gamma0)
   }
   const R vdotbstarr = ustar * a + vstarr * bstarr + wstarr * cstarr;
   const R etotstarr =
-    kShareRecip ? ((sr - ur) * etotr - ptotr * ur + ptotstar * ustar + a * (vdotbr - vdotbstarr)) * isr
-                : ((sr - ur) * etotr - ptotr * ur + ptotstar * ustar + a * (vdotbr - vdotbstarr)) / (sr - ustar);
-  const R rsr = kShareRecip ? rsqrt(rstarr) : R(0);
-  const R sqrrstarr = kShareRecip ? rstarr * rsr : sqrt(rstarr);
-  const R calfvenr = kShareRecip ? fabs(a) * rsr : fabs(a) / sqrrstarr;
+    ((sr - ur) * etotr - ptotr * ur + ptotstar * ustar + a * (vdotbr - vdotbstarr)) / (sr - ustar);
+  const R sqrrstarr = sqrt(rstarr);
+  const R calfvenr = fabs(a) / sqrrstarr;
   const R sar = ustar + calfvenr;
 
   R ro, uo, vo, wo, bo, co, ptoto, etoto, vdotbo;
@@ -456,13 +529,10 @@ mhd_hlld(R (&ql)[8], R (&qr)[8], R (&flux)[NF], R gamma0)
   else
   {
     // double-star region (only evaluated when sampled)
-    const R iss = kShareRecip ? R(1) / (sqrrstarl + sqrrstarr) : R(0);
     const R vstarstar =
-      kShareRecip ? (sqrrstarl * vstarl + sqrrstarr * vstarr + sgnm * (bstarr - bstarl)) * iss
-                  : (sqrrstarl * vstarl + sqrrstarr * vstarr + sgnm * (bstarr - bstarl)) / (sqrrstarl + sqrrstarr);
+      (sqrrstarl * vstarl + sqrrstarr * vstarr + sgnm * (bstarr - bstarl)) / (sqrrstarl + sqrrstarr);
     const R wstarstar =
-      kShareRecip ? (sqrrstarl * wstarl + sqrrstarr * wstarr + sgnm * (cstarr - cstarl)) * iss
-                  : (sqrrstarl * wstarl + sqrrstarr * wstarr + sgnm * (cstarr - cstarl)) / (sqrrstarl + sqrrstarr);
+      (sqrrstarl * wstarl + sqrrstarr * wstarr + sgnm * (cstarr - cstarl)) / (sqrrstarl + sqrrstarr);
     const R bstarstar =
       (sqrrstarl * bstarr + sqrrstarr * bstarl + sgnm * sqrrstarl * sqrrstarr * (vstarr - vstarl)) /
       (sqrrstarl + sqrrstarr);
@@ -498,7 +568,7 @@ mhd_hlld(R (&ql)[8], R (&qr)[8], R (&flux)[NF], R gamma0)
 // time: RS = the reference's riemannSolverType (1 llf, 2 hll, 4 hlld)
 template <int RS, class R, int NF>
 __device__ __forceinline__ bool
-mhd_riemann(R (&ql)[8], R (&qr)[8], R (&flux)[NF], R gamma0);
+mhd_riemann(R (&ql)[8], R (&qr)[8], R (&flux)[NF], const MhdConst<R> & C);
 
 // find_mhd_flux (mhd_utils.h:170-231, cIso = 0): conservative state and
 // flux of a face-frame primitive state; components ID, IP, IU, IV, IW and,
@@ -573,14 +643,14 @@ mhd_llf(R (&ql)[8], R (&qr)[8], R (&flux)[NF], R gamma0)
 // false: the FP32 HLLD left this face to its FP64 island (mhd_riemann_f64)
 template <int RS, class R, int NF>
 __device__ __forceinline__ bool
-mhd_riemann(R (&ql)[8], R (&qr)[8], R (&flux)[NF], R gamma0)
+mhd_riemann(R (&ql)[8], R (&qr)[8], R (&flux)[NF], const MhdConst<R> & C)
 {
   if constexpr (RS == 1)
-    mhd_llf<R, NF>(ql, qr, flux, gamma0);
+    mhd_llf<R, NF>(ql, qr, flux, C.gamma0);
   else if constexpr (RS == 2)
-    mhd_hll<R, NF>(ql, qr, flux, gamma0);
+    mhd_hll<R, NF>(ql, qr, flux, C.gamma0);
   else
-    return mhd_hlld<R, NF>(ql, qr, flux, gamma0);
+    return mhd_hlld<R, NF>(ql, qr, flux, C.gamma0, C.entho);
   return true;
 }
 
@@ -601,7 +671,7 @@ mhd_hlld_f64_island(float4 l0, float4 l1, float4 r0, float4 r1, float gamma0)
   double l[8] = { f2d(l0.x), f2d(l0.y), f2d(l0.z), f2d(l0.w), f2d(l1.x), f2d(l1.y), f2d(l1.z), f2d(l1.w) };
   double r[8] = { f2d(r0.x), f2d(r0.y), f2d(r0.z), f2d(r0.w), f2d(r1.x), f2d(r1.y), f2d(r1.z), f2d(r1.w) };
   double f[NF];
-  mhd_hlld<double, NF>(l, r, f, f2d(gamma0));
+  mhd_hlld<double, NF>(l, r, f, f2d(gamma0), 1.0 / (f2d(gamma0) - 1.0));
   HlldFlux32 out;
 #pragma unroll
   for (int i = 0; i < 6; ++i)
@@ -779,6 +849,99 @@ mag_riemann2d_hlld_f32(const EdgeQ<float> & LL, const EdgeQ<float> & RL, const E
   return E;
 }
 
+// mag_riemann2d_hlld (RiemannSolvers_MHD.h:395-627) in the FP64 FMA build: the
+// same emf with about 300 FP64-pipe operations per edge.  a is the same at
+// the two corners of a row (LL, RL and LR, RR), b at the two of a column.  With
+// fx = (S - u) / (S - u*), fy likewise, rho*, A* and B* are products, and the two
+// Alfven speeds of a corner, |a| / sqrt(rho fx) and |A*| / sqrt(rho fx fy), are
+// the root of a^2 max(1, fy) / (rho fx): the larger of two corners' quotients is
+// chosen by products, so a side takes one reciprocal root instead of four.  Of
+// the five cases only the one sampled is computed.
+__device__ __forceinline__ double
+mag_riemann2d_hlld64(const EdgeQ<double> & LL, const EdgeQ<double> & RL, const EdgeQ<double> & LR,
+                     const EdgeQ<double> & RR, double gamma0, double smallc)
+{
+  const double a0 = LL.a, a1 = LR.a, b0 = LL.b, b1 = RL.b;
+  const double a02 = a0 * a0, a12 = a1 * a1, b02 = b0 * b0, b12 = b1 * b1;
+  // total pressure; squares of the fast speeds along x and y
+  long long cx = 0, cy = 0;
+  auto      corner = [&](const EdgeQ<double> & q, double a2, double b2) {
+    const double s = fma(q.c, q.c, a2 + b2), g = gamma0 * q.p, ir = rcp64(q.r);
+    cx = max(cx, __double_as_longlong(fast_num64(g, s, a2) * ir));
+    cy = max(cy, __double_as_longlong(fast_num64(g, s, b2) * ir));
+    return q.p + scale_down64<1>(s);
+  };
+  const double PLL = corner(LL, a02, b02), PRL = corner(RL, a02, b12);
+  const double PLR = corner(LR, a12, b02), PRR = corner(RR, a12, b12);
+  const double cmx = sqrt64(__longlong_as_double(cx)), cmy = sqrt64(__longlong_as_double(cy));
+  auto         lowest = [](double p, double q, double r, double s) {
+    return from_order64(min(min(order64(p), order64(q)), min(order64(r), order64(s))));
+  };
+  auto highest = [](double p, double q, double r, double s) {
+    return from_order64(max(max(order64(p), order64(q)), max(order64(r), order64(s))));
+  };
+  const double SL = lowest(LL.u, LR.u, RL.u, RR.u) - cmx, SR = highest(LL.u, LR.u, RL.u, RR.u) + cmx;
+  const double SB = lowest(LL.v, LR.v, RL.v, RR.v) - cmy, ST = highest(LL.v, LR.v, RL.v, RR.v) + cmy;
+
+  // distances of the corner velocities from the outer waves (positive)
+  const double xLL = LL.u - SL, xLR = LR.u - SL, xRL = SR - RL.u, xRR = SR - RR.u;
+  const double yLL = LL.v - SB, yRL = RL.v - SB, yLR = ST - LR.v, yRR = ST - RR.v;
+  const double D1 = PLL - PRR, D2 = PLR - PRL;
+  double       us, vs;
+  {
+    const double p = LL.r * xLL, q = LR.r * xLR, r = RL.r * xRL, s = RR.r * xRR;
+    us = fma(p, LL.u, fma(q, LR.u, fma(r, RL.u, fma(s, RR.u, D1 + D2)))) * rcp64((p + q) + (r + s));
+  }
+  {
+    const double p = LL.r * yLL, q = LR.r * yLR, r = RL.r * yRL, s = RR.r * yRR;
+    vs = fma(p, LL.v, fma(q, LR.v, fma(r, RL.v, fma(s, RR.v, D1 - D2)))) * rcp64((p + q) + (r + s));
+  }
+  const double iL = rcp64(us - SL), iR = rcp64(SR - us), iB = rcp64(vs - SB), iT = rcp64(ST - vs);
+  const double fxLL = xLL * iL, fxLR = xLR * iL, fxRL = xRL * iR, fxRR = xRR * iR;
+  const double fyLL = yLL * iB, fyRL = yRL * iB, fyLR = yLR * iT, fyRR = yRR * iT;
+
+  // the larger Alfven speed of two corners: sqrt(max(n1 m1 / d1, n2 m2 / d2)), m >= 1
+  auto alfven = [&](double n1, double m1, double d1, double n2, double m2, double d2) {
+    n1 *= max_floor64(m1, 1.0);
+    n2 *= max_floor64(m2, 1.0);
+    const bool first = __double_as_longlong(n1 * d2) >= __double_as_longlong(n2 * d1);
+    return max_floor64(sqrt_ratio64(first ? n1 : n2, first ? d1 : d2), smallc);
+  };
+  const double cL = alfven(a12, fyLR, LR.r * fxLR, a02, fyLL, LL.r * fxLL);
+  const double cR = alfven(a12, fyRR, RR.r * fxRR, a02, fyRL, RL.r * fxRL);
+  const double cB = alfven(b02, fxLL, LL.r * fyLL, b12, fxRL, RL.r * fyRL);
+  const double cT = alfven(b02, fxLR, LR.r * fyLR, b12, fxRR, RR.r * fyRR);
+  auto         below = [](double x) { return negative64(x) ? x : 0.0; };
+  auto         above = [](double x) { return negative64(x) ? 0.0 : x; };
+  const double SAL = below(us - cL), SAR = above(us + cR), SAB = below(vs - cB), SAT = above(vs + cT);
+
+  const bool SLp = !negative64(SL), SRp = !negative64(SR), SBp = !negative64(SB), STp = !negative64(ST);
+  if (SBp || !STp)
+  {
+    // supersonic along y: the x fan of the corners on that side
+    const EdgeQ<double> &l = SBp ? LL : LR, &r = SBp ? RL : RR;
+    const double         b_l = l.b, b_r = r.b;
+    if (SLp || !SRp)
+      return SLp ? l.u * l.b - l.v * l.a : r.u * r.b - r.v * r.a;
+    const double El = us * (b_l * (SBp ? fxLL : fxLR)) - l.v * l.a, Er = us * (b_r * (SBp ? fxRL : fxRR)) - r.v * r.a;
+    return (SAR * El - SAL * Er + SAR * SAL * (b_r - b_l)) * rcp64(SAR - SAL);
+  }
+  if (SLp || !SRp)
+  {
+    const EdgeQ<double> &b = SLp ? LL : RL, &t = SLp ? LR : RR;
+    const double         Eb = b.u * b.b - vs * (b.a * (SLp ? fyLL : fyRL)), Et = t.u * t.b - vs * (t.a * (SLp ? fyLR : fyRR));
+    return (SAT * Eb - SAB * Et - SAT * SAB * (t.a - b.a)) * rcp64(SAT - SAB);
+  }
+  const double ALL = a0 * fyLL, ARL = a0 * fyRL, ALR = a1 * fyLR, ARR = a1 * fyRR;
+  const double BLL = b0 * fxLL, BLR = b0 * fxLR, BRL = b1 * fxRL, BRR = b1 * fxRR;
+  const double ELL = us * BLL - vs * ALL, ERL = us * BRL - vs * ARL;
+  const double ELR = us * BLR - vs * ALR, ERR = us * BRR - vs * ARR;
+  const double e1 = SAB * ERR - SAT * ERL, e2 = SAB * ELR - SAT * ELL;
+  const double dA = SAR * (ARR - ARL) - SAL * (ALR - ALL), dB = SAT * (BRR - BLR) - SAB * (BRL - BLL);
+  const double e = fma(SAR * SAL, dB, fma(-(SAT * SAB), dA, SAL * e1 - SAR * e2));
+  return e * (rcp64(SAR - SAL) * rcp64(SAT - SAB));
+}
+
 // mag_riemann2d_hlld (RiemannSolvers_MHD.h:395-627); corners LL, RL, LR, RR
 template <class R>
 __device__ __forceinline__ R
@@ -787,21 +950,14 @@ mag_riemann2d_hlld(const EdgeQ<R> & LL, const EdgeQ<R> & RL, const EdgeQ<R> & LR
 {
   if constexpr (sizeof(R) == 4)
     return mag_riemann2d_hlld_f32(LL, RL, LR, RR, ELL, ERL, ELR, ERR, gamma0, smallc);
+  else if constexpr (kFast64<R>)
+    return mag_riemann2d_hlld64(LL, RL, LR, RR, gamma0, smallc);
   else
   {
-  // fast speed of a corner state along x or y; the FP64 FMA build returns its
-  // square (before the outer square root, see mhd_speed_fast_sq) and takes one
-  // square root of the largest
+  // fast speed of a corner state along x or y
   auto fast = [gamma0](const EdgeQ<R> & q, bool ydir) {
     const R b2 = q.a * q.a + q.b * q.b + q.c * q.c;
     const R bn = ydir ? q.b : q.a;
-    if constexpr (kShareRecip)
-    {
-      const R ir = R(1) / q.r;
-      const R c2 = gamma0 * q.p * ir;
-      const R d2 = R(0.5) * (b2 * ir + c2);
-      return d2 + sqrt(d2 * d2 - c2 * bn * bn * ir);
-    }
     const R c2 = gamma0 * q.p / q.r;
     const R d2 = R(0.5) * (b2 / q.r + c2);
     return sqrt(d2 + sqrt(d2 * d2 - c2 * bn * bn / q.r));
@@ -816,9 +972,7 @@ mag_riemann2d_hlld(const EdgeQ<R> & LL, const EdgeQ<R> & RL, const EdgeQ<R> & LR
   const R cFastLLy = fast(LL, true), cFastLRy = fast(LR, true);
   const R cFastRLy = fast(RL, true), cFastRRy = fast(RR, true);
 
-  R cmx = fmax4(cFastLLx, cFastLRx, cFastRLx, cFastRRx), cmy = fmax4(cFastLLy, cFastLRy, cFastRLy, cFastRRy);
-  if constexpr (kShareRecip)
-    cmx = sqrt(cmx), cmy = sqrt(cmy);
+  const R cmx = fmax4(cFastLLx, cFastLRx, cFastRLx, cFastRRx), cmy = fmax4(cFastLLy, cFastLRy, cFastRLy, cFastRRy);
   const R SL = fmin4(uLL, uLR, uRL, uRR) - cmx;
   const R SR = fmax4(uLL, uLR, uRL, uRR) + cmx;
   const R SB = fmin4(vLL, vLR, vRL, vRR) - cmy;
@@ -845,15 +999,11 @@ mag_riemann2d_hlld(const EdgeQ<R> & LL, const EdgeQ<R> & RL, const EdgeQ<R> & LR
     (rcLLy * vLL + rcLRy * vLR + rcRLy * vRL + rcRRy * vRR + (PtotLL - PtotLR + PtotRL - PtotRR)) /
     (rcLLy + rcLRy + rcRLy + rcRRy);
 
-  // quotients by the six shared denominators: divided in the exact build (the
-  // reference's expressions), one reciprocal each in the FMA build
   const R dSLu = SL - ustar, dSRu = SR - ustar, dSBv = SB - vstar, dSTv = ST - vstar;
-  const R iSLu = kShareRecip ? R(1) / dSLu : R(0), iSRu = kShareRecip ? R(1) / dSRu : R(0);
-  const R iSBv = kShareRecip ? R(1) / dSBv : R(0), iSTv = kShareRecip ? R(1) / dSTv : R(0);
-  auto q_SLu = [&](R x) { return kShareRecip ? x * iSLu : x / dSLu; };
-  auto q_SRu = [&](R x) { return kShareRecip ? x * iSRu : x / dSRu; };
-  auto q_SBv = [&](R x) { return kShareRecip ? x * iSBv : x / dSBv; };
-  auto q_STv = [&](R x) { return kShareRecip ? x * iSTv : x / dSTv; };
+  auto q_SLu = [&](R x) { return x / dSLu; };
+  auto q_SRu = [&](R x) { return x / dSRu; };
+  auto q_SBv = [&](R x) { return x / dSBv; };
+  auto q_STv = [&](R x) { return x / dSTv; };
   const R rstarLLx = q_SLu(rLL * (SL - uLL));
   const R BstarLL = q_SLu(bLL * (SL - uLL));
   const R rstarLLy = q_SBv(rLL * (SB - vLL));
@@ -890,9 +1040,7 @@ mag_riemann2d_hlld(const EdgeQ<R> & LL, const EdgeQ<R> & RL, const EdgeQ<R> & LR
   const R EstarRRy = uRR * bRR - vstar * AstarRR;
   const R EstarRR = ustar * BstarRR - vstar * AstarRR;
 
-  // |B| / sqrt(rho*): the reference's quotient in the exact build; one
-  // reciprocal square root (CUDA's rsqrt) in the FMA build
-  auto b_over_sqrt = [](R b, R r) { return kShareRecip ? fabs(b) * rsqrt(r) : fabs(b) / sqrt(r); };
+  auto b_over_sqrt = [](R b, R r) { return fabs(b) / sqrt(r); };
   const R calfvenL = fmax5(b_over_sqrt(aLR, rstarLRx), b_over_sqrt(AstarLR, rstarLR),
                            b_over_sqrt(aLL, rstarLLx), b_over_sqrt(AstarLL, rstarLL), smallc);
   const R calfvenR = fmax5(b_over_sqrt(aRR, rstarRRx), b_over_sqrt(AstarRR, rstarRR),
@@ -907,9 +1055,8 @@ mag_riemann2d_hlld(const EdgeQ<R> & LL, const EdgeQ<R> & RL, const EdgeQ<R> & LR
   const R SAB = fmin(vstar - calfvenB, R(0));
   const R SAT = fmax(vstar + calfvenT, R(0));
   const R dA = SAR - SAL, dB = SAT - SAB;
-  const R iA = kShareRecip ? R(1) / dA : R(0), iB = kShareRecip ? R(1) / dB : R(0);
-  auto q_A = [&](R x) { return kShareRecip ? x * iA : x / dA; };
-  auto q_B = [&](R x) { return kShareRecip ? x * iB : x / dB; };
+  auto q_A = [&](R x) { return x / dA; };
+  auto q_B = [&](R x) { return x / dB; };
 
   const R AstarT = q_A(SAR * AstarRR - SAL * AstarLR);
   const R AstarB = q_A(SAR * AstarRL - SAL * AstarLL);
@@ -964,14 +1111,16 @@ mhd_emf_corners(const EdgeCorner<R> & RT, const EdgeCorner<R> & RB, const EdgeCo
   LL.p = RT.p, RL.p = LT.p, LR.p = RB.p, RR.p = LB.p;
   LL.u = RT.u, RL.u = LT.u, LR.u = RB.u, RR.u = LB.u;
   LL.v = RT.v, RL.v = LT.v, LR.v = RB.v, RR.v = LB.v;
-  LL.a = R(0.5) * (RT.a + LT.a);
-  RL.a = R(0.5) * (RT.a + LT.a);
-  LR.a = R(0.5) * (RB.a + LB.a);
-  RR.a = R(0.5) * (RB.a + LB.a);
-  LL.b = R(0.5) * (RT.b + RB.b);
-  RL.b = R(0.5) * (LT.b + LB.b);
-  LR.b = R(0.5) * (RT.b + RB.b);
-  RR.b = R(0.5) * (LT.b + LB.b);
+  auto half = [](R x) {
+    if constexpr (kFast64<R>)
+      return scale_down64<1>(x);
+    else
+      return R(0.5) * x;
+  };
+  LL.a = RL.a = half(RT.a + LT.a);
+  LR.a = RR.a = half(RB.a + LB.a);
+  LL.b = LR.b = half(RT.b + RB.b);
+  RL.b = RR.b = half(LT.b + LB.b);
   LL.c = RT.c, RL.c = LT.c, LR.c = RB.c, RR.c = LB.c;
   const R ELL = LL.u * LL.b - LL.v * LL.a;
   const R ERL = RL.u * RL.b - RL.v * RL.a;
@@ -1004,6 +1153,12 @@ template <class R>
 __device__ __forceinline__ void
 floor_state(R (&q)[8], R smallr, R smallp)
 {
+  if constexpr (kFast64<R>)
+  {
+    q[ID] = max_floor64(q[ID], smallr);
+    q[IP] = max_floor64(q[IP], smallp);
+    return;
+  }
   q[ID] = fmax(smallr, q[ID]);
   q[IP] = fmax(smallp, q[IP]);
 }
@@ -1131,8 +1286,16 @@ edge_corner_acc(const ACC & T, int d, int p1, int p2, R smallr, R smallp)
   auto sg2 = [](R x) { return S2 > 0 ? x : -x; };
   auto hyd = [&](int f) { return T(f) + (sg1(T(t_hslope(p1, f))) + sg2(T(t_hslope(p2, f)))); };
   EdgeCorner<R> e;
-  e.r = fmax(smallr, hyd(T_R));
-  e.p = fmax(smallp, hyd(T_P));
+  if constexpr (kFast64<R>)
+  {
+    e.r = max_floor64(hyd(T_R), smallr);
+    e.p = max_floor64(hyd(T_P), smallp);
+  }
+  else
+  {
+    e.r = fmax(smallr, hyd(T_R));
+    e.p = fmax(smallp, hyd(T_P));
+  }
   e.u = hyd(T_U + p1);
   e.v = hyd(T_U + p2);
   e.a = T(t_bface(p1, S1 > 0)) + sg2(T(t_bfslope(p1, S1 > 0, p2)));

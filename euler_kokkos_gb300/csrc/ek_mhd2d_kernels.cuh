@@ -40,6 +40,12 @@ template <class R>
 __device__ __forceinline__ void
 floor2d(R & r, R & p, R smallr, R smallp)
 {
+  if constexpr (kFast64<R>)
+  {
+    r = max_floor64(r, smallr);
+    p = floor_ratio64(p, r, smallp);
+    return;
+  }
   r = fmax(smallr, r);
   p = fmax(smallp * r, p);
 }
@@ -150,14 +156,12 @@ mhd2d_dt_kernel(const void * __restrict__ U, KParams P, DevClock * clk, int step
       cfy = sqrt_a(d2 + sqrt_a(d2 * d2 - cr * b * b));
       tmax = fmax(tmax, (cfx + fabsf(q[IU])) * P.idx + (cfy + fabsf(q[IV])) * P.idy);
     }
-    else if constexpr (kShareRecip)
+    else if constexpr (kFast64<R>)
     {
-      // FP64 FMA build: one reciprocal of the density, host-prepared 1/dx
-      const R id = R(1) / d, c2 = C.gamma0 * p * id;
-      const R d2 = R(0.5) * (b2 * id + c2), cr = c2 * id;
-      cfx = sqrt(d2 + sqrt(d2 * d2 - cr * a * a));
-      cfy = sqrt(d2 + sqrt(d2 * d2 - cr * b * b));
-      tmax = fmax(tmax, (cfx + fabs(q[IU])) * P.idxd + (cfy + fabs(q[IV])) * P.idyd);
+      // FP64 FMA build: host-prepared 1/dx
+      cfx = sqrt_ratio64(fast_num64(C.gamma0 * p, b2, a * a), d);
+      cfy = sqrt_ratio64(fast_num64(C.gamma0 * p, b2, b * b), d);
+      tmax = max_cand(tmax, (cfx + fabs(q[IU])) * P.idxd + (cfy + fabs(q[IV])) * P.idyd);
     }
     else
     {
@@ -220,10 +224,12 @@ trace2d_compact(const R * sQ, const R * sB, int qx, int qy, int bx, int by, R dt
     for (int dj = 0; dj < 2; ++dj)
     {
       const int x0 = qx + di - 1, y0 = qy + dj - 1;
-      const R   u = R(0.25) * (Qv(IU, x0, y0) + Qv(IU, x0, y0 + 1) + Qv(IU, x0 + 1, y0) + Qv(IU, x0 + 1, y0 + 1));
-      const R   v = R(0.25) * (Qv(IV, x0, y0) + Qv(IV, x0, y0 + 1) + Qv(IV, x0 + 1, y0) + Qv(IV, x0 + 1, y0 + 1));
-      const R   A = R(0.5) * (Bv(0, bx + di, by + dj - 1) + Bv(0, bx + di, by + dj));
-      const R   B = R(0.5) * (Bv(1, bx + di - 1, by + dj) + Bv(1, bx + di, by + dj));
+      // FP64 FMA build: 8 E from the sums (the factor goes into dt/dx below)
+      const R   quarter = kFast64<R> ? R(1) : R(0.25), half = kFast64<R> ? R(1) : R(0.5);
+      const R   u = quarter * (Qv(IU, x0, y0) + Qv(IU, x0, y0 + 1) + Qv(IU, x0 + 1, y0) + Qv(IU, x0 + 1, y0 + 1));
+      const R   v = quarter * (Qv(IV, x0, y0) + Qv(IV, x0, y0 + 1) + Qv(IV, x0 + 1, y0) + Qv(IV, x0 + 1, y0 + 1));
+      const R   A = half * (Bv(0, bx + di, by + dj - 1) + Bv(0, bx + di, by + dj));
+      const R   B = half * (Bv(1, bx + di - 1, by + dj) + Bv(1, bx + di, by + dj));
       Ez[di][dj] = u * B - v * A;
     }
   const R ELL = Ez[0][0], ELR = Ez[0][1], ERL = Ez[1][0], ERR = Ez[1][1];
@@ -241,62 +247,90 @@ trace2d_compact(const R * sQ, const R * sB, int qx, int qy, int bx, int by, R dt
 #pragma unroll
   for (int vv = 0; vv < 8; ++vv)
   {
-    dqx[vv] = slope1<R>(q[vv], Qv(vv, qx + 1, qy), Qv(vv, qx - 1, qy), st);
-    dqy[vv] = slope1<R>(q[vv], Qv(vv, qx, qy + 1), Qv(vv, qx, qy - 1), st);
+    dqx[vv] = slope_h<R>(q[vv], Qv(vv, qx + 1, qy), Qv(vv, qx - 1, qy), st);
+    dqy[vv] = slope_h<R>(q[vv], Qv(vv, qx, qy + 1), Qv(vv, qx, qy - 1), st);
   }
-  const R drx = dqx[ID] * R(0.5), dpx = dqx[IP] * R(0.5), dux = dqx[IU] * R(0.5), dvx = dqx[IV] * R(0.5),
-          dwx = dqx[IW] * R(0.5), dCx = dqx[IC] * R(0.5), dBx = dqx[IB] * R(0.5);
-  const R dry = dqy[ID] * R(0.5), dpy = dqy[IP] * R(0.5), duy = dqy[IU] * R(0.5), dvy = dqy[IV] * R(0.5),
-          dwy = dqy[IW] * R(0.5), dCy = dqy[IC] * R(0.5), dAy = dqy[IA] * R(0.5);
+  // half slopes (the FP64 FMA build's slope_h returns them)
+  const R hs = kFast64<R> ? R(1) : R(0.5);
+  const R drx = dqx[ID] * hs, dpx = dqx[IP] * hs, dux = dqx[IU] * hs, dvx = dqx[IV] * hs,
+          dwx = dqx[IW] * hs, dCx = dqx[IC] * hs, dBx = dqx[IB] * hs;
+  const R dry = dqy[ID] * hs, dpy = dqy[IP] * hs, duy = dqy[IU] * hs, dvy = dqy[IV] * hs,
+          dwy = dqy[IW] * hs, dCy = dqy[IC] * hs, dAy = dqy[IA] * hs;
 
   // transverse face-field slopes (slope_unsplit_mhd_2d, MHDBaseFunctor2D.h:455-518)
-  const R dALy = R(0.5) * slope1<R>(Bv(0, bx, by), Bv(0, bx, by + 1), Bv(0, bx, by - 1), st);
-  const R dBLx = R(0.5) * slope1<R>(Bv(1, bx, by), Bv(1, bx + 1, by), Bv(1, bx - 1, by), st);
-  const R dARy = R(0.5) * slope1<R>(Bv(0, bx + 1, by), Bv(0, bx + 1, by + 1), Bv(0, bx + 1, by - 1), st);
-  const R dBRx = R(0.5) * slope1<R>(Bv(1, bx, by + 1), Bv(1, bx + 1, by + 1), Bv(1, bx - 1, by + 1), st);
+  const R dALy = hs * slope_h<R>(Bv(0, bx, by), Bv(0, bx, by + 1), Bv(0, bx, by - 1), st);
+  const R dBLx = hs * slope_h<R>(Bv(1, bx, by), Bv(1, bx + 1, by), Bv(1, bx - 1, by), st);
+  const R dARy = hs * slope_h<R>(Bv(0, bx + 1, by), Bv(0, bx + 1, by + 1), Bv(0, bx + 1, by - 1), st);
+  const R dBRx = hs * slope_h<R>(Bv(1, bx, by + 1), Bv(1, bx + 1, by + 1), Bv(1, bx - 1, by + 1), st);
 
-  const R dAx = R(0.5) * (AR - AL);
-  const R dBy = R(0.5) * (BR - BL);
+  R dAx, dBy;
+  if constexpr (kFast64<R>)
+    dAx = scale_down64<1>(AR - AL), dBy = scale_down64<1>(BR - BL);
+  else
+    dAx = R(0.5) * (AR - AL), dBy = R(0.5) * (BR - BL);
   const R gamma = C.gamma0;
 
-  // source terms (MHDBaseFunctor2D.h:969-995)
-  R su0, sv0, sw0;
-  if constexpr (sizeof(R) == 4)
+  // source terms (MHDBaseFunctor2D.h:969-995) and the advanced state
+  R o[V_N];
+  if constexpr (kFast64<R>)
   {
-    const float ir = rcp_a(r);
-    su0 = (-u * dux - dpx * ir - B * dBx * ir - Cc * dCx * ir) * dtdx + (-v * duy + B * dAy * ir) * dtdy;
-    sv0 = (-u * dvx + A * dBx * ir) * dtdx + (-v * dvy - dpy * ir - A * dAy * ir - Cc * dCy * ir) * dtdy;
-    sw0 = (-u * dwx + A * dCx * ir) * dtdx + (-v * dwy + B * dCy * ir) * dtdy;
+    // FP64 FMA build: FMA chains onto the state, B / rho once
+    const R ir = rcp64(r), Ai = A * ir, Bi = B * ir, Ci = Cc * ir, gp = gamma * p;
+    auto    adv = [&](R q0, R fx, R fy) { return fma(-fy, dtdy, fma(-fx, dtdx, q0)); };
+    o[V_R] = adv(r, fma(u, drx, dux * r), fma(v, dry, dvy * r));
+    o[V_P] = adv(p, fma(u, dpx, dux * gp), fma(v, dpy, dvy * gp));
+    o[V_U] = adv(u, fma(u, dux, fma(ir, dpx, fma(Bi, dBx, Ci * dCx))), fma(v, duy, -(Bi * dAy)));
+    o[V_V] = adv(v, fma(u, dvx, -(Ai * dBx)), fma(v, dvy, fma(ir, dpy, fma(Ai, dAy, Ci * dCy))));
+    o[V_W] = adv(w, fma(u, dwx, -(Ai * dCx)), fma(v, dwy, -(Bi * dCy)));
+    o[V_A] = fma(fma(u, dBy, fma(B, duy, fma(-v, dAy, -(A * dvy)))), dtdy, A);
+    o[V_B] = fma(fma(v, dAx, fma(A, dvx, fma(-u, dBx, -(B * dux)))), dtdx, B);
+    o[V_C] = fma(fma(w, dAx, fma(A, dwx, fma(-u, dCx, -(Cc * dux)))), dtdx,
+                 fma(fma(w, dBy, fma(B, dwy, fma(-v, dCy, -(Cc * dvy)))), dtdy, Cc));
+    const R ex = dtdx * R(0.0625), ey = dtdy * R(0.0625);
+    o[V_AL] = fma(ELR - ELL, ey, AL);
+    o[V_AR] = fma(ERR - ERL, ey, AR);
+    o[V_BL] = fma(ELL - ERL, ex, BL);
+    o[V_BR] = fma(ELR - ERR, ex, BR);
   }
   else
   {
-    su0 = (-u * dux - dpx / r - B * dBx / r - Cc * dCx / r) * dtdx + (-v * duy + B * dAy / r) * dtdy;
-    sv0 = (-u * dvx + A * dBx / r) * dtdx + (-v * dvy - dpy / r - A * dAy / r - Cc * dCy / r) * dtdy;
-    sw0 = (-u * dwx + A * dCx / r) * dtdx + (-v * dwy + B * dCy / r) * dtdy;
-  }
-  const R sr0 = (-u * drx - dux * r) * dtdx + (-v * dry - dvy * r) * dtdy;
-  const R sp0 = (-u * dpx - dux * gamma * p) * dtdx + (-v * dpy - dvy * gamma * p) * dtdy;
-  const R sA0 = (u * dBy + B * duy - v * dAy - A * dvy) * dtdy;
-  const R sB0 = (-u * dBx - B * dux + v * dAx + A * dvx) * dtdx;
-  const R sC0 = (w * dAx + A * dwx - u * dCx - Cc * dux) * dtdx + (-v * dCy - Cc * dvy + w * dBy + B * dwy) * dtdy;
-  const R sAL0 = +(ELR - ELL) * R(0.5) * dtdy;
-  const R sAR0 = +(ERR - ERL) * R(0.5) * dtdy;
-  const R sBL0 = -(ERL - ELL) * R(0.5) * dtdx;
-  const R sBR0 = -(ERR - ELR) * R(0.5) * dtdx;
+    R su0, sv0, sw0;
+    if constexpr (sizeof(R) == 4)
+    {
+      const float ir = rcp_a(r);
+      su0 = (-u * dux - dpx * ir - B * dBx * ir - Cc * dCx * ir) * dtdx + (-v * duy + B * dAy * ir) * dtdy;
+      sv0 = (-u * dvx + A * dBx * ir) * dtdx + (-v * dvy - dpy * ir - A * dAy * ir - Cc * dCy * ir) * dtdy;
+      sw0 = (-u * dwx + A * dCx * ir) * dtdx + (-v * dwy + B * dCy * ir) * dtdy;
+    }
+    else
+    {
+      su0 = (-u * dux - dpx / r - B * dBx / r - Cc * dCx / r) * dtdx + (-v * duy + B * dAy / r) * dtdy;
+      sv0 = (-u * dvx + A * dBx / r) * dtdx + (-v * dvy - dpy / r - A * dAy / r - Cc * dCy / r) * dtdy;
+      sw0 = (-u * dwx + A * dCx / r) * dtdx + (-v * dwy + B * dCy / r) * dtdy;
+    }
+    const R sr0 = (-u * drx - dux * r) * dtdx + (-v * dry - dvy * r) * dtdy;
+    const R sp0 = (-u * dpx - dux * gamma * p) * dtdx + (-v * dpy - dvy * gamma * p) * dtdy;
+    const R sA0 = (u * dBy + B * duy - v * dAy - A * dvy) * dtdy;
+    const R sB0 = (-u * dBx - B * dux + v * dAx + A * dvx) * dtdx;
+    const R sC0 = (w * dAx + A * dwx - u * dCx - Cc * dux) * dtdx + (-v * dCy - Cc * dvy + w * dBy + B * dwy) * dtdy;
+    const R sAL0 = +(ELR - ELL) * R(0.5) * dtdy;
+    const R sAR0 = +(ERR - ERL) * R(0.5) * dtdy;
+    const R sBL0 = -(ERL - ELL) * R(0.5) * dtdx;
+    const R sBR0 = -(ERR - ELR) * R(0.5) * dtdx;
 
-  R o[V_N];
-  o[V_R] = r + sr0;
-  o[V_U] = u + su0;
-  o[V_V] = v + sv0;
-  o[V_W] = w + sw0;
-  o[V_P] = p + sp0;
-  o[V_A] = A + sA0;
-  o[V_B] = B + sB0;
-  o[V_C] = Cc + sC0;
-  o[V_AL] = AL + sAL0;
-  o[V_AR] = AR + sAR0;
-  o[V_BL] = BL + sBL0;
-  o[V_BR] = BR + sBR0;
+    o[V_R] = r + sr0;
+    o[V_U] = u + su0;
+    o[V_V] = v + sv0;
+    o[V_W] = w + sw0;
+    o[V_P] = p + sp0;
+    o[V_A] = A + sA0;
+    o[V_B] = B + sB0;
+    o[V_C] = Cc + sC0;
+    o[V_AL] = AL + sAL0;
+    o[V_AR] = AR + sAR0;
+    o[V_BL] = BL + sBL0;
+    o[V_BR] = BR + sBR0;
+  }
   o[V_DRX] = drx, o[V_DPX] = dpx, o[V_DUX] = dux, o[V_DVX] = dvx, o[V_DWX] = dwx, o[V_DCX] = dCx, o[V_DBX] = dBx;
   o[V_DRY] = dry, o[V_DPY] = dpy, o[V_DUY] = duy, o[V_DVY] = dvy, o[V_DWY] = dwy, o[V_DCY] = dCy, o[V_DAY] = dAy;
   o[V_DALY] = dALy, o[V_DBLX] = dBLx, o[V_DARY] = dARy, o[V_DBRX] = dBRx;
@@ -400,7 +434,7 @@ mhd2d_tile(const void * __restrict__ Uin, void * __restrict__ Uout, const KParam
     R ql[8], qr[8], fl[6];
     face2d_state<R, true>(TS(i - (d == 0), j - (d == 1)), T::PL, d, ql, sr, sp);
     face2d_state<R, false>(TS(i, j), T::PL, d, qr, sr, sp);
-    if (!mhd_riemann<RS, R, 6>(ql, qr, fl, C.gamma0))
+    if (!mhd_riemann<RS, R, 6>(ql, qr, fl, C))
     {
       // ill-conditioned star state in FP32 (mixed HLLD only)
       if constexpr (REPAIR)
