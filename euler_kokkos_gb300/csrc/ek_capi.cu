@@ -14,6 +14,7 @@
 #include <cuda_runtime.h>
 
 #include "../../include/ek_gb300.h"
+#include "ek_chunk.h"
 #include "ek_internal.h"
 #include "ek_launch.h"
 
@@ -28,11 +29,6 @@ fail(ek_status s, const std::string & msg)
   return s;
 }
 } // namespace ek_internal
-
-// planes per CTA column of the 3D kernels when the parameters leave it at 0
-#ifndef EK_KCHUNK_DEFAULT
-#define EK_KCHUNK_DEFAULT 32
-#endif
 
 using ek_internal::fail;
 using KParams = ekc::KParams;
@@ -215,6 +211,44 @@ validate(const ek_params & p)
   return EK_OK;
 }
 
+int
+sm_count()
+{
+  static int sms_of[64] = {};
+  int        dev = 0, sms = 0;
+  if (cudaGetDevice(&dev) == cudaSuccess && dev >= 0 && dev < 64)
+  {
+    sms = __atomic_load_n(&sms_of[dev], __ATOMIC_RELAXED);
+    if (sms == 0 && cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) == cudaSuccess)
+      __atomic_store_n(&sms_of[dev], sms, __ATOMIC_RELAXED);
+  }
+  return sms > 0 ? sms : 1;
+}
+
+// planes per CTA of the 3D kernels: the caller's (kchunk > 0), else by the
+// grid's tiles and the device's SMs
+static void
+set_chunks(const ek_params & p, ekc::KParams & k)
+{
+  k.kchunk = k.kchunk_trace = p.kchunk > 0 ? p.kchunk : 1;
+  if (p.kchunk > 0 || p.dim == 2)
+    return;
+  const int  sms = sm_count();
+  const bool f64 = p.precision == EK_PREC_FP64;
+  auto       tiles = [](int nx, int ny, int tx, int ty) { return (long long)((nx + tx - 1) / tx) * ((ny + ty - 1) / ty); };
+  if (!p.mhd)
+  {
+    k.kchunk = ekc::choose_chunk(tiles(k.nx, k.ny, EK_H3_TX, EK_H3_TY), k.nz, sms,
+                                 f64 ? ekc::kChunkHydro64 : ekc::kChunkHydro32);
+    return;
+  }
+  k.kchunk = f64 ? ekc::choose_chunk(tiles(k.nx, k.ny, EK_MU_TX_F64, EK_MU_TY_F64), k.nz, sms, ekc::kChunkUpdate64)
+                 : ekc::choose_chunk(tiles(k.nx, k.ny, EK_MU_TX, EK_MU_TY), k.nz, sms, ekc::kChunkUpdate32);
+  k.kchunk_trace = ekc::choose_chunk(f64 ? tiles(k.nx + 2, k.ny + 2, EK_MT_TX_F64, EK_MT_TY_F64)
+                                         : tiles(k.nx + 2, k.ny + 2, EK_MT_TX, EK_MT_TY),
+                                     k.nz + 2, sms, f64 ? ekc::kChunkTrace64 : ekc::kChunkTrace32);
+}
+
 ekc::KParams
 make_kparams(const ek_params & p)
 {
@@ -245,7 +279,7 @@ make_kparams(const ek_params & p)
   k.tEnd = p.tEnd;
   k.cIso = p.cIso;
   k.riemann = p.riemann;
-  k.kchunk = p.kchunk > 0 ? p.kchunk : (k.nz <= EK_KCHUNK_DEFAULT ? k.nz : EK_KCHUNK_DEFAULT);
+  set_chunks(p, k);
   k.gamma0f = (float)p.gamma0;
   k.smallrf = (float)p.smallr;
   k.smallcf = (float)p.smallc;

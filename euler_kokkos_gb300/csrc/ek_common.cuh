@@ -53,7 +53,8 @@ struct KParams
   double    dx, dy, dz;
   double    gamma0, smallr, smallc, smallp, slope_type, cfl, tEnd, cIso;
   int       riemann;
-  int       kchunk; // interior planes per CTA (3D kernels)
+  int       kchunk;       // interior planes per CTA (3D kernels)
+  int       kchunk_trace; // trace planes per CTA (3D MHD trace kernel)
   // FP32 copies prepared on the host, so that mixed kernels do no per-thread
   // FP64 arithmetic (one FP64 instruction costs 64 FP32 ones on GB300)
   float     gamma0f, smallrf, smallcf, smallpf, slopef;
@@ -193,7 +194,7 @@ using namespace ekc;
 #define EK_MU_MINB_F32 8
 #endif
 #ifndef EK_MU_MINB_F64
-#define EK_MU_MINB_F64 1
+#define EK_MU_MINB_F64 2
 #endif
 #ifndef EK_M2_MINB_F32
 #define EK_M2_MINB_F32 0
@@ -227,6 +228,24 @@ using namespace ekc;
 #endif
 #ifndef EK_MU_TY
 #define EK_MU_TY 8
+#endif
+// The FP64 MHD kernels: bound by the FP64 pipe they gain nothing from longer
+// rows, and smaller tiles fill the SMs of small grids and balance the others.
+// Best times over the planes per CTA (us): update 32 x 8 / 16 x 8: 242 / 242 at
+// 32^3, 675 / 536 at 48^3, 1272 / 1282 at 64^3, 2437 / 2440 at 96 x 80 x 70 (256
+// threads on a 16 x 8 tile: 211, 527, 1327, 2502); trace 16 x 8 / 8 x 8: 89 / 72
+// at 32^3, 398 / 361 at 64^3, 999 / 1003 at 96^3.
+#ifndef EK_MU_TX_F64
+#define EK_MU_TX_F64 16
+#endif
+#ifndef EK_MU_TY_F64
+#define EK_MU_TY_F64 8
+#endif
+#ifndef EK_MT_TX_F64
+#define EK_MT_TX_F64 8
+#endif
+#ifndef EK_MT_TY_F64
+#define EK_MT_TY_F64 8
 #endif
 #ifndef EK_M2_TX
 #define EK_M2_TX 16

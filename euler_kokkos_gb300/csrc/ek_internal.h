@@ -12,6 +12,8 @@ namespace ek_internal
 ek_status fail(ek_status s, const std::string & msg);
 // parameter checks shared by the single solver and the ensemble
 ek_status validate(const ek_params & p);
+// SMs of the current device (looked up once per device)
+int sm_count();
 // kernel parameters of a run
 ekc::KParams make_kparams(const ek_params & p);
 // device bytes of one state in the run's precision

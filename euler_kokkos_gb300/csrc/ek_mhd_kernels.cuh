@@ -460,8 +460,8 @@ mhd_trace_kernel(const void * __restrict__ U, R * __restrict__ trace, KParams P,
   const int gw = P.gw;
   // trace cells span global [gw-1, n+gw] in each direction
   const int c0 = gw - 1 + blockIdx.x * TX, d0 = gw - 1 + blockIdx.y * TY;
-  const int k0 = gw - 1 + blockIdx.z * P.kchunk;
-  const int k1 = min(k0 + P.kchunk, P.nz + gw + 1);
+  const int k0 = gw - 1 + blockIdx.z * P.kchunk_trace;
+  const int k1 = min(k0 + P.kchunk_trace, P.nz + gw + 1);
   const int nti = P.nx + 2, ntj = P.ny + 2; // trace cells per row / column
   // planes whose gathered x/y window [c0-1, c0+TX+1] x [d0-1, d0+TY+1] lies in
   // the interior need no boundary mapping: plain offsets, no sign flips
@@ -1189,8 +1189,15 @@ mhd_update_smem(int TX, int TY, bool stage)
                       2 * (TX + 1) * (TY + 1) + 2 * (TX + 1) * TY + 2 * TX * (TY + 1));
 }
 
-constexpr int MT_TX = EK_MT_TX, MT_TY = EK_MT_TY; // trace tile
-constexpr int MU_TX = EK_MU_TX, MU_TY = EK_MU_TY; // update tile
+constexpr int MU_TX = EK_MU_TX, MU_TY = EK_MU_TY; // update tile of the mixed form and its repair list
+template <class R>
+constexpr int kMuTX = sizeof(R) == 8 ? EK_MU_TX_F64 : MU_TX;
+template <class R>
+constexpr int kMuTY = sizeof(R) == 8 ? EK_MU_TY_F64 : MU_TY;
+template <class R>
+constexpr int kMtTX = sizeof(R) == 8 ? EK_MT_TX_F64 : EK_MT_TX;
+template <class R>
+constexpr int kMtTY = sizeof(R) == 8 ? EK_MT_TY_F64 : EK_MT_TY;
 
 // bytes of the compact trace in the work buffer (256-byte rounded)
 inline size_t
@@ -1247,14 +1254,15 @@ mhd_step_t(int phase, const void * Uin, void * Uout, void * work, const KParams 
   // 2. trace
   if (phase == 1)
   {
-    auto       k = mhd_trace_kernel<S, R, MT_TX, MT_TY>;
-    const int  sm = (int)mhd_trace_smem<S, R>(MT_TX, MT_TY);
+    constexpr int TX = kMtTX<R>, TY = kMtTY<R>;
+    auto          k = mhd_trace_kernel<S, R, TX, TY>;
+    const int     sm = (int)mhd_trace_smem<S, R>(TX, TY);
     cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, sm);
     if (e != cudaSuccess)
       return e;
     const int nt = P.nz + 2;
-    dim3      grid((P.nx + 2 + MT_TX - 1) / MT_TX, (P.ny + 2 + MT_TY - 1) / MT_TY, (nt + P.kchunk - 1) / P.kchunk);
-    k<<<grid, MT_TX * MT_TY, sm, st>>>(Uin, mhd_trace_of<R>(work, P), P, clk, step);
+    dim3      grid((P.nx + 2 + TX - 1) / TX, (P.ny + 2 + TY - 1) / TY, (nt + P.kchunk_trace - 1) / P.kchunk_trace);
+    k<<<grid, TX * TY, sm, st>>>(Uin, mhd_trace_of<R>(work, P), P, clk, step);
     return cudaGetLastError();
   }
   // 4. the repair pass of the mixed HLLD form (after phase 2)
@@ -1280,17 +1288,18 @@ mhd_step_t(int phase, const void * Uin, void * Uout, void * work, const KParams 
   //    for the HLLD solver); the face Riemann solver is a template parameter;
   //    the mixed HLLD form lists tiles for phase 3, which must follow
   {
-    auto k = P.riemann == 1   ? mhd_update_kernel<S, R, MU_TX, MU_TY, false, 1>
-             : P.riemann == 2 ? mhd_update_kernel<S, R, MU_TX, MU_TY, false, 2>
-             : P.mhd_stage    ? mhd_update_kernel<S, R, MU_TX, MU_TY, true, 4>
-                              : mhd_update_kernel<S, R, MU_TX, MU_TY, false, 4>;
-    const int  sm = (int)mhd_update_smem<R>(MU_TX, MU_TY, P.mhd_stage != 0 && P.riemann == 4);
+    constexpr int TX = kMuTX<R>, TY = kMuTY<R>;
+    auto k = P.riemann == 1   ? mhd_update_kernel<S, R, TX, TY, false, 1>
+             : P.riemann == 2 ? mhd_update_kernel<S, R, TX, TY, false, 2>
+             : P.mhd_stage    ? mhd_update_kernel<S, R, TX, TY, true, 4>
+                              : mhd_update_kernel<S, R, TX, TY, false, 4>;
+    const int  sm = (int)mhd_update_smem<R>(TX, TY, P.mhd_stage != 0 && P.riemann == 4);
     cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, sm);
     if (e != cudaSuccess)
       return e;
-    dim3 grid((P.nx + MU_TX - 1) / MU_TX, (P.ny + MU_TY - 1) / MU_TY, (P.nz + P.kchunk - 1) / P.kchunk);
+    dim3 grid((P.nx + TX - 1) / TX, (P.ny + TY - 1) / TY, (P.nz + P.kchunk - 1) / P.kchunk);
     int * repair = sizeof(R) == 4 && P.riemann == 4 ? (int *)work : nullptr;
-    k<<<grid, MU_TX * MU_TY, sm, st>>>(Uin, Uout, mhd_trace_of<R>(work, P), P, clk, step, cfl_next ? 1 : 0, repair);
+    k<<<grid, TX * TY, sm, st>>>(Uin, Uout, mhd_trace_of<R>(work, P), P, clk, step, cfl_next ? 1 : 0, repair);
     return cudaGetLastError();
   }
 }

@@ -1,9 +1,8 @@
-"""Tuning of the step kernels: tile shapes, resident CTAs per SM, planes per
-CTA column.
+"""Tuning of the step kernels: tile shapes and resident CTAs per SM.
 
 The tile shapes and register budgets are compile-time parameters of the CUDA
 kernels (EK_*_TX/TY and EK_*_MINB_* in csrc/ek_common.cuh); the planes per CTA
-column of the 3D kernels is a run-time parameter.  ``python -m
+of the 3D kernels follow from the grid (csrc/ek_chunk.h).  ``python -m
 euler_kokkos_gb300.tuning`` builds the library once per candidate set into
 ``_build/tune/<i>/``, times every kernel family on its workload through the C
 ABI (CUDA events around each launch: ek_solver_set_profiling /
@@ -12,7 +11,7 @@ the choice to ``tuning.json`` beside this file, which build() turns into -D
 flags.  The workloads are the benchmark's sizes (3D blast and Orszag-Tang
 256^3, 2D Orszag-Tang 4096^2, the 512-instance Kelvin-Helmholtz ensemble):
 the best tile depends on the grid.  The objective is the mixed-precision (FP32) kernel time, the
-performance form; the FP64 build uses the same shapes.  Run it on the GPU it
+performance form; the FP64 MHD kernels have shapes of their own (EK_*_F64).  Run it on the GPU it
 tunes for; it needs nvcc and a few minutes.
 """
 
@@ -54,7 +53,6 @@ CANDIDATES = {
               {"EK_M2_TX": "16", "EK_M2_TY": "16", "EK_M2_MINB_F32": "3"},
               {"EK_M2_TX": "16", "EK_M2_TY": "16", "EK_M2_MINB_F32": "4"}],
 }
-KCHUNKS = (16, 32, 64)
 
 
 def load_flags():
@@ -63,10 +61,7 @@ def load_flags():
         return []
     with open(TUNING_FILE) as f:
         cfg = json.load(f)
-    flags = ["-D%s=%s" % (k, v) for k, v in sorted(cfg.get("flags", {}).items())]
-    if cfg.get("kchunk"):
-        flags.append("-DEK_KCHUNK_DEFAULT=%d" % int(cfg["kchunk"]))
-    return flags
+    return ["-D%s=%s" % (k, v) for k, v in sorted(cfg.get("flags", {}).items())]
 
 
 # ---------------------------------------------------------------------------
@@ -115,12 +110,11 @@ def measure(families):
         res["hydro2d"] = _ensemble_ms(ek, P)
     if "hydro3d" in families:
         ini, U0 = P.blast_3d(n=256, nsteps=10 ** 6)
-        res["hydro3d"] = {str(k): _kernel_ms(ek, ini, U0, [("step", 0)], 8, kchunk=k)["step"] for k in KCHUNKS}
+        res["hydro3d"] = _kernel_ms(ek, ini, U0, [("step", 0)], 8)["step"]
     if "mhd_trace" in families or "mhd_update" in families:
         ini, U0 = P.orszag_tang_3d(n=256, nsteps=10 ** 6)
-        r = {str(k): _kernel_ms(ek, ini, U0, [("update", 0), ("trace", 1)], 4, kchunk=k) for k in KCHUNKS}
-        res["mhd_trace"] = {k: v["trace"] for k, v in r.items()}
-        res["mhd_update"] = {k: v["update"] for k, v in r.items()}
+        r = _kernel_ms(ek, ini, U0, [("update", 0), ("trace", 1)], 4)
+        res["mhd_trace"], res["mhd_update"] = r["trace"], r["update"]
     if "mhd2d" in families:
         ini, U0 = P.orszag_tang_2d(n=4096, nsteps=10 ** 6)
         res["mhd2d"] = _kernel_ms(ek, ini, U0, [("step", 0)], 6)["step"]
@@ -166,24 +160,18 @@ def tune(parallel_builds=3):
             raise RuntimeError("variant %d failed to run:\n%s" % (i, r.stdout.decode(errors="replace")))
         results.append(json.loads(r.stdout.decode().strip().splitlines()[-1]))
         print("variant", i, json.dumps(results[-1]), flush=True)
-    # best candidate per family; the 3D families also pick the planes per column
-    flags, chosen, kchunk_score = {}, {}, {k: 0.0 for k in KCHUNKS}
+    # best candidate per family
+    flags, chosen = {}, {}
     for fam, cands in CANDIDATES.items():
         best = None
         for i in range(len(cands)):
-            v = results[i][fam]
-            t = min(x for x in v.values() if x) if isinstance(v, dict) else v
+            t = results[i][fam]
             if t and (best is None or t < best[0]):
                 best = (t, i)
         chosen[fam] = {"candidate": best[1], "ms": best[0], "flags": cands[best[1]],
                        "all_ms": [results[i][fam] for i in range(len(cands))]}
         flags.update(cands[best[1]])
-        v = results[best[1]][fam]
-        if isinstance(v, dict):
-            for k in KCHUNKS:
-                kchunk_score[k] += v[str(k)] or 1e30
-    kchunk = min(KCHUNKS, key=lambda k: kchunk_score[k])
-    cfg = {"flags": flags, "kchunk": kchunk, "families": chosen,
+    cfg = {"flags": flags, "families": chosen,
            "tuned_on": _gpu_name(), "date": time.strftime("%Y-%m-%d")}
     with open(TUNING_FILE, "w") as f:
         json.dump(cfg, f, indent=1, sort_keys=True)
