@@ -233,7 +233,7 @@ set_chunks(const ek_params & p, ekc::KParams & k)
   k.kchunk = k.kchunk_trace = p.kchunk > 0 ? p.kchunk : 1;
   if (p.kchunk > 0 || p.dim == 2)
     return;
-  const int  sms = sm_count();
+  const int  sms = k.sms;
   const bool f64 = p.precision == EK_PREC_FP64;
   auto       tiles = [](int nx, int ny, int tx, int ty) { return (long long)((nx + tx - 1) / tx) * ((ny + ty - 1) / ty); };
   if (!p.mhd)
@@ -279,6 +279,7 @@ make_kparams(const ek_params & p)
   k.tEnd = p.tEnd;
   k.cIso = p.cIso;
   k.riemann = p.riemann;
+  k.sms = sm_count();
   set_chunks(p, k);
   k.gamma0f = (float)p.gamma0;
   k.smallrf = (float)p.smallr;

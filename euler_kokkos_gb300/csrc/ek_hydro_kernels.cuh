@@ -49,12 +49,12 @@ hydro_const(const KParams & P)
 // boundary conditions.
 // When the whole (TX+4) x (TY+4) halo of the tile and plane gk lie inside the
 // interior (direct), the boundary mapping is the identity and is skipped.
-template <class S, class R, int NV, int TX, int TY>
+template <class S, class R, int NV, int TX, int TY, int NT = TX * TY>
 __device__ __forceinline__ void
 load_q_plane(const S * __restrict__ U, const KParams & P, const HydroConst<R> & C, int gi0, int gj0,
              int gk, R * sQ, bool direct = false)
 {
-  constexpr int HX = TX + 4, HY = TY + 4, NT = TX * TY;
+  constexpr int HX = TX + 4, HY = TY + 4;
   for (int c = threadIdx.x; c < HX * HY; c += NT)
   {
     const int hx = c % HX, hy = c / HX;
@@ -141,12 +141,14 @@ cell_slopes(const R * q0, const R * qm, const R * qp, int hx, int hy, R st, R (&
 // ensemble's prefetch); otherwise it is loaded here.
 // pre: the step scalars computed for the whole instance (the ensemble), else
 // thread 0 computes them for this CTA.
-template <class S, class R, int TX, int TY, int RS = 3, bool GRAV = false, bool LOADED = false>
+// NT threads: one per cell, or more (a multiple of 32 per part), so that the
+// ring cells run beside the interior ones and the faces take fewer rounds.
+template <class S, class R, int TX, int TY, int NT, int RS = 3, bool GRAV = false, bool LOADED = false>
 __device__ __forceinline__ void
 hydro2d_tile(const S * __restrict__ Uin, S * __restrict__ Uout, const KParams & P, DevClock * clk,
              int step, int bx, int by, unsigned char * smem_raw, const StepScalars<R> * pre = nullptr)
 {
-  constexpr int NV = 4, HX = TX + 4, HY = TY + 4, NT = TX * TY;
+  constexpr int NV = 4, HX = TX + 4, HY = TY + 4, CELLS = TX * TY;
   constexpr int FX = TX + 2; // face-state rows in x: cells -1..TX
   R * sQ = reinterpret_cast<R *>(smem_raw);  // [NV][HY][HX]
   R * sXm = sQ + NV * HY * HX;               // XMIN state of cells -1..TX, then x-flux
@@ -191,12 +193,13 @@ hydro2d_tile(const S * __restrict__ Uin, S * __restrict__ Uout, const KParams & 
   const int gi0 = P.gw + bx * TX, gj0 = P.gw + by * TY;
   if constexpr (!LOADED)
   {
-    load_q_plane<S, R, NV, TX, TY>(Uin, P, C, gi0, gj0, 0, sQ);
+    load_q_plane<S, R, NV, TX, TY, NT>(Uin, P, C, gi0, gj0, 0, sQ);
     __syncthreads();
   }
 
   const int tx = threadIdx.x % TX, ty = threadIdx.x / TX;
   // traces of the interior cell
+  if (NT == CELLS || threadIdx.x < CELLS)
   {
     R c[NV], dX[NV], dY[NV], dZ[NV], s[NV], f[NV];
     cell_slopes<R, NV, HX, HY>(sQ, sQ, sQ, tx + 2, ty + 2, C.slope_type, c, dX, dY, dZ, false);
@@ -232,7 +235,8 @@ hydro2d_tile(const S * __restrict__ Uin, S * __restrict__ Uout, const KParams & 
       sYp[(v * (TY + 2) + ty + 1) * TX + tx] = f[v];
   }
   // ring cells: only the face state facing the tile
-  for (int r = threadIdx.x; r < 2 * (TX + TY); r += NT)
+  constexpr int RING = 2 * (TX + TY), RT = NT > CELLS ? NT - CELLS : NT; // threads for them
+  for (int r = NT > CELLS ? (int)threadIdx.x - CELLS : (int)threadIdx.x; r >= 0 && r < RING; r += RT)
   {
     int cx, cy, kind; // kind 0: left (XMAX), 1: right (XMIN), 2: bottom (YMAX), 3: top (YMIN)
     if (r < TY)
@@ -280,54 +284,40 @@ hydro2d_tile(const S * __restrict__ Uin, S * __restrict__ Uout, const KParams & 
   }
   __syncthreads();
 
-  // fluxes: x-face i (left face of cell i) from XMAX(i-1), XMIN(i); stored
-  // scaled by dt/dx (flux_scaled) into the XMIN slot of cell i (HydroRunFunctors2D.h:653-661)
-  for (int fidx = threadIdx.x; fidx < (TX + 1) * TY; fidx += NT)
+  // fluxes: x-face i (left face of cell i) from XMAX(i-1), XMIN(i), y-faces
+  // likewise (IU and IV swapped around the solver, HydroRunFunctors2D.h:653-661,
+  // 741-758), as one work list; stored scaled by dt/dx (flux_scaled) into the
+  // MIN slot of cell i
+  constexpr int NFX = (TX + 1) * TY, NFY = TX * (TY + 1);
+  for (int fidx = threadIdx.x; fidx < NFX + NFY; fidx += NT)
   {
-    const int i = fidx % (TX + 1), j = fidx / (TX + 1);
-    R         ql[NV], qr[NV], fl[NV];
+    const bool ydir = fidx >= NFX;
+    const int  g = ydir ? fidx - NFX : fidx;
+    const int  i = ydir ? g % TX : g % (TX + 1), j = ydir ? g / TX : g / (TX + 1);
+    const R *  lsrc = ydir ? sYp + j * TX + i : sXp + j * FX + i;
+    R *        rsrc = ydir ? sYm + (j + 1) * TX + i : sXm + j * FX + i + 1;
+    const int  vs = ydir ? (TY + 2) * TX : TY * FX; // variable stride
+    // slot of the face frame's variable v
+    auto slot = [&](int v) { return (v < IU ? v : (ydir ? IU + IV - v : v)) * vs; };
+    R    ql[NV], qr[NV], fl[NV];
 #pragma unroll
     for (int v = 0; v < NV; ++v)
     {
-      ql[v] = sXp[(v * TY + j) * FX + i];
-      qr[v] = sXm[(v * TY + j) * FX + i + 1];
+      ql[v] = lsrc[slot(v)];
+      qr[v] = rsrc[slot(v)];
     }
     hydro_riemann<RS, R, NV>(ql, qr, fl, C);
+    const R dtd = ydir ? dtdy : dtdx;
 #pragma unroll
     for (int v = 0; v < NV; ++v)
-      sXm[(v * TY + j) * FX + i + 1] = flux_scaled(fl[v], dtdx);
-  }
-  // y-faces: swap IU/IV around the solver (HydroRunFunctors2D.h:741-758)
-  for (int fidx = threadIdx.x; fidx < TX * (TY + 1); fidx += NT)
-  {
-    const int i = fidx % TX, j = fidx / TX;
-    R         ql[NV], qr[NV], fl[NV];
-#pragma unroll
-    for (int v = 0; v < NV; ++v)
-    {
-      ql[v] = sYp[(v * (TY + 2) + j) * TX + i];
-      qr[v] = sYm[(v * (TY + 2) + j + 1) * TX + i];
-    }
-    R tmp = ql[IU];
-    ql[IU] = ql[IV];
-    ql[IV] = tmp;
-    tmp = qr[IU];
-    qr[IU] = qr[IV];
-    qr[IV] = tmp;
-    hydro_riemann<RS, R, NV>(ql, qr, fl, C);
-    tmp = fl[IU];
-    fl[IU] = fl[IV];
-    fl[IV] = tmp;
-#pragma unroll
-    for (int v = 0; v < NV; ++v)
-      sYm[(v * (TY + 2) + j + 1) * TX + i] = flux_scaled(fl[v], dtdy);
+      rsrc[slot(v)] = flux_scaled(fl[v], dtd);
   }
   __syncthreads();
 
   // update (UpdateFunctor2D, HydroRunFunctors2D.h:809-836), in its order
   const int gi = gi0 + tx, gj = gj0 + ty;
   R tmax = R(-INFINITY);
-  if (gi < P.nx + P.gw && gj < P.ny + P.gw)
+  if ((NT == CELLS || threadIdx.x < CELLS) && gi < P.nx + P.gw && gj < P.ny + P.gw)
   {
     const long long off = (long long)gj * P.isize + gi;
     R               u[NV], rho_old = R(0);
@@ -368,12 +358,12 @@ hydro2d_tile(const S * __restrict__ Uin, S * __restrict__ Uout, const KParams & 
     step_commit(clk, step, t, dt);
 }
 
-template <class S, class R, int TX, int TY, int RS, bool GRAV>
-__global__ void __launch_bounds__(TX * TY)
+template <class S, class R, int TX, int TY, int NT, int RS, bool GRAV>
+__global__ void __launch_bounds__(NT)
 hydro2d_step(const S * __restrict__ Uin, S * __restrict__ Uout, KParams P, DevClock * clk, int step)
 {
   extern __shared__ __align__(16) unsigned char smem_raw[];
-  hydro2d_tile<S, R, TX, TY, RS, GRAV>(Uin, Uout, P, clk, step, blockIdx.x, blockIdx.y, smem_raw);
+  hydro2d_tile<S, R, TX, TY, NT, RS, GRAV>(Uin, Uout, P, clk, step, blockIdx.x, blockIdx.y, smem_raw);
   finalize_step(clk, P, step + 1); // the next step's dt, once its CFL key is complete
 }
 
@@ -478,7 +468,7 @@ ensemble2d_step(const EnsInstance * __restrict__ insts, const EnsTile * __restri
     if (t + gridDim.x < ntiles)
       issue(t + gridDim.x);
     __syncthreads(); // the primitive plane is complete
-    hydro2d_tile<S, R, TX, TY, 3, false, true>((const S *)in.U[step % 2], (S *)in.U[(step + 1) % 2], in.P,
+    hydro2d_tile<S, R, TX, TY, TX * TY, 3, false, true>((const S *)in.U[step % 2], (S *)in.U[(step + 1) % 2], in.P,
                                                 in.clk, step, w.bx, w.by, smem_raw, scal + w.inst);
     __syncthreads(); // shared tiles are reused by the next work item
   }

@@ -13,15 +13,15 @@ namespace EK_NS
 
 namespace
 {
-constexpr int H2_TX = EK_H2_TX, H2_TY = EK_H2_TY;
+constexpr int H2_TX = EK_H2_TX, H2_TY = EK_H2_TY; // the ensemble's tile
 constexpr int H3_TX = EK_H3_TX, H3_TY = EK_H3_TY;
 
-template <class R>
+template <class R, int TX = H2_TX, int TY = H2_TY>
 constexpr size_t
 hydro2d_smem()
 {
-  constexpr int NV = 4, HX = H2_TX + 4, HY = H2_TY + 4;
-  return sizeof(R) * (NV * HY * HX + 2 * NV * H2_TY * (H2_TX + 2) + 2 * NV * (H2_TY + 2) * H2_TX);
+  constexpr int NV = 4, HX = TX + 4, HY = TY + 4;
+  return sizeof(R) * (NV * HY * HX + 2 * NV * TY * (TX + 2) + 2 * NV * (TY + 2) * TX);
 }
 template <class R>
 constexpr size_t
@@ -33,6 +33,20 @@ hydro3d_smem()
                       2 * NV * (H3_TY + 2) * H3_TX);
 }
 
+template <class S, class R, int TX, int TY, int NT, int RS, bool GRAV>
+cudaError_t
+hydro2d_step_tiled(const void * Uin, void * Uout, const KParams & P, DevClock * clk, int step, cudaStream_t st)
+{
+  auto        k = hydro2d_step<S, R, TX, TY, NT, RS, GRAV>;
+  size_t      sm = hydro2d_smem<R, TX, TY>();
+  cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
+  if (e != cudaSuccess)
+    return e;
+  dim3 grid((P.nx + TX - 1) / TX, (P.ny + TY - 1) / TY, 1);
+  k<<<grid, NT, sm, st>>>((const S *)Uin, (S *)Uout, P, clk, step);
+  return cudaGetLastError();
+}
+
 template <class S, class R, int RS, bool GRAV>
 cudaError_t
 hydro_step_rs(int dim, const void * Uin, void * Uout, const KParams & P, DevClock * clk, int step,
@@ -40,14 +54,23 @@ hydro_step_rs(int dim, const void * Uin, void * Uout, const KParams & P, DevCloc
 {
   if (dim == 2)
   {
-    auto   k = hydro2d_step<S, R, H2_TX, H2_TY, RS, GRAV>;
-    size_t sm = hydro2d_smem<R>();
-    cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
-    if (e != cudaSuccess)
-      return e;
-    dim3 grid((P.nx + H2_TX - 1) / H2_TX, (P.ny + H2_TY - 1) / H2_TY, 1);
-    k<<<grid, H2_TX * H2_TY, sm, st>>>((const S *)Uin, (S *)Uout, P, clk, step);
-    return cudaGetLastError();
+    // Tiles of the single solver (us per step).  Mixed: 32 x 8 (2048^2: 170;
+    // 32 x 16 180, 16 x 16 177, 64 x 4 183).  FP64, bound by the FP64 pipe: 16 x
+    // 16 on large grids (512^2: 145; 32 x 16 166, 32 x 8 156); where 8 x 8 tiles
+    // make at most six CTAs per SM, those, since a warp's chain of FP64
+    // instructions (64 cycles each on its quarter of the SM) then sets the time
+    // (64^2: 19 against 31; 200 x 136: 28 against 30; 256 x 200, 5.3 CTAs per SM:
+    // 47 against 49; 256^2, 6.7: 51 against 49).  The threads beyond one per
+    // cell take the ring cells and let every phase of the small tile finish in
+    // one round (64^2: 29 with one per cell).
+    if constexpr (sizeof(R) == 4)
+      return hydro2d_step_tiled<S, R, 32, 8, 256, RS, GRAV>(Uin, Uout, P, clk, step, st);
+    else
+    {
+      const long long small = (long long)((P.nx + 7) / 8) * ((P.ny + 7) / 8);
+      return small <= 6ll * P.sms ? hydro2d_step_tiled<S, R, 8, 8, 160, RS, GRAV>(Uin, Uout, P, clk, step, st)
+                                  : hydro2d_step_tiled<S, R, 16, 16, 320, RS, GRAV>(Uin, Uout, P, clk, step, st);
+    }
   }
   if constexpr (RS == 2)
   {
