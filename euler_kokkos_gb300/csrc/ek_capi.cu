@@ -838,11 +838,15 @@ launch_step(ek_solver * s, int step)
     return launch_one(s, 0, 0, step);
   if (s->p.dim == 2)
   {
-    ek_status st = launch_one(s, 2, 0, step); // CFL of the step
+    // CFL of the step: only before the first one after the state was set
+    ek_status st = EK_OK;
+    if (s->cfl_step != step)
+      st = launch_one(s, 2, 0, step);
     if (st == EK_OK)
-      st = launch_one(s, 0, 1, step); // trace, fluxes, emf, update
+      st = launch_one(s, 0, 1, step); // trace, fluxes, emf, update, and the next step's CFL
     if (st == EK_OK && has_repair(s))
-      st = launch_one(s, 3, 2, step); // the listed tiles with FP64 star states
+      st = launch_one(s, 3, 2, step); // the listed tiles with FP64 star states; completes the CFL
+    s->cfl_step = st == EK_OK ? step + 1 : -1;
     return st;
   }
   // CFL of the step: only when no update kernel computed it (the first step

@@ -664,8 +664,10 @@ step_scalars(const KParams & P, const DevClock * clk, int step, StepScalars<R> *
 // dt/dx ratios in FP64 once, for the step's kernels to read (step_consts), so
 // that no block of those kernels runs the divisions behind a barrier.  The
 // clock fields written by other blocks are read through volatile loads.
+// repair: the HLLD repair pass's list, if any; when tiles are listed the pass
+// completes the key, and computes the constants.
 __device__ __forceinline__ void
-finalize_step(DevClock * clk, const KParams & P, int step)
+finalize_step(DevClock * clk, const KParams & P, int step, const int * repair = nullptr)
 {
   __shared__ int last;
   __syncthreads();
@@ -681,7 +683,10 @@ finalize_step(DevClock * clk, const KParams & P, int step)
   {
     __threadfence();
     volatile DevClock * v = clk;
-    StepConsts          c;
+    clk->fin[s] = 0;
+    if (repair && *(const volatile int *)repair != 0)
+      return;
+    StepConsts c;
     c.step = step;
     c.active = 0;
     c.t = c.dt = c.dtdx = c.dtdy = c.dtdz = 0.0;
@@ -700,7 +705,6 @@ finalize_step(DevClock * clk, const KParams & P, int step)
       c.dtdz = d / P.dz;
     }
     clk->sc[s] = c;
-    clk->fin[s] = 0;
   }
 }
 // the constants of `step`; false when the step must not run (or they were

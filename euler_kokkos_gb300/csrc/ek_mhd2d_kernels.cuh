@@ -112,6 +112,39 @@ load_mhd2d_cell(const MhdState<S> & m, const KParams & P, const SrcCell & s, R (
   bz = load_face<S>(m, P, s, 2);
 }
 
+// CFL candidate of a cell: find_speed_info<TWO_D>, x and y only (mhd_utils.h:319-366)
+template <class R>
+__device__ __forceinline__ R
+mhd2d_invdt(const R (&q)[8], const MhdConst<R> & C, const KParams & P)
+{
+  const R d = q[ID], p = q[IP], a = q[IA], b = q[IB], cc = q[IC];
+  const R b2 = a * a + b * b + cc * cc;
+  R       cfx, cfy;
+  if constexpr (sizeof(R) == 4)
+  {
+    const float id = rcp_a(d), c2 = C.gamma0 * p * id;
+    const float d2 = 0.5f * (b2 * id + c2), cr = c2 * id;
+    cfx = sqrt_a(d2 + sqrt_a(d2 * d2 - cr * a * a));
+    cfy = sqrt_a(d2 + sqrt_a(d2 * d2 - cr * b * b));
+    return (cfx + fabsf(q[IU])) * P.idx + (cfy + fabsf(q[IV])) * P.idy;
+  }
+  else if constexpr (kFast64<R>)
+  {
+    // FP64 FMA build: host-prepared 1/dx
+    cfx = sqrt_ratio64(fast_num64(C.gamma0 * p, b2, a * a), d);
+    cfy = sqrt_ratio64(fast_num64(C.gamma0 * p, b2, b * b), d);
+    return (cfx + fabs(q[IU])) * P.idxd + (cfy + fabs(q[IV])) * P.idyd;
+  }
+  else
+  {
+    const R c2 = C.gamma0 * p / d;
+    const R d2 = R(0.5) * (b2 / d + c2);
+    cfx = sqrt(d2 + sqrt(d2 * d2 - c2 * a * a / d));
+    cfy = sqrt(d2 + sqrt(d2 * d2 - c2 * b * b / d));
+    return (cfx + fabs(q[IU])) / P.dx + (cfy + fabs(q[IV])) / P.dy;
+  }
+}
+
 // ---------------------------------------------------------------------------
 // 1. CFL reduction of the step
 // ---------------------------------------------------------------------------
@@ -144,33 +177,7 @@ mhd2d_dt_kernel(const void * __restrict__ U, KParams P, DevClock * clk, int step
       a[0] = bl0, a[1] = bl1, a[2] = bz;
       b[0] = br0, b[1] = br1, b[2] = 0.0;
     });
-    // find_speed_info<TWO_D>: x and y only (mhd_utils.h:319-366)
-    const R d = q[ID], p = q[IP], a = q[IA], b = q[IB], cc = q[IC];
-    const R b2 = a * a + b * b + cc * cc;
-    R       cfx, cfy;
-    if constexpr (sizeof(R) == 4)
-    {
-      const float id = rcp_a(d), c2 = C.gamma0 * p * id;
-      const float d2 = 0.5f * (b2 * id + c2), cr = c2 * id;
-      cfx = sqrt_a(d2 + sqrt_a(d2 * d2 - cr * a * a));
-      cfy = sqrt_a(d2 + sqrt_a(d2 * d2 - cr * b * b));
-      tmax = fmax(tmax, (cfx + fabsf(q[IU])) * P.idx + (cfy + fabsf(q[IV])) * P.idy);
-    }
-    else if constexpr (kFast64<R>)
-    {
-      // FP64 FMA build: host-prepared 1/dx
-      cfx = sqrt_ratio64(fast_num64(C.gamma0 * p, b2, a * a), d);
-      cfy = sqrt_ratio64(fast_num64(C.gamma0 * p, b2, b * b), d);
-      tmax = max_cand(tmax, (cfx + fabs(q[IU])) * P.idxd + (cfy + fabs(q[IV])) * P.idyd);
-    }
-    else
-    {
-      const R c2 = C.gamma0 * p / d;
-      const R d2 = R(0.5) * (b2 / d + c2);
-      cfx = sqrt(d2 + sqrt(d2 * d2 - c2 * a * a / d));
-      cfy = sqrt(d2 + sqrt(d2 * d2 - c2 * b * b / d));
-      tmax = fmax(tmax, (cfx + fabs(q[IU])) / P.dx + (cfy + fabs(q[IV])) / P.dy);
-    }
+    tmax = max_cand(tmax, mhd2d_invdt<R>(q, C, P));
   });
   block_max_commit<256>(cand_key((double)tmax), key ? key : &clk->key[step % 3]);
   if (!key)
@@ -347,8 +354,8 @@ trace2d_compact(const R * sQ, const R * sB, int qx, int qy, int bx, int by, R dt
 // [4..] tiles).
 template <class S, class R, int TX, int TY, int RS, bool REPAIR>
 __device__ __forceinline__ void
-mhd2d_tile(const void * __restrict__ Uin, void * __restrict__ Uout, const KParams & P, const StepConsts & sc,
-           int bx, int by, int * repair)
+mhd2d_tile(const void * __restrict__ Uin, void * __restrict__ Uout, const KParams & P, DevClock * clk, int step,
+           const StepConsts & sc, int bx, int by, int * repair)
 {
   using T = Mhd2dTile<TX, TY>;
   constexpr int NT = TX * TY;
@@ -476,12 +483,20 @@ mhd2d_tile(const void * __restrict__ Uin, void * __restrict__ Uout, const KParam
   //    MHDRunFunctors2D.h:1572-1700), in the reference's order per variable
   const int tx = threadIdx.x % TX, ty = threadIdx.x / TX;
   const int gi = i0 + tx, gj = j0 + ty;
-  if (gi < ihi && gj < jhi)
+  const bool own = gi < ihi && gj < jhi;
+  // the next step's CFL: the final face fields of the tile's cells and, beside
+  // them, of its +1 column and row (over the trace, which is no longer read)
+  double * sBxL = reinterpret_cast<double *>(sT); // [TY][TX]
+  double * sByL = sBxL + TX * TY;                // [TY][TX]
+  double * sBxE = sByL + TX * TY;                // [TY] Bx(i0 + TX) or of the domain's end
+  double * sByE = sBxE + TY;                     // [TX]
+  R        u[5];
+  double   bx_n = 0.0, by_n = 0.0, bz_n = 0.0;
+  if (own)
   {
     const long long st = P.vstride;
     const long long off = (long long)gj * P.isize + gi;
     const int       fx0 = ty * (TX + 1) + tx, fy0 = ty * TX + tx, e0 = ty * (TX + 1) + tx;
-    R               u[5];
 #pragma unroll
     for (int v = 0; v < 5; ++v)
       u[v] = (R)ldg(m.h + v * st + off);
@@ -505,19 +520,33 @@ mhd2d_tile(const void * __restrict__ Uin, void * __restrict__ Uout, const KParam
     S * hout = (S *)Uout;
 #pragma unroll
     for (int v = 0; v < 5; ++v)
+    {
       hout[v * st + off] = (S)u[v];
+      u[v] = (R)(S)u[v];
+    }
 
     double * bout = sizeof(S) == 8 ? (double *)Uout + 5 * P.vstride : mixed_bfield(Uout, P);
     double   bx = m.b[0 * st + off], by = m.b[1 * st + off], bz = m.b[2 * st + off];
     const R  e00 = sE[e0], e01 = sE[e0 + TX + 1], e10 = sE[e0 + 1];
+    // CT increments of a face field, also for the faces beyond the tile
+    auto ct = [&](double b, R ep, R em, R ratio, double dratio) {
+      if constexpr (sizeof(R) == 8)
+        return b + (ep - em) * ratio;
+      else
+        return fma(f2d(ep) - f2d(em), dratio, b);
+    };
+    auto ct_sub = [&](double b, R ep, R em, R ratio, double dratio) {
+      if constexpr (sizeof(R) == 8)
+        return b - (ep - em) * ratio;
+      else
+        return fma(f2d(em) - f2d(ep), dratio, b);
+    };
     if constexpr (sizeof(R) == 8)
     {
       bz += sFx[5 * T::FXS + fx0] * dtdx;
       bz -= sFx[5 * T::FXS + fx0 + 1] * dtdx;
       bz += sFy[5 * T::FYS + fy0] * dtdy;
       bz -= sFy[5 * T::FYS + fy0 + TX] * dtdy;
-      bx += (e01 - e00) * dtdy;
-      by -= (e10 - e00) * dtdx;
     }
     else
     {
@@ -531,15 +560,58 @@ mhd2d_tile(const void * __restrict__ Uin, void * __restrict__ Uout, const KParam
       bzf += sFy[5 * T::FYS + fy0] * dtdy;
       bzf -= sFy[5 * T::FYS + fy0 + TX] * dtdy;
       bz = f2d(bzf);
-      bx = fma(f2d(e01) - f2d(e00), ddtdy, bx);
-      by = fma(f2d(e00) - f2d(e10), ddtdx, by);
     }
+    bx = ct(bx, e01, e00, dtdy, ddtdy);
+    by = ct_sub(by, e10, e00, dtdx, ddtdx);
     bout[0 * st + off] = bx;
     bout[1 * st + off] = by;
     bout[2 * st + off] = bz;
+    bx_n = bx, by_n = by, bz_n = bz;
+    const int c = ty * TX + tx;
+    sBxL[c] = bx;
+    sByL[c] = by;
+    // the face beyond the domain's end follows the next step's ghost fill:
+    // outflow copies, a reflecting wall negates, periodic takes the CT update
+    // there (the update of the first interior face, from the same inputs)
+    auto high_face = [](int bc, double own_b, double ct_b) {
+      return bc == BC_PERIODIC ? ct_b : (bc == BC_DIRICHLET ? -own_b : own_b);
+    };
+    const R e11 = sE[e0 + TX + 2];
+    if (tx == TX - 1 || gi + 1 == ihi)
+    {
+      const bool   end = gi + 1 == ihi;
+      const double b1 = ct(end ? load_face<S>(m, P, src_cell(P, gi + 1, gj, 0), 0) : ldg(m.b + off + 1), e11, e10, dtdy, ddtdy);
+      sBxE[ty] = end ? high_face(P.bc[1], bx, b1) : b1;
+    }
+    if (ty == TY - 1 || gj + 1 == jhi)
+    {
+      const bool   end = gj + 1 == jhi;
+      const double b1 =
+        ct_sub(end ? load_face<S>(m, P, src_cell(P, gi, gj + 1, 0), 1) : ldg(m.b + st + off + P.isize), e11, e01, dtdx, ddtdx);
+      sByE[tx] = end ? high_face(P.bc[3], by, b1) : b1;
+    }
   }
-  // s_dirty was last written before the barrier that ends phase D
-  if (kFlag && threadIdx.x == 0 && s_dirty)
+  __syncthreads();
+  // F. CFL candidate of the updated cell (ConvertToPrimitivesFunctor2D_MHD and
+  //    ComputeDtFunctor2D_MHD on the next step's state, as mhd2d_dt_kernel
+  //    computes them); a tile for the repair pass commits none
+  const bool dirty = kFlag && s_dirty != 0; // last written before the barrier that ends phase D
+  R          tmax = R(-INFINITY);
+  if (own)
+  {
+    const int    c = ty * TX + tx;
+    const double bxr = tx + 1 < TX && gi + 1 < ihi ? sBxL[c + 1] : sBxE[ty];
+    const double byr = ty + 1 < TY && gj + 1 < jhi ? sByL[c + TX] : sByE[tx];
+    R            bl[3] = { to_r<R>(bx_n), to_r<R>(by_n), to_r<R>(bz_n) }, br[3] = { to_r<R>(bxr), to_r<R>(byr), R(0) }, q[8];
+    mhd_constoprim<R>(u, bl, br, q, C, [&](double (&a)[3], double (&b)[3]) {
+      a[0] = bx_n, a[1] = by_n, a[2] = bz_n;
+      b[0] = bxr, b[1] = byr, b[2] = 0.0;
+    });
+    tmax = mhd2d_invdt<R>(q, C, P);
+  }
+  if (!dirty)
+    block_max_commit<NT>(cand_key((double)tmax), &clk->key[(step + 1) % 3]);
+  else if (threadIdx.x == 0)
     repair[kRepairHead + atomicAdd(&repair[0], 1)] = by * ((P.nx + TX - 1) / TX) + bx;
 }
 
@@ -553,9 +625,10 @@ mhd2d_step_kernel(const void * __restrict__ Uin, void * __restrict__ Uout, KPara
   StepConsts sc;
   if (!step_consts(clk, step, sc))
     return;
-  mhd2d_tile<S, R, TX, TY, RS, false>(Uin, Uout, P, sc, blockIdx.x, blockIdx.y, repair);
+  mhd2d_tile<S, R, TX, TY, RS, false>(Uin, Uout, P, clk, step, sc, blockIdx.x, blockIdx.y, repair);
   if (blockIdx.x == 0 && blockIdx.y == 0 && threadIdx.x == 0)
     step_commit(clk, step, sc.t, sc.dt);
+  finalize_step(clk, P, step + 1, repair); // the next step's dt, once its CFL key is complete
 }
 
 // After the step kernel of the mixed HLLD form: recomputes the tiles it
@@ -570,14 +643,17 @@ mhd2d_repair_kernel(const void * __restrict__ Uin, void * __restrict__ Uout, KPa
   if (!step_consts(clk, step, sc))
     return;
   const int n = repair[0];
+  if (n == 0)
+    return; // most steps: nothing listed, and the step kernel computed the next step's dt
   const int gx = (P.nx + TX - 1) / TX;
   for (int e = blockIdx.x; e < n; e += gridDim.x)
   {
     const int tile = repair[kRepairHead + e];
-    mhd2d_tile<S, R, TX, TY, 4, true>(Uin, Uout, P, sc, tile % gx, tile / gx, repair);
+    mhd2d_tile<S, R, TX, TY, 4, true>(Uin, Uout, P, clk, step, sc, tile % gx, tile / gx, repair);
     __syncthreads(); // shared memory of the next tile
   }
   repair_list_release(repair);
+  finalize_step(clk, P, step + 1);
 }
 
 constexpr int M2_TX = EK_M2_TX, M2_TY = EK_M2_TY;

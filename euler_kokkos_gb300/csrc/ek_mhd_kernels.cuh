@@ -1086,8 +1086,8 @@ mhd_update_tile(const void * __restrict__ Uin, void * __restrict__ Uout, const R
 }
 
 // One launch per step: the tile columns of the grid.  repair: the tile list
-// of the mixed HLLD form (null otherwise), whose repair kernel then completes
-// the next step's CFL key.
+// of the mixed HLLD form (null otherwise); if tiles are listed, the repair
+// kernel completes the next step's CFL key.
 template <class S, class R, int TX, int TY, bool STAGE, int RS>
 __global__ void __launch_bounds__(TX * TY, EK_MINB(R, EK_MU_MINB_F32, EK_MU_MINB_F64))
 mhd_update_kernel(const void * __restrict__ Uin, void * __restrict__ Uout, const R * __restrict__ trace,
@@ -1100,8 +1100,8 @@ mhd_update_kernel(const void * __restrict__ Uin, void * __restrict__ Uout, const
                                                    blockIdx.y, blockIdx.z, repair);
   if (blockIdx.x == 0 && blockIdx.y == 0 && blockIdx.z == 0 && threadIdx.x == 0)
     step_commit(clk, step, sc.t, sc.dt);
-  if (cfl_next && !repair)
-    finalize_step(clk, P, step + 1); // the next step's dt, once its CFL key is complete
+  if (cfl_next)
+    finalize_step(clk, P, step + 1, repair); // the next step's dt, once its CFL key is complete
 }
 
 // The last block of a launch of the repair kernel: true once, after every block
@@ -1140,6 +1140,8 @@ mhd_repair_kernel(const void * __restrict__ Uin, void * __restrict__ Uout, const
   if (!step_consts(clk, step, sc))
     return;
   const int n = repair[0];
+  if (n == 0)
+    return; // most steps: nothing listed, and the update kernel computed the next step's dt
   const int gx = (P.nx + TX - 1) / TX, gy = (P.ny + TY - 1) / TY;
   for (int e = blockIdx.x; e < n; e += gridDim.x)
   {
