@@ -346,19 +346,19 @@ trace2d_compact(const R * sQ, const R * sB, int qx, int qy, int bx, int by, R dt
     out[f * ost] = o[f];
 }
 
+// NT threads, one per cell or more (fewer rounds in the phases of a small tile).
 // One tile of the step: the cells [i0, i0+TX) x [j0, j0+TY) of tile (bx, by),
 // written from the step's input state only.  REPAIR: the faces whose FP32
 // HLLD star state is ill-conditioned are solved in FP64 (the repair kernel);
 // otherwise such a face lists the tile for that kernel (repair list as in
 // the 3D update kernel: [0] count, [1] blocks done, [2..3] tiles repaired,
 // [4..] tiles).
-template <class S, class R, int TX, int TY, int RS, bool REPAIR>
+template <class S, class R, int TX, int TY, int NT, int RS, bool REPAIR>
 __device__ __forceinline__ void
 mhd2d_tile(const void * __restrict__ Uin, void * __restrict__ Uout, const KParams & P, DevClock * clk, int step,
            const StepConsts & sc, int bx, int by, int * repair)
 {
   using T = Mhd2dTile<TX, TY>;
-  constexpr int NT = TX * TY;
   extern __shared__ __align__(16) unsigned char smem_raw[];
   R * sT = reinterpret_cast<R *>(smem_raw); // [V_N][YE][XE] compact trace
   R * sB = sT + T::TRACE;                   // [2][BY][BX] face fields IA, IB
@@ -483,7 +483,7 @@ mhd2d_tile(const void * __restrict__ Uin, void * __restrict__ Uout, const KParam
   //    MHDRunFunctors2D.h:1572-1700), in the reference's order per variable
   const int tx = threadIdx.x % TX, ty = threadIdx.x / TX;
   const int gi = i0 + tx, gj = j0 + ty;
-  const bool own = gi < ihi && gj < jhi;
+  const bool own = ty < TY && gi < ihi && gj < jhi; // the first TX * TY threads
   // the next step's CFL: the final face fields of the tile's cells and, beside
   // them, of its +1 column and row (over the trace, which is no longer read)
   double * sBxL = reinterpret_cast<double *>(sT); // [TY][TX]
@@ -617,15 +617,15 @@ mhd2d_tile(const void * __restrict__ Uin, void * __restrict__ Uout, const KParam
 
 // One launch per step: the tiles of the grid.  repair: the tile list of the
 // mixed HLLD form (null otherwise), for the repair kernel that follows.
-template <class S, class R, int TX, int TY, int RS>
-__global__ void __launch_bounds__(TX * TY, EK_MINB(R, EK_M2_MINB_F32, EK_M2_MINB_F64))
+template <class S, class R, int TX, int TY, int NT, int RS>
+__global__ void __launch_bounds__(NT, EK_MINB(R, EK_M2_MINB_F32, EK_M2_MINB_F64))
 mhd2d_step_kernel(const void * __restrict__ Uin, void * __restrict__ Uout, KParams P, DevClock * clk,
                   int step, int * repair)
 {
   StepConsts sc;
   if (!step_consts(clk, step, sc))
     return;
-  mhd2d_tile<S, R, TX, TY, RS, false>(Uin, Uout, P, clk, step, sc, blockIdx.x, blockIdx.y, repair);
+  mhd2d_tile<S, R, TX, TY, NT, RS, false>(Uin, Uout, P, clk, step, sc, blockIdx.x, blockIdx.y, repair);
   if (blockIdx.x == 0 && blockIdx.y == 0 && threadIdx.x == 0)
     step_commit(clk, step, sc.t, sc.dt);
   finalize_step(clk, P, step + 1, repair); // the next step's dt, once its CFL key is complete
@@ -649,7 +649,7 @@ mhd2d_repair_kernel(const void * __restrict__ Uin, void * __restrict__ Uout, KPa
   for (int e = blockIdx.x; e < n; e += gridDim.x)
   {
     const int tile = repair[kRepairHead + e];
-    mhd2d_tile<S, R, TX, TY, 4, true>(Uin, Uout, P, clk, step, sc, tile % gx, tile / gx, repair);
+    mhd2d_tile<S, R, TX, TY, TX * TY, 4, true>(Uin, Uout, P, clk, step, sc, tile % gx, tile / gx, repair);
     __syncthreads(); // shared memory of the next tile
   }
   repair_list_release(repair);
@@ -662,6 +662,23 @@ inline long long
 mhd2d_tiles(const KParams & P)
 {
   return (long long)((P.nx + M2_TX - 1) / M2_TX) * ((P.ny + M2_TY - 1) / M2_TY);
+}
+
+template <class S, class R, int TX, int TY, int NT>
+cudaError_t
+mhd2d_step_tiled(const void * Uin, void * Uout, void * work, const KParams & P, DevClock * clk, int step, cudaStream_t st)
+{
+  auto k = P.riemann == 1   ? mhd2d_step_kernel<S, R, TX, TY, NT, 1>
+           : P.riemann == 2 ? mhd2d_step_kernel<S, R, TX, TY, NT, 2>
+                            : mhd2d_step_kernel<S, R, TX, TY, NT, 4>;
+  const int   sm = (int)mhd2d_smem<R>(TX, TY);
+  cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, sm);
+  if (e != cudaSuccess)
+    return e;
+  dim3  grid((P.nx + TX - 1) / TX, (P.ny + TY - 1) / TY, 1);
+  int * repair = sizeof(R) == 4 && P.riemann == 4 ? (int *)work : nullptr;
+  k<<<grid, NT, sm, st>>>(Uin, Uout, P, clk, step, repair);
+  return cudaGetLastError();
 }
 
 template <class S, class R>
@@ -692,17 +709,23 @@ mhd2d_step_t(int phase, const void * Uin, void * Uout, void * work, const KParam
       return cudaGetLastError();
     }
   }
-  auto k = P.riemann == 1   ? mhd2d_step_kernel<S, R, M2_TX, M2_TY, 1>
-           : P.riemann == 2 ? mhd2d_step_kernel<S, R, M2_TX, M2_TY, 2>
-                            : mhd2d_step_kernel<S, R, M2_TX, M2_TY, 4>;
-  const int   sm = (int)mhd2d_smem<R>(M2_TX, M2_TY);
-  cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, sm);
-  if (e != cudaSuccess)
-    return e;
-  dim3  grid((P.nx + M2_TX - 1) / M2_TX, (P.ny + M2_TY - 1) / M2_TY, 1);
-  int * repair = sizeof(R) == 4 && P.riemann == 4 ? (int *)work : nullptr;
-  k<<<grid, M2_TX * M2_TY, sm, st>>>(Uin, Uout, P, clk, step, repair);
-  return cudaGetLastError();
+  // Mixed: 16 x 16 at every size.  FP64 (us per step; a tile's time is set by
+  // its chain of FP64 instructions, so a whole wave of CTAs counts): 8 x 8 with
+  // 128 threads up to three CTAs per SM (64^2: 50; 16 x 8 82, 16 x 16 117; 200 x
+  // 136: 102, 117, 117), 16 x 8 up to the three that fit in shared memory (256 x
+  // 200: 164; 8 x 8 210, 16 x 16 205), then 16 x 16 (256^2: 205; 16 x 8 314;
+  // 512^2: 692 and 774).
+  if constexpr (sizeof(R) == 4)
+    return mhd2d_step_tiled<S, R, M2_TX, M2_TY, M2_TX * M2_TY>(Uin, Uout, work, P, clk, step, st);
+  else
+  {
+    auto tiles = [&](int tx, int ty) { return (long long)((P.nx + tx - 1) / tx) * ((P.ny + ty - 1) / ty); };
+    if (tiles(8, 8) <= 3ll * P.sms)
+      return mhd2d_step_tiled<S, R, 8, 8, 128>(Uin, Uout, work, P, clk, step, st);
+    if (tiles(16, 8) <= 3ll * P.sms)
+      return mhd2d_step_tiled<S, R, 16, 8, 128>(Uin, Uout, work, P, clk, step, st);
+    return mhd2d_step_tiled<S, R, M2_TX, M2_TY, M2_TX * M2_TY>(Uin, Uout, work, P, clk, step, st);
+  }
 }
 
 // the repair pass's tile list of the mixed form (cleared by the caller before

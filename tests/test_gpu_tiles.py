@@ -14,6 +14,8 @@ pytestmark = pytest.mark.gpu
 
 # 2D: 8 x 8 tiles up to six per SM (240^2: 900 tiles on 152 SMs), 16 x 16 above (248 x 240: 930)
 CASES = [(2, False, s) for s in [(2, 2, 1), (8, 8, 1), (9, 7, 1), (17, 16, 1), (240, 240, 1), (248, 240, 1), (257, 241, 1)]]
+# 2D MHD: 8 x 8 up to three per SM (170 x 165: 462 tiles, 160 x 160: 400), 16 x 8 up to three (240 x 240: 450), then 16 x 16
+CASES += [(2, True, s) for s in [(3, 3, 1), (8, 9, 1), (17, 8, 1), (160, 160, 1), (170, 165, 1), (240, 240, 1), (250, 243, 1)]]
 # 3D: planes per CTA from the grid (kchunk 0)
 CASES += [(3, False, s) for s in [(2, 2, 2), (16, 16, 33), (17, 33, 9)]]
 CASES += [(3, True, s) for s in [(3, 3, 3), (16, 8, 21), (33, 9, 14)]]
