@@ -67,6 +67,7 @@ struct ek_solver
   std::vector<std::pair<int, std::pair<cudaEvent_t, cudaEvent_t>>> ev_pending;
   double                   kernel_ms[4] = { 0, 0, 0, 0 };
   long long                kernel_n[4] = { 0, 0, 0, 0 };
+  bool                     passes = false; // the FP64 step in passes (work: their workspace)
   bool                     owns = true; // false: a view into an ensemble's buffers
   // 3D MHD: the step whose CFL the last update kernel computed (-1: none)
   int                      cfl_step = -1;
@@ -365,7 +366,26 @@ ek_solver_create(const ek_params * params, ek_solver ** out)
     e = cudaMalloc((void **)&s->dtlog, sizeof(double) * s->dtcap);
   if (e == cudaSuccess)
     e = cudaMalloc((void **)&s->scratch3, 3 * sizeof(double));
-  if (e == cudaSuccess && p.mhd)
+  // FP64: the step in passes with a bounded workspace, where the grid is not too
+  // small for it (pass_bytes 0); if the workspace does not fit beside the states,
+  // the tile kernels, which need none
+  if (e == cudaSuccess && s->prec == EK_PREC_FP64)
+  {
+    s->work_bytes = ek_fast::pass_bytes(p.dim, p.mhd, k);
+    if (s->work_bytes)
+    {
+      e = cudaMalloc(&s->work, s->work_bytes);
+      s->passes = e == cudaSuccess;
+      if (e == cudaErrorMemoryAllocation)
+      {
+        cudaGetLastError();
+        s->work = nullptr;
+        s->work_bytes = 0;
+        e = cudaSuccess;
+      }
+    }
+  }
+  if (e == cudaSuccess && p.mhd && !s->passes)
   {
     if (p.dim == 3)
       s->work_bytes = s->exact ? ek_exact::mhd_work_bytes(s->prec, k) : ek_fast::mhd_work_bytes(s->prec, k);
@@ -807,7 +827,10 @@ launch_one(ek_solver * s, int kernel_id, int phase, int step)
     cudaEventRecord(e0, s->stream);
   }
   cudaError_t e;
-  if (s->p.mhd && s->p.dim == 2)
+  if (s->p.mhd && s->passes)
+    e = s->exact ? ek_exact::mhd_passes(s->p.dim, phase, in, outp, s->work, s->kp, s->clk, step, s->stream)
+                 : ek_fast::mhd_passes(s->p.dim, phase, in, outp, s->work, s->kp, s->clk, step, s->stream);
+  else if (s->p.mhd && s->p.dim == 2)
     e = s->exact ? ek_exact::mhd2d_step(s->prec, phase, in, outp, s->work, s->kp, s->clk, step, s->stream)
                  : ek_fast::mhd2d_step(s->prec, phase, in, outp, s->work, s->kp, s->clk, step, s->stream);
   else if (s->p.mhd)
@@ -816,8 +839,8 @@ launch_one(ek_solver * s, int kernel_id, int phase, int step)
   else
   {
     const CUtensorMap * tm = s->has_tmap ? &s->tmap[step % 2] : nullptr;
-    e = s->exact ? ek_exact::hydro_step(s->p.dim, s->prec, in, outp, s->kp, s->clk, step, tm, s->stream)
-                 : ek_fast::hydro_step(s->p.dim, s->prec, in, outp, s->kp, s->clk, step, tm, s->stream);
+    e = s->exact ? ek_exact::hydro_step(s->p.dim, s->prec, in, outp, s->work, s->kp, s->clk, step, tm, s->stream)
+                 : ek_fast::hydro_step(s->p.dim, s->prec, in, outp, s->work, s->kp, s->clk, step, tm, s->stream);
   }
   if (s->profiling)
   {
@@ -834,6 +857,16 @@ launch_one(ek_solver * s, int kernel_id, int phase, int step)
 static ek_status
 launch_step(ek_solver * s, int step)
 {
+  if (s->passes)
+  {
+    ek_status st = EK_OK;
+    if (s->p.mhd)
+      st = launch_one(s, 2, 0, step); // primitives, CFL of the step, electric field
+    if (st == EK_OK)
+      st = launch_one(s, 0, 1, step);
+    s->launches += ek_fast::pass_launches(s->p.dim, s->p.mhd, s->kp) - (s->p.mhd ? 2 : 1);
+    return st;
+  }
   if (!s->p.mhd)
     return launch_one(s, 0, 0, step);
   if (s->p.dim == 2)

@@ -470,15 +470,29 @@ from_order64(long long b)
 {
   return __longlong_as_double(b ^ ((b >> 63) & 0x7fffffffffffffffll));
 }
-// x / 2^K by the exponent (exact); the product where the result or x is not normal
+// |x| (fabs and unary minus can become FP64 additions)
+__device__ __forceinline__ double
+abs64(double x)
+{
+  return with_hi(hi32(x) & 0x7fffffff, x);
+}
+// x / 2 by the exponent; where that leaves the normal range, by a shift of the
+// significand (exact but for the last subnormal bit, which is cut)
+__device__ __forceinline__ double
+half64(double x)
+{
+  const long long b = __double_as_longlong(x), m = b & 0x7fffffffffffffffll;
+  const long long h = m >= 0x7ff0000000000000ll ? m : (m >= 0x0020000000000000ll ? m - 0x0010000000000000ll : m >> 1);
+  return __longlong_as_double(h | (b ^ m));
+}
+// x / 2^K for x >= 0 by the exponent; zero below 2^(K - 1021)
 template <int K>
 __device__ __forceinline__ double
-scale_down64(double x)
+scale_pos64(double x)
 {
   const int hi = hi32(x);
-  if ((unsigned)(hi & 0x7fffffff) - (unsigned)((K + 1) << 20) < (unsigned)((0x7ff - K - 1) << 20))
-    return with_hi(hi - (K << 20), x);
-  return x * (1.0 / (1 << K));
+  const bool tiny = hi < ((K + 1) << 20);
+  return __hiloint2double(tiny ? 0 : hi - (K << 20), tiny ? 0 : __double2loint(x));
 }
 // max(p, d floor) for d > 0: the product only where the high words say that
 // p / d may be below 2 floor

@@ -59,12 +59,13 @@ __device__ __forceinline__ double
 half_slope64(double q, double qp, double qm, double st)
 {
   const double dl = q - qm, dr = qp - q;
-  const double m = min_pos64(fabs(dl), fabs(dr));
+  const double m = min_pos64(abs64(dl), abs64(dr));
   double       h;
-  if (st == 1.0)
-    h = scale_down64<1>(m);
-  else if (st == 2.0)
-    h = min_pos64(m, scale_down64<2>(fabs(qp - qm)));
+  const int    lim = hi32(st); // 1.0 or 2.0 by the high word: a comparison would be an FP64 instruction
+  if (lim == 0x3ff00000)
+    h = scale_pos64<1>(m);
+  else if (lim == 0x40000000)
+    h = min_pos64(m, scale_pos64<2>(abs64(qp - qm)));
   else
     h = 0.0;
   // the sign of dl, or zero
@@ -345,7 +346,7 @@ hllc64(const double (&ql)[NV], const double (&qr)[NV], double (&flux)[NV], const
     kl += ql[IW] * ql[IW];
     kr += qr[IW] * qr[IW];
   }
-  const double el = fma(pl, C.entho, scale_down64<1>(rl) * kl), er = fma(pr, C.entho, scale_down64<1>(rr) * kr);
+  const double el = fma(pl, C.entho, scale_pos64<1>(rl) * kl), er = fma(pr, C.entho, scale_pos64<1>(rr) * kr);
 
   const bool   lbig = __double_as_longlong(pl * rr) >= __double_as_longlong(pr * rl);
   const double cmax = max_floor64(sqrt_ratio64(C.gamma0 * (lbig ? pl : pr), lbig ? rl : rr), C.smallc);
@@ -555,10 +556,10 @@ riemann_approx64(const double (&ql)[NV], const double (&qr)[NV], double (&flux)[
     const double gl = xl * wl * rcp64(xl + cl), gr = xr * wr * rcp64(xr + cr);
     const double dv = fma(-dr, yr, fma(-dl, yl, du)); // u_l* - u_r*
     double       delp = (gr + gr) * gl * rcp64(gr + gl) * dv;
-    delp = negative64(delp + p) ? -p : delp;
+    delp = negative64(delp + p) ? flip64(p, true) : delp;
     p += delp;
     // |delp / (p + smallpp)| > 1e-6
-    if (__double_as_longlong(fabs(delp)) <= __double_as_longlong(fabs((p + C.smallpp) * 1e-6)))
+    if (__double_as_longlong(abs64(delp)) <= __double_as_longlong(abs64((p + C.smallpp) * 1e-6)))
     {
       const double x2l = fma(kl, p - pl, cl), x2r = fma(kr, p - pr, cr);
       yl = rsqrt64(x2l);
@@ -572,10 +573,10 @@ riemann_approx64(const double (&ql)[NV], const double (&qr)[NV], double (&flux)[
   const bool   left = !negative64(us);
   const double ro = left ? rl : rr, po = left ? pl : pr, wo = left ? wl : wr, yo = left ? yl : yr;
   const double uo = flip64(left ? ul : ur, !left), ss = flip64(us, !left); // sgnm u
-  const double co = max_floor64(sqrt_ratio64(fabs(C.gamma0 * po), ro), C.smallc);
+  const double co = max_floor64(sqrt_ratio64(abs64(C.gamma0 * po), ro), C.smallc);
   // rho / (1 + rho (p_o - p*) / w^2)
   const double rs = max_floor64(ro * rcp64(fma(ro * (po - p), yo * yo, 1.0)), C.smallr);
-  const double cs = max_floor64(sqrt_ratio64(fabs(C.gamma0 * p), rs), C.smallc);
+  const double cs = max_floor64(sqrt_ratio64(abs64(C.gamma0 * p), rs), C.smallc);
   double       spout = co - uo, spin = cs - ss;
   if (p >= po)
     spin = spout = fma(wo, rcp64(ro), -uo); // shock

@@ -5,8 +5,10 @@
 
 #include "ek_launch.h"
 #include "ek_hydro_kernels.cuh"
+#include "ek_hydro_passes.cuh"
 #include "ek_mhd_kernels.cuh"
 #include "ek_mhd2d_kernels.cuh"
+#include "ek_mhd_passes.cuh"
 
 namespace EK_NS
 {
@@ -49,20 +51,28 @@ hydro2d_step_tiled(const void * Uin, void * Uout, const KParams & P, DevClock * 
 
 template <class S, class R, int RS, bool GRAV>
 cudaError_t
-hydro_step_rs(int dim, const void * Uin, void * Uout, const KParams & P, DevClock * clk, int step,
+hydro_step_rs(int dim, const void * Uin, void * Uout, void * work, const KParams & P, DevClock * clk, int step,
               const CUtensorMap * tmap, cudaStream_t st)
 {
+  if constexpr (sizeof(R) == 8)
+    if (work)
+    {
+      if (dim == 2)
+        return hydro_step_passes<4, RS, GRAV>(Uin, Uout, work, P, clk, step, st);
+      if constexpr (RS != 2)
+        return hydro_step_passes<5, RS, GRAV>(Uin, Uout, work, P, clk, step, st);
+    }
   if (dim == 2)
   {
     // Tiles of the single solver (us per step).  Mixed: 32 x 8 (2048^2: 170;
-    // 32 x 16 180, 16 x 16 177, 64 x 4 183).  FP64, bound by the FP64 pipe: 16 x
-    // 16 on large grids (512^2: 145; 32 x 16 166, 32 x 8 156); where 8 x 8 tiles
-    // make at most six CTAs per SM, those, since a warp's chain of FP64
-    // instructions (64 cycles each on its quarter of the SM) then sets the time
-    // (64^2: 19 against 31; 200 x 136: 28 against 30; 256 x 200, 5.3 CTAs per SM:
-    // 47 against 49; 256^2, 6.7: 51 against 49).  The threads beyond one per
-    // cell take the ring cells and let every phase of the small tile finish in
-    // one round (64^2: 29 with one per cell).
+    // 32 x 16 180, 16 x 16 177, 64 x 4 183).  FP64, on grids too small for the
+    // passes: 8 x 8 where they make at most six CTAs per SM, since a warp's
+    // chain of FP64 instructions (64 cycles each on its quarter of the SM) then
+    // sets the time (64^2: 19 against 31; 200 x 136: 28 against 30; 256 x 200,
+    // 5.3 CTAs per SM: 47 against 49; 256^2, 6.7: 51 against 49), else 16 x 16
+    // (512^2: 145; 32 x 16 166, 32 x 8 156).  The threads beyond one per cell
+    // take the ring cells and let every phase of the small tile finish in one
+    // round (64^2: 29 with one per cell).
     if constexpr (sizeof(R) == 4)
       return hydro2d_step_tiled<S, R, 32, 8, 256, RS, GRAV>(Uin, Uout, P, clk, step, st);
     else
@@ -100,26 +110,26 @@ hydro_step_rs(int dim, const void * Uin, void * Uout, const KParams & P, DevCloc
 // kernels
 template <class S, class R, bool GRAV>
 cudaError_t
-hydro_step_g(int dim, const void * Uin, void * Uout, const KParams & P, DevClock * clk, int step,
+hydro_step_g(int dim, const void * Uin, void * Uout, void * work, const KParams & P, DevClock * clk, int step,
              const CUtensorMap * tmap, cudaStream_t st)
 {
   switch (P.riemann)
   {
-    case 0: return hydro_step_rs<S, R, 0, GRAV>(dim, Uin, Uout, P, clk, step, tmap, st);
-    case 1: return hydro_step_rs<S, R, 1, GRAV>(dim, Uin, Uout, P, clk, step, tmap, st);
-    case 2: return hydro_step_rs<S, R, 2, GRAV>(dim, Uin, Uout, P, clk, step, tmap, st);
-    case 3: return hydro_step_rs<S, R, 3, GRAV>(dim, Uin, Uout, P, clk, step, tmap, st);
+    case 0: return hydro_step_rs<S, R, 0, GRAV>(dim, Uin, Uout, work, P, clk, step, tmap, st);
+    case 1: return hydro_step_rs<S, R, 1, GRAV>(dim, Uin, Uout, work, P, clk, step, tmap, st);
+    case 2: return hydro_step_rs<S, R, 2, GRAV>(dim, Uin, Uout, work, P, clk, step, tmap, st);
+    case 3: return hydro_step_rs<S, R, 3, GRAV>(dim, Uin, Uout, work, P, clk, step, tmap, st);
   }
   return cudaErrorNotSupported;
 }
 
 template <class S, class R>
 cudaError_t
-hydro_step_t(int dim, const void * Uin, void * Uout, const KParams & P, DevClock * clk, int step,
+hydro_step_t(int dim, const void * Uin, void * Uout, void * work, const KParams & P, DevClock * clk, int step,
              const CUtensorMap * tmap, cudaStream_t st)
 {
-  return P.grav ? hydro_step_g<S, R, true>(dim, Uin, Uout, P, clk, step, tmap, st)
-                : hydro_step_g<S, R, false>(dim, Uin, Uout, P, clk, step, tmap, st);
+  return P.grav ? hydro_step_g<S, R, true>(dim, Uin, Uout, work, P, clk, step, tmap, st)
+                : hydro_step_g<S, R, false>(dim, Uin, Uout, work, P, clk, step, tmap, st);
 }
 
 template <class S, class R>
@@ -141,17 +151,17 @@ hydro_dt_t(int dim, const void * U, const KParams & P, unsigned long long * key,
 } // namespace
 
 cudaError_t
-hydro_step(int dim, int prec, const void * Uin, void * Uout, const KParams & P, DevClock * clk,
+hydro_step(int dim, int prec, const void * Uin, void * Uout, void * work, const KParams & P, DevClock * clk,
            int step, const CUtensorMap * tmap, cudaStream_t st)
 {
 #ifdef EK_EXACT_ONLY
   if (prec != 0)
     return cudaErrorNotSupported;
-  return hydro_step_t<double, double>(dim, Uin, Uout, P, clk, step, tmap, st);
+  return hydro_step_t<double, double>(dim, Uin, Uout, work, P, clk, step, tmap, st);
 #else
   if (prec == 0)
-    return hydro_step_t<double, double>(dim, Uin, Uout, P, clk, step, tmap, st);
-  return hydro_step_t<float, float>(dim, Uin, Uout, P, clk, step, tmap, st);
+    return hydro_step_t<double, double>(dim, Uin, Uout, work, P, clk, step, tmap, st);
+  return hydro_step_t<float, float>(dim, Uin, Uout, work, P, clk, step, tmap, st);
 #endif
 }
 

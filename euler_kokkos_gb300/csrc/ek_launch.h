@@ -15,7 +15,8 @@
   using ekc::DevClock;                                                                              \
   /* prec: 0 FP64, 1 mixed.  Uin/Uout device state arrays. */                                      \
   /* tmap: tensor map of Uin for the 3D kernel's staged planes, or null */                        \
-  cudaError_t hydro_step(int dim, int prec, const void * Uin, void * Uout, const KParams & P,        \
+  /* work: workspace of pass_bytes (FP64: the step in passes), or null (tile kernels) */            \
+  cudaError_t hydro_step(int dim, int prec, const void * Uin, void * Uout, void * work, const KParams & P, \
                          DevClock * clk, int step, const CUtensorMap * tmap, cudaStream_t st);      \
   /* fin: also compute the step constants of step fin_step from key (the last block) */           \
   cudaError_t hydro_dt(int dim, int prec, const void * U, const KParams & P,                       \
@@ -40,6 +41,14 @@
   cudaError_t ensemble2d_step(int prec, const ekc::EnsInstance * insts, int n, const ekc::EnsTile * tiles, \
                               int ntiles, int * stepc, void * scal, int grid, cudaStream_t st);     \
   int         ensemble2d_grid(int prec);                                                            \
+  /* the FP64 MHD step in passes: phase 0 (primitives, CFL, electric field), 1 (trace, fluxes, */   \
+  /* emfs, update); work: workspace of pass_bytes */                                                \
+  cudaError_t mhd_passes(int dim, int phase, const void * Uin, void * Uout, void * work,            \
+                         const KParams & P, DevClock * clk, int step, cudaStream_t st);             \
+  /* the FP64 step in passes: bytes of its workspace (0: the grid is too small for it, the tile */  \
+  /* kernels are used), kernels per step */                                                         \
+  size_t      pass_bytes(int dim, int mhd, const KParams & P);                                      \
+  int         pass_launches(int dim, int mhd, const KParams & P);                                   \
   }
 
 EK_DECLARE_LAUNCHERS(ek_exact)

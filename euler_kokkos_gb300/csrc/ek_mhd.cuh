@@ -25,7 +25,7 @@ struct MhdConst
 __device__ __forceinline__ double
 fast_num64(double gp, double b2, double bn2)
 {
-  const double s = scale_down64<1>(b2 + gp);
+  const double s = scale_pos64<1>(b2 + gp);
   return s + sqrt64(max_floor64(fma(s, s, -(gp * bn2)), 0.0));
 }
 
@@ -111,9 +111,9 @@ mhd_constoprim(const R (&u)[5], const R (&bl)[3], const R (&br)[3], R (&q)[8], c
     q[IU] = u[IU] * id;
     q[IV] = u[IV] * id;
     q[IW] = u[IW] * id;
-    q[IA] = scale_down64<1>(bl[0] + br[0]);
-    q[IB] = scale_down64<1>(bl[1] + br[1]);
-    q[IC] = scale_down64<1>(bl[2] + br[2]);
+    q[IA] = half64(bl[0] + br[0]);
+    q[IB] = half64(bl[1] + br[1]);
+    q[IC] = half64(bl[2] + br[2]);
     const R k2 = q[IU] * q[IU] + q[IV] * q[IV] + q[IW] * q[IW];
     const R b2 = q[IA] * q[IA] + q[IB] * q[IB] + q[IC] * q[IC];
     q[IP] = floor_ratio64((C.gamma0 - R(1)) * fma(R(-0.5) * d, k2, fma(R(-0.5), b2, u[IP])), d, C.smallp);
@@ -317,17 +317,17 @@ template <int NF>
 __device__ __forceinline__ void
 mhd_hlld64(const double (&ql)[8], const double (&qr)[8], double (&flux)[NF], double gamma0, double entho)
 {
-  const double a = scale_down64<1>(ql[IA] + qr[IA]), a2 = a * a;
+  const double a = half64(ql[IA] + qr[IA]), a2 = a * a;
   struct Side
   {
     double pt, et, vb, n; // total pressure and energy, v.B, rho c_fast^2
   };
   auto side = [&](const double (&q)[8]) {
     Side         s;
-    const double b2 = fma(q[IC], q[IC], fma(q[IB], q[IB], a2)), em = scale_down64<1>(b2);
+    const double b2 = fma(q[IC], q[IC], fma(q[IB], q[IB], a2)), em = scale_pos64<1>(b2);
     const double k2 = fma(q[IW], q[IW], fma(q[IV], q[IV], q[IU] * q[IU]));
     s.pt = q[IP] + em;
-    s.et = fma(q[IP], entho, fma(scale_down64<1>(q[ID]), k2, em));
+    s.et = fma(q[IP], entho, fma(scale_pos64<1>(q[ID]), k2, em));
     s.vb = fma(q[IW], q[IC], fma(q[IV], q[IB], q[IU] * a));
     s.n = fast_num64(gamma0 * q[IP], b2, a2);
     return s;
@@ -356,7 +356,7 @@ mhd_hlld64(const double (&ql)[8], const double (&qr)[8], double (&flux)[NF], dou
     t.r = rd * is;
     const double es = fma(rd, sus, -a2), e = fma(rd, dS, -a2), ie = rcp64(es);
     const bool   deg = positive64(a2) &&
-                     __double_as_longlong(fabs(es - a2)) <= __double_as_longlong(1e-8 * a2);
+                     __double_as_longlong(abs64(es - a2)) <= __double_as_longlong(1e-8 * a2);
     const double h = deg ? 0.0 : a * du * ie, f = deg ? 1.0 : e * ie;
     t.v = fma(-q[IB], h, q[IV]);
     t.w = fma(-q[IC], h, q[IW]);
@@ -366,7 +366,7 @@ mhd_hlld64(const double (&ql)[8], const double (&qr)[8], double (&flux)[NF], dou
     t.et = fma(a, s.vb - t.vb, fma(-s.pt, q[IU], fma(dS, s.et, psus))) * is;
     const double y = rsqrt64(t.r);
     t.sq = t.r * y;
-    t.al = fabs(a) * y;
+    t.al = abs64(a) * y;
     return t;
   };
   const Star   Ls = star(ql, L, sl, flip64(al, true), flip64(rcl, true), w), Rs = star(qr, R, sr, ar, rcr, us - ur);
@@ -869,7 +869,7 @@ mag_riemann2d_hlld64(const EdgeQ<double> & LL, const EdgeQ<double> & RL, const E
     const double s = fma(q.c, q.c, a2 + b2), g = gamma0 * q.p, ir = rcp64(q.r);
     cx = max(cx, __double_as_longlong(fast_num64(g, s, a2) * ir));
     cy = max(cy, __double_as_longlong(fast_num64(g, s, b2) * ir));
-    return q.p + scale_down64<1>(s);
+    return q.p + scale_pos64<1>(s);
   };
   const double PLL = corner(LL, a02, b02), PRL = corner(RL, a02, b12);
   const double PLR = corner(LR, a12, b02), PRR = corner(RR, a12, b12);
@@ -1113,7 +1113,7 @@ mhd_emf_corners(const EdgeCorner<R> & RT, const EdgeCorner<R> & RB, const EdgeCo
   LL.v = RT.v, RL.v = LT.v, LR.v = RB.v, RR.v = LB.v;
   auto half = [](R x) {
     if constexpr (kFast64<R>)
-      return scale_down64<1>(x);
+      return half64(x);
     else
       return R(0.5) * x;
   };

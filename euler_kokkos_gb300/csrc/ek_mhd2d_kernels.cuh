@@ -211,35 +211,55 @@ mhd2d_smem(int TX, int TY)
   return sizeof(R) * (V_N * XE * YE + (BQ > FE ? BQ : FE));
 }
 
-// trace_unsplit_mhd_2d (MHDBaseFunctor2D.h:775-1114) of the cell at Q tile
-// coordinates (qx, qy) / B tile coordinates (bx, by), written as the compact
-// trace with field stride ost.
+// The z electric field at the low corner of a cell (MHDBaseFunctor2D.h:816-835)
+// from the primitives Q(v, i, j) and face fields B(f, i, j) around it; FP64 FMA
+// build: 8 E from the sums (the factor goes into the trace's dt/dx).
+template <class R, class ACC>
+__device__ __forceinline__ R
+corner_ez(const ACC & A_, int i, int j)
+{
+  const R quarter = kFast64<R> ? R(1) : R(0.25), half = kFast64<R> ? R(1) : R(0.5);
+  auto    sum4 = [&](int v) { return A_.Q(v, i - 1, j - 1) + A_.Q(v, i - 1, j) + A_.Q(v, i, j - 1) + A_.Q(v, i, j); };
+  const R u = quarter * sum4(IU), v = quarter * sum4(IV);
+  const R A = half * (A_.B(0, i, j - 1) + A_.B(0, i, j));
+  const R B = half * (A_.B(1, i - 1, j) + A_.B(1, i, j));
+  return u * B - v * A;
+}
+
+// the shared planes of the tile kernel around a cell
 template <class R, int TX, int TY>
-__device__ __forceinline__ void
-trace2d_compact(const R * sQ, const R * sB, int qx, int qy, int bx, int by, R dtdx, R dtdy,
-                const MhdConst<R> & C, R * out, int ost)
+struct Tile2dAcc
 {
   using T = Mhd2dTile<TX, TY>;
-  auto Qv = [&](int v, int x, int y) { return sQ[(v * T::QY + y) * T::QX + x]; };
-  auto Bv = [&](int c, int x, int y) { return sB[(c * T::BY + y) * T::BX + x]; };
+  const R * q; // at the cell
+  const R * b;
+  __device__ __forceinline__ R
+  Q(int v, int i, int j) const
+  {
+    return q[(v * T::QY + j) * T::QX + i];
+  }
+  __device__ __forceinline__ R
+  B(int f, int i, int j) const
+  {
+    return b[(f * T::BY + j) * T::BX + i];
+  }
+  __device__ __forceinline__ R
+  E(int i, int j) const
+  {
+    return corner_ez<R>(*this, i, j);
+  }
+};
 
-  // edge electric fields around the cell (MHDBaseFunctor2D.h:816-835)
-  R Ez[2][2];
-#pragma unroll
-  for (int di = 0; di < 2; ++di)
-#pragma unroll
-    for (int dj = 0; dj < 2; ++dj)
-    {
-      const int x0 = qx + di - 1, y0 = qy + dj - 1;
-      // FP64 FMA build: 8 E from the sums (the factor goes into dt/dx below)
-      const R   quarter = kFast64<R> ? R(1) : R(0.25), half = kFast64<R> ? R(1) : R(0.5);
-      const R   u = quarter * (Qv(IU, x0, y0) + Qv(IU, x0, y0 + 1) + Qv(IU, x0 + 1, y0) + Qv(IU, x0 + 1, y0 + 1));
-      const R   v = quarter * (Qv(IV, x0, y0) + Qv(IV, x0, y0 + 1) + Qv(IV, x0 + 1, y0) + Qv(IV, x0 + 1, y0 + 1));
-      const R   A = half * (Bv(0, bx + di, by + dj - 1) + Bv(0, bx + di, by + dj));
-      const R   B = half * (Bv(1, bx + di - 1, by + dj) + Bv(1, bx + di, by + dj));
-      Ez[di][dj] = u * B - v * A;
-    }
-  const R ELL = Ez[0][0], ELR = Ez[0][1], ERL = Ez[1][0], ERR = Ez[1][1];
+// trace_unsplit_mhd_2d (MHDBaseFunctor2D.h:775-1114) of one cell, written as the
+// compact trace with field stride ost.
+template <class R, class ACC>
+__device__ __forceinline__ void
+trace2d_compact(const ACC & A_, R dtdx, R dtdy, const MhdConst<R> & C, R * out, long long ost)
+{
+  auto Qv = [&](int v, int x, int y) { return A_.Q(v, x, y); };
+  auto Bv = [&](int c, int x, int y) { return A_.B(c, x, y); };
+  constexpr int qx = 0, qy = 0, bx = 0, by = 0;
+  const R ELL = A_.E(0, 0), ELR = A_.E(0, 1), ERL = A_.E(1, 0), ERR = A_.E(1, 1);
 
   R q[8];
 #pragma unroll
@@ -272,7 +292,7 @@ trace2d_compact(const R * sQ, const R * sB, int qx, int qy, int bx, int by, R dt
 
   R dAx, dBy;
   if constexpr (kFast64<R>)
-    dAx = scale_down64<1>(AR - AL), dBy = scale_down64<1>(BR - BL);
+    dAx = half64(AR - AL), dBy = half64(BR - BL);
   else
     dAx = R(0.5) * (AR - AL), dBy = R(0.5) * (BR - BL);
   const R gamma = C.gamma0;
@@ -414,7 +434,8 @@ mhd2d_tile(const void * __restrict__ Uin, void * __restrict__ Uout, const KParam
   for (int c = threadIdx.x; c < T::PL; c += NT)
   {
     const int x = c % T::XE, y = c / T::XE;
-    trace2d_compact<R, TX, TY>(sQ, sB, x + 1, y + 1, x + 1, y + 1, dtdx, dtdy, C, sT + c, T::PL);
+    trace2d_compact<R>(Tile2dAcc<R, TX, TY>{ sQ + (y + 1) * T::QX + x + 1, sB + (y + 1) * T::BX + x + 1 }, dtdx, dtdy, C,
+                       sT + c, T::PL);
   }
   __syncthreads();
 
@@ -709,23 +730,13 @@ mhd2d_step_t(int phase, const void * Uin, void * Uout, void * work, const KParam
       return cudaGetLastError();
     }
   }
-  // Mixed: 16 x 16 at every size.  FP64 (us per step; a tile's time is set by
-  // its chain of FP64 instructions, so a whole wave of CTAs counts): 8 x 8 with
-  // 128 threads up to three CTAs per SM (64^2: 50; 16 x 8 82, 16 x 16 117; 200 x
-  // 136: 102, 117, 117), 16 x 8 up to the three that fit in shared memory (256 x
-  // 200: 164; 8 x 8 210, 16 x 16 205), then 16 x 16 (256^2: 205; 16 x 8 314;
-  // 512^2: 692 and 774).
+  // Mixed: 16 x 16 at every size.  FP64, on grids too small for the passes: 8 x
+  // 8 with 128 threads (64^2: 50 us; 16 x 8 82, 16 x 16 117; 200 x 136: 102, 117,
+  // 117), since a tile's chain of FP64 instructions sets its time.
   if constexpr (sizeof(R) == 4)
     return mhd2d_step_tiled<S, R, M2_TX, M2_TY, M2_TX * M2_TY>(Uin, Uout, work, P, clk, step, st);
   else
-  {
-    auto tiles = [&](int tx, int ty) { return (long long)((P.nx + tx - 1) / tx) * ((P.ny + ty - 1) / ty); };
-    if (tiles(8, 8) <= 3ll * P.sms)
-      return mhd2d_step_tiled<S, R, 8, 8, 128>(Uin, Uout, work, P, clk, step, st);
-    if (tiles(16, 8) <= 3ll * P.sms)
-      return mhd2d_step_tiled<S, R, 16, 8, 128>(Uin, Uout, work, P, clk, step, st);
-    return mhd2d_step_tiled<S, R, M2_TX, M2_TY, M2_TX * M2_TY>(Uin, Uout, work, P, clk, step, st);
-  }
+    return mhd2d_step_tiled<S, R, 8, 8, 128>(Uin, Uout, work, P, clk, step, st);
 }
 
 // the repair pass's tile list of the mixed form (cleared by the caller before

@@ -217,92 +217,94 @@ struct TraceTile
   static constexpr int EX = TX + 1, EY = TY + 1, EP = 3 * EX * EY;
 };
 
+// The shared planes of the tile kernel around cell (tx, ty): Q(v, i, j, k),
+// B(f, i, j, k) and E(d, i, j, k) at the offset (i, j, k) from the cell.
 template <class R, int TX, int TY>
-__device__ __forceinline__ void
-trace_cell_compact(const R * sB, int bslot[4], const R * sQ, int qslot[3], const R * sE,
-                   int eslot[2], int tx, int ty, R dtdx, R dtdy, R dtdz, const MhdConst<R> & C,
-                   R * out)
+struct TileTraceAcc
 {
   using T = TraceTile<TX, TY>;
-  // local tile coordinates of the cell in each buffer
-  const int qx = tx + 1, qy = ty + 1; // sQ
-  const int bx = tx + 1, by = ty + 1; // sB
-  const int ex = tx, ey = ty;         // sE
-  const R * Q0 = sQ + qslot[1] * T::QP;
-  const R * Qm = sQ + qslot[0] * T::QP;
-  const R * Qp = sQ + qslot[2] * T::QP;
-  auto Qv = [&](const R * pl, int v, int x, int y) { return pl[(v * T::QY + y) * T::QX + x]; };
-  auto Bv = [&](int slot, int comp, int x, int y) {
-    return sB[bslot[slot] * T::BP + (comp * T::BY + y) * T::BX + x];
-  };
-  auto Ev = [&](int slot, int comp, int x, int y) {
-    return sE[eslot[slot] * T::EP + (comp * T::EY + y) * T::EX + x];
-  };
+  const R * q[3]; // planes k-1..k+1, at the cell
+  const R * b[3];
+  const R * e[2]; // planes k, k+1
+  __device__ __forceinline__
+  TileTraceAcc(const R * sB, const int (&bslot)[4], const R * sQ, const int (&qslot)[3], const R * sE,
+               const int (&eslot)[2], int tx, int ty)
+  {
+#pragma unroll
+    for (int p = 0; p < 3; ++p)
+    {
+      q[p] = sQ + qslot[p] * T::QP + (ty + 1) * T::QX + tx + 1;
+      b[p] = sB + bslot[p] * T::BP + (ty + 1) * T::BX + tx + 1;
+    }
+#pragma unroll
+    for (int p = 0; p < 2; ++p)
+      e[p] = sE + eslot[p] * T::EP + ty * T::EX + tx;
+  }
+  __device__ __forceinline__ R
+  Q(int v, int i, int j, int k) const
+  {
+    return q[k + 1][(v * T::QY + j) * T::QX + i];
+  }
+  __device__ __forceinline__ R
+  B(int f, int i, int j, int k) const
+  {
+    return b[k + 1][(f * T::BY + j) * T::BX + i];
+  }
+  __device__ __forceinline__ R
+  E(int d, int i, int j, int k) const
+  {
+    return e[k][(d * T::EY + j) * T::EX + i];
+  }
+};
+
+// The compact trace of one cell (trace_unsplit_mhd_3d_simpler) from the
+// primitives, face fields and edge fields around it.
+template <class R, class ACC>
+__device__ __forceinline__ void
+trace_state(const ACC & A_, R dtdx, R dtdy, R dtdz, const MhdConst<R> & C, R (&o)[T_N])
+{
 
   // hydro slopes (slope_unsplit_hydro_3d, MHDBaseFunctor3D.h:340-470); the
   // z-slope of IC uses qMinusY as the reference does (unused by the trace)
   R q[8], dq[3][8];
 #pragma unroll
   for (int v = 0; v < 8; ++v)
-    q[v] = Qv(Q0, v, qx, qy);
-  if (C.slope_type == R(1) || C.slope_type == R(2))
-  {
+    q[v] = A_.Q(v, 0, 0, 0);
 #pragma unroll
-    for (int v = 0; v < 8; ++v)
-    {
-      dq[0][v] = slope_h<R>(q[v], Qv(Q0, v, qx + 1, qy), Qv(Q0, v, qx - 1, qy), C.slope_type);
-      dq[1][v] = slope_h<R>(q[v], Qv(Q0, v, qx, qy + 1), Qv(Q0, v, qx, qy - 1), C.slope_type);
-      dq[2][v] = slope_h<R>(q[v], Qv(Qp, v, qx, qy), v == IC ? Qv(Q0, v, qx, qy - 1) : Qv(Qm, v, qx, qy),
-                           C.slope_type);
-    }
-  }
-  else
+  for (int v = 0; v < 8; ++v)
   {
-#pragma unroll
-    for (int v = 0; v < 8; ++v)
-      dq[0][v] = dq[1][v] = dq[2][v] = R(0);
+    dq[0][v] = slope_h<R>(q[v], A_.Q(v, 1, 0, 0), A_.Q(v, -1, 0, 0), C.slope_type);
+    dq[1][v] = slope_h<R>(q[v], A_.Q(v, 0, 1, 0), A_.Q(v, 0, -1, 0), C.slope_type);
+    dq[2][v] = slope_h<R>(q[v], A_.Q(v, 0, 0, 1), v == IC ? A_.Q(v, 0, -1, 0) : A_.Q(v, 0, 0, -1), C.slope_type);
   }
-  // face fields of the cell (bfNb, MHDRunFunctors3D.h:790-795); planes: 0 k-1, 1 k, 2 k+1
-  const R AL = (R)Bv(1, 0, bx, by), AR = (R)Bv(1, 0, bx + 1, by);
-  const R BL = (R)Bv(1, 1, bx, by), BR = (R)Bv(1, 1, bx, by + 1);
-  const R CL = (R)Bv(1, 2, bx, by), CR = (R)Bv(2, 2, bx, by);
-  // transverse face-field slopes (slope_unsplit_mhd_3d, MHDBaseFunctor3D.h:563-668)
-  const R xst = fmin(C.slope_type, R(2.0));
-  auto    sA = [&](int x, int y, bool zdir) {
-    const R b = (R)Bv(1, 0, x, y);
-    return zdir ? slope_h<R>(b, (R)Bv(2, 0, x, y), (R)Bv(0, 0, x, y), xst)
-                   : slope_h<R>(b, (R)Bv(1, 0, x, y + 1), (R)Bv(1, 0, x, y - 1), xst);
-  };
-  auto sBf = [&](int x, int y, bool zdir) {
-    const R b = (R)Bv(1, 1, x, y);
-    return zdir ? slope_h<R>(b, (R)Bv(2, 1, x, y), (R)Bv(0, 1, x, y), xst)
-                : slope_h<R>(b, (R)Bv(1, 1, x + 1, y), (R)Bv(1, 1, x - 1, y), xst);
-  };
-  auto sC = [&](int slot, int x, int y, bool ydir) {
-    const R b = (R)Bv(slot, 2, x, y);
-    return ydir ? slope_h<R>(b, (R)Bv(slot, 2, x, y + 1), (R)Bv(slot, 2, x, y - 1), xst)
-                : slope_h<R>(b, (R)Bv(slot, 2, x + 1, y), (R)Bv(slot, 2, x - 1, y), xst);
+  // face fields of the cell (bfNb, MHDRunFunctors3D.h:790-795)
+  const R AL = A_.B(0, 0, 0, 0), AR = A_.B(0, 1, 0, 0);
+  const R BL = A_.B(1, 0, 0, 0), BR = A_.B(1, 0, 1, 0);
+  const R CL = A_.B(2, 0, 0, 0), CR = A_.B(2, 0, 0, 1);
+  // transverse face-field slopes (slope_unsplit_mhd_3d, MHDBaseFunctor3D.h:563-668):
+  // of component f at (i, j, k) along e
+  const R xst = C.slope_type; // 1 or 2 (the reference takes the smaller of it and 2)
+  auto    sB = [&](int f, int i, int j, int k, int e) {
+    const int di = e == 0, dj = e == 1, dk = e == 2;
+    return slope_h<R>(A_.B(f, i, j, k), A_.B(f, i + di, j + dj, k + dk), A_.B(f, i - di, j - dj, k - dk), xst);
   };
   R dbf[12];
-  dbf[0] = sA(bx, by, false);      // DeltaA(i,j,k).y
-  dbf[1] = sA(bx, by, true);       // DeltaA(i,j,k).z
-  dbf[2] = sBf(bx, by, false);     // DeltaB(i,j,k).x
-  dbf[3] = sBf(bx, by, true);      // DeltaB(i,j,k).z
-  dbf[4] = sC(1, bx, by, false);   // DeltaC(i,j,k).x
-  dbf[5] = sC(1, bx, by, true);    // DeltaC(i,j,k).y
-  dbf[6] = sA(bx + 1, by, false);  // DeltaA(i+1,j,k).y
-  dbf[7] = sA(bx + 1, by, true);   // DeltaA(i+1,j,k).z
-  dbf[8] = sBf(bx, by + 1, false); // DeltaB(i,j+1,k).x
-  dbf[9] = sBf(bx, by + 1, true);  // DeltaB(i,j+1,k).z
-  dbf[10] = sC(2, bx, by, false);  // DeltaC(i,j,k+1).x
-  dbf[11] = sC(2, bx, by, true);   // DeltaC(i,j,k+1).y
+  dbf[0] = sB(0, 0, 0, 0, 1);  // DeltaA(i,j,k).y
+  dbf[1] = sB(0, 0, 0, 0, 2);  // DeltaA(i,j,k).z
+  dbf[2] = sB(1, 0, 0, 0, 0);  // DeltaB(i,j,k).x
+  dbf[3] = sB(1, 0, 0, 0, 2);  // DeltaB(i,j,k).z
+  dbf[4] = sB(2, 0, 0, 0, 0);  // DeltaC(i,j,k).x
+  dbf[5] = sB(2, 0, 0, 0, 1);  // DeltaC(i,j,k).y
+  dbf[6] = sB(0, 1, 0, 0, 1);  // DeltaA(i+1,j,k).y
+  dbf[7] = sB(0, 1, 0, 0, 2);  // DeltaA(i+1,j,k).z
+  dbf[8] = sB(1, 0, 1, 0, 0);  // DeltaB(i,j+1,k).x
+  dbf[9] = sB(1, 0, 1, 0, 2);  // DeltaB(i,j+1,k).z
+  dbf[10] = sB(2, 0, 0, 1, 0); // DeltaC(i,j,k+1).x
+  dbf[11] = sB(2, 0, 0, 1, 1); // DeltaC(i,j,k+1).y
   // edge electric fields around the cell (MHDRunFunctors3D.h:808-823)
-  const R ELL = Ev(0, 0, ex, ey), ELR = Ev(1, 0, ex, ey), ERL = Ev(0, 0, ex, ey + 1),
-          ERR = Ev(1, 0, ex, ey + 1);
-  const R FLL = Ev(0, 1, ex, ey), FLR = Ev(1, 1, ex, ey), FRL = Ev(0, 1, ex + 1, ey),
-          FRR = Ev(1, 1, ex + 1, ey);
-  const R GLL = Ev(0, 2, ex, ey), GLR = Ev(0, 2, ex, ey + 1), GRL = Ev(0, 2, ex + 1, ey),
-          GRR = Ev(0, 2, ex + 1, ey + 1);
+  const R ELL = A_.E(0, 0, 0, 0), ELR = A_.E(0, 0, 0, 1), ERL = A_.E(0, 0, 1, 0), ERR = A_.E(0, 0, 1, 1);
+  const R FLL = A_.E(1, 0, 0, 0), FLR = A_.E(1, 0, 0, 1), FRL = A_.E(1, 1, 0, 0), FRR = A_.E(1, 1, 0, 1);
+  const R GLL = A_.E(2, 0, 0, 0), GLR = A_.E(2, 0, 1, 0), GRL = A_.E(2, 1, 0, 0), GRR = A_.E(2, 1, 1, 0);
 
   // trace_unsplit_mhd_3d_simpler (MHDBaseFunctor3D.h:751-917), Omega0 = 0
   R r = q[ID], p = q[IP], u = q[IU], v = q[IV], w = q[IW], A = q[IA], B = q[IB], Cc = q[IC];
@@ -323,12 +325,11 @@ trace_cell_compact(const R * sB, int bslot[4], const R * sQ, int qslot[3], const
           dBRz = hs * dbf[9], dCRx = hs * dbf[10], dCRy = hs * dbf[11];
   R dAx, dBy, dCz;
   if constexpr (kFast64<R>)
-    dAx = scale_down64<1>(AR - AL), dBy = scale_down64<1>(BR - BL), dCz = scale_down64<1>(CR - CL);
+    dAx = half64(AR - AL), dBy = half64(BR - BL), dCz = half64(CR - CL);
   else
     dAx = R(0.5) * (AR - AL), dBy = R(0.5) * (BR - BL), dCz = R(0.5) * (CR - CL);
   const R gamma = C.gamma0;
   const R C_ = Cc;
-  R       o[T_N];
   if constexpr (kFast64<R>)
   {
     // FP64 FMA build: FMA chains onto the state, B / rho once; the edge
@@ -418,7 +419,14 @@ trace_cell_compact(const R * sB, int bslot[4], const R * sQ, int qslot[3], const
   o[T_DCLY] = dCLy;
   o[T_DARY] = dARy, o[T_DARZ] = dARz, o[T_DBRX] = dBRx, o[T_DBRZ] = dBRz, o[T_DCRX] = dCRx,
   o[T_DCRY] = dCRy;
-  // one 16-byte store per quad (the last quad's spare fields are zero)
+}
+
+// one cell's compact trace: one 16-byte store per quad (the last quad's spare
+// fields are zero)
+template <class R>
+__device__ __forceinline__ void
+store_trace(const R (&o)[T_N], R * out)
+{
 #pragma unroll
   for (int q = 0; q < kTQuads<R>; ++q)
   {
@@ -650,8 +658,9 @@ mhd_trace_kernel(const void * __restrict__ U, R * __restrict__ trace, KParams P,
       int bslot[4] = { bsl(k - 1), bsl(k), bsl(k + 1), bsl(k + 2) };
       int qslot[3] = { qsl(k - 1), qsl(k), qsl(k + 1) };
       int eslot[2] = { esl(k), esl(k + 1) };
-      trace_cell_compact<R, TX, TY>(sB, bslot, sQ, qslot, sE, eslot, tx, ty, dtdx, dtdy, dtdz, C,
-                                    trace_cell(trace, tg, gw, c0 + tx, d0 + ty, k));
+      R   o[T_N];
+      trace_state<R>(TileTraceAcc<R, TX, TY>(sB, bslot, sQ, qslot, sE, eslot, tx, ty), dtdx, dtdy, dtdz, C, o);
+      store_trace<R>(o, trace_cell(trace, tg, gw, c0 + tx, d0 + ty, k));
     }
     __syncthreads();
   }

@@ -43,7 +43,7 @@ errors(int spread)
     at_most(3, fabs(sqrt_ratio64(n, d) / sqrt(n / d) - 1.0));
     // scaling and slopes are exact: any difference counts as 2^53
     const double a = flip64(n, z & 1), b = flip64(d, z & 2), c = flip64(value(mix(z + 2), spread / 2), z & 4);
-    at_most(4, scale_down64<1>(a) == 0.5 * a && scale_down64<2>(b) == 0.25 * b ? 0.0 : 1.0);
+    at_most(4, half64(a) == 0.5 * a && scale_pos64<2>(d) == 0.25 * d && abs64(a) == fabs(a) ? 0.0 : 1.0);
     for (int st = 0; st < 3; ++st)
     {
       const double dl = st * (a - b), dr = st * (c - a), dc = 0.5 * (c - b);
@@ -62,8 +62,9 @@ specials()
   const bool   ok = rcp64(0.0) == inf && rcp64(-0.0) == -inf && rcp64(inf) == 0.0 && isnan(rcp64(NAN)) &&
                   rsqrt64(0.0) == inf && rsqrt64(inf) == 0.0 && isnan(rsqrt64(-1.0)) && isnan(rsqrt64(NAN)) &&
                   sqrt64(0.0) == 0.0 && sqrt64(inf) == inf && isnan(sqrt64(-1.0)) && isnan(sqrt64(NAN)) &&
-                  sqrt_ratio64(0.0, 2.0) == 0.0 && isnan(sqrt_ratio64(NAN, 1.0)) && isnan(scale_down64<1>(NAN)) &&
-                  scale_down64<1>(inf) == inf && scale_down64<2>(0.0) == 0.0 && scale_down64<1>(5e-324) == 0.0 &&
+                  sqrt_ratio64(0.0, 2.0) == 0.0 && isnan(sqrt_ratio64(NAN, 1.0)) && isnan(half64(NAN)) &&
+                  half64(inf) == inf && half64(-0.0) == 0.0 && half64(5e-324) == 0.0 && half64(-3e-308) == -1.5e-308 &&
+                  scale_pos64<2>(0.0) == 0.0 &&
                   max_cand64(1.0, NAN) == 1.0 && max_cand64(-inf, 2.0) == 2.0 && floor_ratio64(-3.0, 8.0, 1e-20) == 8e-20;
   g_out[7] = ok ? 0.0 : 1.0;
 }

@@ -1,4 +1,4 @@
-"""The kernels' tile and chunk choices: grids at the edges of the tiles and on
+"""The kernels' choices by grid: sizes at the edges of tiles and blocks and on
 both sides of the lines between them, exact build against the oracle (bitwise)
 and FP64 FMA build within its tolerances."""
 
@@ -12,13 +12,15 @@ from helpers import interior, rel_linf
 
 pytestmark = pytest.mark.gpu
 
-# 2D: 8 x 8 tiles up to six per SM (240^2: 900 tiles on 152 SMs), 16 x 16 above (248 x 240: 930)
-CASES = [(2, False, s) for s in [(2, 2, 1), (8, 8, 1), (9, 7, 1), (17, 16, 1), (240, 240, 1), (248, 240, 1), (257, 241, 1)]]
-# 2D MHD: 8 x 8 up to three per SM (170 x 165: 462 tiles, 160 x 160: 400), 16 x 8 up to three (240 x 240: 450), then 16 x 16
-CASES += [(2, True, s) for s in [(3, 3, 1), (8, 9, 1), (17, 8, 1), (160, 160, 1), (170, 165, 1), (240, 240, 1), (250, 243, 1)]]
-# 3D: planes per CTA from the grid (kchunk 0)
-CASES += [(3, False, s) for s in [(2, 2, 2), (16, 16, 33), (17, 33, 9)]]
-CASES += [(3, True, s) for s in [(3, 3, 3), (16, 8, 21), (33, 9, 14)]]
+# 2D hydro: 8 x 8 tiles up to six per SM (240^2: 900 tiles on 152 SMs), 16 x 16 above (248 x 240: 930), passes from
+# 2^18 cells (512^2)
+CASES = [(2, False, s) for s in [(2, 2, 1), (8, 8, 1), (9, 7, 1), (17, 16, 1), (240, 240, 1), (248, 240, 1), (511, 513, 1),
+                                 (512, 512, 1)]]
+# 2D MHD: 8 x 8 tiles up to three per SM (170 x 160: 440), then passes
+CASES += [(2, True, s) for s in [(3, 3, 1), (8, 9, 1), (17, 8, 1), (170, 160, 1), (171, 178, 1)]]
+# 3D: passes; blocks of 128 threads
+CASES += [(3, False, s) for s in [(2, 2, 2), (16, 16, 33), (17, 33, 9), (127, 2, 3)]]
+CASES += [(3, True, s) for s in [(3, 3, 3), (16, 8, 21), (33, 9, 14), (129, 3, 4)]]
 
 
 @pytest.mark.parametrize("dim,mhd,n", CASES, ids=["%s%dd_%dx%dx%d" % ("mhd" if m else "hydro", d, *n) for d, m, n in CASES])
@@ -37,3 +39,24 @@ def test_tiles_match_the_oracle(dim, mhd, n):
             assert np.array_equal(U, ref) and np.array_equal(d, dts)
         else:
             assert np.max(rel_linf(U, ref)[[0, 1]]) <= 1e-11 and np.max(np.abs(d / dts - 1)) <= 1e-13
+
+
+@pytest.mark.parametrize("mhd", [False, True], ids=["hydro", "mhd"])
+def test_slabs_do_not_show(mhd):
+    """A grid whose workspace takes several slabs of passes (the trace of 262144-cell planes, 1 GiB a slab): the mixed
+    form's tile kernels are the independent result, within the mixed form's tolerance, and symmetric halves of a
+    z-periodic state stay equal bit for bit across the slab boundaries."""
+    ini, U0 = P.smooth_random(dim=3, mhd=mhd, nx=512, ny=512, nz=10, seed=3, nsteps=2)
+    gw = 3 if mhd else 2
+    k = np.arange(10 + 2 * gw)
+    U0 = np.ascontiguousarray(U0[:, (k - gw) % 2 + gw])  # period two in z
+    if mhd:
+        U0[7] = 0.0
+    with ek.Solver(ek.params_from_ini(ini)) as s, ek.Solver(ek.params_from_ini(ini, precision=ek.EK_PREC_MIXED)) as m:
+        s.set_state(U0)
+        m.set_state(U0)
+        assert s.run(2) == m.run(2) == 2
+        U, V = interior(s.get_state(), gw, 3), interior(m.get_state(), gw, 3)
+    for z in range(2, 10):
+        assert np.array_equal(U[:, z], U[:, z % 2])
+    assert np.abs(U[0] - V[0]).sum() / np.abs(U[0]).sum() <= 1e-5
