@@ -353,6 +353,7 @@ hydro2d_tile(const S * __restrict__ Uin, S * __restrict__ Uout, const KParams & 
     else
       tmax = max_cand(tmax, hydro_invdt<R, NV>(us, C, P));
   }
+  chain_next();
   block_max_commit<NT>(cand_key((double)tmax), &clk->key[(step + 1) % 3]);
   if (bx == 0 && by == 0 && threadIdx.x == 0)
     step_commit(clk, step, t, dt);
@@ -848,6 +849,7 @@ hydro3d_step(const S * __restrict__ Uin, S * __restrict__ Uout, KParams P, DevCl
     }
     __syncthreads(); // ring slot and face buffers are reused next plane
   }
+  chain_next();
   block_max_commit<NT>(cand_key((double)tmax), &clk->key[(step + 1) % 3]);
   if (blockIdx.x == 0 && blockIdx.y == 0 && blockIdx.z == 0 && threadIdx.x == 0)
     step_commit(clk, step, t, dt);

@@ -67,7 +67,8 @@ template <int NV>
 __global__ void __launch_bounds__(kPassThreads)
 hydro_prims_pass(const double * __restrict__ U, const KParams P, const DevClock * clk, int step, HydroSlab<NV> S)
 {
-  if (!clk->sc[step % 3].active || clk->sc[step % 3].step != step)
+  StepConsts sc;
+  if (!step_consts(clk, step, sc))
     return;
   const long long c = pass_index(), n = S.box(4);
   if (c >= n)
@@ -83,6 +84,7 @@ hydro_prims_pass(const double * __restrict__ U, const KParams P, const DevClock 
 #pragma unroll
   for (int v = 0; v < NV; ++v)
     S.q[v * n + c] = q[v];
+  chain_next();
 }
 
 template <int NV, bool GRAV>
@@ -178,6 +180,7 @@ hydro_trace_pass(const KParams P, const DevClock * clk, int step, HydroSlab<NV> 
         out[((2 * a + h) * NV + v) * ns] = f[v];
     }
   }
+  chain_next();
 }
 
 // faces of one axis, padded to whole blocks: (nx + 1) ny nz along x and so on
@@ -230,6 +233,7 @@ hydro_flux_pass(const KParams P, const DevClock * clk, int step, HydroSlab<NV> S
 #pragma unroll
   for (int v = 0; v < NV; ++v)
     out[var(v) * nf] = flux_scaled(fl[v], dtd);
+  chain_next();
 }
 
 template <int NV, bool GRAV>
@@ -285,6 +289,7 @@ hydro_update_pass(const double * __restrict__ Uin, double * __restrict__ Uout, c
     else
       tmax = hydro_invdt<double, NV>(u, C, P);
   }
+  chain_next();
   block_max_commit<kPassThreads>(cand_key(tmax), &clk->key[(step + 1) % 3]);
   if (!S.last)
     return;
@@ -340,12 +345,18 @@ hydro_step_passes(const void * Uin, void * Uout, void * work, const KParams & P,
     long long           fb = 0;
     for (int a = 0; a < DIM; ++a)
       fb += face_blocks(S, a);
-    hydro_prims_pass<NV><<<blocks(S.box(4)), kPassThreads, 0, st>>>(in, P, clk, step, S);
-    hydro_trace_pass<NV, GRAV><<<blocks(cells + ring), kPassThreads, 0, st>>>(P, clk, step, S);
-    hydro_flux_pass<NV, RS><<<(unsigned)fb, kPassThreads, 0, st>>>(P, clk, step, S);
-    hydro_update_pass<NV, GRAV><<<blocks(cells), kPassThreads, 0, st>>>(in, (double *)Uout, P, clk, step, S);
+    cudaError_t e = launch_chained(hydro_prims_pass<NV>, blocks(S.box(4)), kPassThreads, 0, st, in, P, clk, step, S);
+    if (e == cudaSuccess)
+      e = launch_chained(hydro_trace_pass<NV, GRAV>, blocks(cells + ring), kPassThreads, 0, st, P, clk, step, S);
+    if (e == cudaSuccess)
+      e = launch_chained(hydro_flux_pass<NV, RS>, (unsigned)fb, kPassThreads, 0, st, P, clk, step, S);
+    if (e == cudaSuccess)
+      e = launch_chained(hydro_update_pass<NV, GRAV>, blocks(cells), kPassThreads, 0, st, in, (double *)Uout, P, clk,
+                         step, S);
+    if (e != cudaSuccess)
+      return e;
   }
-  return cudaGetLastError();
+  return cudaSuccess;
 }
 
 } // namespace EK_NS

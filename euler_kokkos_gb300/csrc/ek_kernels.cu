@@ -45,8 +45,8 @@ hydro2d_step_tiled(const void * Uin, void * Uout, const KParams & P, DevClock * 
   if (e != cudaSuccess)
     return e;
   dim3 grid((P.nx + TX - 1) / TX, (P.ny + TY - 1) / TY, 1);
-  k<<<grid, NT, sm, st>>>((const S *)Uin, (S *)Uout, P, clk, step);
-  return cudaGetLastError();
+  const bool chained = sizeof(R) == 4 || chain_tiles(P, (long long)grid.x * grid.y);
+  return launch_step_kernel(chained, k, grid, NT, sm, st, (const S *)Uin, (S *)Uout, P, clk, step);
 }
 
 template <class S, class R, int RS, bool GRAV>
@@ -101,8 +101,7 @@ hydro_step_rs(int dim, const void * Uin, void * Uout, void * work, const KParams
     std::memset(&m, 0, sizeof m);
     if (tmap)
       m = *tmap;
-    k<<<grid, H3_TX * H3_TY, sm, st>>>((const S *)Uin, (S *)Uout, P, clk, step, m);
-    return cudaGetLastError();
+    return launch_chained(k, grid, H3_TX * H3_TY, sm, st, (const S *)Uin, (S *)Uout, P, clk, step, m);
   }
 }
 

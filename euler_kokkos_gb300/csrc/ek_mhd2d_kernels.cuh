@@ -630,6 +630,7 @@ mhd2d_tile(const void * __restrict__ Uin, void * __restrict__ Uout, const KParam
     });
     tmax = mhd2d_invdt<R>(q, C, P);
   }
+  chain_next();
   if (!dirty)
     block_max_commit<NT>(cand_key((double)tmax), &clk->key[(step + 1) % 3]);
   else if (threadIdx.x == 0)
@@ -698,8 +699,8 @@ mhd2d_step_tiled(const void * Uin, void * Uout, void * work, const KParams & P, 
     return e;
   dim3  grid((P.nx + TX - 1) / TX, (P.ny + TY - 1) / TY, 1);
   int * repair = sizeof(R) == 4 && P.riemann == 4 ? (int *)work : nullptr;
-  k<<<grid, NT, sm, st>>>(Uin, Uout, P, clk, step, repair);
-  return cudaGetLastError();
+  const bool chained = sizeof(R) == 4 || chain_tiles(P, (long long)grid.x * grid.y);
+  return launch_step_kernel(chained, k, grid, NT, sm, st, Uin, Uout, P, clk, step, repair);
 }
 
 template <class S, class R>
@@ -726,8 +727,7 @@ mhd2d_step_t(int phase, const void * Uin, void * Uout, void * work, const KParam
       cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, sm);
       if (e != cudaSuccess)
         return e;
-      k<<<repair_grid(mhd2d_tiles(P)), M2_TX * M2_TY, sm, st>>>(Uin, Uout, P, clk, step, (int *)work);
-      return cudaGetLastError();
+      return launch_chained(k, repair_grid(mhd2d_tiles(P)), M2_TX * M2_TY, sm, st, Uin, Uout, P, clk, step, (int *)work);
     }
   }
   // Mixed: 16 x 16 at every size.  FP64, on grids too small for the passes: 8 x

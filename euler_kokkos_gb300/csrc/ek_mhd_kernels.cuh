@@ -664,6 +664,7 @@ mhd_trace_kernel(const void * __restrict__ U, R * __restrict__ trace, KParams P,
     }
     __syncthreads();
   }
+  chain_next();
   cp_async_wait_all(); // no copy may land after the block has left
 }
 
@@ -1084,6 +1085,7 @@ mhd_update_tile(const void * __restrict__ Uin, void * __restrict__ Uout, const R
                              bz1 };
       cfl_cell(u, bl, br);
     }
+    chain_next();
     if (!dirty)
       block_max_commit<NT>(cand_key((double)tmax), &clk->key[(step + 1) % 3]);
   }
@@ -1273,8 +1275,7 @@ mhd_step_t(int phase, const void * Uin, void * Uout, void * work, const KParams 
       return e;
     const int nt = P.nz + 2;
     dim3      grid((P.nx + 2 + TX - 1) / TX, (P.ny + 2 + TY - 1) / TY, (nt + P.kchunk_trace - 1) / P.kchunk_trace);
-    k<<<grid, TX * TY, sm, st>>>(Uin, mhd_trace_of<R>(work, P), P, clk, step);
-    return cudaGetLastError();
+    return launch_chained(k, grid, TX * TY, sm, st, Uin, mhd_trace_of<R>(work, P), P, clk, step);
   }
   // 4. the repair pass of the mixed HLLD form (after phase 2)
   if (phase == 3)
@@ -1290,9 +1291,8 @@ mhd_step_t(int phase, const void * Uin, void * Uout, void * work, const KParams 
       cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, sm);
       if (e != cudaSuccess)
         return e;
-      k<<<repair_grid(repair_tiles(P, MU_TX, MU_TY)), MU_TX * MU_TY, sm, st>>>(
-        Uin, Uout, mhd_trace_of<R>(work, P), P, clk, step, cfl_next ? 1 : 0, (int *)work);
-      return cudaGetLastError();
+      return launch_chained(k, repair_grid(repair_tiles(P, MU_TX, MU_TY)), MU_TX * MU_TY, sm, st, Uin, Uout,
+                            mhd_trace_of<R>(work, P), P, clk, step, cfl_next ? 1 : 0, (int *)work);
     }
   }
   // 3. fluxes, emfs, update (trace read through L1, or staged in shared memory
@@ -1310,8 +1310,8 @@ mhd_step_t(int phase, const void * Uin, void * Uout, void * work, const KParams 
       return e;
     dim3 grid((P.nx + TX - 1) / TX, (P.ny + TY - 1) / TY, (P.nz + P.kchunk - 1) / P.kchunk);
     int * repair = sizeof(R) == 4 && P.riemann == 4 ? (int *)work : nullptr;
-    k<<<grid, TX * TY, sm, st>>>(Uin, Uout, mhd_trace_of<R>(work, P), P, clk, step, cfl_next ? 1 : 0, repair);
-    return cudaGetLastError();
+    return launch_chained(k, grid, TX * TY, sm, st, Uin, Uout, mhd_trace_of<R>(work, P), P, clk, step, cfl_next ? 1 : 0,
+                          repair);
   }
 }
 

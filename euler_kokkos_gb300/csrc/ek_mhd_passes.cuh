@@ -62,6 +62,7 @@ template <int DIM>
 __global__ void __launch_bounds__(kPassThreads)
 mhd_prims_pass(const void * __restrict__ U, const KParams P, DevClock * clk, int step, MhdSlab<DIM> S)
 {
+  chain_begin();
   // a step that must not run (finished, or an earlier one did not run)
   if (clk->sid[step % 3] != step || clk->t[step % 3] >= P.tEnd - 1e-14)
     return;
@@ -109,6 +110,7 @@ mhd_prims_pass(const void * __restrict__ U, const KParams P, DevClock * clk, int
       }
     }
   }
+  chain_next();
   block_max_commit<kPassThreads>(cand_key(tmax), &clk->key[step % 3]);
   finalize_step(clk, P, step); // dt and its ratios for the other passes
 }
@@ -188,6 +190,7 @@ mhd_efield_pass(const KParams P, const DevClock * clk, int step, MhdSlab<DIM> S)
     B = half * (A_.B(1, -1, 0, 0) + A_.B(1, 0, 0, 0));
     S.e[2 * P.vstride + o] = uu * B - vv * A;
   }
+  chain_next();
 }
 
 template <int DIM>
@@ -215,6 +218,7 @@ mhd_trace_pass(const KParams P, const DevClock * clk, int step, MhdSlab<DIM> S)
     for (int f = 0; f < T_N; ++f)
       S.t[f * n + c] = o[f];
   }
+  chain_next();
 }
 
 // Blocks of pass 3: the edges (the longer problem) by axis, then the faces,
@@ -312,6 +316,7 @@ mhd_flux_pass(const KParams P, const DevClock * clk, int step, MhdSlab<DIM> S)
     const int w = v == IU ? IU + d : (v == IU + d ? (int)IU : v);
     S.f[(d * MhdSlab<DIM>::NF + w) * nf + out] = fl[v];
   }
+  chain_next();
 }
 
 template <int DIM>
@@ -377,6 +382,7 @@ mhd_update_pass(const double * __restrict__ Uin, double * __restrict__ Uout, con
   Uout[5 * st + off] = bx;
   Uout[6 * st + off] = by;
   Uout[7 * st + off] = bz;
+  chain_next();
 }
 
 template <int DIM>
@@ -427,9 +433,10 @@ mhd_passes_t(int phase, const void * Uin, void * Uout, void * work, const KParam
   {
     const MhdSlab<DIM> S = mhd_slab<DIM>(P, 0, n, work);
     auto all = [&](int w) { return (long long)(P.nx + w) * (P.ny + w) * (DIM == 3 ? P.nz + w : 1); };
-    mhd_prims_pass<DIM><<<blocks(all(5)), kPassThreads, 0, st>>>(Uin, P, clk, step, S);
-    mhd_efield_pass<DIM><<<blocks(all(3)), kPassThreads, 0, st>>>(P, clk, step, S);
-    return cudaGetLastError();
+    cudaError_t e = launch_chained(mhd_prims_pass<DIM>, blocks(all(5)), kPassThreads, 0, st, Uin, P, clk, step, S);
+    if (e == cudaSuccess)
+      e = launch_chained(mhd_efield_pass<DIM>, blocks(all(3)), kPassThreads, 0, st, P, clk, step, S);
+    return e;
   }
   for (int first = 0; first < N; first += n)
   {
@@ -437,12 +444,17 @@ mhd_passes_t(int phase, const void * Uin, void * Uout, void * work, const KParam
     long long          fb = 0;
     for (int kind = 0; kind < 6; ++kind)
       fb += mhd_kind_blocks(S, kind);
-    mhd_trace_pass<DIM><<<blocks(S.box(2)), kPassThreads, 0, st>>>(P, clk, step, S);
     auto flux = P.riemann == 1 ? mhd_flux_pass<DIM, 1> : P.riemann == 2 ? mhd_flux_pass<DIM, 2> : mhd_flux_pass<DIM, 4>;
-    flux<<<(unsigned)fb, kPassThreads, 0, st>>>(P, clk, step, S);
-    mhd_update_pass<DIM><<<blocks(S.box(0)), kPassThreads, 0, st>>>((const double *)Uin, (double *)Uout, P, clk, step, S);
+    cudaError_t e = launch_chained(mhd_trace_pass<DIM>, blocks(S.box(2)), kPassThreads, 0, st, P, clk, step, S);
+    if (e == cudaSuccess)
+      e = launch_chained(flux, (unsigned)fb, kPassThreads, 0, st, P, clk, step, S);
+    if (e == cudaSuccess)
+      e = launch_chained(mhd_update_pass<DIM>, blocks(S.box(0)), kPassThreads, 0, st, (const double *)Uin, (double *)Uout,
+                         P, clk, step, S);
+    if (e != cudaSuccess)
+      return e;
   }
-  return cudaGetLastError();
+  return cudaSuccess;
 }
 
 // Workspace of the FP64 step in passes.  0 for the small 2D grids, where one
