@@ -295,6 +295,7 @@ make_kparams(const ek_params & p)
   k.idzd = 1.0 / (p.dim == 3 ? p.dz : 1.0);
   k.mhd_stage = p.mhd_stage;
   k.entho = 1.0 / (p.gamma0 - 1.0);
+  k.enthof = (float)k.entho;
   k.gamma6 = p.gamma6;
   k.smallpp = p.smallpp;
   k.gamma6f = (float)p.gamma6;

@@ -63,6 +63,7 @@ struct KParams
   double    idxd, idyd, idzd; // 1/dx, 1/dy, 1/dz in FP64 (FP64 FMA build's CFL)
   int       mhd_stage;     // MHD update: stage the trace planes in shared memory
   double    entho;           // 1 / (gamma0 - 1)
+  float     enthof;
   double    gamma6, smallpp; // riemann_approx constants (HydroParams.cpp:353-356)
   float     gamma6f, smallppf;
   // static gravity (hydro; GravityParams.h:22-37): the field is gfield
@@ -316,6 +317,13 @@ sqrt_a(float x)
   float r;
   asm("sqrt.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x));
   return r;
+}
+// sqrt(n / d) for n >= 0, d > 0 in FP32, one reciprocal square root; NaN (which
+// fmaxf drops) where n d underflows
+__device__ __forceinline__ float
+sqrt_ratio_a(float n, float d)
+{
+  return n * rsqrt_a(n * d);
 }
 
 // Packed FP32 pairs: one instruction computes two lanes (sm_100 and later).

@@ -186,39 +186,38 @@ constexpr float kHlldStarTol = 1.0f / 16384.0f;
 // solved in FP64 (flux is not written)
 template <int NF>
 __device__ __forceinline__ bool
-mhd_hlld_f32(const float (&ql)[8], const float (&qr)[8], float (&flux)[NF], float gamma0)
+mhd_hlld_f32(const float (&ql)[8], const float (&qr)[8], float (&flux)[NF], float gamma0, float entho)
 {
   // left state in lane x, right state in lane y
-  const float  entho = rcp_a(gamma0 - 1.0f);
   const float  a = 0.5f * (ql[IA] + qr[IA]);
   const float  sgnm = (a >= 0.f) ? 1.f : -1.f;
   const float  a2 = a * a;
   const float2 A = f2s(a), A2 = f2s(a2), H = f2s(0.5f);
   const float2 r = f2(ql[ID], qr[ID]), p = f2(ql[IP], qr[IP]), u = f2(ql[IU], qr[IU]);
   const float2 v = f2(ql[IV], qr[IV]), w = f2(ql[IW], qr[IW]), b = f2(ql[IB], qr[IB]), c = f2(ql[IC], qr[IC]);
-  const float2 bsq = fma2(c, c, fma2(b, b, A2));                         // a^2 + b^2 + c^2
+  const float2 bt2 = fma2(c, c, mul2(b, b)), bsq = add2(bt2, A2);
   const float2 ecin = mul2(mul2(H, fma2(w, w, fma2(v, v, mul2(u, u)))), r);
   const float2 emag = mul2(H, bsq);
   const float2 etot = add2(fma2(p, f2s(entho), ecin), emag);
   const float2 ptot = add2(p, emag);
   const float2 vdotb = fma2(w, c, fma2(v, b, mul2(u, A)));
 
-  // fast magnetosonic speeds (find_speed_fast, the normal field a)
-  const float2 id = f2(rcp_a(r.x), rcp_a(r.y));
-  const float2 c2 = mul2(mul2(f2s(gamma0), p), id);
-  const float2 d2 = mul2(H, fma2(bsq, id, c2));
-  const float2 dq = fma2(d2, d2, neg2(mul2(mul2(c2, A2), id)));
-  const float2 cq = add2(d2, f2(sqrt_a(dq.x), sqrt_a(dq.y)));
-  const float  cmax = sqrt_a(fmaxf(cq.x, cq.y)); // the larger fast speed
+  // the larger fast magnetosonic speed (find_speed_fast, the normal field a):
+  // rho c^2 of both sides, the discriminant as (B^2 - gamma p)^2 / 4 + gamma p
+  // Bt^2, which does not cancel; the quotients compared by products
+  const float2 g = mul2(f2s(gamma0), p), h = mul2(H, add2(bsq, g)), hm = fma2(g, f2s(-0.5f), emag);
+  const float2 dq = fma2(g, bt2, mul2(hm, hm));
+  const float2 n = add2(h, f2(sqrt_a(dq.x), sqrt_a(dq.y)));
+  const bool   lbig = n.x * r.y >= n.y * r.x;
+  const float  cmax = sqrt_ratio_a(lbig ? n.x : n.y, lbig ? r.x : r.y);
   const float  sl = fminf(u.x, u.y) - cmax;
   const float  sr = fmaxf(u.x, u.y) + cmax;
   const float2 S = f2(sl, sr);
   const float2 su = sub2(S, u);  // S - u
   const float2 rsu = mul2(r, su); // rho (S - u): -rcl, rcr
-  const float  rcl = -rsu.x, rcr = rsu.y;
-  const float  irc = rcp_a(rcr + rcl);
-  const float  ustar = (rcr * u.y + rcl * u.x + (ptot.x - ptot.y)) * irc;
-  const float  ptotstar = (rcr * ptot.x + rcl * ptot.y + rcl * rcr * (u.x - u.y)) * irc;
+  // u* = u_l + w, p* = p_l - rcl w
+  const float  w0 = (ptot.x - ptot.y - rsu.y * (u.x - u.y)) * rcp_a(rsu.y - rsu.x);
+  const float  ustar = u.x + w0, ptotstar = fmaf(rsu.x, w0, ptot.x);
   const float2 US = f2s(ustar);
   const float2 sus = sub2(S, US);
   // the star-state denominators; the face goes to FP64 when one is
@@ -420,7 +419,7 @@ __device__ __forceinline__ bool
 mhd_hlld(R (&ql)[8], R (&qr)[8], R (&flux)[NF], R gamma0, R entho)
 {
   if constexpr (sizeof(R) == 4)
-    return mhd_hlld_f32<NF>(ql, qr, flux, gamma0);
+    return mhd_hlld_f32<NF>(ql, qr, flux, gamma0, entho);
   else if constexpr (kFast64<R>)
   {
     mhd_hlld64<NF>(ql, qr, flux, gamma0, entho);
@@ -731,122 +730,98 @@ struct EdgeQ
   R r, p, u, v, a, b, c;
 };
 
-// mag_riemann2d_hlld in FP32 for the mixed form: one reciprocal per corner
-// density and per shared denominator, |B| / sqrt(rho*) as reciprocal square
-// roots; the reference's branch-free selection of the emf.
+// mag_riemann2d_hlld in FP32 for the mixed form, in the algebra of the FP64 FMA
+// build's (below), with the left and right corners of a row in the lanes of
+// packed pairs (rows LL, RL and LR, RR; a is the same along a row, b along a
+// column).  The discriminant of the fast speed is taken as (B^2 - gamma p)^2 / 4
+// + gamma p Bt^2, which does not cancel.  20 special-function instructions
+// instead of 38, and of the five cases only the one sampled.  Issue bounds the
+// kernels that call it (62 to 68 % busy): with the HLLD fluxes' algebra above,
+// update kernel at 256^3 2605 -> 2524 us, 2D step at 2048^2 495 -> 483 us.
 __device__ __forceinline__ float
 mag_riemann2d_hlld_f32(const EdgeQ<float> & LL, const EdgeQ<float> & RL, const EdgeQ<float> & LR,
-                       const EdgeQ<float> & RR, float ELL, float ERL, float ELR, float ERR, float gamma0,
-                       float smallc)
+                       const EdgeQ<float> & RR, float gamma0, float smallc)
 {
-  // squares of the fast speeds along x and y (before the outer square root:
-  // one square root of the largest of the four corners', below)
-  auto fast2 = [gamma0](const EdgeQ<float> & q, float & cx, float & cy) {
-    const float ir = rcp_a(q.r);
-    const float c2 = gamma0 * q.p * ir;
-    const float d2 = 0.5f * ((q.a * q.a + q.b * q.b + q.c * q.c) * ir + c2);
-    const float dd = d2 * d2, cr = c2 * ir;
-    cx = d2 + sqrt_a(dd - cr * q.a * q.a);
-    cy = d2 + sqrt_a(dd - cr * q.b * q.b);
+  const float  a0 = LL.a, a1 = LR.a, a02 = a0 * a0, a12 = a1 * a1;
+  const float2 b = f2(LL.b, RL.b), bb = mul2(b, b);
+  struct Row
+  {
+    float2 r, u, v, pt;
   };
-  const float rLL = LL.r, pLL = LL.p, uLL = LL.u, vLL = LL.v, aLL = LL.a, bLL = LL.b, cLL = LL.c;
-  const float rLR = LR.r, pLR = LR.p, uLR = LR.u, vLR = LR.v, aLR = LR.a, bLR = LR.b, cLR = LR.c;
-  const float rRL = RL.r, pRL = RL.p, uRL = RL.u, vRL = RL.v, aRL = RL.a, bRL = RL.b, cRL = RL.c;
-  const float rRR = RR.r, pRR = RR.p, uRR = RR.u, vRR = RR.v, aRR = RR.a, bRR = RR.b, cRR = RR.c;
-  float cLLx, cLLy, cLRx, cLRy, cRLx, cRLy, cRRx, cRRy;
-  fast2(LL, cLLx, cLLy);
-  fast2(LR, cLRx, cLRy);
-  fast2(RL, cRLx, cRLy);
-  fast2(RR, cRRx, cRRy);
-  const float cmx = sqrt_a(fmax4(cLLx, cLRx, cRLx, cRRx)), cmy = sqrt_a(fmax4(cLLy, cLRy, cRLy, cRRy));
-  const float SL = fmin4(uLL, uLR, uRL, uRR) - cmx;
-  const float SR = fmax4(uLL, uLR, uRL, uRR) + cmx;
-  const float SB = fmin4(vLL, vLR, vRL, vRR) - cmy;
-  const float ST = fmax4(vLL, vLR, vRL, vRR) + cmy;
+  float cx = 0.f, cy = 0.f; // squares of the largest fast speeds along x and y
+  auto  row = [&](const EdgeQ<float> & l, const EdgeQ<float> & r, float a2) {
+    Row w;
+    w.r = f2(l.r, r.r), w.u = f2(l.u, r.u), w.v = f2(l.v, r.v);
+    const float2 p = f2(l.p, r.p), c = f2(l.c, r.c), c2 = mul2(c, c);
+    const float2 btx = add2(c2, bb), bty = add2(c2, f2s(a2)), b2 = add2(btx, f2s(a2)); // transverse to x, to y; B^2
+    const float2 g = mul2(f2s(gamma0), p), h = mul2(f2s(0.5f), add2(b2, g)), m = fma2(g, f2s(-0.5f), mul2(f2s(0.5f), b2));
+    const float2 mm = mul2(m, m), dx = fma2(g, btx, mm), dy = fma2(g, bty, mm);
+    const float2 ir = f2(rcp_a(w.r.x), rcp_a(w.r.y));
+    const float2 fx = mul2(add2(h, f2(sqrt_a(dx.x), sqrt_a(dx.y))), ir);
+    const float2 fy = mul2(add2(h, f2(sqrt_a(dy.x), sqrt_a(dy.y))), ir);
+    cx = fmaxf(cx, fmaxf(fx.x, fx.y));
+    cy = fmaxf(cy, fmaxf(fy.x, fy.y));
+    w.pt = fma2(f2s(0.5f), b2, p);
+    return w;
+  };
+  const Row   B = row(LL, RL, a02), T = row(LR, RR, a12);
+  const float cmx = sqrt_a(cx), cmy = sqrt_a(cy);
+  const float SL = fminf(fminf(B.u.x, B.u.y), fminf(T.u.x, T.u.y)) - cmx;
+  const float SR = fmaxf(fmaxf(B.u.x, B.u.y), fmaxf(T.u.x, T.u.y)) + cmx;
+  const float SB = fminf(fminf(B.v.x, B.v.y), fminf(T.v.x, T.v.y)) - cmy;
+  const float ST = fmaxf(fmaxf(B.v.x, B.v.y), fmaxf(T.v.x, T.v.y)) + cmy;
 
-  const float PtotLL = pLL + 0.5f * (aLL * aLL + bLL * bLL + cLL * cLL);
-  const float PtotLR = pLR + 0.5f * (aLR * aLR + bLR * bLR + cLR * cLR);
-  const float PtotRL = pRL + 0.5f * (aRL * aRL + bRL * bRL + cRL * cRL);
-  const float PtotRR = pRR + 0.5f * (aRR * aRR + bRR * bRR + cRR * cRR);
+  // distances of the corner velocities from the outer waves (positive)
+  const float2 sgn = f2(1.f, -1.f), S = f2(-SL, SR);
+  const float2 xB = fma2(B.u, sgn, S), xT = fma2(T.u, sgn, S);
+  const float2 yB = add2(B.v, f2s(-SB)), yT = fma2(T.v, f2s(-1.f), f2s(ST));
+  const float2 wB = mul2(B.r, xB), wT = mul2(T.r, xT), ps = add2(B.pt, T.pt), pd = sub2(B.pt, T.pt);
+  const float2 un = fma2(wB, B.u, mul2(wT, T.u)), ud = add2(wB, wT);
+  const float  us = (un.x + un.y + (ps.x - ps.y)) * rcp_a(ud.x + ud.y);
+  const float2 zB = mul2(B.r, yB), zT = mul2(T.r, yT);
+  const float2 vn = fma2(zB, B.v, mul2(zT, T.v)), vd = add2(zB, zT);
+  const float  vs = (vn.x + vn.y + (pd.x + pd.y)) * rcp_a(vd.x + vd.y);
+  const float2 iX = f2(rcp_a(us - SL), rcp_a(SR - us));
+  const float  iB = rcp_a(vs - SB), iT = rcp_a(ST - vs);
+  const float2 fxB = mul2(xB, iX), fxT = mul2(xT, iX), fyB = mul2(yB, f2s(iB)), fyT = mul2(yT, f2s(iT));
 
-  const float rcLLx = rLL * (uLL - SL), rcRLx = rRL * (SR - uRL);
-  const float rcLRx = rLR * (uLR - SL), rcRRx = rRR * (SR - uRR);
-  const float rcLLy = rLL * (vLL - SB), rcLRy = rLR * (ST - vLR);
-  const float rcRLy = rRL * (vRL - SB), rcRRy = rRR * (ST - vRR);
+  // the larger Alfven speed of two corners: sqrt(max(n1 / d1, n2 / d2))
+  auto larger = [smallc](float n1, float d1, float n2, float d2) {
+    const bool first = n1 * d2 >= n2 * d1;
+    return fmaxf(sqrt_ratio_a(first ? n1 : n2, first ? d1 : d2), smallc);
+  };
+  const float2 dxB = mul2(wB, iX), dxT = mul2(wT, iX), dyB = mul2(zB, f2s(iB)), dyT = mul2(zT, f2s(iT));
+  const float  cL = larger(a12 * fmaxf(fyT.x, 1.f), dxT.x, a02 * fmaxf(fyB.x, 1.f), dxB.x);
+  const float  cR = larger(a12 * fmaxf(fyT.y, 1.f), dxT.y, a02 * fmaxf(fyB.y, 1.f), dxB.y);
+  const float  cB = larger(bb.x * fmaxf(fxB.x, 1.f), dyB.x, bb.y * fmaxf(fxB.y, 1.f), dyB.y);
+  const float  cT = larger(bb.x * fmaxf(fxT.x, 1.f), dyT.x, bb.y * fmaxf(fxT.y, 1.f), dyT.y);
+  const float  SAL = fminf(us - cL, 0.f), SAR = fmaxf(us + cR, 0.f);
+  const float  SAB = fminf(vs - cB, 0.f), SAT = fmaxf(vs + cT, 0.f);
 
-  const float ustar = (rcLLx * uLL + rcLRx * uLR + rcRLx * uRL + rcRRx * uRR + (PtotLL - PtotRL + PtotLR - PtotRR)) *
-                      rcp_a(rcLLx + rcLRx + rcRLx + rcRRx);
-  const float vstar = (rcLLy * vLL + rcLRy * vLR + rcRLy * vRL + rcRRy * vRR + (PtotLL - PtotLR + PtotRL - PtotRR)) *
-                      rcp_a(rcLLy + rcLRy + rcRLy + rcRRy);
-  const float iL = rcp_a(SL - ustar), iR = rcp_a(SR - ustar), iB = rcp_a(SB - vstar), iT = rcp_a(ST - vstar);
-
-  // star states of corner (r, u, v, a, b) against the x-side factor fx and y-side factor fy
-  const float fxLL = (SL - uLL) * iL, fyLL = (SB - vLL) * iB;
-  const float fxLR = (SL - uLR) * iL, fyLR = (ST - vLR) * iT;
-  const float fxRL = (SR - uRL) * iR, fyRL = (SB - vRL) * iB;
-  const float fxRR = (SR - uRR) * iR, fyRR = (ST - vRR) * iT;
-
-  const float rstarLLx = rLL * fxLL, BstarLL = bLL * fxLL, rstarLLy = rLL * fyLL, AstarLL = aLL * fyLL;
-  const float rstarLL = rstarLLx * fyLL;
-  const float EstarLLx = ustar * BstarLL - vLL * aLL, EstarLLy = uLL * bLL - vstar * AstarLL;
-  const float EstarLL = ustar * BstarLL - vstar * AstarLL;
-  const float rstarLRx = rLR * fxLR, BstarLR = bLR * fxLR, rstarLRy = rLR * fyLR, AstarLR = aLR * fyLR;
-  const float rstarLR = rstarLRx * fyLR;
-  const float EstarLRx = ustar * BstarLR - vLR * aLR, EstarLRy = uLR * bLR - vstar * AstarLR;
-  const float EstarLR = ustar * BstarLR - vstar * AstarLR;
-  const float rstarRLx = rRL * fxRL, BstarRL = bRL * fxRL, rstarRLy = rRL * fyRL, AstarRL = aRL * fyRL;
-  const float rstarRL = rstarRLx * fyRL;
-  const float EstarRLx = ustar * BstarRL - vRL * aRL, EstarRLy = uRL * bRL - vstar * AstarRL;
-  const float EstarRL = ustar * BstarRL - vstar * AstarRL;
-  const float rstarRRx = rRR * fxRR, BstarRR = bRR * fxRR, rstarRRy = rRR * fyRR, AstarRR = aRR * fyRR;
-  const float rstarRR = rstarRRx * fyRR;
-  const float EstarRRx = ustar * BstarRR - vRR * aRR, EstarRRy = uRR * bRR - vstar * AstarRR;
-  const float EstarRR = ustar * BstarRR - vstar * AstarRR;
-
-  const float qLL = rsqrt_a(rstarLL), qLR = rsqrt_a(rstarLR), qRL = rsqrt_a(rstarRL), qRR = rsqrt_a(rstarRR);
-  const float calfvenL = fmax5(fabsf(aLR) * rsqrt_a(rstarLRx), fabsf(AstarLR) * qLR,
-                               fabsf(aLL) * rsqrt_a(rstarLLx), fabsf(AstarLL) * qLL, smallc);
-  const float calfvenR = fmax5(fabsf(aRR) * rsqrt_a(rstarRRx), fabsf(AstarRR) * qRR,
-                               fabsf(aRL) * rsqrt_a(rstarRLx), fabsf(AstarRL) * qRL, smallc);
-  const float calfvenB = fmax5(fabsf(bLL) * rsqrt_a(rstarLLy), fabsf(BstarLL) * qLL,
-                               fabsf(bRL) * rsqrt_a(rstarRLy), fabsf(BstarRL) * qRL, smallc);
-  const float calfvenT = fmax5(fabsf(bLR) * rsqrt_a(rstarLRy), fabsf(BstarLR) * qLR,
-                               fabsf(bRR) * rsqrt_a(rstarRRy), fabsf(BstarRR) * qRR, smallc);
-
-  const float SAL = fminf(ustar - calfvenL, 0.f);
-  const float SAR = fmaxf(ustar + calfvenR, 0.f);
-  const float SAB = fminf(vstar - calfvenB, 0.f);
-  const float SAT = fmaxf(vstar + calfvenT, 0.f);
-  const float iAx = rcp_a(SAR - SAL), iAy = rcp_a(SAT - SAB);
-
-  const float AstarT = (SAR * AstarRR - SAL * AstarLR) * iAx;
-  const float AstarB = (SAR * AstarRL - SAL * AstarLL) * iAx;
-  const float BstarR = (SAT * BstarRR - SAB * BstarRL) * iAy;
-  const float BstarL = (SAT * BstarLR - SAB * BstarLL) * iAy;
-
-  // the reference's sign masks (1 + copysign(1, S)) / 2 as sign-bit tests and
-  // its mask-weighted sums as selects: exactly one term of each sum is live
-  const bool SBp = !signbit(SB), STp = !signbit(ST), SLp = !signbit(SL), SRp = !signbit(SR);
-  float      E = 0.f, tmpE;
-
-  tmpE = (SAL * SAB * EstarRR - SAL * SAT * EstarRL - SAR * SAB * EstarLR + SAR * SAT * EstarLL) * iAx * iAy -
-         SAT * SAB * iAy * (AstarT - AstarB) + SAR * SAL * iAx * (BstarR - BstarL);
-  E += (!SBp && STp && !SLp && SRp) ? tmpE : 0.f;
-
-  tmpE = (SAR * EstarLLx - SAL * EstarRLx + SAR * SAL * (bRL - bLL)) * iAx;
-  tmpE = SLp ? ELL : (!SRp ? ERL : tmpE);
-  E += SBp ? tmpE : 0.f;
-
-  tmpE = (SAR * EstarLRx - SAL * EstarRRx + SAR * SAL * (bRR - bLR)) * iAx;
-  tmpE = SLp ? ELR : (!SRp ? ERR : tmpE);
-  E += (!SBp && !STp) ? tmpE : 0.f;
-
-  tmpE = (SAT * EstarLLy - SAB * EstarLRy - SAT * SAB * (aLR - aLL)) * iAy;
-  E += (!SBp && STp && SLp) ? tmpE : 0.f;
-
-  tmpE = (SAT * EstarRLy - SAB * EstarRRy - SAT * SAB * (aRR - aRL)) * iAy;
-  E += (!SBp && STp && !SLp && !SRp) ? tmpE : 0.f;
-  return E;
+  const bool SLp = !signbit(SL), SRp = !signbit(SR), SBp = !signbit(SB), STp = !signbit(ST);
+  if (SBp || !STp)
+  {
+    // supersonic along y: the x fan of the corners on that side
+    const float2 u = SBp ? B.u : T.u, v = SBp ? B.v : T.v, fx = SBp ? fxB : fxT;
+    const float  a = SBp ? a0 : a1;
+    if (SLp || !SRp)
+      return SLp ? u.x * b.x - v.x * a : u.y * b.y - v.y * a;
+    const float El = us * (b.x * fx.x) - v.x * a, Er = us * (b.y * fx.y) - v.y * a;
+    return (SAR * El - SAL * Er + SAR * SAL * (b.y - b.x)) * rcp_a(SAR - SAL);
+  }
+  if (SLp || !SRp)
+  {
+    const float uB = SLp ? B.u.x : B.u.y, uT = SLp ? T.u.x : T.u.y, fB = SLp ? fyB.x : fyB.y, fT = SLp ? fyT.x : fyT.y;
+    const float bs = SLp ? b.x : b.y;
+    const float Eb = uB * bs - vs * (a0 * fB), Et = uT * bs - vs * (a1 * fT);
+    return (SAT * Eb - SAB * Et - SAT * SAB * (a1 - a0)) * rcp_a(SAT - SAB);
+  }
+  const float2 AB = mul2(f2s(a0), fyB), AT = mul2(f2s(a1), fyT), BB = mul2(b, fxB), BT = mul2(b, fxT);
+  const float2 EB = fma2(f2s(us), BB, mul2(f2s(-vs), AB)), ET = fma2(f2s(us), BT, mul2(f2s(-vs), AT));
+  const float2 e = fma2(f2s(SAB), ET, mul2(f2s(-SAT), EB)), dA = sub2(AT, AB);
+  const float  dB = SAT * (BT.y - BT.x) - SAB * (BB.y - BB.x);
+  const float  m = SAL * e.y - SAR * e.x - SAT * SAB * (SAR * dA.y - SAL * dA.x) + SAR * SAL * dB;
+  return m * (rcp_a(SAR - SAL) * rcp_a(SAT - SAB));
 }
 
 // mag_riemann2d_hlld (RiemannSolvers_MHD.h:395-627) in the FP64 FMA build: the
@@ -949,7 +924,7 @@ mag_riemann2d_hlld(const EdgeQ<R> & LL, const EdgeQ<R> & RL, const EdgeQ<R> & LR
                    const EdgeQ<R> & RR, R ELL, R ERL, R ELR, R ERR, R gamma0, R smallc)
 {
   if constexpr (sizeof(R) == 4)
-    return mag_riemann2d_hlld_f32(LL, RL, LR, RR, ELL, ERL, ELR, ERR, gamma0, smallc);
+    return mag_riemann2d_hlld_f32(LL, RL, LR, RR, gamma0, smallc);
   else if constexpr (kFast64<R>)
     return mag_riemann2d_hlld64(LL, RL, LR, RR, gamma0, smallc);
   else

@@ -47,7 +47,7 @@ mhd_const(const KParams & P)
     C.smallp = P.smallpf;
     C.smallc = P.smallcf;
     C.slope_type = P.slopef;
-    C.entho = (R)P.entho;
+    C.entho = P.enthof;
   }
   return C;
 }
