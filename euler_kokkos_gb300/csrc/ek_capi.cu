@@ -1204,12 +1204,10 @@ struct ek_ensemble
   double *                 dtlogs = nullptr;
   ekc::EnsInstance *       d_insts = nullptr;
   ekc::EnsTile *           d_tiles = nullptr;
-  int *                    d_step = nullptr;
   double *                 d_totals = nullptr;
-  void *                   d_scalars = nullptr; // per-instance step scalars (64 B each)
   int                      ntiles = 0;
-  int                      grid = 0;
-  int                      step = 0; // host copy of the device step counter
+  int                      rows = 1; // of a warp's run (choose_rows)
+  int                      step = 0; // steps launched
   long long                cells = 0;
   long long                launches = 0;
   cudaGraph_t              graph = nullptr;
@@ -1237,9 +1235,7 @@ ek_ensemble_destroy(ek_ensemble * e)
   cudaFree(e->dtlogs);
   cudaFree(e->d_insts);
   cudaFree(e->d_tiles);
-  cudaFree(e->d_step);
   cudaFree(e->d_totals);
-  cudaFree(e->d_scalars);
   if (e->stream)
     cudaStreamDestroy(e->stream);
   delete e;
@@ -1303,15 +1299,16 @@ ek_ensemble_create(const ek_params * params, int n, ek_ensemble ** out)
   if (err == cudaSuccess)
     err = cudaMalloc((void **)&e->d_insts, sizeof(ekc::EnsInstance) * n);
   if (err == cudaSuccess)
-    err = cudaMalloc((void **)&e->d_step, sizeof(int));
-  if (err == cudaSuccess)
-    err = cudaMemsetAsync(e->d_step, 0, sizeof(int), e->stream);
-  if (err == cudaSuccess)
     err = cudaMalloc((void **)&e->d_totals, 2 * sizeof(double) * n);
   std::vector<ekc::EnsInstance> h_insts(n);
   std::vector<ekc::EnsTile>     tiles;
   if (err == cudaSuccess)
   {
+    std::vector<int> nx(n), ny(n);
+    for (int i = 0; i < n; ++i)
+      nx[i] = params[i].nx, ny[i] = params[i].ny;
+    e->rows = ekc::choose_rows(nx.data(), ny.data(), n, ek_internal::sm_count(),
+                               e->prec == EK_PREC_FP64 ? ekc::kChunkRows64 : ekc::kChunkRows32);
     for (int i = 0; i < n; ++i)
     {
       ek_solver * v = new ek_solver();
@@ -1334,16 +1331,15 @@ ek_ensemble_create(const ek_params * params, int n, ek_ensemble ** out)
       h_insts[i].U[0] = v->U[0];
       h_insts[i].U[1] = v->U[1];
       h_insts[i].clk = v->clk;
-      // tiles of the 2D step kernel, instance-major
-      const int tx = (params[i].nx + EK_H2_TX - 1) / EK_H2_TX, ty = (params[i].ny + EK_H2_TY - 1) / EK_H2_TY;
+      // tiles of the step kernel, instance-major
+      const int tx = ekc::row_strips(params[i].nx), ty = ekc::row_groups(params[i].ny, e->rows);
+      h_insts[i].tiles = (unsigned)(tx * ty);
       for (int by = 0; by < ty; ++by)
         for (int bx = 0; bx < tx; ++bx)
           tiles.push_back({ i, bx, by });
     }
     e->ntiles = (int)tiles.size();
     err = cudaMalloc((void **)&e->d_tiles, sizeof(ekc::EnsTile) * tiles.size());
-    if (err == cudaSuccess)
-      err = cudaMalloc(&e->d_scalars, 64 * (size_t)n);
   }
   if (err == cudaSuccess)
     err = cudaMemcpyAsync(e->d_insts, h_insts.data(), sizeof(ekc::EnsInstance) * n, cudaMemcpyHostToDevice,
@@ -1359,7 +1355,6 @@ ek_ensemble_create(const ek_params * params, int n, ek_ensemble ** out)
     ek_ensemble_destroy(e);
     return st;
   }
-  e->grid = e->exact ? ek_exact::ensemble2d_grid(e->prec) : ek_fast::ensemble2d_grid(e->prec);
   *out = e;
   return EK_OK;
 }
@@ -1392,10 +1387,8 @@ ensemble_launch_steps(ek_ensemble * e, int nsteps)
 {
   for (int k = 0; k < nsteps; ++k)
   {
-    cudaError_t err = e->exact ? ek_exact::ensemble2d_step(e->prec, e->d_insts, e->n, e->d_tiles, e->ntiles,
-                                                           e->d_step, e->d_scalars, e->grid, e->stream)
-                               : ek_fast::ensemble2d_step(e->prec, e->d_insts, e->n, e->d_tiles, e->ntiles,
-                                                          e->d_step, e->d_scalars, e->grid, e->stream);
+    cudaError_t err = e->exact ? ek_exact::ensemble2d_step(e->prec, e->d_insts, e->d_tiles, e->ntiles, e->rows, e->stream)
+                               : ek_fast::ensemble2d_step(e->prec, e->d_insts, e->d_tiles, e->ntiles, e->rows, e->stream);
     if (err != cudaSuccess)
       return cuda_fail(err, "ensemble step");
   }
@@ -1441,7 +1434,7 @@ ek_ensemble_run(ek_ensemble * e, int nsteps, int use_graph)
     }
     EK_CUDA(cudaGraphLaunch(e->graph_exec, e->stream), "graph launch");
   }
-  e->launches += 3LL * nsteps;
+  e->launches += nsteps;
   e->step += nsteps;
   return EK_OK;
 }
@@ -1490,7 +1483,7 @@ ek_ensemble_totals(ek_ensemble * e, double * out)
 {
   if (!e || !out)
     return fail(EK_ERR_INVALID, "ek_ensemble_totals: bad argument");
-  EK_CUDA(ek_fast::ensemble_totals(e->prec, e->d_insts, e->n, e->d_step, e->d_totals, e->stream), "totals");
+  EK_CUDA(ek_fast::ensemble_totals(e->prec, e->d_insts, e->n, e->step, e->d_totals, e->stream), "totals");
   EK_CUDA(cudaMemcpyAsync(out, e->d_totals, 2 * sizeof(double) * e->n, cudaMemcpyDeviceToHost, e->stream),
           "totals");
   EK_CUDA(cudaStreamSynchronize(e->stream), "totals");
@@ -1513,7 +1506,7 @@ ek_ensemble_info(ek_ensemble * e, long long * interior_cells, int * tiles, int *
   if (tiles)
     *tiles = e->ntiles;
   if (grid)
-    *grid = e->grid;
+    *grid = e->ntiles; // one CTA per tile
   if (launches)
     *launches = e->launches;
   return EK_OK;

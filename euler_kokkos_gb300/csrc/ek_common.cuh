@@ -108,6 +108,7 @@ struct DevClock
   double             last_dt;   // dt of the last step taken (read with the clock)
   StepConsts         sc[3];     // per slot, by the last block of the CFL kernel
   unsigned int       fin[3];    // blocks of that kernel done (reset by the last)
+  int                next;      // the step whose constants were computed last
 };
 
 enum : int
@@ -122,6 +123,7 @@ struct EnsInstance
   KParams    P;
   void *     U[2]; // ping-pong states
   DevClock * clk;
+  unsigned   tiles; // of the work list
 };
 struct EnsTile
 {
@@ -204,15 +206,12 @@ using namespace ekc;
 #ifndef EK_M2_MINB_F64
 #define EK_M2_MINB_F64 0
 #endif
+#ifndef EK_H2_MINB_F32
+#define EK_H2_MINB_F32 5
+#endif
 #define EK_MINB(R, F32, F64) (sizeof(R) == 4 ? (F32) : (F64))
 // Tile shapes (output cells per CTA in x, y) of the step kernels; the
 // defaults are the measured best, euler_kokkos_gb300/tuning.py re-tunes them.
-#ifndef EK_H2_TX
-#define EK_H2_TX 32
-#endif
-#ifndef EK_H2_TY
-#define EK_H2_TY 8
-#endif
 #ifndef EK_H3_TX
 #define EK_H3_TX 32
 #endif
@@ -634,62 +633,16 @@ ldg(const T * p)
   return __ldg(p);
 }
 
-// dt at the start of a step, SolverBase::compute_dt (SolverBase.cpp:124-154).
-// Returns false when the step must not run: the simulation is finished
-// (SolverBase::finished, t >= tEnd - 1e-14, SolverBase.cpp:170-176) or an
-// earlier launched step did not run (its slot was never committed).
-__device__ __forceinline__ bool
-step_dt(const KParams & P, const DevClock * clk, int step, double * t, double * dt)
-{
-  const int s = step % 3;
-  if (clk->sid[s] != step)
-    return false;
-  const double invDt = dkey_inv(clk->key[s]);
-  double       d = P.cfl / invDt;
-  const double tt = clk->t[s];
-  if (tt + d > P.tEnd)
-    d = P.tEnd - tt;
-  *t = tt;
-  *dt = d;
-  return !(tt >= P.tEnd - 1e-14);
-}
-
-// Step scalars computed once per CTA by thread 0 and shared: dt and the
-// dt/dx ratios (the FP64 divisions would otherwise run in every thread).
-template <class R>
-struct StepScalars
-{
-  double t, dt;
-  R      dtdx, dtdy, dtdz;
-  int    active;
-};
-template <class R>
-__device__ __forceinline__ bool
-step_scalars(const KParams & P, const DevClock * clk, int step, StepScalars<R> * sh)
-{
-  if (threadIdx.x == 0)
-  {
-    double t, dt;
-    sh->active = step_dt(P, clk, step, &t, &dt) ? 1 : 0;
-    sh->t = t;
-    sh->dt = dt;
-    sh->dtdx = (R)(dt / P.dx);
-    sh->dtdy = (R)(dt / P.dy);
-    sh->dtdz = (R)(dt / P.dz);
-  }
-  __syncthreads();
-  return sh->active != 0;
-}
-
 // Called by every block of the kernel that completes the CFL key of `step`
 // (after its atomicMax): the last block to finish computes the step's dt and
 // dt/dx ratios in FP64 once, for the step's kernels to read (step_consts), so
 // that no block of those kernels runs the divisions behind a barrier.  The
 // clock fields written by other blocks are read through volatile loads.
 // repair: the HLLD repair pass's list, if any; when tiles are listed the pass
-// completes the key, and computes the constants.
+// completes the key, and computes the constants.  blocks: their number, where it
+// is not the grid's.
 __device__ __forceinline__ void
-finalize_step(DevClock * clk, const KParams & P, int step, const int * repair = nullptr)
+finalize_step(DevClock * clk, const KParams & P, int step, const int * repair = nullptr, unsigned blocks = 0)
 {
   __shared__ int last;
   __syncthreads();
@@ -697,7 +650,7 @@ finalize_step(DevClock * clk, const KParams & P, int step, const int * repair = 
   if (threadIdx.x == 0)
   {
     __threadfence();
-    const unsigned nb = gridDim.x * gridDim.y * gridDim.z;
+    const unsigned nb = blocks ? blocks : gridDim.x * gridDim.y * gridDim.z;
     last = atomicAdd(&clk->fin[s], 1u) == nb - 1;
   }
   __syncthreads();
@@ -712,7 +665,11 @@ finalize_step(DevClock * clk, const KParams & P, int step, const int * repair = 
     c.step = step;
     c.active = 0;
     c.t = c.dt = c.dtdx = c.dtdy = c.dtdz = 0.0;
-    if (v->sid[s] == step) // step_dt's arithmetic
+    // dt at the start of a step, SolverBase::compute_dt (SolverBase.cpp:124-154);
+    // the step must not run when the simulation is finished (t >= tEnd - 1e-14,
+    // SolverBase.cpp:170-176) or an earlier launched step did not run (its slot
+    // was never committed)
+    if (v->sid[s] == step)
     {
       const double invDt = dkey_inv(v->key[s]);
       double       d = P.cfl / invDt;
@@ -727,6 +684,7 @@ finalize_step(DevClock * clk, const KParams & P, int step, const int * repair = 
       c.dtdz = d / P.dz;
     }
     clk->sc[s] = c;
+    clk->next = step;
   }
 }
 // The kernels of consecutive steps are launched with programmatic stream

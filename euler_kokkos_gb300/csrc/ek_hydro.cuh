@@ -756,9 +756,9 @@ hydro_riemann(const R (&ql)[NV], const R (&qr)[NV], R (&flux)[NV], const HydroCo
 // precision: FP64 keeps the reference's expression; the mixed form uses the
 // FP32 inverse cell sizes.  Threads keep a NaN-ignoring max (fmax, as the
 // reference's reduction) and convert to the FP64 key once.
-template <class R, int NV>
+template <class R, int NV, class PP>
 __device__ __forceinline__ R
-hydro_invdt(const R (&u)[NV], const HydroConst<R> & C, const KParams & P)
+hydro_invdt(const R (&u)[NV], const HydroConst<R> & C, const PP & P)
 {
   R q[NV];
   hydro_prims<R, NV>(u, q, C);

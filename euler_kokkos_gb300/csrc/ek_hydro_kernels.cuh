@@ -143,10 +143,10 @@ cell_slopes(const R * q0, const R * qm, const R * qp, int hx, int hy, R st, R (&
 // thread 0 computes them for this CTA.
 // NT threads: one per cell, or more (a multiple of 32 per part), so that the
 // ring cells run beside the interior ones and the faces take fewer rounds.
-template <class S, class R, int TX, int TY, int NT, int RS = 3, bool GRAV = false, bool LOADED = false>
+template <class S, class R, int TX, int TY, int NT, int RS = 3, bool GRAV = false>
 __device__ __forceinline__ void
 hydro2d_tile(const S * __restrict__ Uin, S * __restrict__ Uout, const KParams & P, DevClock * clk,
-             int step, int bx, int by, unsigned char * smem_raw, const StepScalars<R> * pre = nullptr)
+             int step, int bx, int by, unsigned char * smem_raw)
 {
   constexpr int NV = 4, HX = TX + 4, HY = TY + 4, CELLS = TX * TY;
   constexpr int FX = TX + 2; // face-state rows in x: cells -1..TX
@@ -156,27 +156,11 @@ hydro2d_tile(const S * __restrict__ Uin, S * __restrict__ Uout, const KParams & 
   R * sYm = sXp + NV * TY * FX;              // YMIN state of cells -1..TY, then y-flux
   R * sYp = sYm + NV * (TY + 2) * TX;        // YMAX state
 
-  StepScalars<R> ss;
-  if (pre)
-  {
-    ss = *pre;
-    if (!ss.active)
-      return;
-  }
-  else
-  {
-    StepConsts c; // computed once for the step by the last block of the kernel before
-    if (!step_consts(clk, step, c))
-      return;
-    ss.t = c.t;
-    ss.dt = c.dt;
-    ss.dtdx = to_r<R>(c.dtdx);
-    ss.dtdy = to_r<R>(c.dtdy);
-    ss.dtdz = to_r<R>(c.dtdz);
-    ss.active = 1;
-  }
-  const double        t = ss.t, dt = ss.dt;
-  const R             dtdx = ss.dtdx, dtdy = ss.dtdy;
+  StepConsts sc; // computed once for the step by the last block of the kernel before
+  if (!step_consts(clk, step, sc))
+    return;
+  const double        t = sc.t, dt = sc.dt;
+  const R             dtdx = to_r<R>(sc.dtdx), dtdy = to_r<R>(sc.dtdy);
   const bool          same_xy = dtdx == dtdy; // square cells: one time-advanced state for all faces
   const HydroConst<R> C = hydro_const<R>(P);
   const R             hdt = (R)(0.5 * dt);
@@ -191,11 +175,8 @@ hydro2d_tile(const S * __restrict__ Uin, S * __restrict__ Uout, const KParams & 
   };
 
   const int gi0 = P.gw + bx * TX, gj0 = P.gw + by * TY;
-  if constexpr (!LOADED)
-  {
-    load_q_plane<S, R, NV, TX, TY, NT>(Uin, P, C, gi0, gj0, 0, sQ);
-    __syncthreads();
-  }
+  load_q_plane<S, R, NV, TX, TY, NT>(Uin, P, C, gi0, gj0, 0, sQ);
+  __syncthreads();
 
   const int tx = threadIdx.x % TX, ty = threadIdx.x / TX;
   // traces of the interior cell
@@ -367,148 +348,6 @@ hydro2d_step(const S * __restrict__ Uin, S * __restrict__ Uout, KParams P, DevCl
   hydro2d_tile<S, R, TX, TY, NT, RS, GRAV>(Uin, Uout, P, clk, step, blockIdx.x, blockIdx.y, smem_raw);
   finalize_step(clk, P, step + 1); // the next step's dt, once its CFL key is complete
 }
-
-// ---------------------------------------------------------------------------
-// Ensemble of independent 2D runs (uneven grids, own dt each): a persistent
-// kernel walks the flat (instance, tile) work list; one launch = one step of
-// every instance.  No inter-block waits.
-// ---------------------------------------------------------------------------
-// raw conserved variables of a tile's (TX+4) x (TY+4) halo plane, gathered
-// from the boundary-mapped cells by per-thread asynchronous copies
-template <class S, int NV, int TX, int TY>
-__device__ __forceinline__ void
-issue_raw_plane(const S * __restrict__ U, const KParams & P, int gi0, int gj0, S * raw)
-{
-  constexpr int HX = TX + 4, HY = TY + 4, NT = TX * TY;
-  for (int c = threadIdx.x; c < HX * HY; c += NT)
-  {
-    const SrcCell s = src_cell(P, gi0 - 2 + c % HX, gj0 - 2 + c / HX, 0);
-#pragma unroll
-    for (int v = 0; v < NV; ++v)
-      cp_async<sizeof(S)>(raw + v * HY * HX + c, U + v * P.vstride + s.off);
-  }
-}
-// ... and, once this thread's copies landed, the primitives of the cells it
-// copied (reflecting walls flip the normal velocity, as load_q_plane does)
-template <class S, class R, int NV, int TX, int TY>
-__device__ __forceinline__ void
-convert_raw_plane(const S * raw, const KParams & P, const HydroConst<R> & C, int gi0, int gj0, R * sQ)
-{
-  constexpr int HX = TX + 4, HY = TY + 4, NT = TX * TY;
-  for (int c = threadIdx.x; c < HX * HY; c += NT)
-  {
-    const SrcCell s = src_cell(P, gi0 - 2 + c % HX, gj0 - 2 + c / HX, 0);
-    R             u[NV], q[NV];
-#pragma unroll
-    for (int v = 0; v < NV; ++v)
-      u[v] = neg_if((R)raw[v * HY * HX + c], flips(s, v, 0));
-    hydro_prims<R, NV>(u, q, C);
-#pragma unroll
-    for (int v = 0; v < NV; ++v)
-      sQ[v * HY * HX + c] = q[v];
-  }
-}
-
-template <class S, class R, int TX, int TY>
-__host__ __device__ constexpr size_t
-ensemble_raw_bytes()
-{
-  return sizeof(S) * 4 * (TX + 4) * (TY + 4);
-}
-
-// The step scalars (active, t, dt, dt/dx, dt/dy) of every instance, once per
-// step: the FP64 divisions run in one thread per instance, not per tile.
-template <class R>
-__global__ void
-ensemble_scalars_kernel(const EnsInstance * __restrict__ insts, int n, const int * __restrict__ stepc,
-                        StepScalars<R> * __restrict__ out)
-{
-  const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= n)
-    return;
-  const KParams & P = insts[i].P;
-  double          t = 0.0, dt = 0.0;
-  StepScalars<R>  s;
-  s.active = step_dt(P, insts[i].clk, *stepc, &t, &dt) ? 1 : 0;
-  s.t = t;
-  s.dt = dt;
-  s.dtdx = (R)(dt / P.dx);
-  s.dtdy = (R)(dt / P.dy);
-  s.dtdz = (R)(dt / P.dz);
-  out[i] = s;
-}
-
-template <class S, class R, int TX, int TY>
-__global__ void __launch_bounds__(TX * TY)
-ensemble2d_step(const EnsInstance * __restrict__ insts, const EnsTile * __restrict__ tiles, int ntiles,
-                const int * __restrict__ stepc, size_t tile_smem, const StepScalars<R> * __restrict__ scal)
-{
-  extern __shared__ __align__(16) unsigned char smem_raw[];
-  // raw staging of the next work item's plane, after the tile's own buffers
-  S * raw = reinterpret_cast<S *>(smem_raw + tile_smem);
-  // the step number lives in device memory (advanced by ensemble_advance after
-  // every step), so a captured sequence of steps can be replayed as is
-  const int step = *stepc;
-  // the plane of work item t is gathered while item t - gridDim.x computes
-  auto issue = [&](int t) {
-    const EnsTile       w = tiles[t];
-    const EnsInstance & in = insts[w.inst];
-    issue_raw_plane<S, 4, TX, TY>((const S *)in.U[step % 2], in.P, in.P.gw + w.bx * TX, in.P.gw + w.by * TY, raw);
-    cp_async_commit();
-  };
-  if (blockIdx.x < ntiles)
-    issue(blockIdx.x);
-  for (int t = blockIdx.x; t < ntiles; t += gridDim.x)
-  {
-    const EnsTile       w = tiles[t];
-    const EnsInstance & in = insts[w.inst];
-    const int           gi0 = in.P.gw + w.bx * TX, gj0 = in.P.gw + w.by * TY;
-    cp_async_wait_all();
-    convert_raw_plane<S, R, 4, TX, TY>(raw, in.P, hydro_const<R>(in.P), gi0, gj0, reinterpret_cast<R *>(smem_raw));
-    // every thread converted the cells it copied: the staging is free again
-    if (t + gridDim.x < ntiles)
-      issue(t + gridDim.x);
-    __syncthreads(); // the primitive plane is complete
-    hydro2d_tile<S, R, TX, TY, TX * TY, 3, false, true>((const S *)in.U[step % 2], (S *)in.U[(step + 1) % 2], in.P,
-                                                in.clk, step, w.bx, w.by, smem_raw, scal + w.inst);
-    __syncthreads(); // shared tiles are reused by the next work item
-  }
-  cp_async_wait_all(); // no copy may land after the block has left
-}
-
-__global__ void
-ensemble_advance(int * stepc)
-{
-  *stepc += 1;
-}
-
-// FP64 mass and total energy of every instance (blockIdx.y = instance)
-template <class S>
-__global__ void
-ensemble_totals_kernel(const EnsInstance * __restrict__ insts, const int * __restrict__ stepc,
-                       double * __restrict__ out)
-{
-  const EnsInstance & in = insts[blockIdx.y];
-  const KParams &     P = in.P;
-  const S *           U = (const S *)in.U[*stepc % 2];
-  double              m = 0.0, e = 0.0;
-  for_interior_rows(P, [&](int i, int j, int) {
-    const long long off = (long long)j * P.isize + i;
-    m += (double)U[off];
-    e += (double)U[P.vstride + off];
-  });
-  for (int o = 16; o > 0; o >>= 1)
-  {
-    m += __shfl_xor_sync(0xffffffffu, m, o);
-    e += __shfl_xor_sync(0xffffffffu, e, o);
-  }
-  if ((threadIdx.x & 31) == 0)
-  {
-    atomicAdd(out + 2 * blockIdx.y, m);
-    atomicAdd(out + 2 * blockIdx.y + 1, e);
-  }
-}
-
 
 // ---------------------------------------------------------------------------
 // 3D: one CTA = a TX x TY column of interior cells marching over kchunk planes

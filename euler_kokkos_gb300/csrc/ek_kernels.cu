@@ -6,6 +6,7 @@
 #include "ek_launch.h"
 #include "ek_hydro_kernels.cuh"
 #include "ek_hydro_passes.cuh"
+#include "ek_hydro_rows.cuh"
 #include "ek_mhd_kernels.cuh"
 #include "ek_mhd2d_kernels.cuh"
 #include "ek_mhd_passes.cuh"
@@ -15,10 +16,9 @@ namespace EK_NS
 
 namespace
 {
-constexpr int H2_TX = EK_H2_TX, H2_TY = EK_H2_TY; // the ensemble's tile
 constexpr int H3_TX = EK_H3_TX, H3_TY = EK_H3_TY;
 
-template <class R, int TX = H2_TX, int TY = H2_TY>
+template <class R, int TX, int TY>
 constexpr size_t
 hydro2d_smem()
 {
@@ -45,7 +45,7 @@ hydro2d_step_tiled(const void * Uin, void * Uout, const KParams & P, DevClock * 
   if (e != cudaSuccess)
     return e;
   dim3 grid((P.nx + TX - 1) / TX, (P.ny + TY - 1) / TY, 1);
-  const bool chained = sizeof(R) == 4 || chain_tiles(P, (long long)grid.x * grid.y);
+  const bool chained = chain_tiles(P, (long long)grid.x * grid.y);
   return launch_step_kernel(chained, k, grid, NT, sm, st, (const S *)Uin, (S *)Uout, P, clk, step);
 }
 
@@ -64,17 +64,21 @@ hydro_step_rs(int dim, const void * Uin, void * Uout, void * work, const KParams
     }
   if (dim == 2)
   {
-    // Tiles of the single solver (us per step).  Mixed: 32 x 8 (2048^2: 170;
-    // 32 x 16 180, 16 x 16 177, 64 x 4 183).  FP64, on grids too small for the
-    // passes: 8 x 8 where they make at most six CTAs per SM, since a warp's
-    // chain of FP64 instructions (64 cycles each on its quarter of the SM) then
-    // sets the time (64^2: 19 against 31; 200 x 136: 28 against 30; 256 x 200,
-    // 5.3 CTAs per SM: 47 against 49; 256^2, 6.7: 51 against 49), else 16 x 16
-    // (512^2: 145; 32 x 16 166, 32 x 8 156).  The threads beyond one per cell
-    // take the ring cells and let every phase of the small tile finish in one
-    // round (64^2: 29 with one per cell).
+    // Mixed: marching warps (us per step, against 32 x 8 tiles: 64^2 8.8 / 12.4,
+    // 512^2 14.1 / 18.5, 1022 x 518 21 / 30, 2048^2 91 / 170).  FP64, on grids too
+    // small for the passes: 8 x 8 tiles where they make at most six CTAs per SM,
+    // since a warp's chain of FP64 instructions (64 cycles each on its quarter of
+    // the SM) then sets the time (64^2: 19 against 31; 200 x 136: 28 against 30;
+    // 256 x 200, 5.3 CTAs per SM: 47 against 49; 256^2, 6.7: 51 against 49), else
+    // 16 x 16 (512^2: 145; 32 x 16 166, 32 x 8 156).  The threads beyond one per
+    // cell take the ring cells and let every phase of the small tile finish in
+    // one round (64^2: 29 with one per cell).
     if constexpr (sizeof(R) == 4)
-      return hydro2d_step_tiled<S, R, 32, 8, 256, RS, GRAV>(Uin, Uout, P, clk, step, st);
+    {
+      const int rows = ekc::choose_rows(&P.nx, &P.ny, 1, P.sms, ekc::kChunkRows32);
+      return launch_chained(hydro2d_rows_step<S, R, RS, GRAV>, dim3(ekc::row_strips(P.nx), ekc::row_groups(P.ny, rows)),
+                            32 * kRowWarps, 0, st, (const S *)Uin, (S *)Uout, P, clk, step, rows);
+    }
     else
     {
       const long long small = (long long)((P.nx + 7) / 8) * ((P.ny + 7) / 8);
@@ -179,69 +183,18 @@ hydro_dt(int dim, int prec, const void * U, const KParams & P, unsigned long lon
 #endif
 }
 
-namespace
-{
-template <class S, class R>
 cudaError_t
-ensemble2d_t(const EnsInstance * insts, int n, const EnsTile * tiles, int ntiles, int * stepc, void * scal,
-             int grid, cudaStream_t st)
+ensemble2d_step(int prec, const EnsInstance * insts, const EnsTile * tiles, int ntiles, int rows, cudaStream_t st)
 {
-  static_assert(sizeof(StepScalars<R>) <= 64, "per-instance step scalars are allocated 64 bytes each");
-  StepScalars<R> * sc = static_cast<StepScalars<R> *>(scal);
-  ensemble_scalars_kernel<R><<<(n + 127) / 128, 128, 0, st>>>(insts, n, stepc, sc);
-  cudaError_t e = cudaGetLastError();
-  if (e != cudaSuccess)
-    return e;
-  auto   k = ensemble2d_step<S, R, H2_TX, H2_TY>;
-  size_t sm = hydro2d_smem<R>() + ensemble_raw_bytes<S, R, H2_TX, H2_TY>();
-  e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
-  if (e != cudaSuccess)
-    return e;
-  k<<<grid, H2_TX * H2_TY, sm, st>>>(insts, tiles, ntiles, stepc, hydro2d_smem<R>(), sc);
-  e = cudaGetLastError();
-  if (e != cudaSuccess)
-    return e;
-  ensemble_advance<<<1, 1, 0, st>>>(stepc);
-  return cudaGetLastError();
-}
-template <class S, class R>
-int
-ensemble2d_grid_t()
-{
-  auto   k = ensemble2d_step<S, R, H2_TX, H2_TY>;
-  size_t sm = hydro2d_smem<R>() + ensemble_raw_bytes<S, R, H2_TX, H2_TY>();
-  cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
-  int per_sm = 0, dev = 0, nsm = 0;
-  cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k, H2_TX * H2_TY, sm);
-  cudaGetDevice(&dev);
-  cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev);
-  return (per_sm > 0 ? per_sm : 1) * (nsm > 0 ? nsm : 1);
-}
-} // namespace
-
-cudaError_t
-ensemble2d_step(int prec, const EnsInstance * insts, int n, const EnsTile * tiles, int ntiles, int * stepc,
-                void * scal, int grid, cudaStream_t st)
-{
+  const dim3 grid((unsigned)ntiles);
 #ifdef EK_EXACT_ONLY
   if (prec != 0)
     return cudaErrorNotSupported;
-  return ensemble2d_t<double, double>(insts, n, tiles, ntiles, stepc, scal, grid, st);
 #else
-  if (prec == 0)
-    return ensemble2d_t<double, double>(insts, n, tiles, ntiles, stepc, scal, grid, st);
-  return ensemble2d_t<float, float>(insts, n, tiles, ntiles, stepc, scal, grid, st);
+  if (prec != 0)
+    return launch_chained(ensemble2d_step<float, float>, grid, 32 * kRowWarps, 0, st, insts, tiles, rows);
 #endif
-}
-
-int
-ensemble2d_grid(int prec)
-{
-#ifdef EK_EXACT_ONLY
-  return ensemble2d_grid_t<double, double>();
-#else
-  return prec == 0 ? ensemble2d_grid_t<double, double>() : ensemble2d_grid_t<float, float>();
-#endif
+  return launch_chained(ensemble2d_step<double, double>, grid, 32 * kRowWarps, 0, st, insts, tiles, rows);
 }
 
 #ifndef EK_EXACT_ONLY
@@ -458,7 +411,7 @@ convert_stage(bool to_state, int prec, int layout, double * stage, void * U, con
 }
 
 cudaError_t
-ensemble_totals(int prec, const EnsInstance * insts, int n, const int * stepc, double * out,
+ensemble_totals(int prec, const EnsInstance * insts, int n, int step, double * out,
                 cudaStream_t st)
 {
   cudaError_t e = cudaMemsetAsync(out, 0, 2 * sizeof(double) * n, st);
@@ -466,9 +419,9 @@ ensemble_totals(int prec, const EnsInstance * insts, int n, const int * stepc, d
     return e;
   dim3 grid(16, n);
   if (prec == 0)
-    ensemble_totals_kernel<double><<<grid, 256, 0, st>>>(insts, stepc, out);
+    ensemble_totals_kernel<double><<<grid, 256, 0, st>>>(insts, step, out);
   else
-    ensemble_totals_kernel<float><<<grid, 256, 0, st>>>(insts, stepc, out);
+    ensemble_totals_kernel<float><<<grid, 256, 0, st>>>(insts, step, out);
   return cudaGetLastError();
 }
 

@@ -36,11 +36,9 @@
   size_t      mhd2d_work_bytes(int prec, const KParams & P);                                        \
   cudaError_t mhd2d_dt(int prec, const void * U, const KParams & P, unsigned long long * key,       \
                        cudaStream_t st);                                                            \
-  /* one step of every instance of a 2D hydro ensemble (persistent kernel) */                       \
-  /* scal: per-instance step scalars (n entries of 64 bytes), written by the step */                \
-  cudaError_t ensemble2d_step(int prec, const ekc::EnsInstance * insts, int n, const ekc::EnsTile * tiles, \
-                              int ntiles, int * stepc, void * scal, int grid, cudaStream_t st);     \
-  int         ensemble2d_grid(int prec);                                                            \
+  /* one step of every instance of a 2D hydro ensemble; rows: of a warp's run (choose_rows) */          \
+  cudaError_t ensemble2d_step(int prec, const ekc::EnsInstance * insts, const ekc::EnsTile * tiles,  \
+                              int ntiles, int rows, cudaStream_t st);                                \
   /* the FP64 MHD step in passes: phase 0 (primitives, CFL, electric field), 1 (trace, fluxes, */   \
   /* emfs, update); work: workspace of pass_bytes */                                                \
   cudaError_t mhd_passes(int dim, int phase, const void * Uin, void * Uout, void * work,            \
@@ -61,7 +59,7 @@ using ekc::KParams;
 cudaError_t fill_ghosts(int prec, void * U, const KParams & P, int nbvar, cudaStream_t st);
 cudaError_t totals(int prec, const void * U, const KParams & P, int nbvar, double * out3,
                    cudaStream_t st);
-cudaError_t ensemble_totals(int prec, const ekc::EnsInstance * insts, int n, const int * stepc,
+cudaError_t ensemble_totals(int prec, const ekc::EnsInstance * insts, int n, int step,
                             double * out, cudaStream_t st);
 // Host FP64 arrays <-> device state.  Elements [first, first + count) of a
 // host array in the caller's layout (0 LayoutLeft, 1 LayoutRight; nbvar

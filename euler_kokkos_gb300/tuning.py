@@ -28,9 +28,7 @@ TUNING_FILE = os.path.join(HERE, "tuning.json")
 
 # Candidate sets per kernel family; candidate 0 is the built-in default.
 CANDIDATES = {
-    "hydro2d": [{"EK_H2_TX": "32", "EK_H2_TY": "8"}, {"EK_H2_TX": "32", "EK_H2_TY": "4"}, {"EK_H2_TX": "64", "EK_H2_TY": "4"},
-                {"EK_H2_TX": "16", "EK_H2_TY": "16"}, {"EK_H2_TX": "64", "EK_H2_TY": "8"},
-                {"EK_H2_TX": "16", "EK_H2_TY": "8"}, {"EK_H2_TX": "32", "EK_H2_TY": "16"}],
+    "hydro2d": [{"EK_H2_MINB_F32": "5"}, {"EK_H2_MINB_F32": "6"}, {"EK_H2_MINB_F32": "4"}, {"EK_H2_MINB_F32": "7"}],
     "hydro3d": [{"EK_H3_TX": "32", "EK_H3_TY": "8", "EK_H3_MINB_F32": "4", "EK_H3_MINB_F64": "2"},
                 {"EK_H3_TX": "32", "EK_H3_TY": "4", "EK_H3_MINB_F32": "8", "EK_H3_MINB_F64": "4"},
                 {"EK_H3_TX": "64", "EK_H3_TY": "4", "EK_H3_MINB_F32": "4", "EK_H3_MINB_F64": "2"},
@@ -105,7 +103,7 @@ def measure(families):
 
     res = {}
     if "hydro2d" in families:
-        # the 2D tile serves the single solver and the ensemble; the batched
+        # the march serves the single solver and the ensemble; the batched
         # Kelvin-Helmholtz ensemble is the benchmark that uses it
         res["hydro2d"] = _ensemble_ms(ek, P)
     if "hydro3d" in families:

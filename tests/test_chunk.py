@@ -12,10 +12,19 @@ PROGRAM = r"""
 #include "ek_chunk.h"
 #include <cstdio>
 #include <cstdlib>
+#include <initializer_list>
 int main(int, char ** a)
 {
   const ekc::ChunkModel m[6] = { ekc::kChunkHydro64, ekc::kChunkHydro32, ekc::kChunkTrace64, ekc::kChunkTrace32,
                                  ekc::kChunkUpdate64, ekc::kChunkUpdate32 };
+  if (atoi(a[3]) < 0) // rows of the 2D marches: nx, ny, -sms
+  {
+    const int nx[2] = { atoi(a[1]), atoi(a[1]) }, ny[2] = { atoi(a[2]), atoi(a[2]) };
+    for (int n = 1; n <= 2; ++n)
+      for (auto & x : { ekc::kChunkRows64, ekc::kChunkRows32 })
+        std::printf("%d ", ekc::choose_rows(nx, ny, n, -atoi(a[3]), x));
+    return 0;
+  }
   for (auto & x : m)
     std::printf("%d ", ekc::choose_chunk(atoll(a[1]), atoi(a[2]), atoi(a[3]), x));
 }
@@ -43,3 +52,12 @@ def test_chunks_cover_the_planes(program, columns, planes, sms):
             assert kc == 1
         if columns >= 1000 * sms:  # plenty of tiles: no repeated end planes
             assert kc == planes
+
+
+@pytest.mark.parametrize("nx,ny", [(1, 1), (2, 2), (64, 64), (28, 10_000_000), (1, 4_000_000), (1022, 518), (30000, 20000)])
+def test_runs_of_rows(program, nx, ny):
+    for rows in map(int, subprocess.run([program, str(nx), str(ny), "-152"], check=True, capture_output=True,
+                                        text=True).stdout.split()):
+        assert 1 <= rows <= min(ny, 64) and -(-ny // (4 * rows)) <= 65535
+        if nx * ny <= 64 * 64:  # few warps: one row each
+            assert rows == 1

@@ -41,6 +41,42 @@ def test_tiles_match_the_oracle(dim, mhd, n):
             assert np.max(rel_linf(U, ref)[[0, 1]]) <= 1e-11 and np.max(np.abs(d / dts - 1)) <= 1e-13
 
 
+# 2D marches: strips of 28 columns, four runs of rows per CTA
+ROW_SIZES = [(2, 2), (27, 5), (28, 8), (29, 9), (57, 3), (5, 131), (84, 33)]
+
+
+@pytest.mark.parametrize("more", [0, 12], ids=["one row", "longer runs"])
+def test_marching_warps_match_the_oracle(more):
+    """An ensemble's instances run the march: bitwise in the exact build, with runs of one row (few cells) and longer
+    ones (the added instances)."""
+    cases = [P.smooth_random(dim=2, nx=x, ny=y, seed=x + y, bc=(1, 2, 3, 3, 1, 1) if x % 2 else (3, 3, 2, 1, 1, 1), nsteps=3)
+             for x, y in ROW_SIZES + more * [(128, 130)]]
+    with ek.Ensemble([ek.params_from_ini(ini, exact_fp=1) for ini, _ in cases]) as e:
+        for i, (_, U0) in enumerate(cases):
+            e.set_state(i, U0)
+        e.run(3)
+        e.synchronize()
+        for i, (ini, U0) in enumerate(cases[:len(ROW_SIZES) + 1]):
+            o = eko.Oracle(eko.params_from_ini(ini), U0)
+            dts = o.run(3)
+            assert np.array_equal(e.dt_history(i), dts), i
+            assert np.array_equal(interior(e.get_state(i), 2, 2), interior(o.state(), 2, 2)), i
+
+
+@pytest.mark.parametrize("n", ROW_SIZES + [(400, 301)])
+def test_mixed_marching_warps(n):
+    ini, U0 = P.smooth_random(dim=2, nx=n[0], ny=n[1], seed=sum(n), bc=(1, 2, 3, 3, 1, 1), nsteps=3)
+    o = eko.Oracle(eko.params_from_ini(ini), U0)
+    o.run(3)
+    ref = interior(o.state(), 2, 2)
+    with ek.Solver(ek.params_from_ini(ini, precision=ek.EK_PREC_MIXED)) as s:
+        s.set_state(U0)
+        assert s.run(3) == 3
+        U = interior(s.get_state(), 2, 2)
+    for v in (0, 1):  # density and energy, the mixed form's bound
+        assert np.abs(U[v] - ref[v]).sum() / np.abs(ref[v]).sum() <= 1e-5
+
+
 @pytest.mark.parametrize("mhd", [False, True], ids=["hydro", "mhd"])
 def test_slabs_do_not_show(mhd):
     """A grid whose workspace takes several slabs of passes (the trace of 262144-cell planes, 1 GiB a slab): the mixed
