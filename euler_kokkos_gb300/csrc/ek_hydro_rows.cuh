@@ -12,7 +12,8 @@
 // (678 instructions a cell with runs of 8).  Issue bounds large grids (57 to 73 %
 // busy, 20 warps per SM at 96 registers; at 80, 24 warps, 2 % slower), the chain
 // of one row, 0.6 us, small ones.  us per step, tile / march: mixed 64^2 12.4 /
-// 8.8, 512^2 18.5 / 14.1, 1022 x 518 29.6 / 21.3, 2048^2 182 / 91; ensemble of 32
+// 8.7, 512^2 18.5 / 13.6, 1022 x 518 29.6 / 20.3, 2048^2 182 / 85 (the first and
+// last row in the loop, by branches: 14.4, 22.2, 91); ensemble of 32
 // runs of 64^2 to 256^2 mixed 42 / 31, FP64 852 / 551.
 #pragma once
 
@@ -91,14 +92,14 @@ hydro2d_rows(const S * __restrict__ Uin, S * __restrict__ Uout, const PP & P, co
     prims(wb, qb);
     prims(next, qc);
   }
-  R top[NV], acc[NV], rho_old = R(0); // state above row r - 1; its update so far
-  for (int r = -1; r <= n; ++r)
-  {
-    const bool inner = r >= 0 && r < n;
-    if (r < n)
+  R top[NV], acc[NV] = {}, rho_old = R(0); // state above row r - 1; its update so far
+  // one row; the first (-1) and the last (n) only for the states that face the run
+  auto row = [&](int r, auto part) {
+    constexpr bool first = part.value < 0, last = part.value > 0, inner = !first && !last;
+    if constexpr (!last)
       load(j0 + r + 2, next);
     S u0[NV];
-    if (inner)
+    if constexpr (inner)
     {
       const S * in = Uin + (long long)(P.gw + j0 + r) * P.isize + si;
 #pragma unroll
@@ -128,7 +129,7 @@ hydro2d_rows(const S * __restrict__ Uin, S * __restrict__ Uout, const PP & P, co
     }
     FaceStates<R, NV> F(qb, s, dtdx, C.smallr);
     R                 fx[NV];
-    if (inner)
+    if constexpr (inner)
     {
       // x flux through the low face of the cell
       R l[NV], h[NV];
@@ -149,7 +150,7 @@ hydro2d_rows(const S * __restrict__ Uin, S * __restrict__ Uout, const PP & P, co
     }
     F.turn(dtdy, same_xy);
     R fy[NV];
-    if (r >= 0)
+    if constexpr (!first)
     {
       // y flux through the low face, IU and IV swapped around the solver
       R l[NV], h[NV], f[NV];
@@ -168,21 +169,21 @@ hydro2d_rows(const S * __restrict__ Uin, S * __restrict__ Uout, const PP & P, co
       for (int v = 0; v < NV; ++v)
         fy[v] = flux_scaled(f[v < IU ? v : IU + IV - v], dtdy);
     }
-    if (r >= 1)
+    if constexpr (!first)
     {
-      // row r - 1 is complete (UpdateFunctor2D, HydroRunFunctors2D.h:809-836, in its order)
+      // row r - 1 is complete (of r = 0: nothing) (UpdateFunctor2D, HydroRunFunctors2D.h:809-836, in its order)
 #pragma unroll
       for (int v = 0; v < NV; ++v)
         acc[v] = sub_flux(acc[v], fy[v], dtdy);
-      const int gj = P.gw + j0 + r - 1;
-      R         g[3];
+      const int          gj = P.gw + j0 + r - 1;
+      [[maybe_unused]] R g[3];
       if constexpr (GRAV)
       {
         // gravity source term after the flux update (SolverHydroMuscl.cpp:245-252)
         grav_at<S, R, NV>(P, P.gw + i, gj, 0, g);
         grav_source<R, NV>(acc, rho_old, g, hdt, C);
       }
-      if (mine)
+      if (mine && r >= 1)
       {
         // the next step's dt is computed on the stored (possibly rounded) state
         S * out = Uout + (long long)gj * P.isize + P.gw + i;
@@ -199,7 +200,7 @@ hydro2d_rows(const S * __restrict__ Uin, S * __restrict__ Uout, const PP & P, co
           tmax = max_cand(tmax, hydro_invdt<R, NV>(us, C, P));
       }
     }
-    if (inner)
+    if constexpr (inner)
     {
 #pragma unroll
       for (int v = 0; v < NV; ++v)
@@ -212,17 +213,25 @@ hydro2d_rows(const S * __restrict__ Uin, S * __restrict__ Uout, const PP & P, co
         acc[v] = add_flux(x, fy[v], dtdy);
       }
     }
-    F.get(dY, true, top);
-    if (kick)
-      grav_kick<R, NV>(top, hg);
-#pragma unroll
-    for (int v = 0; v < NV; ++v)
+    if constexpr (!last)
     {
-      qa[v] = qb[v];
-      qb[v] = qc[v];
+      F.get(dY, true, top);
+      if (kick)
+        grav_kick<R, NV>(top, hg);
+#pragma unroll
+      for (int v = 0; v < NV; ++v)
+      {
+        qa[v] = qb[v];
+        qb[v] = qc[v];
+      }
+      prims(next, qc);
     }
-    prims(next, qc);
-  }
+  };
+  row(-1, std::integral_constant<int, -1>());
+#pragma unroll 1
+  for (int r = 0; r < n; ++r)
+    row(r, std::integral_constant<int, 0>());
+  row(n, std::integral_constant<int, 1>());
   return tmax;
 }
 
