@@ -8,6 +8,7 @@
 #include <cstdio>
 #include <cstdlib>
 #include <cstring>
+#include <mutex>
 #include <string>
 #include <vector>
 
@@ -34,6 +35,75 @@ using ek_internal::fail;
 using KParams = ekc::KParams;
 using DevClock = ekc::DevClock;
 
+// Device staging of host FP64 arrays (set/get state), at most kStageElems.  One
+// transfer at a time: an ensemble's instances share one.
+struct Stage
+{
+  double *   buf = nullptr;
+  long long  elems = 0;
+  std::mutex lock;
+};
+
+// Page-locked memory for the host's copies of device clocks: a read through it
+// takes 5 us less than through pageable memory (next_iteration of 64^2 31 -> 25
+// us), but to lock and unlock a page takes 330 us, so that one block of 128
+// slots serves the process.  Slots beyond them are null (the reads then go
+// through pageable memory).
+struct ClockSlots
+{
+  static constexpr int kSlots = 128, kBytes = 512;
+  static_assert(sizeof(DevClock) <= kBytes, "a slot holds a clock");
+  std::mutex lock;
+  char *     block = nullptr;
+  unsigned   generation = 0; // of the block
+  bool       used[kSlots];
+
+  DevClock * take(unsigned & gen)
+  {
+    std::lock_guard<std::mutex> hold(lock);
+    if (block)
+    {
+      // a device reset frees page-locked memory too
+      cudaPointerAttributes at;
+      if (cudaPointerGetAttributes(&at, block) != cudaSuccess || at.type != cudaMemoryTypeHost)
+        block = nullptr;
+    }
+    if (!block)
+    {
+      if (cudaMallocHost((void **)&block, (size_t)kSlots * kBytes) != cudaSuccess)
+        block = nullptr;
+      std::memset(used, 0, sizeof used);
+      ++generation;
+    }
+    cudaGetLastError(); // of the calls above
+    gen = generation;
+    for (int i = 0; block && i < kSlots; ++i)
+      if (!used[i])
+      {
+        used[i] = true;
+        return reinterpret_cast<DevClock *>(block + i * kBytes);
+      }
+    return nullptr;
+  }
+  void give(DevClock * p, unsigned gen)
+  {
+    std::lock_guard<std::mutex> hold(lock);
+    if (p && gen == generation)
+      used[(reinterpret_cast<char *>(p) - block) / kBytes] = false;
+  }
+};
+static ClockSlots g_clock_slots;
+
+// One reader at a time: an ensemble's instances share one.
+struct HostClock
+{
+  DevClock * p = nullptr;
+  unsigned   generation = 0;
+  std::mutex lock;
+  void       take() { p = g_clock_slots.take(generation); }
+  ~HostClock() { g_clock_slots.give(p, generation); }
+};
+
 struct ek_solver
 {
   ek_params     p;
@@ -59,8 +129,10 @@ struct ek_solver
   int           iteration = 0;
   bool          has_state = false;
   long long     launches = 0;
-  double *      stage = nullptr; // device staging of host FP64 arrays (set/get state)
-  long long     stage_elems = 0;
+  Stage *       stage = &own_stage; // an ensemble's views share the ensemble's
+  Stage         own_stage;
+  HostClock *   h_clk = &own_clk;
+  HostClock     own_clk;
   // kernel timing (ek_solver_set_profiling)
   bool                     profiling = false;
   std::vector<cudaEvent_t> ev_pool;            // recycled events
@@ -404,6 +476,8 @@ ek_solver_create(const ek_params * params, ek_solver ** out)
   if (e == cudaSuccess && !p.mhd && p.dim == 3 && !p.no_tma)
     s->has_tmap = ek_fast::hydro3d_tensor_map(s->prec, s->U[0], k, &s->tmap[0]) &&
                   ek_fast::hydro3d_tensor_map(s->prec, s->U[1], k, &s->tmap[1]);
+  if (e == cudaSuccess)
+    s->own_clk.take();
   if (e != cudaSuccess)
   {
     ek_status st = cuda_fail(e, "ek_solver_create");
@@ -422,7 +496,6 @@ ek_solver_destroy(ek_solver * s)
   if (!s->owns)
   {
     drain_events(s);
-    cudaFree(s->stage);
     delete s;
     return EK_OK;
   }
@@ -435,7 +508,7 @@ ek_solver_destroy(ek_solver * s)
   cudaFree(s->dtlog);
   cudaFree(s->scratch3);
   cudaFree(s->gfield);
-  cudaFree(s->stage);
+  cudaFree(s->own_stage.buf);
   drain_events(s);
   for (auto e : s->ev_pool)
     cudaEventDestroy(e);
@@ -453,28 +526,17 @@ ek_solver_destroy(ek_solver * s)
 static const long long kStageElems = 1LL << 25; // 32 Mi doubles (256 MB)
 
 static ek_status
-ensure_stage(ek_solver * s, long long total)
+ensure_stage(Stage & g, long long total)
 {
   const long long want = total < kStageElems ? total : kStageElems;
-  if (s->stage_elems >= want)
+  if (g.elems >= want)
     return EK_OK;
-  cudaFree(s->stage);
-  s->stage = nullptr;
-  s->stage_elems = 0;
-  EK_CUDA(cudaMalloc((void **)&s->stage, sizeof(double) * (size_t)want), "staging buffer");
-  s->stage_elems = want;
+  cudaFree(g.buf);
+  g.buf = nullptr;
+  g.elems = 0;
+  EK_CUDA(cudaMalloc((void **)&g.buf, sizeof(double) * (size_t)want), "staging buffer");
+  g.elems = want;
   return EK_OK;
-}
-
-// views into an ensemble keep no staging buffer between calls
-static void
-release_stage(ek_solver * s)
-{
-  if (s->owns)
-    return;
-  cudaFree(s->stage);
-  s->stage = nullptr;
-  s->stage_elems = 0;
 }
 
 static ek_status
@@ -487,20 +549,21 @@ host_to_state(ek_solver * s, const double * U, int layout, void * dev)
     EK_CUDA(cudaStreamSynchronize(s->stream), "upload");
     return EK_OK;
   }
-  ek_status st = ensure_stage(s, total);
+  Stage &                     g = *s->stage;
+  std::lock_guard<std::mutex> hold(g.lock);
+  ek_status                   st = ensure_stage(g, total);
   if (st != EK_OK)
     return st;
-  for (long long first = 0; first < total; first += s->stage_elems)
+  for (long long first = 0; first < total; first += g.elems)
   {
-    const long long cnt = total - first < s->stage_elems ? total - first : s->stage_elems;
-    EK_CUDA(cudaMemcpyAsync(s->stage, U + first, sizeof(double) * (size_t)cnt, cudaMemcpyHostToDevice, s->stream),
+    const long long cnt = total - first < g.elems ? total - first : g.elems;
+    EK_CUDA(cudaMemcpyAsync(g.buf, U + first, sizeof(double) * (size_t)cnt, cudaMemcpyHostToDevice, s->stream),
             "upload");
-    EK_CUDA(ek_fast::convert_stage(true, s->prec, layout, s->stage, dev, s->kp, s->p.nbvar, first, cnt, s->stream),
+    EK_CUDA(ek_fast::convert_stage(true, s->prec, layout, g.buf, dev, s->kp, s->p.nbvar, first, cnt, s->stream),
             "upload");
     s->launches += 1;
   }
   EK_CUDA(cudaStreamSynchronize(s->stream), "upload");
-  release_stage(s);
   return EK_OK;
 }
 
@@ -514,21 +577,22 @@ state_to_host(ek_solver * s, const void * dev, double * U, int layout)
     EK_CUDA(cudaStreamSynchronize(s->stream), "download");
     return EK_OK;
   }
-  ek_status st = ensure_stage(s, total);
+  Stage &                     g = *s->stage;
+  std::lock_guard<std::mutex> hold(g.lock);
+  ek_status                   st = ensure_stage(g, total);
   if (st != EK_OK)
     return st;
-  for (long long first = 0; first < total; first += s->stage_elems)
+  for (long long first = 0; first < total; first += g.elems)
   {
-    const long long cnt = total - first < s->stage_elems ? total - first : s->stage_elems;
-    EK_CUDA(ek_fast::convert_stage(false, s->prec, layout, s->stage, const_cast<void *>(dev), s->kp, s->p.nbvar,
+    const long long cnt = total - first < g.elems ? total - first : g.elems;
+    EK_CUDA(ek_fast::convert_stage(false, s->prec, layout, g.buf, const_cast<void *>(dev), s->kp, s->p.nbvar,
                                    first, cnt, s->stream),
             "download");
     s->launches += 1;
-    EK_CUDA(cudaMemcpyAsync(U + first, s->stage, sizeof(double) * (size_t)cnt, cudaMemcpyDeviceToHost, s->stream),
+    EK_CUDA(cudaMemcpyAsync(U + first, g.buf, sizeof(double) * (size_t)cnt, cudaMemcpyDeviceToHost, s->stream),
             "download");
   }
   EK_CUDA(cudaStreamSynchronize(s->stream), "download");
-  release_stage(s);
   return EK_OK;
 }
 
@@ -592,6 +656,16 @@ reset_clock(ek_solver * s, double t0)
 static ek_status
 read_clock(ek_solver * s, DevClock * h)
 {
+  HostClock & c = *s->h_clk;
+  if (c.p)
+  {
+    // by way of page-locked memory, which the copy engine writes itself
+    std::lock_guard<std::mutex> hold(c.lock);
+    EK_CUDA(cudaMemcpyAsync(c.p, s->clk, sizeof *h, cudaMemcpyDeviceToHost, s->stream), "clock read");
+    EK_CUDA(cudaStreamSynchronize(s->stream), "clock read");
+    *h = *c.p;
+    return EK_OK;
+  }
   EK_CUDA(cudaMemcpyAsync(h, s->clk, sizeof *h, cudaMemcpyDeviceToHost, s->stream), "clock read");
   EK_CUDA(cudaStreamSynchronize(s->stream), "clock read");
   return EK_OK;
@@ -1205,6 +1279,8 @@ struct ek_ensemble
   ekc::EnsInstance *       d_insts = nullptr;
   ekc::EnsTile *           d_tiles = nullptr;
   double *                 d_totals = nullptr;
+  HostClock                h_clk;              // of the instances' clock reads
+  Stage                    stage;              // of the instances' transfers
   int                      ntiles = 0;
   int                      rows = 1; // of a warp's run (choose_rows)
   int                      step = 0; // steps launched
@@ -1236,6 +1312,7 @@ ek_ensemble_destroy(ek_ensemble * e)
   cudaFree(e->d_insts);
   cudaFree(e->d_tiles);
   cudaFree(e->d_totals);
+  cudaFree(e->stage.buf);
   if (e->stream)
     cudaStreamDestroy(e->stream);
   delete e;
@@ -1304,6 +1381,7 @@ ek_ensemble_create(const ek_params * params, int n, ek_ensemble ** out)
   std::vector<ekc::EnsTile>     tiles;
   if (err == cudaSuccess)
   {
+    e->h_clk.take();
     std::vector<int> nx(n), ny(n);
     for (int i = 0; i < n; ++i)
       nx[i] = params[i].nx, ny[i] = params[i].ny;
@@ -1326,6 +1404,8 @@ ek_ensemble_create(const ek_params * params, int n, ek_ensemble ** out)
       v->dtlog = e->dtlogs + (size_t)i * dtcap;
       v->dtcap = dtcap;
       v->scratch3 = nullptr;
+      v->stage = &e->stage;
+      v->h_clk = &e->h_clk;
       e->views.push_back(v);
       h_insts[i].P = v->kp;
       h_insts[i].U[0] = v->U[0];
