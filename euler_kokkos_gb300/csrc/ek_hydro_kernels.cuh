@@ -118,17 +118,31 @@ __device__ __forceinline__ void
 cell_slopes(const R * q0, const R * qm, const R * qp, int hx, int hy, R st, R (&c)[NV], R (&dX)[NV],
             R (&dY)[NV], R (&dZ)[NV], bool three_d)
 {
+  constexpr int V = HY * HX;
+  const int     o = hy * HX + hx;
+  R             lo[NV], hi[NV];
+  auto          get = [&](const R * p, R(&x)[NV]) {
 #pragma unroll
-  for (int v = 0; v < NV; ++v)
+    for (int v = 0; v < NV; ++v)
+      x[v] = p[v * V];
+  };
+  get(q0 + o, c);
+  get(q0 + o - 1, lo);
+  get(q0 + o + 1, hi);
+  slopes_h<R, NV>(c, hi, lo, st, dX);
+  get(q0 + o - HX, lo);
+  get(q0 + o + HX, hi);
+  slopes_h<R, NV>(c, hi, lo, st, dY);
+  if (three_d)
   {
-    const R * p = q0 + v * HY * HX;
-    const R   x = p[hy * HX + hx];
-    c[v] = x;
-    dX[v] = slope_h<R>(x, p[hy * HX + hx + 1], p[hy * HX + hx - 1], st);
-    dY[v] = slope_h<R>(x, p[(hy + 1) * HX + hx], p[(hy - 1) * HX + hx], st);
-    if (three_d)
-      dZ[v] = slope_h<R>(x, qp[(v * HY + hy) * HX + hx], qm[(v * HY + hy) * HX + hx], st);
-    else
+    get(qm + o, lo);
+    get(qp + o, hi);
+    slopes_h<R, NV>(c, hi, lo, st, dZ);
+  }
+  else
+  {
+#pragma unroll
+    for (int v = 0; v < NV; ++v)
       dZ[v] = R(0);
   }
 }
