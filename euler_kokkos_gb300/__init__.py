@@ -416,7 +416,7 @@ class Solver:
 
 
 class Ensemble:
-    """Independent Hydro_Muscl_2D runs stepped together by one persistent
+    """Independent Hydro_Muscl_2D runs stepped together by one
     kernel per step (optionally replayed from a CUDA graph)."""
 
     def __init__(self, params_list):

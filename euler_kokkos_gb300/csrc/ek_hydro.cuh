@@ -374,7 +374,10 @@ template <class R>
 __device__ __forceinline__ R
 flux_scaled(R f, R dtd)
 {
-  return kFast64<R> ? f : f * dtd;
+  if constexpr (sizeof(R) == 4)
+    return __fmul_rn(f, dtd); // rounded: both cells of a face take the same value, whichever code adds it
+  else
+    return kFast64<R> ? f : f * dtd;
 }
 template <class R>
 __device__ __forceinline__ R

@@ -2,8 +2,8 @@
 // device arrays that allocates no device memory.
 //
 // The step: boundaries of U_in (by index mapping), the CFL dt of that state,
-// the trace, fluxes, emfs and update into U_out -- the same kernels as a step
-// of ek_solver_next_iteration.
+// the trace, fluxes, emfs and update into U_out by the tile kernels
+// (a step of ek_solver_next_iteration does the same arithmetic in passes).
 //
 // Which callers cannot allocate, and why: a host code that hands the library
 // only the two state arrays of the step and keeps every other byte of device

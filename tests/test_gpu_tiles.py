@@ -63,6 +63,27 @@ def test_marching_warps_match_the_oracle(more):
             assert np.array_equal(interior(e.get_state(i), 2, 2), interior(o.state(), 2, 2)), i
 
 
+@pytest.mark.parametrize("prec", [ek.EK_PREC_FP64, ek.EK_PREC_MIXED], ids=["fp64", "mixed"])
+def test_runs_of_rows_do_not_show(prec):
+    """A cell's result does not depend on the rows per run: the same instances beside few and many others, bitwise, and
+    no mass is lost at the ends of runs."""
+    cases = [P.smooth_random(dim=2, nx=x, ny=y, seed=x + y, bc=(3, 3, 3, 3, 1, 1), nsteps=20) for x, y in ROW_SIZES + [(100, 120)]]
+    out = []
+    for more in (0, 40):
+        with ek.Ensemble([ek.params_from_ini(ini, precision=prec) for ini, _ in cases + more * cases[-1:]]) as e:
+            for i, (_, U0) in enumerate(cases + more * cases[-1:]):
+                e.set_state(i, U0)
+            e.run(20)
+            e.synchronize()
+            out.append([(e.get_state(i), e.dt_history(i)) for i in range(len(cases))])
+    for (U, d), (V, f), (_, U0) in zip(*out, cases):
+        assert np.array_equal(U, V) and np.array_equal(d, f)
+        # 20 updates of n cells, each rounded to half an ulp of about its value
+        n, m = interior(U, 2, 2)[0].size, interior(U0, 2, 2)[0].sum()
+        ulp = 2.0 ** -52 if prec == ek.EK_PREC_FP64 else 2.0 ** -23
+        assert abs(interior(U, 2, 2)[0].sum() / m - 1) <= 20 * 8 * ulp / np.sqrt(n) + 8 * ulp
+
+
 @pytest.mark.parametrize("n", ROW_SIZES + [(400, 301)])
 def test_mixed_marching_warps(n):
     ini, U0 = P.smooth_random(dim=2, nx=n[0], ny=n[1], seed=sum(n), bc=(1, 2, 3, 3, 1, 1), nsteps=3)
