@@ -640,7 +640,7 @@ mhd2d_tile(const void * __restrict__ Uin, void * __restrict__ Uout, const KParam
 // One launch per step: the tiles of the grid.  repair: the tile list of the
 // mixed HLLD form (null otherwise), for the repair kernel that follows.
 template <class S, class R, int TX, int TY, int NT, int RS>
-__global__ void __launch_bounds__(NT, EK_MINB(R, EK_M2_MINB_F32, EK_M2_MINB_F64))
+__global__ void __launch_bounds__(NT, EK_MINB(R, NT < 256 ? 0 : EK_M2_MINB_F32, EK_M2_MINB_F64))
 mhd2d_step_kernel(const void * __restrict__ Uin, void * __restrict__ Uout, KParams P, DevClock * clk,
                   int step, int * repair)
 {
@@ -656,8 +656,8 @@ mhd2d_step_kernel(const void * __restrict__ Uin, void * __restrict__ Uout, KPara
 // After the step kernel of the mixed HLLD form: recomputes the tiles it
 // listed with the ill-conditioned faces solved in FP64 (tiles are independent
 // within a step, so this replaces their output), then clears the list.
-template <class S, class R, int TX, int TY>
-__global__ void __launch_bounds__(TX * TY, EK_MINB(R, EK_M2_MINB_F32, EK_M2_MINB_F64))
+template <class S, class R, int TX, int TY, int NT>
+__global__ void __launch_bounds__(NT, EK_MINB(R, NT < 256 ? 0 : EK_M2_MINB_F32, EK_M2_MINB_F64))
 mhd2d_repair_kernel(const void * __restrict__ Uin, void * __restrict__ Uout, KParams P, DevClock * clk,
                     int step, int * repair)
 {
@@ -671,7 +671,7 @@ mhd2d_repair_kernel(const void * __restrict__ Uin, void * __restrict__ Uout, KPa
   for (int e = blockIdx.x; e < n; e += gridDim.x)
   {
     const int tile = repair[kRepairHead + e];
-    mhd2d_tile<S, R, TX, TY, TX * TY, 4, true>(Uin, Uout, P, clk, step, sc, tile % gx, tile / gx, repair);
+    mhd2d_tile<S, R, TX, TY, NT, 4, true>(Uin, Uout, P, clk, step, sc, tile % gx, tile / gx, repair);
     __syncthreads(); // shared memory of the next tile
   }
   repair_list_release(repair);
@@ -681,9 +681,18 @@ mhd2d_repair_kernel(const void * __restrict__ Uin, void * __restrict__ Uout, KPa
 constexpr int M2_TX = EK_M2_TX, M2_TY = EK_M2_TY;
 
 inline long long
-mhd2d_tiles(const KParams & P)
+mhd2d_tiles(const KParams & P, int TX, int TY)
 {
-  return (long long)((P.nx + M2_TX - 1) / M2_TX) * ((P.ny + M2_TY - 1) / M2_TY);
+  return (long long)((P.nx + TX - 1) / TX) * ((P.ny + TY - 1) / TY);
+}
+// Mixed: 8 x 8 tiles with 128 threads while they make at most seven CTAs per SM:
+// a tile's phases, one after another, then set the time (us per step, 16 x 16 /
+// 8 x 8: 64^2 17.2 / 14.1, 128^2 17.5 / 14.7, 256^2 20.0 / 18.7), above it the
+// repeated halo work does (512^2, 27 CTAs per SM: 40.0 / 52.2).
+inline bool
+mhd2d_small(const KParams & P)
+{
+  return mhd2d_tiles(P, 8, 8) <= 7ll * P.sms;
 }
 
 template <class S, class R, int TX, int TY, int NT>
@@ -701,6 +710,18 @@ mhd2d_step_tiled(const void * Uin, void * Uout, void * work, const KParams & P, 
   int * repair = sizeof(R) == 4 && P.riemann == 4 ? (int *)work : nullptr;
   const bool chained = sizeof(R) == 4 || chain_tiles(P, (long long)grid.x * grid.y);
   return launch_step_kernel(chained, k, grid, NT, sm, st, Uin, Uout, P, clk, step, repair);
+}
+
+template <class S, class R, int TX, int TY, int NT>
+cudaError_t
+mhd2d_repair_tiled(const void * Uin, void * Uout, void * work, const KParams & P, DevClock * clk, int step, cudaStream_t st)
+{
+  auto        k = mhd2d_repair_kernel<S, R, TX, TY, NT>;
+  const int   sm = (int)mhd2d_smem<R>(TX, TY);
+  cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, sm);
+  if (e != cudaSuccess)
+    return e;
+  return launch_chained(k, repair_grid(mhd2d_tiles(P, TX, TY)), NT, sm, st, Uin, Uout, P, clk, step, (int *)work);
 }
 
 template <class S, class R>
@@ -722,19 +743,16 @@ mhd2d_step_t(int phase, const void * Uin, void * Uout, void * work, const KParam
     {
       if (P.riemann != 4)
         return cudaErrorNotSupported;
-      auto        k = mhd2d_repair_kernel<S, R, M2_TX, M2_TY>;
-      const int   sm = (int)mhd2d_smem<R>(M2_TX, M2_TY);
-      cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, sm);
-      if (e != cudaSuccess)
-        return e;
-      return launch_chained(k, repair_grid(mhd2d_tiles(P)), M2_TX * M2_TY, sm, st, Uin, Uout, P, clk, step, (int *)work);
+      return mhd2d_small(P) ? mhd2d_repair_tiled<S, R, 8, 8, 128>(Uin, Uout, work, P, clk, step, st)
+                            : mhd2d_repair_tiled<S, R, M2_TX, M2_TY, M2_TX * M2_TY>(Uin, Uout, work, P, clk, step, st);
     }
   }
-  // Mixed: 16 x 16 at every size.  FP64, on grids too small for the passes: 8 x
+  // Mixed: 16 x 16, small grids 8 x 8 (mhd2d_small).  FP64, on grids too small for the passes: 8 x
   // 8 with 128 threads (64^2: 50 us; 16 x 8 82, 16 x 16 117; 200 x 136: 102, 117,
   // 117), since a tile's chain of FP64 instructions sets its time.
   if constexpr (sizeof(R) == 4)
-    return mhd2d_step_tiled<S, R, M2_TX, M2_TY, M2_TX * M2_TY>(Uin, Uout, work, P, clk, step, st);
+    return mhd2d_small(P) ? mhd2d_step_tiled<S, R, 8, 8, 128>(Uin, Uout, work, P, clk, step, st)
+                          : mhd2d_step_tiled<S, R, M2_TX, M2_TY, M2_TX * M2_TY>(Uin, Uout, work, P, clk, step, st);
   else
     return mhd2d_step_tiled<S, R, 8, 8, 128>(Uin, Uout, work, P, clk, step, st);
 }
@@ -744,7 +762,8 @@ mhd2d_step_t(int phase, const void * Uin, void * Uout, void * work, const KParam
 size_t
 mhd2d_work_bytes(int prec, const KParams & P)
 {
-  return prec == 0 ? 0 : sizeof(int) * (size_t)(kRepairHead + mhd2d_tiles(P));
+  return prec == 0 ? 0
+                   : sizeof(int) * (size_t)(kRepairHead + (mhd2d_small(P) ? mhd2d_tiles(P, 8, 8) : mhd2d_tiles(P, M2_TX, M2_TY)));
 }
 
 // one MHD 2D step = phase 0 (CFL), 1 (fused trace, fluxes, emf, update),

@@ -98,6 +98,33 @@ def test_mixed_marching_warps(n):
         assert np.abs(U[v] - ref[v]).sum() / np.abs(ref[v]).sum() <= 1e-5
 
 
+# mixed 2D MHD: 8 x 8 tiles up to seven per SM (264 x 256: 1056), 16 x 16 above (272 x 266: 1156)
+@pytest.mark.parametrize("n", [(3, 3), (8, 9), (17, 8), (33, 25), (264, 256), (272, 266)])
+def test_mixed_mhd2d_tiles(n):
+    ini, U0 = P.smooth_random(dim=2, mhd=True, nx=n[0], ny=n[1], seed=sum(n), bc=(1, 2, 3, 3, 1, 1), nsteps=3)
+    o = eko.Oracle(eko.params_from_ini(ini), U0)
+    o.run(3)
+    ref = interior(o.state(), 3, 2)
+    with ek.Solver(ek.params_from_ini(ini, precision=ek.EK_PREC_MIXED)) as s:
+        s.set_state(U0)
+        assert s.run(3) == 3
+        U = interior(s.get_state(), 3, 2)
+    for v in (0, 1):  # density and energy, the mixed form's bound
+        assert np.abs(U[v] - ref[v]).sum() / np.abs(ref[v]).sum() <= 1e-5
+
+
+def test_mixed_mhd2d_repair_in_16x16_tiles():
+    # the repair test's low-beta blast (tests/test_gpu_mhd2d.py) on a grid of 16 x 16 tiles
+    ini, U0 = P.mhd_blast_2d(n=272, nsteps=30)
+    with ek.Solver(ek.params_from_ini(ini, precision=ek.EK_PREC_MIXED)) as s, ek.Solver(ek.params_from_ini(ini)) as d:
+        s.set_state(U0)
+        d.set_state(U0)
+        assert s.run(30) == d.run(30) == 30
+        U, V = interior(s.get_state(), 3, 2), interior(d.get_state(), 3, 2)
+    for v in (0, 1):
+        assert np.abs(U[v] - V[v]).sum() / np.abs(V[v]).sum() <= 1e-5
+
+
 @pytest.mark.parametrize("mhd", [False, True], ids=["hydro", "mhd"])
 def test_slabs_do_not_show(mhd):
     """A grid whose workspace takes several slabs of passes (the trace of 262144-cell planes, 1 GiB a slab): the mixed
