@@ -1,4 +1,4 @@
-// Fused hydro step kernels (2D tile, 3D tile marching in z).
+// Fused hydro step kernels (2D tile; 3D tile marching in z, the mixed form's).
 //
 // One launch performs the whole implementationVersion=0 step of
 // SolverHydroMuscl::godunov_unsplit_impl (SolverHydroMuscl.cpp:214-243,
@@ -148,13 +148,9 @@ cell_slopes(const R * q0, const R * qm, const R * qp, int hx, int hy, R st, R (&
 }
 
 // ---------------------------------------------------------------------------
-// 2D: one CTA = one TX x TY tile of interior cells.  hydro2d_tile is the tile
-// body shared by the single-solver kernel and the ensemble kernel.
+// 2D, FP64 grids too small for the passes: one CTA = one TX x TY tile of
+// interior cells.
 // ---------------------------------------------------------------------------
-// LOADED: the caller already stored the tile's primitive plane in sQ (the
-// ensemble's prefetch); otherwise it is loaded here.
-// pre: the step scalars computed for the whole instance (the ensemble), else
-// thread 0 computes them for this CTA.
 // NT threads: one per cell, or more (a multiple of 32 per part), so that the
 // ring cells run beside the interior ones and the faces take fewer rounds.
 template <class S, class R, int TX, int TY, int NT, int RS = 3, bool GRAV = false>

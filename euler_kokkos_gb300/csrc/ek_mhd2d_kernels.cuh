@@ -1,5 +1,5 @@
-// MHD 2D (SolverMHDMuscl<2>, implementationVersion 0) on GB300: two kernels
-// per step.
+// MHD 2D (SolverMHDMuscl<2>, implementationVersion 0) on GB300: one kernel per
+// step, after a CFL kernel before the first one.
 //   1. mhd2d_dt_kernel    primitive variables of the boundary-mapped state and
 //                         the CFL max-reduction (ConvertToPrimitivesFunctor2D_MHD
 //                         + ComputeDtFunctor2D_MHD, MHDRunFunctors2D.h:16-160);
@@ -11,8 +11,8 @@
 //                         numbers per cell in shared memory, HLLD fluxes on
 //                         the x and y faces, the 2D-HLLD emf on the z edges,
 //                         then the hydro, Bz and face-field update
-//                         (SolverMHDMuscl.cpp:369-420).
-// The state is read from HBM in 1 and 2 and written once in 2.
+//                         (SolverMHDMuscl.cpp:369-420) and the next step's CFL.
+// The state is read from HBM and written once in 2.
 #pragma once
 
 #include "ek_mhd_kernels.cuh"

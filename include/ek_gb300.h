@@ -79,7 +79,7 @@ typedef struct ek_params
   int    precision; /* ek_precision; [gb300] precision = fp64 | mixed */
   int    exact_fp;  /* 1: FP64 kernels with the reference's arithmetic, no FMA contraction and
                        every division, bitwise equal to it ([gb300] exact = 1) */
-  int    kchunk;    /* 3D planes per CTA column (0: automatic; [gb300] kchunk) */
+  int    kchunk;    /* 3D planes per CTA column of the tile kernels (0: automatic; [gb300] kchunk) */
   int    mhd_stage; /* MHD update kernel stages the trace planes in shared memory ([gb300] mhd_stage) */
   char   solver_name[32];
   char   problem[32];
@@ -233,7 +233,7 @@ ek_status ek_solver_load_restart(ek_solver * s, const char * path, int reset_tim
  * Ensembles of independent Hydro_Muscl_2D runs (no counterpart in the
  * reference, which runs one problem per process): every instance has its own
  * grid size, parameters, boundary conditions and time step.  One step of all
- * instances is one persistent kernel over a flat (instance, tile) work list;
+ * instances is one kernel launch over a flat (instance, tile) work list;
  * ek_ensemble_run can capture the steps in a CUDA graph and replay it.
  * ------------------------------------------------------------------------- */
 typedef struct ek_ensemble ek_ensemble;
@@ -254,7 +254,7 @@ ek_status ek_ensemble_time(ek_ensemble * e, int i, double * t, double * dt, int 
 ek_status ek_ensemble_dt_history(ek_ensemble * e, int i, double * dts, int n);
 /* FP64 totals per instance: out[2i] mass, out[2i+1] total energy */
 ek_status ek_ensemble_totals(ek_ensemble * e, double * out);
-/* interior cells over all instances, work tiles per step, persistent grid size,
+/* interior cells over all instances, work tiles per step, grid size,
  * kernel launches issued */
 ek_status ek_ensemble_info(ek_ensemble * e, long long * interior_cells, int * tiles, int * grid,
                            long long * launches);
@@ -266,8 +266,8 @@ ek_status ek_ensemble_stream(ek_ensemble * e, void ** stream);
  * every byte of device memory in their own pool (a Kokkos memory space, an
  * embedding code that budgets the whole HBM) and hand the step only its two
  * state arrays, and for which a cudaMalloc / cudaFree pair per step (each
- * synchronising the device) is not acceptable.  It runs the same kernels as a
- * step of ek_solver_next_iteration.
+ * synchronising the device) is not acceptable.  It runs the tile kernels (a
+ * step of ek_solver_next_iteration does the same arithmetic in passes).
  *
  * The step's temporary (the 47 x FP64 per-cell compact trace) lives in one
  * static device array of EK_NOALLOC_SCRATCH_BYTES, held by every GPU context
