@@ -317,13 +317,6 @@ sqrt_a(float x)
   asm("sqrt.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x));
   return r;
 }
-// sqrt(n / d) for n >= 0, d > 0 in FP32, one reciprocal square root; NaN (which
-// fmaxf drops) where n d underflows
-__device__ __forceinline__ float
-sqrt_ratio_a(float n, float d)
-{
-  return n * rsqrt_a(n * d);
-}
 
 // Packed FP32 pairs: one instruction computes two lanes (sm_100 and later).
 // The mixed form's solvers put the left and right states of a face in the two

@@ -202,14 +202,14 @@ mhd_hlld_f32(const float (&ql)[8], const float (&qr)[8], float (&flux)[NF], floa
   const float2 ptot = add2(p, emag);
   const float2 vdotb = fma2(w, c, fma2(v, b, mul2(u, A)));
 
-  // the larger fast magnetosonic speed (find_speed_fast, the normal field a):
-  // rho c^2 of both sides, the discriminant as (B^2 - gamma p)^2 / 4 + gamma p
-  // Bt^2, which does not cancel; the quotients compared by products
-  const float2 g = mul2(f2s(gamma0), p), h = mul2(H, add2(bsq, g)), hm = fma2(g, f2s(-0.5f), emag);
-  const float2 dq = fma2(g, bt2, mul2(hm, hm));
-  const float2 n = add2(h, f2(sqrt_a(dq.x), sqrt_a(dq.y)));
-  const bool   lbig = n.x * r.y >= n.y * r.x;
-  const float  cmax = sqrt_ratio_a(lbig ? n.x : n.y, lbig ? r.x : r.y);
+  // the larger fast magnetosonic speed (find_speed_fast, the normal field a), the
+  // discriminant as (B^2 - gamma p)^2 / 4 + gamma p Bt^2, which does not cancel.
+  // All terms divided by the density first: squares of pressures, or a pressure
+  // times a density, leave FP32's range where the speeds are ordinary
+  const float2 id = f2(rcp_a(r.x), rcp_a(r.y)), g = mul2(mul2(f2s(gamma0), p), id);
+  const float2 h = mul2(H, fma2(bsq, id, g)), hm = sub2(h, g);
+  const float2 dq = fma2(g, mul2(bt2, id), mul2(hm, hm)), n = add2(h, f2(sqrt_a(dq.x), sqrt_a(dq.y)));
+  const float  cmax = sqrt_a(fmaxf(n.x, n.y));
   const float  sl = fminf(u.x, u.y) - cmax;
   const float  sr = fmaxf(u.x, u.y) + cmax;
   const float2 S = f2(sl, sr);
@@ -734,10 +734,13 @@ struct EdgeQ
 // build's (below), with the left and right corners of a row in the lanes of
 // packed pairs (rows LL, RL and LR, RR; a is the same along a row, b along a
 // column).  The discriminant of the fast speed is taken as (B^2 - gamma p)^2 / 4
-// + gamma p Bt^2, which does not cancel.  20 special-function instructions
-// instead of 38, and of the five cases only the one sampled.  Issue bounds the
+// + gamma p Bt^2, which does not cancel.  26 special-function instructions, and of
+// the five cases only the one sampled.  Issue bounds the
 // kernels that call it (62 to 68 % busy): with the HLLD fluxes' algebra above,
-// update kernel at 256^3 2605 -> 2524 us, 2D step at 2048^2 495 -> 483 us.
+// update kernel at 256^3 2605 -> 2524 us, 2D step at 2048^2 495 -> 483 us.  Speeds
+// are formed from quotients by the density (a step at 256^3 3.84 -> 3.85 ms, at
+// 2048^2 503 -> 506 us against squares of pressures and products with densities,
+// which overflow and underflow where speeds do not).
 __device__ __forceinline__ float
 mag_riemann2d_hlld_f32(const EdgeQ<float> & LL, const EdgeQ<float> & RL, const EdgeQ<float> & LR,
                        const EdgeQ<float> & RR, float gamma0, float smallc)
@@ -746,7 +749,7 @@ mag_riemann2d_hlld_f32(const EdgeQ<float> & LL, const EdgeQ<float> & RL, const E
   const float2 b = f2(LL.b, RL.b), bb = mul2(b, b);
   struct Row
   {
-    float2 r, u, v, pt;
+    float2 r, u, v, pt, ir;
   };
   float cx = 0.f, cy = 0.f; // squares of the largest fast speeds along x and y
   auto  row = [&](const EdgeQ<float> & l, const EdgeQ<float> & r, float a2) {
@@ -754,11 +757,12 @@ mag_riemann2d_hlld_f32(const EdgeQ<float> & LL, const EdgeQ<float> & RL, const E
     w.r = f2(l.r, r.r), w.u = f2(l.u, r.u), w.v = f2(l.v, r.v);
     const float2 p = f2(l.p, r.p), c = f2(l.c, r.c), c2 = mul2(c, c);
     const float2 btx = add2(c2, bb), bty = add2(c2, f2s(a2)), b2 = add2(btx, f2s(a2)); // transverse to x, to y; B^2
-    const float2 g = mul2(f2s(gamma0), p), h = mul2(f2s(0.5f), add2(b2, g)), m = fma2(g, f2s(-0.5f), mul2(f2s(0.5f), b2));
-    const float2 mm = mul2(m, m), dx = fma2(g, btx, mm), dy = fma2(g, bty, mm);
-    const float2 ir = f2(rcp_a(w.r.x), rcp_a(w.r.y));
-    const float2 fx = mul2(add2(h, f2(sqrt_a(dx.x), sqrt_a(dx.y))), ir);
-    const float2 fy = mul2(add2(h, f2(sqrt_a(dy.x), sqrt_a(dy.y))), ir);
+    // over the density first, as in mhd_hlld_f32
+    const float2 ir = f2(rcp_a(w.r.x), rcp_a(w.r.y)), g = mul2(mul2(f2s(gamma0), p), ir);
+    w.ir = ir;
+    const float2 h = mul2(f2s(0.5f), fma2(b2, ir, g)), m = sub2(h, g), mm = mul2(m, m), gr = mul2(g, ir);
+    const float2 dx = fma2(gr, btx, mm), dy = fma2(gr, bty, mm);
+    const float2 fx = add2(h, f2(sqrt_a(dx.x), sqrt_a(dx.y))), fy = add2(h, f2(sqrt_a(dy.x), sqrt_a(dy.y)));
     cx = fmaxf(cx, fmaxf(fx.x, fx.y));
     cy = fmaxf(cy, fmaxf(fy.x, fy.y));
     w.pt = fma2(f2s(0.5f), b2, p);
@@ -785,16 +789,24 @@ mag_riemann2d_hlld_f32(const EdgeQ<float> & LL, const EdgeQ<float> & RL, const E
   const float  iB = rcp_a(vs - SB), iT = rcp_a(ST - vs);
   const float2 fxB = mul2(xB, iX), fxT = mul2(xT, iX), fyB = mul2(yB, f2s(iB)), fyT = mul2(yT, f2s(iT));
 
-  // the larger Alfven speed of two corners: sqrt(max(n1 / d1, n2 / d2))
+  // The larger Alfven speed of two corners: sqrt(max(n1 / d1, n2 / d2)), the
+  // quotients compared by products, with n and d over the smallest density: n is a
+  // speed's square, not a field's (a field of 1e-19 is an ordinary foot of a
+  // magnetised region, its square is not among FP32's normal numbers) and d at least
+  // about one.  Where n d is below 1e-36 the speed, under 1e-18, is taken as n 1e18.
+  const float s = fmaxf(fmaxf(B.ir.x, B.ir.y), fmaxf(T.ir.x, T.ir.y));
   auto larger = [smallc](float n1, float d1, float n2, float d2) {
-    const bool first = n1 * d2 >= n2 * d1;
-    return fmaxf(sqrt_ratio_a(first ? n1 : n2, first ? d1 : d2), smallc);
+    const bool  first = n1 * d2 >= n2 * d1;
+    const float n = first ? n1 : n2, d = first ? d1 : d2;
+    return fmaxf(n * rsqrt_a(fmaxf(n * d, 1e-36f)), smallc);
   };
-  const float2 dxB = mul2(wB, iX), dxT = mul2(wT, iX), dyB = mul2(zB, f2s(iB)), dyT = mul2(zT, f2s(iT));
-  const float  cL = larger(a12 * fmaxf(fyT.x, 1.f), dxT.x, a02 * fmaxf(fyB.x, 1.f), dxB.x);
-  const float  cR = larger(a12 * fmaxf(fyT.y, 1.f), dxT.y, a02 * fmaxf(fyB.y, 1.f), dxB.y);
-  const float  cB = larger(bb.x * fmaxf(fxB.x, 1.f), dyB.x, bb.y * fmaxf(fxB.y, 1.f), dyB.y);
-  const float  cT = larger(bb.x * fmaxf(fxT.x, 1.f), dyT.x, bb.y * fmaxf(fxT.y, 1.f), dyT.y);
+  const float2 sX = mul2(iX, f2s(s)), bs = mul2(mul2(b, f2s(s)), b);
+  const float  sB = iB * s, sT = iT * s, as0 = a0 * s * a0, as1 = a1 * s * a1;
+  const float2 dxB = mul2(wB, sX), dxT = mul2(wT, sX), dyB = mul2(zB, f2s(sB)), dyT = mul2(zT, f2s(sT));
+  const float  cL = larger(as1 * fmaxf(fyT.x, 1.f), dxT.x, as0 * fmaxf(fyB.x, 1.f), dxB.x);
+  const float  cR = larger(as1 * fmaxf(fyT.y, 1.f), dxT.y, as0 * fmaxf(fyB.y, 1.f), dxB.y);
+  const float  cB = larger(bs.x * fmaxf(fxB.x, 1.f), dyB.x, bs.y * fmaxf(fxB.y, 1.f), dyB.y);
+  const float  cT = larger(bs.x * fmaxf(fxT.x, 1.f), dyT.x, bs.y * fmaxf(fxT.y, 1.f), dyT.y);
   const float  SAL = fminf(us - cL, 0.f), SAR = fmaxf(us + cR, 0.f);
   const float  SAB = fminf(vs - cB, 0.f), SAT = fmaxf(vs + cT, 0.f);
 
