@@ -18,34 +18,12 @@
 #pragma once
 
 #include "ek_hydro_kernels.cuh"
+#include "ek_slabs.h"
 
 namespace EK_NS
 {
 
-// One slab: the interior cells [j0, j0 + ny) in 2D, [k0, k0 + nz) in 3D, and
-// its part of the workspace.  Arrays are [..][variable][cells of the box], x
-// fastest; a box is the slab's cells with 2 (q), 1 (s) or 0 (f, one more on the
-// high side) layers around.
-template <int NV>
-struct HydroSlab
-{
-  static constexpr int DIM = NV == 4 ? 2 : 3;
-  int       nx, ny, nz, j0, k0;
-  int       last; // the step's last slab
-  double *  q;    // primitives
-  double *  s;    // face states [axis][low, high]
-  double *  f;    // fluxes through the low faces [axis]
-  __host__ __device__ long long
-  box(int w) const // cells of a box with w more cells per axis
-  {
-    return (long long)(nx + w) * (ny + w) * (DIM == 3 ? nz + w : 1);
-  }
-  __host__ __device__ long long
-  bytes() const
-  {
-    return (long long)sizeof(double) * NV * (box(4) + 2 * DIM * box(2) + DIM * box(1));
-  }
-};
+using ekc::HydroSlab;
 constexpr int kPassThreads = 128;
 
 __device__ __forceinline__ long long

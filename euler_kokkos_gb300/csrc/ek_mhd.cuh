@@ -6,6 +6,7 @@
 #include <type_traits>
 
 #include "ek_common.cuh"
+#include "ek_slabs.h"
 
 namespace EK_NS
 {
@@ -1179,19 +1180,19 @@ t_bfslope(int f, int right, int e)
 
 // Accessors of a cell's trace fields: A(f) is field f.
 // StrideAcc: field-major storage with stride st (the staged shared-memory
-// planes).  QuadAcc: the HBM trace, 16-byte quads of fields per cell (see
+// planes, the slabs of the FP64 passes).  QuadAcc: the HBM trace, 16-byte quads of fields per cell (see
 // trace_cell); the gathers below read compile-time field indices, so only the
 // quads a face or edge state needs are loaded (the others are never used and
 // their loads are removed), one vector load per quad.
-template <class R>
+template <class R, class I>
 struct StrideAcc
 {
   const R * t;
-  int       st;
+  I         st;
   __device__ __forceinline__ R
   operator()(int f) const
   {
-    return t[f * st];
+    return t[ekc::field_offset(f, st)];
   }
 };
 constexpr int kTraceLanes = 32; // cells per block of the HBM trace
@@ -1253,11 +1254,11 @@ face_state_acc(const ACC & T, int d, R (&q)[8], R smallr, R smallp)
   q[IC] = tb(d == 2 ? 0 : 2);
   floor_state(q, smallr, smallp);
 }
-template <class R, bool PLUS>
+template <class R, bool PLUS, class I>
 __device__ __forceinline__ void
-face_state_dir(const R * t, int st, int d, R (&q)[8], R smallr, R smallp)
+face_state_dir(const R * t, I st, int d, R (&q)[8], R smallr, R smallp)
 {
-  face_state_acc<R, PLUS>(StrideAcc<R>{ t, st }, d, q, smallr, smallp);
+  face_state_acc<R, PLUS>(StrideAcc<R, I>{ t, st }, d, q, smallr, smallp);
 }
 
 // One corner of an edge along d (MHDBaseFunctor3D.h:957-1113).  The
@@ -1290,11 +1291,11 @@ edge_corner_acc(const ACC & T, int d, int p1, int p2, R smallr, R smallp)
   e.c = T(T_A + d) + (sg1(T(t_bslope(p1, d))) + sg2(T(t_bslope(p2, d))));
   return e;
 }
-template <class R, int S1, int S2>
+template <class R, int S1, int S2, class I>
 __device__ __forceinline__ EdgeCorner<R>
-edge_corner(const R * t, int st, int d, int p1, int p2, R smallr, R smallp)
+edge_corner(const R * t, I st, int d, int p1, int p2, R smallr, R smallp)
 {
-  return edge_corner_acc<R, S1, S2>(StrideAcc<R>{ t, st }, d, p1, p2, smallr, smallp);
+  return edge_corner_acc<R, S1, S2>(StrideAcc<R, I>{ t, st }, d, p1, p2, smallr, smallp);
 }
 
 } // namespace EK_NS

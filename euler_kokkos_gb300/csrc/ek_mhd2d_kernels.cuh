@@ -54,13 +54,14 @@ floor2d(R & r, R & p, R smallr, R smallp)
 // right face (qm), otherwise the right state of its left face (qp); y states
 // come in the face frame (IU<->IV and IA<->IB swapped) as the flux functor
 // hands them to the Riemann solver (MHDRunFunctors2D.h:418-466).
-template <class R, bool PLUS>
+template <class R, bool PLUS, class I>
 __device__ __forceinline__ void
-face2d_state(const R * t, int st, int d, R (&q)[8], R smallr, R smallp)
+face2d_state(const R * t, I st, int d, R (&q)[8], R smallr, R smallp)
 {
-  const int ds = V_DRX + 7 * d;
-  auto      h = [&](int f) {
-    const R c = t[f * st], s = t[(ds + f) * st];
+  const int             ds = V_DRX + 7 * d;
+  const StrideAcc<R, I> T{ t, st };
+  auto                  h = [&](int f) {
+    const R c = T(f), s = T(ds + f);
     return PLUS ? c + s : c - s;
   };
   q[ID] = h(V_R);
@@ -68,14 +69,14 @@ face2d_state(const R * t, int st, int d, R (&q)[8], R smallr, R smallp)
   q[IU] = h(V_U + d);
   q[IV] = h(d == 1 ? V_U : V_V);
   q[IW] = h(V_W);
-  q[IA] = t[(d == 0 ? (PLUS ? V_AR : V_AL) : (PLUS ? V_BR : V_BL)) * st];
+  q[IA] = T(d == 0 ? (PLUS ? V_AR : V_AL) : (PLUS ? V_BR : V_BL));
   {
     // transverse in-plane field: B +- dBx (x faces), A +- dAy (y faces)
-    const R c = t[(d == 0 ? V_B : V_A) * st], s = t[(ds + 6) * st];
+    const R c = T(d == 0 ? V_B : V_A), s = T(ds + 6);
     q[IB] = PLUS ? c + s : c - s;
   }
   {
-    const R c = t[V_C * st], s = t[(ds + 5) * st];
+    const R c = T(V_C), s = T(ds + 5);
     q[IC] = PLUS ? c + s : c - s;
   }
   floor2d(q[ID], q[IP], smallr, smallp);
@@ -84,22 +85,23 @@ face2d_state(const R * t, int st, int d, R (&q)[8], R smallr, R smallp)
 // Edge state of a cell at its corner (S1 along x, S2 along y: +1 right/top,
 // -1 left/bottom) with the components compute_emf<EMFZ> reads
 // (MHDBaseFunctor2D.h:1061-1113).
-template <class R, int S1, int S2>
+template <class R, int S1, int S2, class I>
 __device__ __forceinline__ EdgeCorner<R>
-edge2d_corner(const R * t, int st, R smallr, R smallp)
+edge2d_corner(const R * t, I st, R smallr, R smallp)
 {
   auto sg1 = [](R x) { return S1 > 0 ? x : -x; };
   auto sg2 = [](R x) { return S2 > 0 ? x : -x; };
-  auto hyd = [&](int f) { return t[f * st] + (sg1(t[(V_DRX + f) * st]) + sg2(t[(V_DRY + f) * st])); };
+  const StrideAcc<R, I> T{ t, st };
+  auto hyd = [&](int f) { return T(f) + (sg1(T(V_DRX + f)) + sg2(T(V_DRY + f))); };
   EdgeCorner<R> e;
   e.r = hyd(V_R);
   e.p = hyd(V_P);
   floor2d(e.r, e.p, smallr, smallp);
   e.u = hyd(V_U);
   e.v = hyd(V_V);
-  e.a = t[(S1 > 0 ? V_AR : V_AL) * st] + sg2(t[(S1 > 0 ? V_DARY : V_DALY) * st]);
-  e.b = t[(S2 > 0 ? V_BR : V_BL) * st] + sg1(t[(S2 > 0 ? V_DBRX : V_DBLX) * st]);
-  e.c = t[V_C * st] + (sg1(t[V_DCX * st]) + sg2(t[V_DCY * st]));
+  e.a = T(S1 > 0 ? V_AR : V_AL) + sg2(T(S1 > 0 ? V_DARY : V_DALY));
+  e.b = T(S2 > 0 ? V_BR : V_BL) + sg1(T(S2 > 0 ? V_DBRX : V_DBLX));
+  e.c = T(V_C) + (sg1(T(V_DCX)) + sg2(T(V_DCY)));
   return e;
 }
 

@@ -19,44 +19,8 @@
 namespace EK_NS
 {
 
-// The whole grid's arrays, indexed as the state is ([variable][k][j][i] with
-// ghosts), and one slab: interior cells [j0, j0 + ny) in 2D, [k0, k0 + nz) in 3D.
-template <int DIM>
-struct MhdSlab
-{
-  static constexpr int NE = DIM == 3 ? 3 : 1;       // edge fields (2D: z only, the last)
-  static constexpr int NT = DIM == 3 ? (int)T_N : (int)V_N;   // trace fields
-  static constexpr int NF = DIM == 3 ? 5 : 6;       // flux components
-  int       nx, ny, nz, j0, k0;
-  int       last;
-  double *  q;  // [8] primitives
-  double *  b;  // [3] face fields
-  double *  e;  // [NE] edge fields
-  double *  t;  // [NT] trace of the box with one more cell on every side
-  double *  f;  // [DIM][NF] fluxes through the low faces, box with one more on the high side
-  double *  em; // [NE] emfs of the low edges, the same box
-  __host__ __device__ long long
-  box(int w) const
-  {
-    return (long long)(nx + w) * (ny + w) * (DIM == 3 ? nz + w : 1);
-  }
-  __host__ __device__ long long
-  slab_bytes() const
-  {
-    return (long long)sizeof(double) * (NT * box(2) + (DIM * NF + NE) * box(1));
-  }
-  // of the slab's boxes: trace cell and low face / edge of cell (i, j, k)
-  __host__ __device__ long long
-  tcell(int i, int j, int k) const
-  {
-    return ((DIM == 3 ? k + 1 : 0) * (long long)(ny + 2) + (j + 1)) * (nx + 2) + (i + 1);
-  }
-  __host__ __device__ long long
-  face(int i, int j, int k) const
-  {
-    return ((DIM == 3 ? k : 0) * (long long)(ny + 1) + j) * (nx + 1) + i;
-  }
-};
+using ekc::MhdSlab;
+static_assert(MhdSlab<3>::NT == T_N && MhdSlab<2>::NT == V_N, "trace fields");
 
 template <int DIM>
 __global__ void __launch_bounds__(kPassThreads)
@@ -268,7 +232,7 @@ mhd_flux_pass(const KParams P, const DevClock * clk, int step, MhdSlab<DIM> S)
   box_coords((unsigned)c, ex, ey, i, j, k);
   const MhdConst<double> C = mhd_const<double>(P);
   const double           sr = C.smallr, sp = C.smallp;
-  const int              st = (int)S.box(2); // trace field stride
+  const long long        st = S.trace_stride(); // 64 bits: 46 st passes 2^31 on planes of 4000 x 4000
   const long long        nf = S.box(1), out = S.face(i, j, k);
   const double *         t = S.t + S.tcell(i, j, k);
   const int              back[3] = { 1, S.nx + 2, (S.nx + 2) * (S.ny + 2) };
