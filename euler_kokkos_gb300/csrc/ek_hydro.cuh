@@ -426,8 +426,10 @@ hllc64(const double (&ql)[NV], const double (&qr)[NV], double (&flux)[NV], const
   const double w = fma(-rcr, du, pl - pr) * rcp64(rcr + rcl);
   const double us = ul + w, ps = fma(-rcl, w, pl);
 
-  // the star state on the side of the contact (left when u* > 0)
-  const bool   left = positive64(us);
+  // the star state on the side of the contact (left when u* > 0), or the left
+  // state's own side when its wave is the one sampled: without a sound speed the
+  // star state of an expansion is 0 / 0
+  const bool   left = positive64(us) || positive64(SL);
   const double Sk = left ? SL : SR, uk = left ? ul : ur, ek = left ? el : er, pk = left ? pl : pr;
   const double is = rcp64(Sk - us);
   const double rs = (left ? flip64(rcl, true) : rcr) * is;
