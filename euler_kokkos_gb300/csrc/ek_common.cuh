@@ -495,12 +495,14 @@ scale_pos64(double x)
   return __hiloint2double(tiny ? 0 : hi - (K << 20), tiny ? 0 : __double2loint(x));
 }
 // max(p, d floor) for d > 0: the product only where the high words say that
-// p / d may be below 2 floor
+// p / d may be below 2 floor.  They are logarithms of positive normal p alone: a
+// negative p, below any floor (also one of zero), takes the product always, and
+// zero, a subnormal and infinity do.
 __device__ __forceinline__ double
 floor_ratio64(double p, double d, double floor)
 {
-  // a negative p counts as zero (the difference must not wrap)
-  if (max(hi32(p), 0) - hi32(d) < hi32(floor) - 0x3ff00000 + 0x00100000)
+  const int hp = hi32(p);
+  if ((unsigned)(hp - 0x00100000) >= 0x7fe00000u || hp - hi32(d) < hi32(floor) - 0x3ff00000 + 0x00100000)
     p = max_floor64(p, d * floor);
   return p;
 }
