@@ -440,12 +440,14 @@ negative64(double x) // the sign bit
 {
   return hi32(x) < 0;
 }
-// the larger of x (any sign) and f >= 0; the smaller of two non-negative
-// values: the integer order of the bit patterns is the numbers' order
+// the larger of x (any sign) and f >= 0, f where x is a NaN of either sign (as fmax);
+// the smaller of two non-negative values: the integer order of the bit patterns is
+// the numbers' order.  x stays where its bits lie between those of f and infinity.
 __device__ __forceinline__ double
 max_floor64(double x, double f)
 {
-  return __longlong_as_double(max(__double_as_longlong(x), __double_as_longlong(f)));
+  const unsigned long long b = (unsigned long long)__double_as_longlong(f);
+  return (unsigned long long)__double_as_longlong(x) - b <= 0x7ff0000000000000ull - b ? x : f;
 }
 __device__ __forceinline__ double
 min_pos64(double a, double b)
@@ -497,7 +499,7 @@ scale_pos64(double x)
 // max(p, d floor) for d > 0: the product only where the high words say that
 // p / d may be below 2 floor.  They are logarithms of positive normal p alone: a
 // negative p, below any floor (also one of zero), takes the product always, and
-// zero, a subnormal and infinity do.
+// zero, a subnormal, infinity and NaN do.
 __device__ __forceinline__ double
 floor_ratio64(double p, double d, double floor)
 {

@@ -6,7 +6,7 @@
 #include "ek_hydro.cuh"
 using namespace ek_fast;
 
-__device__ unsigned g_bad[1];
+__device__ unsigned g_bad[2];
 
 __device__ void
 same(int k, double x, double y)
@@ -42,13 +42,30 @@ floors()
     }
 }
 
+__global__ void
+nans()
+{
+  const double v[] = { 0.0, 5e-324, 1e-300, 1e-20, 1e-10, 0.3, 1.0, 7.0, 1e200 };
+  for (double f : v)
+    for (long long bits : { 0x7ff8000000000000ll, 0x7ff0000000000001ll, 0x7fffffffffffffffll })
+      for (long long sign : { 0ll, (long long)0x8000000000000000ull })
+      {
+        const double x = __longlong_as_double(bits | sign);
+        same(1, max_floor64(x, f), f);
+        same(1, floor_ratio64(x, 0.3, f), 0.3 * f);
+        same(1, floor_ratio64(x, 1e10, f), 1e10 * f);
+        same(1, max_cand64(f, x), f);
+      }
+}
+
 int
 main()
 {
   floors<<<1, 1>>>();
-  unsigned h[1];
+  nans<<<1, 1>>>();
+  unsigned h[2];
   if (cudaMemcpyFromSymbol(h, g_bad, sizeof h) != cudaSuccess)
     return 1;
-  printf("floors %u\n", h[0]);
+  printf("floors %u\nnan %u\n", h[0], h[1]);
   return 0;
 }

@@ -1,4 +1,5 @@
-"""Floors of the FP64 FMA build: a negative pressure with smallc = 0.  The exact build (the reference's fmax) is
+"""Floors of the FP64 FMA build: a density or energy that is not a number, a
+negative pressure with smallc = 0.  The exact build (the reference's fmax) is
 the result to agree with."""
 
 import os
@@ -47,7 +48,23 @@ def limits(tmp_path_factory):
 
 
 def test_floor_helpers(limits):
-    assert limits["floors"] == 0  # values of fmax
+    assert limits["floors"] == 0 and limits["nan"] == 0  # values of fmax
+
+
+@pytest.mark.parametrize("var", [0, 1], ids=["density", "energy"])
+@pytest.mark.parametrize("sign", [1.0, -1.0])
+@pytest.mark.parametrize("dim,mhd,n", GRIDS, ids=IDS)
+def test_nan_is_floored(dim, mhd, n, var, sign):
+    gw = 3 if mhd else 2
+    ini, U0, at = _state(dim, mhd, n, gw)
+    U0[(slice(2, 5 if U0.shape[0] > 4 else 4),) + at] = 0.0  # a density of smallr with a momentum would be a jet
+    U0[(var,) + at] = np.copysign(np.nan, sign)
+    (Ue, de), (Uf, df) = _both(ini, U0, gw, dim, 2)
+    assert np.array_equal(np.isnan(Ue), np.isnan(Uf))
+    assert np.isnan(Ue).sum() == 1  # the cell itself: its neighbours see the floor
+    ok = ~np.isnan(Ue)
+    assert np.max(rel_linf(np.where(ok, Uf, 0.0), np.where(ok, Ue, 0.0))[[0, 1]]) <= 1e-11
+    assert np.max(np.abs(df / de - 1)) <= 1e-13
 
 
 @pytest.mark.parametrize("dim,mhd,n", GRIDS, ids=IDS)
