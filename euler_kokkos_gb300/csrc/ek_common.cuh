@@ -423,12 +423,37 @@ sqrt64(double x)
   const double q = fma(g * r, fma(r, 0.375, 0.5), g);
   return seed_special(y) ? ((hi32(y) & 0x000fffff) != 0 ? y : x) : q;
 }
-// sqrt(n / d) for n >= 0, d > 0; 0 where n d is below 2^-1021
+// x not in [2^-1021, 2^1022): the results above may be rounded, 0 or infinite
+__device__ __forceinline__ bool
+out_of_range64(double x)
+{
+  return (unsigned)(hi32(x) - 0x00200000) >= 0x7fc00000u;
+}
+__device__ __forceinline__ bool
+both_zero64(double a, double b) // a, b >= 0
+{
+  return (__double_as_longlong(a) | __double_as_longlong(b)) == 0;
+}
+// sqrt(n / d) for n >= 0, d > 0; by the quotient where n d leaves the range (a
+// branch on integer comparisons that ordinary states do not take)
 __device__ __forceinline__ double
 sqrt_ratio64(double n, double d)
 {
-  const double x = n * d, c = n * rsqrt64(x);
-  return (unsigned)hi32(x) < 0x00200000u ? 0.0 : c;
+  const double x = n * d;
+  double       c = n * rsqrt64(x);
+  if (out_of_range64(x))
+    c = both_zero64(n, n) ? 0.0 : sqrt64(n * rcp64(d));
+  return c;
+}
+// the larger of sqrt(n1 / d1) and sqrt(n2 / d2), the quotients compared by products
+__device__ __forceinline__ double
+sqrt_larger_ratio64(double n1, double d1, double n2, double d2)
+{
+  const long long p1 = __double_as_longlong(n1 * d2), p2 = __double_as_longlong(n2 * d1);
+  const bool      first = p1 >= p2;
+  if (out_of_range64(__longlong_as_double(first ? p1 : p2)))
+    return both_zero64(n1, n2) ? 0.0 : sqrt64(fmax(n1 * rcp64(d1), n2 * rcp64(d2)));
+  return sqrt_ratio64(first ? n1 : n2, first ? d1 : d2);
 }
 __device__ __forceinline__ bool
 positive64(double x) // x > 0

@@ -415,8 +415,7 @@ hllc64(const double (&ql)[NV], const double (&qr)[NV], double (&flux)[NV], const
   }
   const double el = fma(pl, C.entho, scale_pos64<1>(rl) * kl), er = fma(pr, C.entho, scale_pos64<1>(rr) * kr);
 
-  const bool   lbig = __double_as_longlong(pl * rr) >= __double_as_longlong(pr * rl);
-  const double cmax = max_floor64(sqrt_ratio64(C.gamma0 * (lbig ? pl : pr), lbig ? rl : rr), C.smallc);
+  const double cmax = max_floor64(sqrt_larger_ratio64(C.gamma0 * pl, rl, C.gamma0 * pr, rr), C.smallc);
 
   const double du = ul - ur;
   const bool   lslow = negative64(du); // ul < ur

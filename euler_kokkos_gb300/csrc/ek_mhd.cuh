@@ -27,7 +27,15 @@ __device__ __forceinline__ double
 fast_num64(double gp, double b2, double bn2)
 {
   const double s = scale_pos64<1>(b2 + gp);
-  return s + sqrt64(max_floor64(fma(s, s, -(gp * bn2)), 0.0));
+  double       n = s + sqrt64(max_floor64(fma(s, s, -(gp * bn2)), 0.0));
+  if ((unsigned)(hi32(s) - 0x20b00000) >= 0x3e800000u)
+  {
+    // beyond 2^-500 to 2^500, where the squares leave the range: scaled by 2^600 or 2^-600
+    const bool   small = hi32(s) < 0x3ff00000;
+    const double f = small ? 0x1p600 : 0x1p-600, t = s * f;
+    n = (t + sqrt64(max_floor64(fma(t, t, -((gp * f) * (bn2 * f))), 0.0))) * (small ? 0x1p-600 : 0x1p600);
+  }
+  return n;
 }
 
 // find_speed_fast<dir> (mhd_utils.h:89-117)
@@ -334,8 +342,7 @@ mhd_hlld64(const double (&ql)[8], const double (&qr)[8], double (&flux)[NF], dou
   };
   const Side   L = side(ql), R = side(qr);
   const double ul = ql[IU], ur = qr[IU];
-  const bool   lbig = __double_as_longlong(L.n * qr[ID]) >= __double_as_longlong(R.n * ql[ID]);
-  const double cmax = sqrt_ratio64(lbig ? L.n : R.n, lbig ? ql[ID] : qr[ID]);
+  const double cmax = sqrt_larger_ratio64(L.n, ql[ID], R.n, qr[ID]);
   const double du = ul - ur;
   const bool   lslow = negative64(du);
   const double sl = (lslow ? ul : ur) - cmax, sr = (lslow ? ur : ul) + cmax;
@@ -892,8 +899,7 @@ mag_riemann2d_hlld64(const EdgeQ<double> & LL, const EdgeQ<double> & RL, const E
   auto alfven = [&](double n1, double m1, double d1, double n2, double m2, double d2) {
     n1 *= max_floor64(m1, 1.0);
     n2 *= max_floor64(m2, 1.0);
-    const bool first = __double_as_longlong(n1 * d2) >= __double_as_longlong(n2 * d1);
-    return max_floor64(sqrt_ratio64(first ? n1 : n2, first ? d1 : d2), smallc);
+    return max_floor64(sqrt_larger_ratio64(n1, d1, n2, d2), smallc);
   };
   const double cL = alfven(a12, fyLR, LR.r * fxLR, a02, fyLL, LL.r * fxLL);
   const double cR = alfven(a12, fyRR, RR.r * fxRR, a02, fyRL, RL.r * fxRL);

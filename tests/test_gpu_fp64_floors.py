@@ -51,6 +51,29 @@ def test_floor_helpers(limits):
     assert limits["floors"] == 0 and limits["nan"] == 0  # values of fmax
 
 
+def test_roots_of_quotients(limits):
+    # as test_gpu_fp64_math.py's ratio, whose bound holds where n d leaves the range too (reciprocal 1.05 and product 0.5,
+    # halved by the root, and the root 1.55); the fast speed: two roots of at most 1.55, sums and the difference, of which
+    # the discriminant is no less than 0.3 of its first term
+    assert limits["ratio"] <= 4.1 and limits["larger"] <= 4.1 and limits["fast"] <= 8
+
+
+# scales beyond the roots of the number range: LLF takes no products of two densities
+@pytest.mark.parametrize("dim,mhd,n", GRIDS, ids=IDS)
+@pytest.mark.parametrize("power", [-512, 520])
+def test_densities_beyond_the_root_of_the_range(dim, mhd, n, power):
+    gw = 3 if mhd else 2
+    ini, U0, _ = _state(dim, mhd, n, gw)
+    ini = ini.replace("riemann=hlld", "riemann=llf").replace("riemann=hllc", "riemann=llf")
+    ini = ini.replace("[hydro]", "[hydro]\nsmallr=0.0")
+    U0 = U0 * 2.0 ** power
+    U0[5:] *= 2.0 ** (-power // 2)
+    (Ue, de), (Uf, df) = _both(ini, U0, gw, dim, 1)
+    assert np.isfinite(Ue).all() and np.isfinite(Uf).all()
+    assert np.max(np.abs(df / de - 1)) <= 1e-13
+    assert np.max(rel_linf(Uf, Ue)[[0, 1]]) <= 1e-11
+
+
 @pytest.mark.parametrize("var", [0, 1], ids=["density", "energy"])
 @pytest.mark.parametrize("sign", [1.0, -1.0])
 @pytest.mark.parametrize("dim,mhd,n", GRIDS, ids=IDS)
