@@ -1372,6 +1372,8 @@ ek_ensemble_create(const ek_params * params, int n, ek_ensemble ** out)
   if (err == cudaSuccess)
     err = cudaMalloc((void **)&e->clocks, sizeof(DevClock) * n);
   if (err == cudaSuccess)
+    err = cudaMemsetAsync(e->clocks, 0, sizeof(DevClock) * n, e->stream); // totals before a state is set
+  if (err == cudaSuccess)
     err = cudaMalloc((void **)&e->dtlogs, sizeof(double) * (size_t)dtcap * n);
   if (err == cudaSuccess)
     err = cudaMalloc((void **)&e->d_insts, sizeof(ekc::EnsInstance) * n);
@@ -1563,7 +1565,7 @@ ek_ensemble_totals(ek_ensemble * e, double * out)
 {
   if (!e || !out)
     return fail(EK_ERR_INVALID, "ek_ensemble_totals: bad argument");
-  EK_CUDA(ek_fast::ensemble_totals(e->prec, e->d_insts, e->n, e->step, e->d_totals, e->stream), "totals");
+  EK_CUDA(ek_fast::ensemble_totals(e->prec, e->d_insts, e->n, e->d_totals, e->stream), "totals");
   EK_CUDA(cudaMemcpyAsync(out, e->d_totals, 2 * sizeof(double) * e->n, cudaMemcpyDeviceToHost, e->stream),
           "totals");
   EK_CUDA(cudaStreamSynchronize(e->stream), "totals");

@@ -292,14 +292,15 @@ ensemble2d_step(const EnsInstance * __restrict__ insts, const EnsTile * __restri
   finalize_step(clk, in.P, step + 1, nullptr, in.tiles);
 }
 
-// FP64 mass and total energy of every instance (blockIdx.y = instance)
+// FP64 mass and total energy of every instance (blockIdx.y = instance), from the
+// buffer of its own last step: an instance at its end time stays in it
 template <class S>
 __global__ void
-ensemble_totals_kernel(const EnsInstance * __restrict__ insts, int step, double * __restrict__ out)
+ensemble_totals_kernel(const EnsInstance * __restrict__ insts, double * __restrict__ out)
 {
   const EnsInstance & in = insts[blockIdx.y];
   const KParams &     P = in.P;
-  const S *           U = (const S *)in.U[step % 2];
+  const S *           U = (const S *)in.U[in.clk->iteration % 2];
   double              m = 0.0, e = 0.0;
   for_interior_rows(P, [&](int i, int j, int) {
     const long long off = (long long)j * P.isize + i;

@@ -411,17 +411,16 @@ convert_stage(bool to_state, int prec, int layout, double * stage, void * U, con
 }
 
 cudaError_t
-ensemble_totals(int prec, const EnsInstance * insts, int n, int step, double * out,
-                cudaStream_t st)
+ensemble_totals(int prec, const EnsInstance * insts, int n, double * out, cudaStream_t st)
 {
   cudaError_t e = cudaMemsetAsync(out, 0, 2 * sizeof(double) * n, st);
   if (e != cudaSuccess)
     return e;
   dim3 grid(16, n);
   if (prec == 0)
-    ensemble_totals_kernel<double><<<grid, 256, 0, st>>>(insts, step, out);
+    ensemble_totals_kernel<double><<<grid, 256, 0, st>>>(insts, out);
   else
-    ensemble_totals_kernel<float><<<grid, 256, 0, st>>>(insts, step, out);
+    ensemble_totals_kernel<float><<<grid, 256, 0, st>>>(insts, out);
   return cudaGetLastError();
 }
 

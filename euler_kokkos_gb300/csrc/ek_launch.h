@@ -59,8 +59,8 @@ using ekc::KParams;
 cudaError_t fill_ghosts(int prec, void * U, const KParams & P, int nbvar, cudaStream_t st);
 cudaError_t totals(int prec, const void * U, const KParams & P, int nbvar, double * out3,
                    cudaStream_t st);
-cudaError_t ensemble_totals(int prec, const ekc::EnsInstance * insts, int n, int step,
-                            double * out, cudaStream_t st);
+cudaError_t ensemble_totals(int prec, const ekc::EnsInstance * insts, int n, double * out,
+                            cudaStream_t st);
 // Host FP64 arrays <-> device state.  Elements [first, first + count) of a
 // host array in the caller's layout (0 LayoutLeft, 1 LayoutRight; nbvar
 // variables) sit in the device staging buffer stage; to_state: convert them
