@@ -440,9 +440,11 @@ ek_solver_create(const ek_params * params, ek_solver ** out)
   if (e == cudaSuccess)
     e = cudaMalloc((void **)&s->scratch3, 3 * sizeof(double));
   // FP64: the step in passes with a bounded workspace, where the grid is not too
-  // small for it (pass_bytes 0); if the workspace does not fit beside the states,
-  // the tile kernels, which need none
-  if (e == cudaSuccess && s->prec == EK_PREC_FP64)
+  // small for it (pass_bytes 0) and no planes per CTA of the 3D tile kernels are
+  // given; if the workspace does not fit beside the states, the tile kernels,
+  // which need none
+  const bool tiles = p.dim == 3 && p.kchunk > 0;
+  if (e == cudaSuccess && s->prec == EK_PREC_FP64 && !tiles)
   {
     s->work_bytes = ek_fast::pass_bytes(p.dim, p.mhd, k);
     if (s->work_bytes)
