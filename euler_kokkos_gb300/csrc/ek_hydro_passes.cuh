@@ -276,8 +276,8 @@ hydro_update_pass(const double * __restrict__ Uin, double * __restrict__ Uout, c
   finalize_step(clk, P, step + 1); // the next step's dt, once its CFL key is complete
 }
 
-// Cells of the last axis per slab: the workspace of a slab stays under
-// kPassBytes (2.6 million 3D cells), the slabs about equal.
+// Workspace of a slab (slab_cells): 2.6 million hydro 3D cells.  A single plane
+// may take more, from 1024 x 1024 (1.3 GB) on.
 constexpr long long kPassBytes = 1ll << 30;
 template <int NV>
 inline HydroSlab<NV>
@@ -299,11 +299,7 @@ template <int NV>
 inline int
 hydro_slab_cells(const KParams & P)
 {
-  const int N = NV == 4 ? P.ny : P.nz;
-  int       n = N;
-  while (n > 1 && hydro_slab<NV>(P, 0, n, nullptr).bytes() > kPassBytes)
-    n = (n + 1) / 2;
-  return n;
+  return ekc::slab_cells(NV == 4 ? P.ny : P.nz, kPassBytes, [&](int n) { return hydro_slab<NV>(P, 0, n, nullptr).bytes(); });
 }
 
 template <int NV, int RS, bool GRAV>

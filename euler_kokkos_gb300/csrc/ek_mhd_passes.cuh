@@ -372,10 +372,7 @@ template <int DIM>
 inline int
 mhd_slab_cells(const KParams & P)
 {
-  int n = DIM == 2 ? P.ny : P.nz;
-  while (n > 1 && mhd_slab<DIM>(P, 0, n, nullptr).slab_bytes() > kPassBytes)
-    n = (n + 1) / 2;
-  return n;
+  return ekc::slab_cells(DIM == 2 ? P.ny : P.nz, kPassBytes, [&](int n) { return mhd_slab<DIM>(P, 0, n, nullptr).slab_bytes(); });
 }
 template <int DIM>
 inline size_t

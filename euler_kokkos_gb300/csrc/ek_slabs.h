@@ -92,4 +92,16 @@ struct MhdSlab
   }
 };
 
+// Cells of the last axis, N in all, per slab: the fewest slabs whose workspace,
+// bytes(cells), is at most `limit` (one cell's may be more), about equal
+template <class Bytes>
+inline int
+slab_cells(int N, long long limit, Bytes bytes)
+{
+  int n = N;
+  for (int slabs = 2; n > 1 && bytes(n) > limit; ++slabs)
+    n = (int)(((long long)N + slabs - 1) / slabs);
+  return n;
+}
+
 } // namespace ekc

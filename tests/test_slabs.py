@@ -59,3 +59,32 @@ def offsets(tmp_path_factory):
 def test_trace_offsets_of_large_planes(offsets, dim, nx, ny, n):
     assert subprocess.run([offsets, str(dim), str(nx), str(ny), str(n)], check=True, capture_output=True,
                           text=True).stdout.strip() == "0"
+
+
+LENGTHS = r"""
+#include "ek_slabs.h"
+#include <cstdio>
+#include <cstdlib>
+int main(int, char ** a)
+{
+  const int       N = atoi(a[1]);
+  const long long limit = atoll(a[2]), cell = atoll(a[3]), fixed = atoll(a[4]);
+  std::printf("%d\n", ekc::slab_cells(N, limit, [&](int n) { return fixed + cell * n; }));
+}
+"""
+
+
+@pytest.fixture(scope="module")
+def lengths(tmp_path_factory):
+    return _compile(tmp_path_factory.mktemp("lengths"), LENGTHS)
+
+
+@pytest.mark.parametrize("N,limit,cell,fixed", [(1, 10, 1, 0), (10, 100, 1, 0), (9, 4, 1, 0), (10, 4, 1, 0), (10, 8, 2, 1),
+                                                (16, 10, 1, 0), (17, 16, 1, 0), (512, 1 << 30, 110 << 20, 200 << 20),
+                                                (7, 3, 5, 0), (100_000, 1000, 7, 3), (2_000_000_000, 1 << 40, 100, 0)])
+def test_slab_lengths(lengths, N, limit, cell, fixed):
+    n = int(subprocess.run([lengths, str(N), str(limit), str(cell), str(fixed)], check=True, capture_output=True,
+                           text=True).stdout)
+    most = max(1, min(N, (limit - fixed) // cell))  # cells that fit
+    assert 1 <= n <= most
+    assert n == -(-N // -(-N // most))  # the fewest slabs, equal but for the rounding
