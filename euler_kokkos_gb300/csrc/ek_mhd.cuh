@@ -23,19 +23,22 @@ struct MhdConst
 // root, which is one sqrt_ratio64 for the largest of several speeds.  The
 // discriminant, (B^2 - gamma p)^2 / 4 + gamma p Bt^2 by its parts, is not
 // negative.
+// beyond 2^-500 to 2^500, where the squares leave the range: scaled by 2^600 or
+// 2^-600 (out of line, so that the callers' registers are not its)
+__device__ __noinline__ double
+fast_num64_scaled(double s, double gp, double bn2)
+{
+  const bool   small = hi32(s) < 0x3ff00000;
+  const double f = small ? 0x1p600 : 0x1p-600, t = s * f;
+  return (t + sqrt64(max_floor64(fma(t, t, -((gp * f) * (bn2 * f))), 0.0))) * (small ? 0x1p-600 : 0x1p600);
+}
 __device__ __forceinline__ double
 fast_num64(double gp, double b2, double bn2)
 {
   const double s = scale_pos64<1>(b2 + gp);
-  double       n = s + sqrt64(max_floor64(fma(s, s, -(gp * bn2)), 0.0));
   if ((unsigned)(hi32(s) - 0x20b00000) >= 0x3e800000u)
-  {
-    // beyond 2^-500 to 2^500, where the squares leave the range: scaled by 2^600 or 2^-600
-    const bool   small = hi32(s) < 0x3ff00000;
-    const double f = small ? 0x1p600 : 0x1p-600, t = s * f;
-    n = (t + sqrt64(max_floor64(fma(t, t, -((gp * f) * (bn2 * f))), 0.0))) * (small ? 0x1p-600 : 0x1p600);
-  }
-  return n;
+    return fast_num64_scaled(s, gp, bn2);
+  return s + sqrt64(max_floor64(fma(s, s, -(gp * bn2)), 0.0));
 }
 
 // find_speed_fast<dir> (mhd_utils.h:89-117)
