@@ -18,6 +18,7 @@
 #include "ek_chunk.h"
 #include "ek_internal.h"
 #include "ek_launch.h"
+#include "ek_slabs.h"
 
 namespace ek_internal
 {
@@ -402,6 +403,51 @@ state_bytes(const ek_params & p, const ekc::KParams & kp)
 }
 } // namespace ek_internal
 
+// The step's workspace, and with it the way the step runs.  FP64: in passes along
+// slabs, where the grid is not too small for them (pass_slab 0) and no planes per
+// CTA of the 3D tile kernels are given; in shorter slabs when the workspace does
+// not fit beside the states.  The tile kernels come last: they need no workspace
+// but in 3D MHD, where it is the trace of the whole grid (384 B a cell in FP64;
+// passes 112 B a cell and a slab).
+static cudaError_t
+place_work(ek_solver * s)
+{
+  const ek_params & p = s->p;
+  KParams &         k = s->kp;
+  cudaError_t       e = cudaSuccess;
+  s->work = nullptr;
+  s->work_bytes = 0;
+  s->passes = false;
+  k.slab = 0;
+  if (s->prec == EK_PREC_FP64 && !(p.dim == 3 && p.kchunk > 0))
+  {
+    k.slab = ekc::place_slab(
+      ek_fast::pass_slab(p.dim, p.mhd, k), [&](int n) { return ek_fast::pass_bytes(p.dim, p.mhd, k, n); },
+      [&](size_t bytes) {
+        e = cudaMalloc(&s->work, bytes);
+        if (e == cudaErrorMemoryAllocation)
+        {
+          cudaGetLastError();
+          e = cudaSuccess;
+          return false;
+        }
+        s->work_bytes = bytes;
+        return true; // other errors end the search
+      });
+    s->passes = k.slab > 0 && e == cudaSuccess;
+  }
+  if (e == cudaSuccess && p.mhd && !s->passes)
+  {
+    if (p.dim == 3)
+      s->work_bytes = s->exact ? ek_exact::mhd_work_bytes(s->prec, k) : ek_fast::mhd_work_bytes(s->prec, k);
+    else
+      s->work_bytes = s->exact ? ek_exact::mhd2d_work_bytes(s->prec, k) : ek_fast::mhd2d_work_bytes(s->prec, k);
+    if (s->work_bytes)
+      e = cudaMalloc(&s->work, s->work_bytes);
+  }
+  return e;
+}
+
 extern "C" ek_status
 ek_solver_create(const ek_params * params, ek_solver ** out)
 {
@@ -439,36 +485,8 @@ ek_solver_create(const ek_params * params, ek_solver ** out)
     e = cudaMalloc((void **)&s->dtlog, sizeof(double) * s->dtcap);
   if (e == cudaSuccess)
     e = cudaMalloc((void **)&s->scratch3, 3 * sizeof(double));
-  // FP64: the step in passes with a bounded workspace, where the grid is not too
-  // small for it (pass_bytes 0) and no planes per CTA of the 3D tile kernels are
-  // given; if the workspace does not fit beside the states, the tile kernels,
-  // which need none
-  const bool tiles = p.dim == 3 && p.kchunk > 0;
-  if (e == cudaSuccess && s->prec == EK_PREC_FP64 && !tiles)
-  {
-    s->work_bytes = ek_fast::pass_bytes(p.dim, p.mhd, k);
-    if (s->work_bytes)
-    {
-      e = cudaMalloc(&s->work, s->work_bytes);
-      s->passes = e == cudaSuccess;
-      if (e == cudaErrorMemoryAllocation)
-      {
-        cudaGetLastError();
-        s->work = nullptr;
-        s->work_bytes = 0;
-        e = cudaSuccess;
-      }
-    }
-  }
-  if (e == cudaSuccess && p.mhd && !s->passes)
-  {
-    if (p.dim == 3)
-      s->work_bytes = s->exact ? ek_exact::mhd_work_bytes(s->prec, k) : ek_fast::mhd_work_bytes(s->prec, k);
-    else
-      s->work_bytes = s->exact ? ek_exact::mhd2d_work_bytes(s->prec, k) : ek_fast::mhd2d_work_bytes(s->prec, k);
-    if (s->work_bytes)
-      e = cudaMalloc(&s->work, s->work_bytes);
-  }
+  if (e == cudaSuccess)
+    e = place_work(s);
   // on the solver's stream: a legacy-stream memset is not ordered before the
   // uploads of the (non-blocking) solver stream
   if (e == cudaSuccess)

@@ -56,6 +56,7 @@ struct KParams
   int       kchunk;       // interior planes per CTA (3D kernels)
   int       kchunk_trace; // trace planes per CTA (3D MHD trace kernel)
   int       sms;          // SMs of the device
+  int       slab;         // cells of the last axis per slab (FP64 steps in passes)
   // FP32 copies prepared on the host, so that mixed kernels do no per-thread
   // FP64 arithmetic (one FP64 instruction costs 64 FP32 ones on GB300)
   float     gamma0f, smallrf, smallcf, smallpf, slopef;

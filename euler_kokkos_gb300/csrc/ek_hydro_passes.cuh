@@ -295,13 +295,6 @@ hydro_slab(const KParams & P, int first, int n, void * work)
   S.f = S.s + 2 * HydroSlab<NV>::DIM * NV * S.box(2);
   return S;
 }
-template <int NV>
-inline int
-hydro_slab_cells(const KParams & P)
-{
-  return ekc::slab_cells(NV == 4 ? P.ny : P.nz, kPassBytes, [&](int n) { return hydro_slab<NV>(P, 0, n, nullptr).bytes(); });
-}
-
 template <int NV, int RS, bool GRAV>
 cudaError_t
 hydro_step_passes(const void * Uin, void * Uout, void * work, const KParams & P, DevClock * clk, int step,
@@ -309,7 +302,7 @@ hydro_step_passes(const void * Uin, void * Uout, void * work, const KParams & P,
 {
   constexpr int DIM = HydroSlab<NV>::DIM;
   const double * in = (const double *)Uin;
-  const int      N = NV == 4 ? P.ny : P.nz, n = hydro_slab_cells<NV>(P);
+  const int      N = NV == 4 ? P.ny : P.nz, n = P.slab;
   auto           blocks = [](long long items) { return (unsigned)((items + kPassThreads - 1) / kPassThreads); };
   for (int first = 0; first < N; first += n)
   {

@@ -43,9 +43,10 @@
   /* emfs, update); work: workspace of pass_bytes */                                                \
   cudaError_t mhd_passes(int dim, int phase, const void * Uin, void * Uout, void * work,            \
                          const KParams & P, DevClock * clk, int step, cudaStream_t st);             \
-  /* the FP64 step in passes: bytes of its workspace (0: the grid is too small for it, the tile */  \
-  /* kernels are used), kernels per step */                                                         \
-  size_t      pass_bytes(int dim, int mhd, const KParams & P);                                      \
+  /* the FP64 step in passes: cells of the last axis per slab (0: the grid is too small for it, */  \
+  /* the tile kernels are used), workspace bytes of slabs of n cells, kernels per step */           \
+  int         pass_slab(int dim, int mhd, const KParams & P);                                       \
+  size_t      pass_bytes(int dim, int mhd, const KParams & P, int n);                               \
   int         pass_launches(int dim, int mhd, const KParams & P);                                   \
   }
 

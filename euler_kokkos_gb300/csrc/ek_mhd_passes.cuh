@@ -368,20 +368,6 @@ mhd_slab(const KParams & P, int first, int n, void * work)
   S.em = S.f + DIM * MhdSlab<DIM>::NF * S.box(1);
   return S;
 }
-template <int DIM>
-inline int
-mhd_slab_cells(const KParams & P)
-{
-  return ekc::slab_cells(DIM == 2 ? P.ny : P.nz, kPassBytes, [&](int n) { return mhd_slab<DIM>(P, 0, n, nullptr).slab_bytes(); });
-}
-template <int DIM>
-inline size_t
-mhd_pass_bytes_t(const KParams & P)
-{
-  return sizeof(double) * (11 + MhdSlab<DIM>::NE) * (size_t)P.vstride +
-         (size_t)mhd_slab<DIM>(P, 0, mhd_slab_cells<DIM>(P), nullptr).slab_bytes();
-}
-
 // one step: phase 0 (passes 0 and 1), phase 1 (passes 2 to 4)
 template <int DIM>
 cudaError_t
@@ -389,7 +375,7 @@ mhd_passes_t(int phase, const void * Uin, void * Uout, void * work, const KParam
              cudaStream_t st)
 {
   auto      blocks = [](long long items) { return (unsigned)((items + kPassThreads - 1) / kPassThreads); };
-  const int N = DIM == 2 ? P.ny : P.nz, n = mhd_slab_cells<DIM>(P);
+  const int N = DIM == 2 ? P.ny : P.nz, n = P.slab;
   if (phase == 0)
   {
     const MhdSlab<DIM> S = mhd_slab<DIM>(P, 0, n, work);
@@ -418,21 +404,33 @@ mhd_passes_t(int phase, const void * Uin, void * Uout, void * work, const KParam
   return cudaSuccess;
 }
 
-// Workspace of the FP64 step in passes.  0 for the small 2D grids, where one
+// Cells of the last axis per slab of the FP64 step in passes.  0 for the small 2D grids, where one
 // tile kernel ends before four or five launches do (us per step, passes /
 // tiles): hydro 64^2 28 / 15, 256^2 49 / 42, 512^2 124 / 126, 1024^2 424 / 464;
 // MHD 64^2 53 / 45, 128^2 72 / 66, 200 x 136 (425 tiles of 8 x 8) 92 / 92, 256^2
 // 153 / 185, 1024^2 1894 / 2348.  3D: hydro 24^3 37 / 64, 33 x 31 x 99 94 / 157,
 // 96^3 610 / 689, 200 x 180 x 160 3915 / 5214; MHD 16^3 71 / 181, 32^3 184 / 296,
 // 64^3 1077 / 1638, 160^3 15993 / 19314.
-size_t
-pass_bytes(int dim, int mhd, const KParams & P)
+int
+pass_slab(int dim, int mhd, const KParams & P)
 {
-  if (dim == 2 && !mhd)
-    return (long long)P.nx * P.ny < (1ll << 18) ? 0 : (size_t)hydro_slab<4>(P, 0, hydro_slab_cells<4>(P), nullptr).bytes();
-  if (dim == 2)
-    return (long long)((P.nx + 7) / 8) * ((P.ny + 7) / 8) <= 3ll * P.sms ? 0 : mhd_pass_bytes_t<2>(P);
-  return mhd ? mhd_pass_bytes_t<3>(P) : (size_t)hydro_slab<5>(P, 0, hydro_slab_cells<5>(P), nullptr).bytes();
+  if (dim == 2 && (mhd ? (long long)((P.nx + 7) / 8) * ((P.ny + 7) / 8) <= 3ll * P.sms : (long long)P.nx * P.ny < (1ll << 18)))
+    return 0;
+  // the MHD arrays of the whole grid do not count towards a slab
+  const long long whole = mhd ? (long long)pass_bytes(dim, mhd, P, 0) : 0;
+  return ekc::slab_cells(dim == 2 ? P.ny : P.nz, kPassBytes,
+                         [&](int n) { return (long long)pass_bytes(dim, mhd, P, n) - whole; });
+}
+// bytes of the workspace for slabs of n cells (MHD, n = 0: of the whole grid's arrays)
+size_t
+pass_bytes(int dim, int mhd, const KParams & P, int n)
+{
+  if (!mhd)
+    return (size_t)(dim == 2 ? hydro_slab<4>(P, 0, n, nullptr).bytes() : hydro_slab<5>(P, 0, n, nullptr).bytes());
+  const size_t whole = sizeof(double) * (11 + (dim == 2 ? MhdSlab<2>::NE : MhdSlab<3>::NE)) * (size_t)P.vstride;
+  if (n == 0)
+    return whole;
+  return whole + (size_t)(dim == 2 ? mhd_slab<2>(P, 0, n, nullptr).slab_bytes() : mhd_slab<3>(P, 0, n, nullptr).slab_bytes());
 }
 cudaError_t
 mhd_passes(int dim, int phase, const void * Uin, void * Uout, void * work, const KParams & P, DevClock * clk, int step,
@@ -445,10 +443,7 @@ mhd_passes(int dim, int phase, const void * Uin, void * Uout, void * work, const
 int
 pass_launches(int dim, int mhd, const KParams & P)
 {
-  const int N = dim == 2 ? P.ny : P.nz;
-  const int n = mhd ? (dim == 2 ? mhd_slab_cells<2>(P) : mhd_slab_cells<3>(P))
-                    : (dim == 2 ? hydro_slab_cells<4>(P) : hydro_slab_cells<5>(P));
-  const int slabs = (N + n - 1) / n;
+  const int N = dim == 2 ? P.ny : P.nz, slabs = (N + P.slab - 1) / P.slab;
   return mhd ? 2 + 3 * slabs : 4 * slabs;
 }
 

@@ -104,4 +104,16 @@ slab_cells(int N, long long limit, Bytes bytes)
   return n;
 }
 
+// A workspace for slabs of n cells or, when it cannot be had, fewer: try_alloc is
+// called with the bytes and tells whether it was.  The cells it holds, 0 for none.
+template <class Bytes, class Try>
+inline int
+place_slab(int n, Bytes bytes, Try try_alloc)
+{
+  for (; n > 0; n = n > 1 ? (n + 1) / 2 : 0)
+    if (try_alloc(bytes(n)))
+      return n;
+  return 0;
+}
+
 } // namespace ekc

@@ -88,3 +88,34 @@ def test_slab_lengths(lengths, N, limit, cell, fixed):
     most = max(1, min(N, (limit - fixed) // cell))  # cells that fit
     assert 1 <= n <= most
     assert n == -(-N // -(-N // most))  # the fewest slabs, equal but for the rounding
+
+
+PLACE = r"""
+#include "ek_slabs.h"
+#include <cstdio>
+#include <cstdlib>
+int main(int, char ** a)
+{
+  const int       n0 = atoi(a[1]);
+  const long long cell = atoll(a[2]), fixed = atoll(a[3]), room = atoll(a[4]);
+  const int       n = ekc::place_slab(n0, [&](int n) { return fixed + cell * n; }, [&](long long bytes) {
+    std::printf("%lld ", bytes);
+    return bytes <= room;
+  });
+  std::printf("-> %d\n", n);
+}
+"""
+
+
+@pytest.fixture(scope="module")
+def place(tmp_path_factory):
+    return _compile(tmp_path_factory.mktemp("place"), PLACE)
+
+
+@pytest.mark.parametrize("n,cell,fixed,room,asked,want", [
+    (9, 10, 5, 100, [95], 9), (9, 10, 5, 94, [95, 55], 5), (9, 10, 5, 20, [95, 55, 35, 25, 15], 1),
+    (9, 10, 5, 14, [95, 55, 35, 25, 15], 0), (1, 10, 5, 15, [15], 1), (1, 10, 5, 3, [15], 0), (0, 10, 5, 100, [], 0)])
+def test_workspace_placement(place, n, cell, fixed, room, asked, want):
+    out = subprocess.run([place, str(n), str(cell), str(fixed), str(room)], check=True, capture_output=True,
+                         text=True).stdout.split("->")
+    assert [int(x) for x in out[0].split()] == asked and int(out[1]) == want
