@@ -191,6 +191,7 @@ drain_events(ek_solver * s)
 static ek_status
 cuda_fail(cudaError_t e, const char * what)
 {
+  cudaGetLastError(); // reported here: the next launch's check must not find it again
   return fail(e == cudaErrorMemoryAllocation ? EK_ERR_NO_MEMORY : EK_ERR_CUDA,
               std::string(what) + ": " + cudaGetErrorString(e));
 }

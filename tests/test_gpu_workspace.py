@@ -67,3 +67,21 @@ def test_workspace_in_shorter_slabs(dim, mhd, room):
         assert np.array_equal(U, V) and np.array_equal(d, f)
     else:
         assert np.max(np.abs(U - V)) <= 1e-11 and np.max(np.abs(d / f - 1)) <= 1e-13
+
+
+@pytest.mark.parametrize("mhd", [False, True], ids=["hydro", "mhd"])
+def test_what_does_not_fit_leaves_the_solver_as_it_was(mhd):
+    """The staging buffer fits in no way: the call is refused, and the solver goes on."""
+    n = (64, 64, 64) if mhd else (96, 96, 96)
+    ini, U0 = P.smooth_random(dim=3, mhd=mhd, nx=n[0], ny=n[1], nz=n[2], seed=7, nsteps=3)
+    p = ek.params_from_ini(ini, kchunk=4)  # tile kernels: no workspace to give way in hydro
+    with ek.Solver(p) as s:
+        s.set_state(U0)
+        assert s.run(1) == 1
+        U = s.get_state()
+        with _left(4 * MB):
+            with pytest.raises(ek.EkError) as err:
+                s.get_state(layout=ek.EK_LAYOUT_RIGHT)
+            assert err.value.status == ek.EK_ERR_NO_MEMORY
+            assert np.array_equal(s.get_state(), U)
+            assert s.run(1) == 1
