@@ -449,6 +449,33 @@ place_work(ek_solver * s)
   return e;
 }
 
+// An allocation of a solver that runs: if it does not fit beside the workspace of
+// the passes, which holds nothing between steps, that is placed anew after it.
+static cudaError_t
+alloc_beside_work(ek_solver * s, void ** ptr, size_t bytes)
+{
+  cudaError_t e = cudaMalloc(ptr, bytes);
+  if (e != cudaErrorMemoryAllocation || !s->passes)
+    return e;
+  cudaGetLastError();
+  *ptr = nullptr;
+  e = cudaStreamSynchronize(s->stream);
+  if (e != cudaSuccess)
+    return e;
+  cudaFree(s->work);
+  s->cfl_step = -1; // as the tile kernels would take over
+  e = cudaMalloc(ptr, bytes);
+  if (e == cudaSuccess && place_work(s) == cudaSuccess)
+    return cudaSuccess;
+  // not both: the workspace where it was
+  cudaGetLastError();
+  if (e == cudaSuccess)
+    cudaFree(*ptr);
+  *ptr = nullptr;
+  place_work(s);
+  return cudaErrorMemoryAllocation;
+}
+
 extern "C" ek_status
 ek_solver_create(const ek_params * params, ek_solver ** out)
 {
@@ -547,7 +574,7 @@ ek_solver_destroy(ek_solver * s)
 static const long long kStageElems = 1LL << 25; // 32 Mi doubles (256 MB)
 
 static ek_status
-ensure_stage(Stage & g, long long total)
+ensure_stage(ek_solver * s, Stage & g, long long total)
 {
   const long long want = total < kStageElems ? total : kStageElems;
   if (g.elems >= want)
@@ -555,7 +582,7 @@ ensure_stage(Stage & g, long long total)
   cudaFree(g.buf);
   g.buf = nullptr;
   g.elems = 0;
-  EK_CUDA(cudaMalloc((void **)&g.buf, sizeof(double) * (size_t)want), "staging buffer");
+  EK_CUDA(alloc_beside_work(s, (void **)&g.buf, sizeof(double) * (size_t)want), "staging buffer");
   g.elems = want;
   return EK_OK;
 }
@@ -572,7 +599,7 @@ host_to_state(ek_solver * s, const double * U, int layout, void * dev)
   }
   Stage &                     g = *s->stage;
   std::lock_guard<std::mutex> hold(g.lock);
-  ek_status                   st = ensure_stage(g, total);
+  ek_status                   st = ensure_stage(s, g, total);
   if (st != EK_OK)
     return st;
   for (long long first = 0; first < total; first += g.elems)
@@ -600,7 +627,7 @@ state_to_host(ek_solver * s, const void * dev, double * U, int layout)
   }
   Stage &                     g = *s->stage;
   std::lock_guard<std::mutex> hold(g.lock);
-  ek_status                   st = ensure_stage(g, total);
+  ek_status                   st = ensure_stage(s, g, total);
   if (st != EK_OK)
     return st;
   for (long long first = 0; first < total; first += g.elems)
@@ -837,7 +864,7 @@ ek_solver_set_gravity_field(ek_solver * s, const double * G, int layout)
     // device copy in the state's precision, LayoutLeft, one plane per component
     const size_t es = s->prec == EK_PREC_FP64 ? sizeof(double) : sizeof(float);
     if (!s->gfield)
-      EK_CUDA(cudaMalloc(&s->gfield, es * (size_t)n * dim), "gravity field");
+      EK_CUDA(alloc_beside_work(s, &s->gfield, es * (size_t)n * dim), "gravity field");
     std::vector<double> h((size_t)n * dim);
     if (layout == EK_LAYOUT_LEFT)
       std::memcpy(h.data(), G, sizeof(double) * h.size());
@@ -953,6 +980,8 @@ launch_one(ek_solver * s, int kernel_id, int phase, int step)
 static ek_status
 launch_step(ek_solver * s, int step)
 {
+  if (s->p.mhd && s->p.dim == 3 && !s->work)
+    return fail(EK_ERR_NO_MEMORY, "no device memory for the step's workspace");
   if (s->passes)
   {
     ek_status st = EK_OK;

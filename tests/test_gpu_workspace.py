@@ -69,6 +69,23 @@ def test_workspace_in_shorter_slabs(dim, mhd, room):
         assert np.max(np.abs(U - V)) <= 1e-11 and np.max(np.abs(d / f - 1)) <= 1e-13
 
 
+def test_staging_beside_the_workspace():
+    """A row-major state goes through a staging buffer, allocated when it is first needed."""
+    p, U0 = _state(False, 3)
+    R = np.ascontiguousarray(np.transpose(U0, (3, 2, 1, 0)))
+    out = []
+    for little in (False, True):
+        with ek.Solver(p) as s:
+            s.set_state(U0)
+            assert s.run(1) == 1
+            with _left(20 * MB) if little else contextlib.nullcontext():
+                s.set_state(R, layout=ek.EK_LAYOUT_RIGHT)  # 45 MB
+                out.append(_run(s))
+                assert np.array_equal(np.transpose(s.get_state(layout=ek.EK_LAYOUT_RIGHT), (3, 2, 1, 0)), out[-1][1])
+    assert out[1][0] > out[0][0]
+    assert np.array_equal(out[0][1], out[1][1]) and np.array_equal(out[0][2], out[1][2])
+
+
 @pytest.mark.parametrize("mhd", [False, True], ids=["hydro", "mhd"])
 def test_what_does_not_fit_leaves_the_solver_as_it_was(mhd):
     """The staging buffer fits in no way: the call is refused, and the solver goes on."""
@@ -85,3 +102,19 @@ def test_what_does_not_fit_leaves_the_solver_as_it_was(mhd):
             assert err.value.status == ek.EK_ERR_NO_MEMORY
             assert np.array_equal(s.get_state(), U)
             assert s.run(1) == 1
+
+
+def test_gravity_field_beside_the_workspace():
+    ini, U0 = P.rayleigh_taylor(dim=3, nx=96, ny=96, nz=96, nsteps=3)
+    p = ek.params_from_ini(ini)
+    G = np.zeros((3,) + U0.shape[1:])
+    G[2] = -0.1 * (1.0 + 0.1 * np.cos(np.arange(U0.shape[1]))[:, None, None])
+    out = []
+    for little in (False, True):
+        with ek.Solver(p) as s:
+            s.set_state(U0)
+            with _left(8 * MB) if little else contextlib.nullcontext():
+                s.set_gravity_field(G)  # 24 MB
+                out.append(_run(s))
+    assert out[1][0] > out[0][0]
+    assert np.array_equal(out[0][1], out[1][1]) and np.array_equal(out[0][2], out[1][2])
