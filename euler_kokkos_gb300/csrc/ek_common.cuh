@@ -56,13 +56,13 @@ struct KParams
   int       kchunk;       // interior planes per CTA (3D kernels)
   int       kchunk_trace; // trace planes per CTA (3D MHD trace kernel)
   int       sms;          // SMs of the device
-  int       slab;         // cells of the last axis per slab (FP64 steps in passes)
   // FP32 copies prepared on the host, so that mixed kernels do no per-thread
   // FP64 arithmetic (one FP64 instruction costs 64 FP32 ones on GB300)
   float     gamma0f, smallrf, smallcf, smallpf, slopef;
   float     idx, idy, idz; // 1/dx, 1/dy, 1/dz
   double    idxd, idyd, idzd; // 1/dx, 1/dy, 1/dz in FP64 (FP64 FMA build's CFL)
   int       mhd_stage;     // MHD update: stage the trace planes in shared memory
+  int       slab;          // cells of the last axis per slab (FP64 steps in passes)
   double    entho;           // 1 / (gamma0 - 1)
   float     enthof;
   double    gamma6, smallpp; // riemann_approx constants (HydroParams.cpp:353-356)
