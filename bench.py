@@ -69,14 +69,14 @@ KERNEL_NAMES = {
 # are in profiles/); a launch's traffic on the bench workload is this figure
 # times its interior cells (these kernels' traffic grows with the cells).
 TRAFFIC_PER_CELL = {
-    ("hydro3d", "mixed"): {"hydro3d_step": 38.0},   # 159.0 + 109.9 MB / 7.08 M cells
+    ("hydro3d", "mixed"): {"hydro3d_step": 37.2},   # 154.7 + 108.9 MB / 7.08 M cells
     ("mhd3d", "mixed"): {"mhd_dt_kernel": 46.0,      # 323 + 3 MB / 7.08 M cells (first step only)
-                         "mhd_trace_kernel": 243.0,  # 375.4 + 1345.0 MB / 7.08 M cells
-                         "mhd_update_kernel": 345.8,  # 2125.8 + 321.4 MB / 7.08 M cells
+                         "mhd_trace_kernel": 242.9,  # 374.0 + 1345.2 MB / 7.08 M cells
+                         "mhd_update_kernel": 353.2,  # 2172.9 + 326.7 MB / 7.08 M cells
                          # with no tile listed (the Orszag-Tang steps) the
                          # repair kernel reads the list head only
                          "mhd_repair_kernel": 0.0},
-    ("mhd2d", "mixed"): {"mhd2d_step_kernel": 78.1,  # 186.4 + 141.0 MB / 4.19 M cells
+    ("mhd2d", "mixed"): {"mhd2d_step_kernel": 77.7,  # 186.3 + 139.7 MB / 4.19 M cells
                          "mhd2d_repair_kernel": 0.0},
 }
 

@@ -55,9 +55,11 @@ choose_chunk(long long columns, int planes, int sms, ChunkModel m)
 
 // The 2D hydro marches: strips of kRowCols columns, CTAs of kRowWarps warps on
 // consecutive runs of rows (a "plane" above is a row of each warp).  Fitted on
-// runs of 1 to 32 rows (us per step, mixed): 64^2 8.9 with 1, 13.2 with 8; 512^2
-// 14.2 with 4, 24.5 with 1; 1022 x 518 20.1 with 8, 40.5 with 1, 32.4 with 32;
-// 2048^2 87.4 with 32, 99.5 with 8, 277 with 1.
+// runs of 1 to 32 rows; us per step, mixed, with 1 / 2 / 4 / 8 / 16 / 32 rows and by
+// the rule: 64^2 7.9 / 8.4 / 9.6 / 11.1 / 16.1 / 24.3, 7.9; 512^2 21.7 / 15.7 / 13.1 /
+// 13.3 / 16.0 / 24.4, 13.2; 1022 x 518 36.8 / 25.7 / 20.2 / 18.7 / 21.4 / 29.5, 19.4;
+// 1024^2 67 / 45 / 33 / 27.6 / 25.5 / 35.5, 27.6; 2048^2 258 / 160 / 114 / 91.9 /
+// 84.1 / 80.5, 84.1.
 constexpr int kRowCols = 28, kRowWarps = 4;
 constexpr ChunkModel kChunkRows64 = { 0.60, 2.0, 8 }, kChunkRows32 = { 0.35, 2.0, 2 };
 inline int

@@ -754,8 +754,10 @@ launch_chained(void (*kernel)(KA...), dim3 grid, int threads, size_t smem, cudaS
 }
 // A tile kernel whose time is a tile's (FP64) and that has one to three tiles
 // per SM is not chained: the blocks brought in early crowd on the SMs that end
-// first (hydro 128^2, 256 tiles: 18.9 us, chained 22.0; MHD 165^2, 441 tiles:
-// 89.0, chained 103.7).
+// first.  us per step by tiles per SM, unchained / chained: hydro 8 x 8, 1.1 18.6 /
+// 17.6, 1.5 19.0 / 19.8, 1.7 19.7 / 22.3, 2.1 24.2 / 24.4, 2.6 24.4 / 26.8, 3.2 29.6 /
+// 29.5; 16 x 16, 1.7 43.1 / 48.5, 2.1 59.6 / 57.2; MHD, 1.1 63.7 / 66.1, 1.7 63.7 /
+// 85.8, 2.1 89.5 / 87.8, 2.6 90.1 / 99.9, 2.9 89.3 / 104.
 inline bool
 chain_tiles(const KParams & P, long long tiles)
 {

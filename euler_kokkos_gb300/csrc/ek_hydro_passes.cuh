@@ -1,8 +1,8 @@
 // FP64 hydro step in passes, each over all its cells or faces.
 //
 // GB300 issues FP64 at 1/64 of the FP32 rate, so the FP64 step's time is its
-// count of FP64 instructions: 0.3 kB a cell and step of memory traffic is
-// nothing beside it (1 Gcell/s x 400 B = 0.4 TB/s of 6.8).  A tile kernel
+// count of FP64 instructions: the passes' 807 B a cell and step (ncu, 96^3) are
+// little beside it (1.5 Gcell/s x 807 B = 1.2 TB/s of 6.8).  A tile kernel
 // repeats work (primitives of the halo 1.56 x, traces of the ring 1.25 x, the
 // planes at a chunk's ends) and its phases wait for one another on few warps.
 // Here every value is computed once, by one thread of a flat launch at full
@@ -12,9 +12,12 @@
 //      state that faces the interior)
 //   3. one Riemann problem per face
 //   4. update, gravity, the next step's CFL
-// along slabs of the last axis, so that the workspace stays bounded.  The
-// arithmetic is that of the tile kernels, function by function (the exact build
-// stays bitwise equal to the reference).
+// along slabs of the last axis, so that the workspace stays bounded (a slab repeats
+// the primitives of two layers on each side and the traces of one: 256 x 256 x 64
+// 1.47 Gcell/s, 512 x 512 x 16, two slabs, 1.36, 1024 x 1024 x 12, a slab a plane,
+// 0.81; the former tile kernel 0.69 to 0.72 on all).  The arithmetic is that of the
+// tile kernels, function by function (the exact build stays bitwise equal to the
+// reference).
 #pragma once
 
 #include "ek_hydro_kernels.cuh"

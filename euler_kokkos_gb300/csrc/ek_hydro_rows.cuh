@@ -12,9 +12,9 @@
 // (678 instructions a cell with runs of 8).  Issue bounds large grids (57 to 73 %
 // busy, 20 warps per SM at 96 registers; at 80, 24 warps, 2 % slower), the chain
 // of one row, 0.6 us, small ones.  us per step, tile / march: mixed 64^2 12.4 /
-// 8.7, 512^2 18.5 / 13.6, 1022 x 518 29.6 / 20.3, 2048^2 182 / 85 (the first and
-// last row in the loop, by branches: 14.4, 22.2, 91); ensemble of 32
-// runs of 64^2 to 256^2 mixed 42 / 31, FP64 852 / 551.
+// 7.9, 512^2 18.5 / 13.2, 1022 x 518 29.6 / 19.4, 2048^2 182 / 84 (the first and
+// last row in the loop, by branches: 8.8, 14.4, 22.2, 91); ensemble of 32
+// runs of 64^2 to 256^2 mixed 42 / 28, FP64 852 / 549.
 #pragma once
 
 #include "ek_chunk.h"

@@ -64,15 +64,16 @@ hydro_step_rs(int dim, const void * Uin, void * Uout, void * work, const KParams
     }
   if (dim == 2)
   {
-    // Mixed: marching warps (us per step, against 32 x 8 tiles: 64^2 8.8 / 12.4,
-    // 512^2 14.1 / 18.5, 1022 x 518 21 / 30, 2048^2 91 / 170).  FP64, on grids too
+    // Mixed: marching warps (us per step, against 32 x 8 tiles: 64^2 7.9 / 12.4,
+    // 512^2 13.2 / 18.5, 1022 x 518 19.4 / 30, 2048^2 84 / 170).  FP64, on grids too
     // small for the passes: 8 x 8 tiles where they make at most six CTAs per SM,
     // since a warp's chain of FP64 instructions (64 cycles each on its quarter of
-    // the SM) then sets the time (64^2: 19 against 31; 200 x 136: 28 against 30;
-    // 256 x 200, 5.3 CTAs per SM: 47 against 49; 256^2, 6.7: 51 against 49), else
-    // 16 x 16 (512^2: 145; 32 x 16 166, 32 x 8 156).  The threads beyond one per
-    // cell take the ring cells and let every phase of the small tile finish in
-    // one round (64^2: 29 with one per cell).
+    // the SM) then sets the time (64^2: 13.4 against 23.9; 200 x 136: 24.8 against
+    // 23.9; 256 x 200, 5.3 CTAs per SM: 40.4 against 42.3; 256^2, 6.7: 43.5 against
+    // 43.1), else 16 x 16 (512 x 500: 125 against 148; 512^2, before the passes, 145,
+    // 32 x 16 166, 32 x 8 156).  The threads beyond one per cell take the ring cells
+    // and let every phase of the small tile finish in one round (64^2, at 19 with
+    // them, 29 with one per cell).
     if constexpr (sizeof(R) == 4)
     {
       const int rows = ekc::choose_rows(&P.nx, &P.ny, 1, P.sms, ekc::kChunkRows32);

@@ -689,8 +689,9 @@ mhd2d_tiles(const KParams & P, int TX, int TY)
 }
 // Mixed: 8 x 8 tiles with 128 threads while they make at most seven CTAs per SM:
 // a tile's phases, one after another, then set the time (us per step, 16 x 16 /
-// 8 x 8: 64^2 17.2 / 14.1, 128^2 17.5 / 14.7, 256^2 20.0 / 18.7), above it the
-// repeated halo work does (512^2, 27 CTAs per SM: 40.0 / 52.2).
+// 8 x 8: 64^2 16.7 / 13.3, 128^2 17.1 / 14.5, 256^2, 6.7 CTAs per SM, 19.2 / 19.0),
+// above it the repeated halo work does (272 x 266, 7.6, 19.2 / 19.5; 512^2, 27, 40.3 /
+// 52.7).
 inline bool
 mhd2d_small(const KParams & P)
 {
@@ -749,9 +750,10 @@ mhd2d_step_t(int phase, const void * Uin, void * Uout, void * work, const KParam
                             : mhd2d_repair_tiled<S, R, M2_TX, M2_TY, M2_TX * M2_TY>(Uin, Uout, work, P, clk, step, st);
     }
   }
-  // Mixed: 16 x 16, small grids 8 x 8 (mhd2d_small).  FP64, on grids too small for the passes: 8 x
-  // 8 with 128 threads (64^2: 50 us; 16 x 8 82, 16 x 16 117; 200 x 136: 102, 117,
-  // 117), since a tile's chain of FP64 instructions sets its time.
+  // Mixed: 16 x 16, small grids 8 x 8 (mhd2d_small).  FP64, on grids too small for
+  // the passes: 8 x 8 with 128 threads (64^2: 50 us; 16 x 8 82, 16 x 16 117; 200 x
+  // 136: 102, 117, 117, when all three were built; now 42 and 89), since a tile's
+  // chain of FP64 instructions sets its time.
   if constexpr (sizeof(R) == 4)
     return mhd2d_small(P) ? mhd2d_step_tiled<S, R, 8, 8, 128>(Uin, Uout, work, P, clk, step, st)
                           : mhd2d_step_tiled<S, R, M2_TX, M2_TY, M2_TX * M2_TY>(Uin, Uout, work, P, clk, step, st);

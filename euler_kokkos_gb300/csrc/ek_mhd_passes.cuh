@@ -404,13 +404,13 @@ mhd_passes_t(int phase, const void * Uin, void * Uout, void * work, const KParam
   return cudaSuccess;
 }
 
-// Cells of the last axis per slab of the FP64 step in passes.  0 for the small 2D grids, where one
-// tile kernel ends before four or five launches do (us per step, passes /
-// tiles): hydro 64^2 28 / 15, 256^2 49 / 42, 512^2 124 / 126, 1024^2 424 / 464;
-// MHD 64^2 53 / 45, 128^2 72 / 66, 200 x 136 (425 tiles of 8 x 8) 92 / 92, 256^2
-// 153 / 185, 1024^2 1894 / 2348.  3D: hydro 24^3 37 / 64, 33 x 31 x 99 94 / 157,
-// 96^3 610 / 689, 200 x 180 x 160 3915 / 5214; MHD 16^3 71 / 181, 32^3 184 / 296,
-// 64^3 1077 / 1638, 160^3 15993 / 19314.
+// Cells of the last axis per slab of the FP64 step in passes.  0 for the small 2D
+// grids, where one tile kernel ends before four or five launches do (us per step,
+// passes / tiles): hydro 64^2 28 / 15, 256^2 49 / 42 (both when the rule was made),
+// 512^2 118 / 125, 1024^2 431 / 467; MHD 64^2 53 / 45, 128^2 72 / 66 (then), 200 x 136
+// (425 tiles of 8 x 8) 89 / 89, 256^2 139 / 201, 1024^2 1861 / 2834.  3D: hydro 24^3 30 /
+// 64, 33 x 31 x 99 89 / 211, 96^3 606 / 711, 200 x 180 x 160 3861 / 5490; MHD 16^3 61 /
+// 179, 32^3 158 / 292, 64^3 1016 / 1587, 160^3 15237 / 19328.
 int
 pass_slab(int dim, int mhd, const KParams & P)
 {

@@ -163,7 +163,8 @@ ek_status ek_solver_dt_history(ek_solver * s, double * dts, int n);
 ek_status ek_solver_totals(ek_solver * s, double out[3]);
 /* Device pointer / byte size of the current state (zero-copy access; the
  * storage type is FP64, or FP32 hydro variables + FP64 face B in the mixed
- * form).  Valid until the next step. */
+ * form).  Valid until the next step, and for reading: the next step's dt may
+ * already have been computed from the state (ek_solver_set_state sets one). */
 ek_status ek_solver_device_state(ek_solver * s, void ** ptr, size_t * bytes);
 /* Block until all work of the solver is done; reports device-side errors. */
 ek_status ek_solver_synchronize(ek_solver * s);
